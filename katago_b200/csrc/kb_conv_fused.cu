@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
   uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(resFull + PP_EPI_WARPS * 2);
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warpIndex(), lane = threadIdx.x & 31;
   const int numTiles = a.g.rowsPad / PP_BM;
   const int grid = (int)gridDim.x;
   const int cpp = a.NP / 64;   // K chunks of GEMM2 per part
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
   }
   else if(warp == 0) {
     // ---------------- TMA producer ----------------
-    if(lane == 0) {
+    if(electOne()) {
       uint32_t s1 = 0, ph1 = 0, s2 = 0, ph2 = 0;
       bool ok = true;
       auto loadW1c = [&](int kc, int row, uint32_t bytes) {
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
   }
   else if(warp == 1) {
     // ---------------- MMA issuer ----------------
-    if(lane == 0) {
+    if(electOne()) {
       const uint32_t descHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);
       const uint32_t a1Lo = ((smemU32(sA1) & 0x3FFFFu) >> 4) | (1u << 16);
       const uint32_t a2Lo = ((smemU32(sA2) & 0x3FFFFu) >> 4) | (1u << 16);
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
       tmaLoad2d(smemU32(sR + (size_t)b * PP_UNIT), &tmS, np * a.NP + nj * 32, nt * PP_BM + q * 32, smemU32(&myRes[b]));
     };
     gridDepWait();
-    if(lane == 0) fetchNext(0);
+    if(electOne()) fetchNext(0);
     __syncwarp();
     for(int t = (int)blockIdx.x; t < numTiles && alive; t += grid, it++) {
       const int m0 = t * PP_BM;
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
           tmemLd32(tmemBase + d1Col + (uint32_t)(j * 32) + ((uint32_t)(q * 32) << 16), r);
           // the slot of the unit after this one held this warp's store before last: it must have been read; then the
           // next residual is requested, so that its latency hides behind this unit's arithmetic
-          if(lane == 0) { bulkWaitRead0(); fetchNext(rs + 1u); }
+          if(electOne()) { bulkWaitRead0(); fetchNext(rs + 1u); }
           __syncwarp();
           bool landed = mbarWait(smemU32(&myRes[slot]), (rs >> 1) & 1u, abortFlag);
           if(!__all_sync(0xffffffffu, landed)) { alive = false; break; }
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
             // this warp's last load of the part: the accumulator may be overwritten by the next part
             tcFenceBefore();
             __syncwarp();
-            if(lane == 0) mbarArrive(smemU32(d1Empty));
+            if(electOne()) mbarArrive(smemU32(d1Empty));
           }
           const int c = p * a.NP + j * 32;  // first output channel of this unit
           float2 v[16];
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
           }
           fenceProxyAsync();
           __syncwarp();
-          if(lane == 0) {
+          if(electOne()) {
             mbarArrive(smemU32(&a2Full[abuf]));
             tmaStore2d(&tmS, smemU32(sR + (size_t)slot * PP_UNIT), c, m0 + q * 32);
             bulkCommit();
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
             }
           }
           // staging: the ring slot that does not hold the residual requested ahead, and the third unit
-          if(lane == 0) bulkWaitRead0();
+          if(electOne()) bulkWaitRead0();
           __syncwarp();
           uint8_t* rawRow = sR + (size_t)((rs + 1u) & 1u) * PP_UNIT + lane * 64;
           uint8_t* actRow = sO + lane * 64;
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
           }
           fenceProxyAsync();
           __syncwarp();
-          if(lane == 0) {
+          if(electOne()) {
             tmaStore2d(&tmRaw2, smemU32(sR + (size_t)((rs + 1u) & 1u) * PP_UNIT), c, m0 + q * 32);
             tmaStore2d(&tmAct2, smemU32(sO), c, m0 + q * 32);
             bulkCommit();
@@ -455,11 +455,11 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
         }
         tcFenceBefore();
         __syncwarp();
-        if(lane == 0) mbarArrive(smemU32(d2Empty));
+        if(electOne()) mbarArrive(smemU32(d2Empty));
       }
     }
     if(!alive && lane == 0 && !*abortFlag) { *abortFlag = 1; atomicCAS(a.status, 0, PP_ERR_EPILOGUE); }
-    if(lane == 0) bulkWaitAll();
+    if(electOne()) bulkWaitAll();
   }
 
   // ---------------- common exit ----------------

@@ -390,7 +390,7 @@ __device__ __forceinline__ bool epilogueTileTma(
     TRACE(threadIdx.x == 64, 1024 + (int)(tileIter & 31u) * 16 + j * 5 + 2);
     // The TMA engine must have read the previous unit's stores before their staging units are written again; that
     // also frees the ring slot before this one for the residual of the same unit of the next tile.
-    if(lane == 0) {
+    if(electOne()) {
       bulkWaitRead0();
       // the slot of the unit before this one is free now: it takes the unit ring-1 ahead of this one
       if(CHAIN) {
@@ -421,7 +421,7 @@ __device__ __forceinline__ bool epilogueTileTma(
     // make the generic-proxy writes visible to the TMA engine, then let lane 0 send the unit out
     fenceProxyAsync();
     __syncwarp();
-    if(lane == 0) {
+    if(electOne()) {
       if(doRaw) tmaStore2d(tmRaw, smemU32(es.sR + (size_t)slot * TC_UNIT_BYTES), c - ep.rawC0, m0 + q * 32);
       if(doAct) tmaStore2d(tmAct, smemU32(es.sO), ACT == KB_ACT_SWIGLU_PAIRS ? (c - ep.actC0) / 2 : c - ep.actC0, m0 + q * 32);
       bulkCommit();
@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
   volatile int* gateTiles = abortFlag + 1;  // per-tile dependencies: how many of this CTA's tiles are known to be ready
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warpIndex(), lane = threadIdx.x & 31;
   const int numNTiles = a.outC / a.BN;
   const int taps = a.kY * a.kX;
   // CTA pair: both CTAs walk the same tile list; a tile is 256 rows, the even CTA (leader) takes the upper 128
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
 
   if(warp == 0) {
     // ---------------- TMA producer ----------------
-    if(lane == 0) {
+    if(electOne()) {
       uint32_t sa = 0, phA = 0, sb = 0, phB = 0;
       bool ok = true;
       // In a pair both CTAs load their own rows of A and their own half of each weight tile; every load signals the
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
     // and the tap offsets are computed once.
     // In a pair only the leader issues; its MMAs read both CTAs' shared memory and write both CTAs' TMEM, and every
     // completion is signalled to the same barrier of both CTAs.
-    if(lane == 0 && leader) {
+    if(leader && electOne()) {
       auto mma = [&](uint32_t d, uint32_t aLo, uint32_t bLo, uint32_t descHi, uint32_t acc) {
         if(PAIR) ummaLoHiPair(d, aLo, bLo, descHi, a.idesc, acc);
         else ummaLoHi(d, aLo, bLo, descHi, a.idesc, acc);
@@ -722,7 +722,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
       const int bIdx = min(m / a.g.PB, a.g.n - 1);
       const float* biasRow = a.ep.biasNC ? a.ep.biasNC + (size_t)bIdx * a.outC : nullptr;
       if(TMA_EPI) {
-        if(a.ep.residual && lane == 0 && it == 0 && es.nU > 0) {
+        if(a.ep.residual && it == 0 && es.nU > 0 && electOne()) {
           // fill the ring; afterwards every unit that drains fetches the unit ring-1 ahead of it
           for(int k = 0; k < es.ring; k++) prefetchResidual<CG>(&tmRes, a, es, (uint32_t)k, tm, q, cg);
         }
@@ -759,11 +759,11 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
       tcFenceBefore();
       __syncwarp();
       TRACE(threadIdx.x == 64, 512 + it * 16 + 3);
-      if(lane == 0) {
+      if(electOne()) {
         if(PAIR) mbarArriveCluster(pairLeaderAddr(smemU32(&accEmpty[buf])));
         else mbarArrive(smemU32(&accEmpty[buf]));
       }
-      if(DEPS && TMA_EPI && a.doneCtr != nullptr && lane == 0) {
+      if(DEPS && TMA_EPI && a.doneCtr != nullptr && electOne()) {
         if(a.kY == 3) {
           // a 3x3 convolution's epilogue warps idle until the next accumulator is full: wait here for this tile's
           // stores to reach memory and report the tile at once
@@ -781,9 +781,9 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
         }
       }
     }
-    if(lane == 0) bulkWaitAll();  // outstanding tile stores must complete before the CTA's shared memory goes away
+    if(electOne()) bulkWaitAll();  // outstanding tile stores must complete before the CTA's shared memory goes away
     if(threadIdx.x == 64) TLT(4);
-    if(DEPS && TMA_EPI && a.doneCtr != nullptr && lane == 0 && prevRowTile >= 0) {
+    if(DEPS && TMA_EPI && a.doneCtr != nullptr && prevRowTile >= 0 && electOne()) {
       redReleaseGpuAdd(a.doneCtr + prevRowTile, 1u);
     }
   }
@@ -889,7 +889,7 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
   volatile int* gateItems = abortFlag + 1;  // how many of this CTA's tiles (over all layers) have their dependencies met
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warpIndex(), lane = threadIdx.x & 31;
   const int grid = (int)gridDim.x;
   const int rowTiles = c.g.rowsPad / TC_BM;
 #ifdef KB_TC_TRACE
@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
 
   if(warp == 0) {
     // ---------------- TMA producer ----------------
-    if(lane == 0) {
+    if(electOne()) {
       uint32_t sa = 0, phA = 0, sb = 0, phB = 0;
       bool ok = true;
       int item = 0, base = 0;
@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
   }
   else if(warp == 1) {
     // ---------------- MMA issuer ----------------
-    if(lane == 0) {
+    if(electOne()) {
       const uint32_t descHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);
       const uint32_t aLoBase = ((smemU32(smemA) & 0x3FFFFu) >> 4) | (1u << 16);
       const uint32_t bLoBase = ((smemU32(smemB) & 0x3FFFFu) >> 4) | (1u << 16);
@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
         const float mk = la.ep.mask ? la.ep.mask[m] : 1.0f;
         const int bIdx = min(m / c.g.PB, c.g.n - 1);
         const float* biasRow = la.ep.biasNC ? la.ep.biasNC + (size_t)bIdx * la.outC : nullptr;
-        if(hasRes && lane == 0 && es.nU > 0) {
+        if(hasRes && es.nU > 0 && electOne()) {
           // The residual may come from a layer of this chain: fetch it only once this tile's dependencies are known to
           // be met (they cover every row the residual unit holds).  The staging slots must be free as well.
           uint32_t spins = 0;
@@ -1111,8 +1111,8 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
         }
         tcFenceBefore();
         __syncwarp();
-        if(lane == 0) mbarArrive(smemU32(&accEmpty[buf]));
-        if(la.doneCtr != nullptr && lane == 0) {
+        if(electOne()) mbarArrive(smemU32(&accEmpty[buf]));
+        if(la.doneCtr != nullptr && electOne()) {
           if(la.kY == 3) {
             // epilogue warps of a 3x3 layer idle until the next accumulator is full: report the tile at once
             bulkWaitAll();
@@ -1128,13 +1128,13 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
           }
         }
       }
-      if(la.doneCtr != nullptr && lane == 0 && prevRowTile >= 0) {
+      if(la.doneCtr != nullptr && prevRowTile >= 0 && electOne()) {
         bulkWaitAll();
         redReleaseGpuAdd(la.doneCtr + prevRowTile, 1u);
       }
       base += numTiles;
     }
-    if(lane == 0) bulkWaitAll();
+    if(electOne()) bulkWaitAll();
     if(threadIdx.x == 64) TLT(4);
   }
   else if(lane == 0) {

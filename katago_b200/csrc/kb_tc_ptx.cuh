@@ -59,6 +59,19 @@ __device__ __forceinline__ bool mbarWait(uint32_t bar, uint32_t parity, volatile
 __device__ __forceinline__ void gridDepWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void gridDepLaunch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// One thread of a converged warp, always the same one.  Where one thread issues TMA or tcgen05 instructions it has to be
+// chosen this way and not by its lane number: only elect.sync tells the compiler that a single thread executes them.
+// Measured with 108 MMAs (M=128, K=16) from one thread, a commit after every four: 112 cycles per MMA for every N up to
+// 192 behind a comparison of the lane number; 64 (N <= 64), 74 (N=128) and 96 (N=192, the tensor pipe's own rate) behind
+// elect.sync.  Without commits 59 cycles against 39 to 49 (N = 16 to 64).
+__device__ __forceinline__ bool electOne() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p)::"memory");
+  return p != 0u;
+}
+// The warp's number in its block, in a form the compiler knows to be the same for the whole warp.
+__device__ __forceinline__ int warpIndex() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ void tmaLoad2d(uint32_t dst, const CUtensorMap* tmap, int c0, int c1, uint32_t bar) {
   asm volatile(
     "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
