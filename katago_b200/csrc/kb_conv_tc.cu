@@ -783,7 +783,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
     }
     if(electOne()) bulkWaitAll();  // outstanding tile stores must complete before the CTA's shared memory goes away
     if(threadIdx.x == 64) TLT(4);
-    if(DEPS && TMA_EPI && a.doneCtr != nullptr && prevRowTile >= 0 && electOne()) {
+    if(DEPS && TMA_EPI && a.doneCtr != nullptr && electOne() && prevRowTile >= 0) {
       redReleaseGpuAdd(a.doneCtr + prevRowTile, 1u);
     }
   }
@@ -1128,7 +1128,7 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
           }
         }
       }
-      if(la.doneCtr != nullptr && prevRowTile >= 0 && electOne()) {
+      if(la.doneCtr != nullptr && electOne() && prevRowTile >= 0) {
         bulkWaitAll();
         redReleaseGpuAdd(la.doneCtr + prevRowTile, 1u);
       }
