@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attentionTcKernel(const __grid_
   uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bars + 5);
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
 
-  const int tid = threadIdx.x, warp = warpIndex(), lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3;        // TMEM lane quarter this warp may read
   const int half = warp >> 2;          // which half of the keys (softmax) / of the output columns this warp handles
   const int row = quarter * 32 + lane; // query row inside the tile
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1) attentionPipeKernel(const __gri
   uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bars + AP_NUM_BARS);
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
 
-  const int tid = threadIdx.x, warp = warpIndex(), lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   AT_TRACE(0);
   if(tid == 0) {
     for(int i = 0; i < AP_NUM_BARS; i++) mbarInit(smemU32(&bars[i]), (i == AP_SM_DONE || (i >= AP_O_FREE && i < AP_P_FREE)) ? 8 : 1);
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1) attentionPipeKernel(const __gri
 
   if(warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-    if(warp == 8 && u1 > u0 && electOne()) {
+    if(warp == 8 && lane == 0 && u1 > u0) {
       // ---------------- issuer: every TMA load and every MMA ----------------
       const uint32_t descHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);  // stride offset | version | SWIZZLE_128B
       auto descLo = [](uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); };
