@@ -21,6 +21,7 @@
 // leave through the common exit, which still frees TMEM.
 #include "kb_conv_dev.cuh"
 #include "kb_tile_table.h"
+#include "kb_conv_small.cuh"
 
 #include <cuda.h>
 #include <cstdio>
@@ -1252,6 +1253,9 @@ struct ConvTcPlan {
   int rowsPadMax;
   int tmaEpi, epiWarpBytes, resRing;
   CUtensorMap tmRes, tmRaw, tmAct;
+  int smallMaps;  // the weight maps of the small-batch kernel exist
+  int small;  // the small-batch kernel (kb_conv_small.cu) can run this convolution
+  ConvSmallShape smallShape;
 };
 
 static int pickBN(int k, int inC, int outC) {
@@ -1324,6 +1328,19 @@ static bool encode2d(
     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
+}
+
+static bool encodeWeights3d(CUtensorMap* tm, int dt, const void* base, int inC, int outC, int taps, int boxRows, int boxTaps) {
+  EncodeTiledFn fn = getEncodeTiled();
+  if(!fn) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)inC, (cuuint64_t)outC, (cuuint64_t)taps};
+  cuuint64_t strides[2] = {(cuuint64_t)inC * 2, (cuuint64_t)inC * 2 * (cuuint64_t)outC};
+  cuuint32_t box[3] = {(cuuint32_t)TC_BK, (cuuint32_t)boxRows, (cuuint32_t)boxTaps};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(
+           tm, dt == DT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides,
+           box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 constexpr int TC_FIXED_SMEM = 2 * 512 * 4 + 96 * 8 + 64 + 1024;  // norm parameters, barriers, TMEM slot, alignment slack
@@ -1405,8 +1422,21 @@ ConvTcPlan* convTcCreate(
   int dev = 0, sms = 148;
   if(cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   p->numSMs = sms;
+  ConvSmallShape& ss = p->smallShape;
+  ss.dt = dt; ss.inC = inC; ss.outC = outC; ss.taps = kY * kX; ss.haloPad = p->haloPad; ss.aRows = p->aRows; ss.tmA = &p->tmA;
+  const int boxTaps = ss.taps == 9 ? 3 : 1;
+  p->smallMaps = encodeWeights3d(&ss.tmB32, dt, w, inC, outC, ss.taps, 32, boxTaps) && encodeWeights3d(&ss.tmB64, dt, w, inC, outC, ss.taps, 64, boxTaps);
+  p->small = 0;
   return p;
 }
+
+// Tile width of the small-batch kernel for this convolution and batch, or 0 if the wide-tile kernel runs it.  Decided by
+// the plan and the number of row tiles alone, so that every launch of a batch size takes the same route.
+static int smallWidth(const ConvTcPlan* p, const Geom& g) {
+  static const bool off = getenv("KB_NO_SMALL") != nullptr && atoi(getenv("KB_NO_SMALL")) != 0;
+  return p->small && !off ? convSmallTileWidth(p->outC, (g.rows + TC_BM - 1) / TC_BM, p->numSMs) : 0;
+}
+bool convTcRunsSmall(const ConvTcPlan* p, const Geom& g) { return p && smallWidth(p, g) > 0; }
 
 void convTcDestroy(ConvTcPlan* p) { delete p; }
 
@@ -1414,7 +1444,7 @@ void convTcDestroy(ConvTcPlan* p) { delete p; }
 // multiple of 32 channels the residual is fetched and the outputs are written by TMA through swizzled
 // shared-memory units; otherwise the epilogue threads access global memory directly.
 bool convTcSetEpilogue(ConvTcPlan* p, const Epilogue& ep) {
-  p->tmaEpi = 0; p->cg = TC_EPI_CG;
+  p->tmaEpi = 0; p->cg = TC_EPI_CG; p->small = 0;
   const bool force = getenv("KB_TC_NO_TMA_EPI") != nullptr && atoi(getenv("KB_TC_NO_TMA_EPI")) != 0;
   auto aligned32 = [](int c0, int c1) { return (c0 % 32) == 0 && (c1 % 32) == 0 && c1 > c0; };
   bool ok = !force && (p->BN % 32) == 0 && p->BN <= 256;
@@ -1471,6 +1501,8 @@ bool convTcSetEpilogue(ConvTcPlan* p, const Epilogue& ep) {
   else if(ep.outAct) enc = enc && encode2d(&p->tmAct, p->dt, ep.outAct, (uint64_t)(ep.actC1 - ep.actC0), rows, (uint64_t)ep.actStride * 2, 32, 32, sw);
   if(!enc) { p->cg = TC_EPI_CG; return needsStaged ? false : sizeRings(p, 0); }
   p->tmaEpi = 1;
+  // the small-batch kernel repeats the arithmetic of the staged epilogue; 3x3 needs two activation slots besides weights
+  p->small = p->smallMaps && convSmallSupports(ep) && 2 * p->aRows * 128 <= 64 * 1024 ? 1 : 0;
   return true;
 }
 
@@ -1496,6 +1528,9 @@ cudaError_t launchConvTc(cudaStream_t st, const ConvTcPlan* p, Geom g, const Epi
   if(ep.outRaw && ((ep.rawStride % 8) || (ep.rawC0 % 16) || (ep.rawC1 % 16))) return cudaErrorInvalidValue;
   if(ep.outAct && ((ep.actStride % 8) || (ep.actC0 % 16) || (ep.actC1 % 16) || ((ep.actC1 - ep.actC0) > 512 && ep.act != KB_ACT_SWIGLU_PAIRS))) return cudaErrorInvalidValue;
   if(ep.residual && (ep.resStride % 8)) return cudaErrorInvalidValue;
+  if(!(deps && (deps->done || deps->wait))) {
+    if(const int bn = smallWidth(p, g)) return launchConvSmall(st, p->smallShape, bn, p->numSMs, g, ep, statusWord);
+  }
   ConvTcArgs a;
   a.g = g; a.ep = ep;
   a.inC = p->inC; a.outC = p->outC; a.kY = p->kY; a.kX = p->kX;

@@ -1044,6 +1044,7 @@ void Engine::planPostPre() {
                        std::to_string(ops_[i + 1].convOutC) + " tcgen05 fused");
       int* status = statusWord_;
       op.run = [plan, status](cudaStream_t st, const Geom& g) { return launchConvPostPre(st, plan, g, status); };
+      op.members.assign(ops_.begin() + (long)i, ops_.begin() + (long)i + 2);
       out.push_back(std::move(op));
       i += 2;
     }
@@ -1104,6 +1105,8 @@ void Engine::planChains() {
       op.cls = classId(classes_[ops_[big].cls].name + " chain x" + std::to_string(j - i));
       int* status = statusWord_;
       op.run = [plan, status](cudaStream_t st, const Geom& g) { return launchConvChain(st, plan, g, status); };
+      op.members.assign(ops_.begin() + (long)i, ops_.begin() + (long)j);
+      op.tileCounters = true;
       out.push_back(std::move(op));
       i = j;
     }
@@ -1162,10 +1165,18 @@ void Engine::launchOpsEager(int n) {
     const int nc = std::min(chunk, n - c0);
     boardOffset_ = c0;
     const Geom g = makeGeom(X_, Y_, nc);
-    if(tileCtr_) cudaCheck(cudaMemsetAsync(tileCtr_, 0, tileCtrBytes_, stream_), "reset of the tile counters");
+    // the tile counters are read by multi-layer launches (small batches have none) and by per-tile dependencies
+    bool counters = tileDeps_;
+    for(const Op& op : ops_) counters = counters || (op.tileCounters && !op.runsSingly(g));
+    if(tileCtr_ && counters) cudaCheck(cudaMemsetAsync(tileCtr_, 0, tileCtrBytes_, stream_), "reset of the tile counters");
     for(size_t i = 0; i < ops_.size(); i++) {
       if(profiling_) cudaCheck(cudaEventRecord(events_[2 * i], stream_), "event record");
-      cudaError_t e = ops_[i].run(stream_, g);
+      cudaError_t e = cudaSuccess;
+      if(ops_[i].runsSingly(g)) {
+        for(const Op& m : ops_[i].members)
+          if(e == cudaSuccess) e = m.run(stream_, g);
+      }
+      else e = ops_[i].run(stream_, g);
       if(e != cudaSuccess) throw CudaError("launch of '" + classes_[ops_[i].cls].name + "' failed: " + cudaGetErrorString(e));
       if(profiling_) cudaCheck(cudaEventRecord(events_[2 * i + 1], stream_), "event record");
     }

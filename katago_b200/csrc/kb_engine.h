@@ -5,6 +5,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <functional>
 #include <map>
@@ -32,6 +33,15 @@ struct Op {
   int cls = 0;                                   // index into Engine::classes (profiling bucket)
   double flops = 0.0, bytes = 0.0;               // algorithmic, per board (scaled by n when accounted)
   std::function<cudaError_t(cudaStream_t, const Geom&)> run;
+  // launches merged into one (multi-layer launches, fused 1x1 pairs): the convolutions themselves, which small batches run
+  // one by one (runsSingly)
+  std::vector<Op> members;
+  bool tileCounters = false;  // the merged launch hands tiles over through the tile counters
+  bool runsSingly(const Geom& g) const {
+    for(const Op& m : members)
+      if(!convTcRunsSmall(m.tcPlan, g)) return false;
+    return !members.empty();
+  }
   // tensor-core convolutions only: what the launch reads and writes, and its per-tile dependency record
   const ConvTcPlan* tcPlan = nullptr;
   Epilogue ep;
@@ -60,7 +70,10 @@ class Engine {
   int precision() const { return dt_; }
   int launchesPerForward(int n) const {
     const int chunk = chunkBoards_ > 0 ? chunkBoards_ : n;
-    return (int)ops_.size() * ((n + chunk - 1) / chunk);
+    const Geom g = makeGeom(X_, Y_, std::min(chunk, n));
+    int perChunk = 0;
+    for(const Op& op : ops_) perChunk += op.runsSingly(g) ? (int)op.members.size() : 1;
+    return perChunk * ((n + chunk - 1) / chunk);
   }
 
   // meta: [n][inMetaC] rows for nets with an SGF metadata encoder (must be non-NULL exactly for those nets)

@@ -195,6 +195,8 @@ struct ConvTcDeps {
 };
 bool convTcDepsCapable(const ConvTcPlan* p);
 int convTcKernelSize(const ConvTcPlan* p);
+// True if a batch of this size runs this convolution in the small-batch kernel: merged launches then make way for single ones.
+bool convTcRunsSmall(const ConvTcPlan* p, const Geom& g);
 // True if the tile table marks this shape for multi-layer launches.
 bool convTcChainPreferred(const ConvTcPlan* p);
 int convTcDoneCount(const ConvTcPlan* p);

@@ -79,6 +79,13 @@ __device__ __forceinline__ void tmaLoad2d(uint32_t dst, const CUtensorMap* tmap,
     : "memory");
 }
 
+__device__ __forceinline__ void tmaLoad3d(uint32_t dst, const CUtensorMap* tmap, int c0, int c1, int c2, uint32_t bar) {
+  asm volatile(
+    "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+    ::"r"(dst), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+    : "memory");
+}
+
 // Tile readiness counters in global memory (per-tile dependencies between consecutive convolutions).
 __device__ __forceinline__ uint32_t ldAcquireGpu(const uint32_t* p) {
   uint32_t v;

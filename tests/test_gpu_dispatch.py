@@ -25,3 +25,26 @@ def test_input_widths_between_chunks(prec, tol, trunk, mid, oracle):
     ref = oracle.eval_layer(blob, x, mask, trunk)
     out = capi.eval_layer(blob, x, mask, trunk, precision=prec)
     assert np.all(np.abs(out - ref) <= tol * np.maximum(np.maximum(np.abs(out), np.abs(ref)), 3.0))
+
+
+@pytest.mark.parametrize("factory,prec,full,edge", [
+    (lambda: mf.make_b18c384nbt(num_blocks=3), capi.PRECISION_FP16, 128, 19),
+    (lambda: mf.make_b18c384nbt(num_blocks=3), capi.PRECISION_BF16, 128, 9),
+    (lambda: mf.make_b28c512nbt(num_blocks=3), capi.PRECISION_BF16, 128, 19),
+    (lambda: mf.make_b28c512nbt(num_blocks=3), capi.PRECISION_FP16, 64, 13),
+    (lambda: mf.make_b6c96(), capi.PRECISION_FP16, 256, 19),
+])
+def test_small_batches_give_the_rows_of_a_full_batch(factory, prec, full, edge):
+    """Small batches run in narrow tiles (kb_conv_small.cu), full ones in wide tiles and merged launches.  The order of an
+    accumulator's additions depends on neither, so a position's outputs are the same bits whatever batch it is in."""
+    model = capi.Model(mf.to_blob(factory()))
+    h = capi.Handle(model, full, nn_x=edge, nn_y=edge, precision=prec)
+    sizes = ([edge, 9, 7, edge] * full)[:full]
+    sp, gl = mf.random_positions(full, seed=61, nn_len=edge, board_sizes=sizes)
+    ref = h.forward(sp, gl)
+    for n in (1, 2, 5, 11, 12, 13, 24, 25, 32, 48):
+        for _ in range(2):  # the eager run and the graph
+            part = h.forward(sp[:n], gl[:n])
+            for k in ref:
+                assert np.array_equal(part[k], ref[k][:n]), (n, k)
+    h.close()
