@@ -321,7 +321,7 @@ ConvSmallKernelFn smallKernelForT(int act) {
 }  // namespace
 
 bool convSmallSupports(const Epilogue& ep) {
-  if(ep.sumsqOut || ep.rowSumsq) return false;
+  if(ep.sumsqOut || ep.rowSumsq || ep.act == KB_ACT_SWIGLU_PAIRS || ep.act == KB_ACT_ROPE_QK) return false;
   return !ep.outAct || smallKernelForT<__half>(ep.act) != nullptr;
 }
 
