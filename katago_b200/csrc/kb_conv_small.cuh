@@ -6,11 +6,15 @@
 
 namespace kb {
 
+// Tile widths the kernel is launched with.
+constexpr int CONV_SMALL_WIDTHS[4] = {16, 32, 64, 96};
+inline int convSmallMapIndex(int BN) { return BN <= 32 ? BN / 16 - 1 : BN / 32; }
+
 struct ConvSmallShape {
   int dt, inC, outC, taps;      // taps: 1 or 9
   int haloPad, aRows;           // of the activation box, as in the convolution's plan
   const CUtensorMap* tmA;       // activations, box of 64 channels x aRows rows
-  CUtensorMap tmB32, tmB64;     // weights [taps][outC][inC], boxes of 64 channels x 32 or 64 rows x 1 or 3 taps
+  CUtensorMap tmB[4];           // weights [taps][outC][inC], boxes of 64 channels x CONV_SMALL_WIDTHS[i] rows x 1 or 3 taps
 };
 
 // True if the kernel has a variant for this epilogue (staged-epilogue convolutions without row sums).

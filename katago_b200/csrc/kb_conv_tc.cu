@@ -513,15 +513,21 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
   tcFenceAfter();
   const uint32_t tmemBase = *tmemSlot;
 
+  // The feeding and the issuing warp of a CTA pair run their loops with all lanes and elect a thread for each batch of
+  // instructions (mbarWaitWarp); those of a single CTA run them inside one elected thread.  Measured both ways: 3x3 256->256
+  // in pairs (b28, batch 512) 182 us with all lanes against 189 with one (with residual), 178 against 179 (without); 3x3
+  // 192->192 for single CTAs 72 against 69, the transformer's net at batch 128 4410 against 4370.
+  auto one = [&]() { return PAIR ? electOne() : true; };
+  auto aborted = [&]() { return PAIR ? warpAny(*abortFlag) : *abortFlag != 0; };
   if(warp == 0) {
     // ---------------- TMA producer ----------------
-    if(electOne()) {
+    if(PAIR || electOne()) {
       uint32_t sa = 0, phA = 0, sb = 0, phB = 0;
-      bool ok = true;
       // In a pair both CTAs load their own rows of A and their own half of each weight tile; every load signals the
       // leader's barrier, on which the leader alone has announced the bytes of both CTAs.
       const uint32_t aBytes = (PAIR ? 2u : 1u) * (uint32_t)a.aSlotBytes, bBytes = (PAIR ? 2u : 1u) * (uint32_t)a.bSlotBytes;
       const int bRow0 = PAIR ? (int)rank * (a.BN / 2) : 0;
+      auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_PRODUCER_TIMEOUT); };
       auto loadA = [&](uint32_t slot, int kc, int m0) {
         const uint32_t bar = smemU32(&fullA[slot]), dst = smemU32(smemA + (size_t)slot * a.aSlotBytes);
         if(leader) mbarExpectTx(bar, aBytes);
@@ -534,83 +540,91 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
         if(PAIR) tmaLoad2dPair(dst, &tmB, kc * TC_BK, row + bRow0, pairLeaderAddr(bar));
         else tmaLoad2d(dst, &tmB, kc * TC_BK, row, bar);
       };
-      if(a.residentB) {
-        // the number of CTAs (pairs) is a multiple of the number of channel tiles, so this CTA always works on the same one
-        const int n0 = (tm.first % numNTiles) * a.BN;
-        for(int kc = 0; kc < a.kChunks; kc++) loadB((uint32_t)kc, kc, n0);
-      }
       // Weight ring: the first tile's first slots are requested before the wait on the preceding kernels as well (the
       // ring starts empty, so the slots need no empty-wait); the main loop below skips those loads.
       int prefilled = 0;
       if(!a.residentB && a.prefillB && !a.jointAB && tm.first < numTiles) {
-        const int n0 = tm.nTile(tm.first) * a.BN;
         const int total = a.kChunks * taps;
         prefilled = a.numB < total ? a.numB : total;
-        for(int i = 0; i < prefilled; i++) loadB((uint32_t)i, i / taps, (i % taps) * a.outC + n0);
+      }
+      if(one()) {
+        if(a.residentB) {
+          // the number of CTAs (pairs) is a multiple of the number of channel tiles, so this CTA always works on the same one
+          const int n0 = (tm.first % numNTiles) * a.BN;
+          for(int kc = 0; kc < a.kChunks; kc++) loadB((uint32_t)kc, kc, n0);
+        }
+        if(prefilled > 0) {
+          const int n0 = tm.nTile(tm.first) * a.BN;
+          for(int i = 0; i < prefilled; i++) loadB((uint32_t)i, i / taps, (i % taps) * a.outC + n0);
+        }
       }
       // everything above touched only weights; the activations belong to the kernels before this one
       const bool tileDeps = DEPS && a.depCtr != nullptr;
       if(!tileDeps) gridDepWait();
       int issuedB = 0;  // weight slots of this CTA in issue order
-      for(int t = tm.first; t < numTiles && ok; t += tm.step) {
+      for(int t = tm.first; t < numTiles && !aborted(); t += tm.step) {
         const int m0 = tm.m0(t), n0 = tm.nTile(t) * a.BN;
         if(tileDeps) {
           // the dependency warp polls the counters ahead of time and publishes how many tiles are ready
           const int need = (t - tm.first) / tm.step + 1;
           uint32_t spins = 0;
           while(*gateTiles < need) {
-            if((++spins & 63u) == 0u && *abortFlag) { ok = false; break; }
+            if((++spins & 63u) == 0u && *abortFlag) break;
           }
-          if(!ok) break;
           asm volatile("fence.acq_rel.cta;" ::: "memory");
           asm volatile("fence.proxy.async.global;" ::: "memory");
         }
         if(t == tm.first) TLT(1);
-        for(int kc = 0; kc < a.kChunks && ok; kc++) {
-          if(!mbarWait(smemU32(&emptyA[sa]), phA ^ 1u, abortFlag)) { ok = false; break; }
+        for(int kc = 0; kc < a.kChunks; kc++) {
+          wait(&emptyA[sa], phA ^ 1u);
           TRACE(true, ((t - tm.first) / tm.step) * 16 + kc);
           if(!PAIR && a.jointAB) {
             // both operands of the step on the activation slot's barrier; the weight slot has the same index
-            const uint32_t bar = smemU32(&fullA[sa]);
-            mbarExpectTx(bar, aBytes + bBytes);
-            tmaLoad2d(smemU32(smemA + (size_t)sa * a.aSlotBytes), &tmA, kc * TC_BK, m0 - a.haloPad, bar);
-            tmaLoad2d(smemU32(smemB + (size_t)sa * a.bSlotBytes), &tmB, kc * TC_BK, n0, bar);
+            if(one()) {
+              const uint32_t bar = smemU32(&fullA[sa]);
+              mbarExpectTx(bar, aBytes + bBytes);
+              tmaLoad2d(smemU32(smemA + (size_t)sa * a.aSlotBytes), &tmA, kc * TC_BK, m0 - a.haloPad, bar);
+              tmaLoad2d(smemU32(smemB + (size_t)sa * a.bSlotBytes), &tmB, kc * TC_BK, n0, bar);
+            }
             if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
             continue;
           }
-          loadA(sa, kc, m0);
+          if(one()) loadA(sa, kc, m0);
           if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
           if(a.residentB) continue;
           for(int tap = 0; tap < taps; tap++, issuedB++) {
             if(issuedB >= prefilled) {
-              if(!mbarWait(smemU32(&emptyB[sb]), phB ^ 1u, abortFlag)) { ok = false; break; }
-              loadB(sb, kc, tap * a.outC + n0);
+              wait(&emptyB[sb], phB ^ 1u);
+              if(one()) loadB(sb, kc, tap * a.outC + n0);
             }
             if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
           }
         }
       }
-      if(!ok && !*abortFlag) { *abortFlag = 1; atomicCAS(a.status, 0, TC_ERR_PRODUCER_TIMEOUT); }
     }
   }
   else if(warp == 1) {
     // ---------------- MMA issuer ----------------
-    // One thread issues every MMA; its instruction stream is the critical path of the main loop, so the
-    // descriptors are kept as 32-bit low words that only need an add per MMA, ring positions wrap by compare,
-    // and the tap offsets are computed once.
+    // This warp's instruction stream is the critical path of the main loop, so the descriptors are kept as 32-bit low
+    // words that only need an add per MMA, ring positions wrap by compare, and the tap offsets are computed once.
     // In a pair only the leader issues; its MMAs read both CTAs' shared memory and write both CTAs' TMEM, and every
     // completion is signalled to the same barrier of both CTAs.
-    if(leader && electOne()) {
-      auto mma = [&](uint32_t d, uint32_t aLo, uint32_t bLo, uint32_t descHi, uint32_t acc) {
-        if(PAIR) ummaLoHiPair(d, aLo, bLo, descHi, a.idesc, acc);
-        else ummaLoHi(d, aLo, bLo, descHi, a.idesc, acc);
-      };
+    if(leader && (PAIR || electOne())) {
+      auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_MMA_TIMEOUT); };
       auto commit = [&](uint64_t* bar) {
         const uint32_t b = smemU32(bar);
         if(PAIR) { ummaCommitPair(b); ummaCommitPair(clusterMapAddr(b, 1u)); }
         else ummaCommit(b);
       };
       const uint32_t descHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);  // stride offset | version | SWIZZLE_128B
+      // the four MMAs of a 64-channel step: advancing K by 16 elements = 32 bytes = 2 units inside the 128-byte swizzle atom
+      auto mma4 = [&](uint32_t d, uint32_t aLo, uint32_t bLo, uint32_t accumulate) {
+#pragma unroll
+        for(int k = 0; k < TC_BK / 16; k++) {
+          if(PAIR) ummaLoHiPair(d, aLo + 2 * k, bLo + 2 * k, descHi, a.idesc, k == 0 ? accumulate : 1u);
+          else ummaLoHi(d, aLo + 2 * k, bLo + 2 * k, descHi, a.idesc, k == 0 ? accumulate : 1u);
+        }
+      };
       const uint32_t aLoBase = ((smemU32(smemA) & 0x3FFFFu) >> 4) | (1u << 16);
       const uint32_t bLoBase = ((smemU32(smemB) & 0x3FFFFu) >> 4) | (1u << 16);
       const uint32_t aSlot16 = (uint32_t)a.aSlotBytes >> 4, bSlot16 = (uint32_t)a.bSlotBytes >> 4;
@@ -622,78 +636,64 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
         tapOff[tap] = (taps == 9) ? (uint32_t)(a.haloPad + dy * a.g.RW + dx) * 8u : 0u;
       }
       uint32_t sa = 0, phA = 0, sb = 0, phB = 0, it = 0;
-      bool ok = true;
-      for(int t = tm.first; t < numTiles && ok; t += tm.step, it++) {
+      for(int t = tm.first; t < numTiles && !aborted(); t += tm.step, it++) {
         const uint32_t buf = it & 1u;
         // wait until the epilogue has drained this accumulator (two tiles ago)
-        if(!mbarWait(smemU32(&accEmpty[buf]), ((it >> 1) & 1u) ^ 1u, abortFlag)) { ok = false; break; }
+        wait(&accEmpty[buf], ((it >> 1) & 1u) ^ 1u);
         tcFenceAfter();
         TRACE(true, 256 + it * 16);
         const uint32_t dTmem = tmemBase + buf * (uint32_t)a.BN;
-        uint32_t accumulate = 0;
-        for(int kc = 0; kc < a.kChunks && ok; kc++) {
-          if(!mbarWait(smemU32(&fullA[sa]), phA, abortFlag)) { ok = false; break; }
+        for(int kc = 0; kc < a.kChunks; kc++) {
+          wait(&fullA[sa], phA);
           if(it == 0 && kc == 0) { TLT(2); TL(8, (unsigned long long)clock64()); }
           TRACE(true, 256 + it * 16 + 1 + kc);
-          const uint32_t aLo = aLoBase + sa * aSlot16;
+          const uint32_t aLo = aLoBase + sa * aSlot16, accumulate = kc > 0 ? 1u : 0u;
           if(taps == 9) {
 #pragma unroll
             for(int tap = 0; tap < 9; tap++) {
-              if(!mbarWait(smemU32(&fullB[sb]), phB, abortFlag)) { ok = false; break; }
+              wait(&fullB[sb], phB);
               tcFenceAfter();
-              const uint32_t aT = aLo + tapOff[tap], bT = bLoBase + sb * bSlot16;
-#pragma unroll
-              for(int k = 0; k < TC_BK / 16; k++) {
-                // advancing K by 16 elements = 32 bytes = 2 units inside the 128-byte swizzle atom
-                mma(dTmem, aT + 2 * k, bT + 2 * k, descHi, accumulate);
-                accumulate = 1;
+              if(one()) {
+                mma4(dTmem, aLo + tapOff[tap], bLoBase + sb * bSlot16, tap == 0 ? accumulate : 1u);
+                commit(&emptyB[sb]);  // frees the weight slot once these MMAs have read it
+                if(tap == 8) commit(&emptyA[sa]);
               }
-              commit(&emptyB[sb]);  // frees the weight slot once these MMAs have read it
               if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
             }
           }
           else if(a.residentB) {
             // weights were loaded once; the barrier of chunk kc completed its only phase during the first tile
-            if(!mbarWait(smemU32(&fullB[kc]), 0u, abortFlag)) { ok = false; break; }
+            if(it == 0) wait(&fullB[kc], 0u);
             tcFenceAfter();
-            const uint32_t bT = bLoBase + (uint32_t)kc * bSlot16;
-#pragma unroll
-            for(int k = 0; k < TC_BK / 16; k++) {
-              mma(dTmem, aLo + 2 * k, bT + 2 * k, descHi, accumulate);
-              accumulate = 1;
+            if(one()) {
+              mma4(dTmem, aLo, bLoBase + (uint32_t)kc * bSlot16, accumulate);
+              commit(&emptyA[sa]);
             }
           }
           else if(!PAIR && a.jointAB) {
-            // the weight chunk arrived on the same barrier as the activation chunk and is released with it below
+            // the weight chunk arrived on the same barrier as the activation chunk and is released with it
             tcFenceAfter();
-            const uint32_t bT = bLoBase + sa * bSlot16;
-#pragma unroll
-            for(int k = 0; k < TC_BK / 16; k++) {
-              mma(dTmem, aLo + 2 * k, bT + 2 * k, descHi, accumulate);
-              accumulate = 1;
+            if(one()) {
+              mma4(dTmem, aLo, bLoBase + sa * bSlot16, accumulate);
+              commit(&emptyA[sa]);
             }
           }
           else {
-            if(!mbarWait(smemU32(&fullB[sb]), phB, abortFlag)) { ok = false; break; }
+            wait(&fullB[sb], phB);
             tcFenceAfter();
-            const uint32_t bT = bLoBase + sb * bSlot16;
-#pragma unroll
-            for(int k = 0; k < TC_BK / 16; k++) {
-              mma(dTmem, aLo + 2 * k, bT + 2 * k, descHi, accumulate);
-              accumulate = 1;
+            if(one()) {
+              mma4(dTmem, aLo, bLoBase + sb * bSlot16, accumulate);
+              commit(&emptyB[sb]);
+              commit(&emptyA[sa]);
             }
-            commit(&emptyB[sb]);
             if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
           }
-          commit(&emptyA[sa]);
           if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
         }
-        if(ok) commit(&accFull[buf]);
-        TLT(3);
-        TL(9, (unsigned long long)clock64());
+        if(one()) commit(&accFull[buf]);
+        { TLT(3); TL(9, (unsigned long long)clock64()); }
         TRACE(true, 256 + it * 16 + 15);
       }
-      if(!ok && !*abortFlag) { *abortFlag = 1; atomicCAS(a.status, 0, TC_ERR_MMA_TIMEOUT); }
     }
   }
   else if(warp < 2 + TC_EPI_WARPS) {
@@ -928,6 +928,8 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
 
   if(warp == 0) {
     // ---------------- TMA producer ----------------
+    // (the loops of this kernel run inside the elected threads: with all lanes in them, as in convTcKernel, chains of four
+    // 192-wide layers took 1.5 to 2 % longer)
     if(electOne()) {
       uint32_t sa = 0, phA = 0, sb = 0, phB = 0;
       bool ok = true;
@@ -1424,8 +1426,9 @@ ConvTcPlan* convTcCreate(
   p->numSMs = sms;
   ConvSmallShape& ss = p->smallShape;
   ss.dt = dt; ss.inC = inC; ss.outC = outC; ss.taps = kY * kX; ss.haloPad = p->haloPad; ss.aRows = p->aRows; ss.tmA = &p->tmA;
-  const int boxTaps = ss.taps == 9 ? 3 : 1;
-  p->smallMaps = encodeWeights3d(&ss.tmB32, dt, w, inC, outC, ss.taps, 32, boxTaps) && encodeWeights3d(&ss.tmB64, dt, w, inC, outC, ss.taps, 64, boxTaps);
+  p->smallMaps = 1;
+  for(int bn : CONV_SMALL_WIDTHS)
+    if(!encodeWeights3d(&ss.tmB[convSmallMapIndex(bn)], dt, w, inC, outC, ss.taps, bn, ss.taps == 9 ? 3 : 1)) p->smallMaps = 0;
   p->small = 0;
   return p;
 }
@@ -1501,8 +1504,8 @@ bool convTcSetEpilogue(ConvTcPlan* p, const Epilogue& ep) {
   else if(ep.outAct) enc = enc && encode2d(&p->tmAct, p->dt, ep.outAct, (uint64_t)(ep.actC1 - ep.actC0), rows, (uint64_t)ep.actStride * 2, 32, 32, sw);
   if(!enc) { p->cg = TC_EPI_CG; return needsStaged ? false : sizeRings(p, 0); }
   p->tmaEpi = 1;
-  // the small-batch kernel repeats the arithmetic of the staged epilogue; 3x3 needs two activation slots besides weights
-  p->small = p->smallMaps && convSmallSupports(ep) && 2 * p->aRows * 128 <= 64 * 1024 ? 1 : 0;
+  // the small-batch kernel repeats the arithmetic of the staged epilogue
+  p->small = p->smallMaps && convSmallSupports(ep) ? 1 : 0;
   return true;
 }
 
