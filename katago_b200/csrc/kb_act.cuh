@@ -1,10 +1,30 @@
-// Fast activation functions for reduced-precision outputs (fp16 / bf16): special-function-unit approximations whose
-// error is far below the output rounding.  The fp32 paths use the accurate library functions instead.
+// Activation functions.  The accurate ones are for the fp32 paths; the fast ones, for reduced-precision outputs (fp16 / bf16),
+// use special-function-unit approximations whose error is far below the output rounding.
 #pragma once
 
 #include "../../include/kb_modelblob.h"
 
 namespace kb {
+
+// Activation functions (eigenbackend.cpp:749-760; MISH_SCALE8 from desc.cpp:402-432).
+__device__ __forceinline__ float mishF(float x) {
+  // x * tanh(softplus(x)), softplus linear above 20
+  float sp = (x > 20.0f) ? x : log1pf(expf(x));
+  return x * tanhf(sp);
+}
+__device__ __forceinline__ float applyActF(float x, int act) {
+  switch(act) {
+    case KB_ACT_RELU: return fmaxf(x, 0.0f);
+    case KB_ACT_MISH: return mishF(x);
+    case KB_ACT_SILU: return x / (1.0f + expf(-x));
+    case KB_ACT_MISH_SCALE8: {
+      float x8 = 8.0f * x;
+      float sp = (x8 > 20.0f) ? x8 : log1pf(expf(x8));
+      return x * tanhf(sp);
+    }
+    default: return x;
+  }
+}
 
 __device__ __forceinline__ float ex2Approx(float x) {
   float y;

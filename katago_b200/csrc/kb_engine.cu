@@ -856,7 +856,8 @@ Engine::Engine(const Model& m, int device, int maxBatch, int X, int Y, int preci
   *statusHost_ = 0;
 
   const bool tcInit = !forceSimt_ && dt_ != DT_F32 && convTcEligible(dt_, 64, m.trunkC, m.initialConv.kY, m.initialConv.kX);
-  inCdev_ = tcInit ? (m.inC + 63) / 64 * 64 : m.inC;
+  // fp32: whole 16-byte pieces per row (convF32Eligible)
+  inCdev_ = tcInit ? (m.inC + 63) / 64 * 64 : (dt_ == DT_F32 ? (m.inC + 3) / 4 * 4 : m.inC);
 
   dSpatial_ = static_cast<float*>(alloc((size_t)maxBatch * S * m.inC * sizeof(float)));
   dGlobal_ = static_cast<float*>(alloc((size_t)maxBatch * m.inGlobalC * sizeof(float)));

@@ -7,6 +7,7 @@
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <cstdint>
+#include <cstdlib>
 
 namespace kb {
 
@@ -101,6 +102,31 @@ cudaError_t launchPackInput(
 cudaError_t launchConvSimt(
   cudaStream_t st, int dt, const void* in, int inStride, int inC, const void* w, int outC, int kY, int kX,
   Geom g, const Epilogue& ep);
+
+// The same for fp32, 1x1 and 3x3, where rows of activations and weights are 16-byte aligned (kb_conv_f32.cu).  Like the
+// tensor-core kernels it relies on the zeros in the padding rows of its input.
+bool convF32Eligible(const void* in, int inStride, int inC, const void* w, int outC, int kY, int kX, const Geom& g);
+cudaError_t launchConvF32(
+  cudaStream_t st, const void* in, int inStride, int inC, const void* w, int outC, int kY, Geom g, const Epilogue& ep);
+
+// Launches a kernel that may become resident while the kernel before it in the stream still runs (programmatic dependent
+// launch).  It has to call gridDepWait() before it touches anything that other kernels of the stream read or write.
+inline bool dependentLaunches() {
+  static const bool on = getenv("KB_NO_PDL") == nullptr;
+  return on;
+}
+template <typename... P, typename... A>
+cudaError_t launchDependent(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  if(dependentLaunches()) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, fn, P(args)...);
+}
 
 // out[r][oc] (+)= act(sum_ic in[r][ic]*w[ic][oc] + bias[oc]); fp32, small row counts (heads, gpool bias, metadata encoder).
 cudaError_t launchMatMulSmall(

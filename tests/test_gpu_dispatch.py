@@ -48,3 +48,21 @@ def test_small_batches_give_the_rows_of_a_full_batch(factory, prec, full, edge):
             for k in ref:
                 assert np.array_equal(part[k], ref[k][:n]), (n, k)
     h.close()
+
+
+@pytest.mark.parametrize("trunk,mid", [(4, 8), (20, 36), (96, 96), (64, 100), (132, 48)])
+@pytest.mark.parametrize("n,ylen,xlen", [(1, 19, 19), (5, 9, 13), (2, 5, 30)])
+def test_fp32_block_widths(trunk, mid, n, ylen, xlen, oracle):
+    """fp32 residual blocks at the edges of the staged kernel's tiles (16-channel slices, 32-channel and 64-row tiles, wide
+    boards with their larger halo).  A sum of K products of order one in fp32 is off by at most about K * 2^-24 of their
+    magnitude: 2 * 9 * 132 * 6e-8 = 1.4e-4 in the worst case and two orders less in practice; 1e-4 as for the other fp32 tests."""
+    g = mf._Gen(500 + trunk + mid)
+    rng = np.random.default_rng(trunk + 7 * mid)
+    mask = np.ones((n, ylen, xlen), np.float32)
+    mask[0, ylen // 2:] = 0
+    layer = mf._gen_ordinary(g, trunk, mid, mf.ACT_MISH)
+    x = rng.standard_normal((n, ylen, xlen, trunk)).astype(np.float32) * mask[..., None]
+    blob = mf.layer_blob(layer)
+    ref = oracle.eval_layer(blob, x, mask, trunk)
+    out = capi.eval_layer(blob, x, mask, trunk, precision=capi.PRECISION_FP32)
+    assert np.abs(out - ref).max() <= 1e-4 * max(1.0, np.abs(ref).max())
