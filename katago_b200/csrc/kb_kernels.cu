@@ -492,8 +492,14 @@ cudaError_t launchBnAct(
 // The middle of a global-pooling block in one launch (eigenbackend.cpp:1188-1211): pooled statistics of the activated gpool
 // branch, the 3*Cg -> Cr matmul that turns them into a per-board bias, and the pass that adds that bias to the regular
 // branch and applies the next norm + activation + mask.  Everything is per board, so a board's CTAs need nothing from
-// other boards: grid (n, GPM_SPLIT); every CTA of a board computes the board's statistics and bias (the second reader of
-// the gpool branch hits L2) and then takes its share of the board's rows.
+// other boards.
+//
+// For a few boards the launch is one dependent chain, so it is cut at its latencies: 512 threads read a board's gpool branch in
+// one round of loads (the padding rows hold zeros and count as points off the board, which saves the point arithmetic), the
+// partial sums meet by shuffles before they meet in shared memory, and a board is split over CTAs by CHANNELS of the regular
+// branch, so that a CTA multiplies only the rows of the matrix it needs (24 KB instead of 147) and has its first rows of the
+// regular branch in registers by then.  Every CTA of a board repeats the pooling, from L2; the number of CTAs per board falls as
+// the number of boards rises.
 // out[oc] = act(sum_k in[k] * wT[oc][k] + bias[oc]) for oc < outC; in and out in shared memory, all warps take part.
 // The weights are stored output-major: a warp takes an output at a time, its lanes stride over k with coalesced loads
 // that are all in flight together (a thread-per-output loop over [k][oc] weights has one dependent chain of K
@@ -528,48 +534,68 @@ __device__ __forceinline__ void blockMatVecT(const float* in, int K, const float
   }
 }
 
-constexpr int GPM_SPLIT = 2;
-constexpr int GPM_THREADS = 256;
+constexpr int GPM_THREADS = 512;
 
+// Cg / 8, the 16-byte pieces of a gpool row, is a power of two up to 32; cPer is a multiple of 8.
 template <typename T>
-__global__ void __launch_bounds__(GPM_THREADS) gpoolMidVec8Kernel(
-  const T* __restrict__ gIn, int gStride, int Cg, const T* __restrict__ rIn, int rStride, int Cr, const float* __restrict__ wT,
+__global__ void __launch_bounds__(GPM_THREADS) gpoolMidKernel(
+  const T* __restrict__ gIn, int gStride, int Cg, const T* __restrict__ rIn, int rStride, int cPer, const float* __restrict__ wT,
   const float* __restrict__ scale, const float* __restrict__ bias, int act, const float* __restrict__ mask,
   const float* __restrict__ maskSum, T* __restrict__ out, int outStride, Geom g) {
-  extern __shared__ float sm[];  // [2][groups][Cg] partial sums / maxima, then pooled [3*Cg], then board bias [Cr]
-  const int n = blockIdx.x;
-  const int vecs = Cg / 8;
-  const int groups = GPM_THREADS / vecs;
-  float* sPooled = sm + 2 * groups * Cg;
+  extern __shared__ float sm[];  // [2][warps][Cg] partial sums / maxima, then pooled [3*Cg], then board bias [cPer]
+  constexpr int WARPS = GPM_THREADS / 32;
+  const int n = blockIdx.x, c0 = blockIdx.y * cPer;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* sPooled = sm + 2 * WARPS * Cg;
   float* sBias = sPooled + 3 * Cg;
+  // (no early start for the launch after this one: it would take SMs from boards that have not started; batch 256 1 % slower)
+  gridDepWait();
+  const size_t board = (size_t)n * g.PB;
+  // the first piece of the regular branch this thread will finish
+  const int rvecs = cPer / 8;
+  const int cv0 = (int)threadIdx.x % rvecs, row0 = (int)threadIdx.x / rvecs, rowStep = GPM_THREADS / rvecs;
+  uint4 first = make_uint4(0u, 0u, 0u, 0u);
+  float firstMask = 0.0f;
+  if((int)threadIdx.x < rowStep * rvecs && row0 < g.PB) {
+    first = *reinterpret_cast<const uint4*>(rIn + (board + row0) * rStride + c0 + cv0 * 8);
+    firstMask = mask[board + row0];
+  }
   {
-    const int cgv = threadIdx.x % vecs, rg = threadIdx.x / vecs;
+    const int vecs = Cg / 8, groups = GPM_THREADS / vecs;
+    const int cv = (int)threadIdx.x % vecs, rg = (int)threadIdx.x / vecs;
     float s[8], mx[8];
 #pragma unroll
     for(int j = 0; j < 8; j++) { s[j] = 0.0f; mx[j] = -1.0f; }
-    if(rg < groups) {
-#pragma unroll 4
-      for(int p = rg; p < g.S; p += groups) {
-        const int y = p / g.X, x = p - y * g.X;
-        const size_t row = (size_t)n * g.PB + (size_t)y * g.RW + x;
-        const uint4 v4 = *reinterpret_cast<const uint4*>(gIn + row * gStride + cgv * 8);
-        const T* ve = reinterpret_cast<const T*>(&v4);
-        const float mOff = mask[row] - 1.0f;
+#pragma unroll 7
+    for(int r = rg; r < g.PB; r += groups) {
+      const uint4 v4 = *reinterpret_cast<const uint4*>(gIn + (board + r) * gStride + cv * 8);
+      const T* ve = reinterpret_cast<const T*>(&v4);
+      const float mOff = mask[board + r] - 1.0f;
 #pragma unroll
-        for(int j = 0; j < 8; j++) {
-          const float v = toF<T>(ve[j]);
-          s[j] += v;
-          mx[j] = fmaxf(mx[j], v + mOff);
-        }
+      for(int j = 0; j < 8; j++) {
+        const float v = toF<T>(ve[j]);
+        s[j] += v;
+        mx[j] = fmaxf(mx[j], v + mOff);
       }
+    }
+    // lanes with the same channels lie `vecs` apart
+    for(int o = 16; o >= vecs; o >>= 1) {
 #pragma unroll
-      for(int j = 0; j < 8; j++) { sm[rg * Cg + cgv * 8 + j] = s[j]; sm[(groups + rg) * Cg + cgv * 8 + j] = mx[j]; }
+      for(int j = 0; j < 8; j++) {
+        s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+        mx[j] = fmaxf(mx[j], __shfl_xor_sync(0xffffffffu, mx[j], o));
+      }
+    }
+    if(lane < vecs) {
+#pragma unroll
+      for(int j = 0; j < 8; j++) { sm[warp * Cg + lane * 8 + j] = s[j]; sm[(WARPS + warp) * Cg + lane * 8 + j] = mx[j]; }
     }
   }
   __syncthreads();
   for(int c = threadIdx.x; c < Cg; c += blockDim.x) {
     float ss = 0.0f, mm = -1.0f;
-    for(int k = 0; k < groups; k++) { ss += sm[k * Cg + c]; mm = fmaxf(mm, sm[(groups + k) * Cg + c]); }
+#pragma unroll
+    for(int k = 0; k < WARPS; k++) { ss += sm[k * Cg + c]; mm = fmaxf(mm, sm[(WARPS + k) * Cg + c]); }
     const float div = maskSum[n];
     const float sq = sqrtf(div);
     const float mean = ss / div;
@@ -578,68 +604,64 @@ __global__ void __launch_bounds__(GPM_THREADS) gpoolMidVec8Kernel(
     sPooled[2 * Cg + c] = mm;
   }
   __syncthreads();
-  blockMatVecT(sPooled, 3 * Cg, wT, Cr, nullptr, KB_ACT_IDENTITY, sBias);
+  blockMatVecT(sPooled, 3 * Cg, wT + (size_t)c0 * 3 * Cg, cPer, nullptr, KB_ACT_IDENTITY, sBias);
   __syncthreads();
-  // this CTA's share of the board's rows (padding rows included: they are written as zeros)
-  const int rvecs = Cr / 8;
-  const int rowsPer = (g.PB + GPM_SPLIT - 1) / GPM_SPLIT;
-  const int r0 = blockIdx.y * rowsPer, r1 = min(g.PB, r0 + rowsPer);
-  const int total = (r1 - r0) * rvecs;
+  // all rows of the board (padding rows included: they are written as zeros)
+  if((int)threadIdx.x >= rowStep * rvecs) return;
+  const int c = c0 + cv0 * 8;
+  const float4* s4 = reinterpret_cast<const float4*>(scale + c);
+  const float4* b4 = reinterpret_cast<const float4*>(bias + c);
+  const float4 s0 = s4[0], s1 = s4[1], e0 = b4[0], e1 = b4[1];
+  const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+  const float bi[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+  float bb[8];
+#pragma unroll
+  for(int j = 0; j < 8; j++) bb[j] = sBias[cv0 * 8 + j];
   constexpr int U = 4;
-  for(int base = threadIdx.x; base < total; base += blockDim.x * U) {
+  for(int rb = row0; rb < g.PB; rb += U * rowStep) {
     uint4 xs[U];
     float mk[U];
 #pragma unroll
     for(int u = 0; u < U; u++) {
-      const int idx = base + u * blockDim.x;
-      const int rr = min(idx, total - 1) / rvecs;
-      const int c = (min(idx, total - 1) - rr * rvecs) * 8;
-      const size_t m = (size_t)n * g.PB + r0 + rr;
-      mk[u] = mask[m];
-      xs[u] = *reinterpret_cast<const uint4*>(rIn + m * rStride + c);
+      const int r = min(rb + u * rowStep, g.PB - 1);
+      if(rb == row0 && u == 0) { xs[u] = first; mk[u] = firstMask; }
+      else { mk[u] = mask[board + r]; xs[u] = *reinterpret_cast<const uint4*>(rIn + (board + r) * rStride + c); }
     }
 #pragma unroll
     for(int u = 0; u < U; u++) {
-    const int idx = base + u * blockDim.x;
-    if(idx >= total) break;
-    const int rr = idx / rvecs;
-    const int c = (idx - rr * rvecs) * 8;
-    const size_t m = (size_t)n * g.PB + r0 + rr;
-    uint4 o = make_uint4(0u, 0u, 0u, 0u);
-    if(mk[u] == 1.0f) {
-      const uint4 x = xs[u];
-      const T* xe = reinterpret_cast<const T*>(&x);
-      T* oe = reinterpret_cast<T*>(&o);
-      const float4* s4 = reinterpret_cast<const float4*>(scale + c);
-      const float4* b4 = reinterpret_cast<const float4*>(bias + c);
-      const float4 s0 = s4[0], s1 = s4[1], c0 = b4[0], c1 = b4[1];
-      const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-      const float bi[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+      const int r = rb + u * rowStep;
+      if(r >= g.PB) break;
+      uint4 o = make_uint4(0u, 0u, 0u, 0u);
+      if(mk[u] == 1.0f) {
+        const T* xe = reinterpret_cast<const T*>(&xs[u]);
+        T* oe = reinterpret_cast<T*>(&o);
 #pragma unroll
-      for(int j = 0; j < 8; j++) oe[j] = fromF<T>(fastAct(fmaf(toF<T>(xe[j]) + sBias[c + j], sc[j], bi[j]), act));
-    }
-    *reinterpret_cast<uint4*>(out + m * outStride + c) = o;
+        for(int j = 0; j < 8; j++) oe[j] = fromF<T>(fastAct(fmaf(toF<T>(xe[j]) + bb[j], sc[j], bi[j]), act));
+      }
+      *reinterpret_cast<uint4*>(out + (board + r) * outStride + c) = o;
     }
   }
 }
 
 bool gpoolMidEligible(int dt, int Cg, int gStride, int Cr, int rStride, int outStride) {
+  const int vecs = Cg / 8;
   return dt != DT_F32 && (Cg % 8) == 0 && (Cr % 8) == 0 && (gStride % 8) == 0 && (rStride % 8) == 0 && (outStride % 8) == 0 &&
-         Cg / 8 <= GPM_THREADS && Cg >= 8;
+         vecs >= 1 && vecs <= 32 && (vecs & (vecs - 1)) == 0 && Cr / 8 <= GPM_THREADS;
 }
 
 cudaError_t launchGPoolMid(
   cudaStream_t st, int dt, const void* gIn, int gStride, int Cg, const void* rIn, int rStride, int Cr, const float* w,
   const float* scale, const float* bias, int act, const float* mask, const float* maskSum, void* out, int outStride, Geom g) {
   if(!gpoolMidEligible(dt, Cg, gStride, Cr, rStride, outStride)) return cudaErrorInvalidValue;
-  const int groups = GPM_THREADS / (Cg / 8);
-  const size_t smem = (size_t)(2 * groups * Cg + 3 * Cg + Cr) * sizeof(float);
-  const dim3 grid(g.n, GPM_SPLIT);
+  // channels per CTA: 32 (a row's 64 bytes are then written whole) while two CTAs per SM are not reached, else twice as many and so on
+  int cPer = Cr % 32 == 0 ? 32 : Cr;
+  while(cPer < Cr && (Cr % (2 * cPer)) == 0 && (long long)g.n * (Cr / cPer) > 296) cPer *= 2;
+  if(cPer < Cr && (long long)g.n * (Cr / cPer) > 296) cPer = Cr;
+  const size_t smem = (size_t)(2 * (GPM_THREADS / 32) * Cg + 3 * Cg + cPer) * sizeof(float);
+  const dim3 grid(g.n, Cr / cPer);
   if(dt == DT_F16)
-    gpoolMidVec8Kernel<__half><<<grid, GPM_THREADS, smem, st>>>((const __half*)gIn, gStride, Cg, (const __half*)rIn, rStride, Cr, w, scale, bias, act, mask, maskSum, (__half*)out, outStride, g);
-  else
-    gpoolMidVec8Kernel<__nv_bfloat16><<<grid, GPM_THREADS, smem, st>>>((const __nv_bfloat16*)gIn, gStride, Cg, (const __nv_bfloat16*)rIn, rStride, Cr, w, scale, bias, act, mask, maskSum, (__nv_bfloat16*)out, outStride, g);
-  return cudaGetLastError();
+    return launchDependent(gpoolMidKernel<__half>, grid, dim3(GPM_THREADS), smem, st, (const __half*)gIn, gStride, Cg, (const __half*)rIn, rStride, cPer, w, scale, bias, act, mask, maskSum, (__half*)out, outStride, g);
+  return launchDependent(gpoolMidKernel<__nv_bfloat16>, grid, dim3(GPM_THREADS), smem, st, (const __nv_bfloat16*)gIn, gStride, Cg, (const __nv_bfloat16*)rIn, rStride, cPer, w, scale, bias, act, mask, maskSum, (__nv_bfloat16*)out, outStride, g);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -66,3 +66,22 @@ def test_fp32_block_widths(trunk, mid, n, ylen, xlen, oracle):
     ref = oracle.eval_layer(blob, x, mask, trunk)
     out = capi.eval_layer(blob, x, mask, trunk, precision=capi.PRECISION_FP32)
     assert np.abs(out - ref).max() <= 1e-4 * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("reg,gp", [(32, 8), (64, 16), (96, 64), (160, 32), (40, 128), (64, 24)])
+@pytest.mark.parametrize("n,edge", [(1, 19), (11, 9), (80, 13)])
+def test_gpool_widths(reg, gp, n, edge, oracle):
+    """Global-pooling blocks at the widths where the fused middle changes its split (channels per CTA, lanes per pooled
+    channel) or is left to the separate kernels (24 pooled channels), for few and for many boards; the tolerance is the
+    reference's reduced-precision layer tolerance (cpp/tests/testnn.cpp:8-15)."""
+    C = 64
+    g = mf._Gen(600 + reg + gp)
+    rng = np.random.default_rng(reg * gp + n)
+    mask = np.ones((n, edge, edge), np.float32)
+    mask[0, :, edge // 2:] = 0
+    layer = mf._gen_gpool(g, C, reg, gp, mf.ACT_MISH)
+    x = rng.standard_normal((n, edge, edge, C)).astype(np.float32) * mask[..., None]
+    blob = mf.layer_blob(layer)
+    ref = oracle.eval_layer(blob, x, mask, C)
+    out = capi.eval_layer(blob, x, mask, C, precision=capi.PRECISION_FP16)
+    assert np.all(np.abs(out - ref) <= 0.03 * np.maximum(np.maximum(np.abs(out), np.abs(ref)), 3.0))
