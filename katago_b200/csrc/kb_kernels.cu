@@ -738,144 +738,197 @@ cudaError_t launchHeadFinal(
 }
 
 // ---------------------------------------------------------------------------------------------
-// Everything of the heads after their first convolutions, one CTA per board (eigenbackend.cpp:1975-2025, 2063-2103): the two
-// poolings, the policy bias, the pass logits, the value MLP, and per board point the policy's norm + activation and
-// final 1x1 convolution and the ownership convolution, written in the caller's frame (inverse board symmetry).
+// Everything of the heads after their first convolutions (eigenbackend.cpp:1975-2025, 2063-2103): the two poolings, the policy
+// bias, the pass logits, the value MLP, and per board point the policy's norm + activation and final 1x1 convolution and the
+// ownership convolution, written in the caller's frame (inverse board symmetry).
+//
+// Two CTAs per board, one for the policy head (g1, p1) and one for the value head (v1): neither needs anything of the other.
+// Like gpoolMidKernel the launch is a dependent chain for a few boards; 512 threads take a board in one or two rounds of loads
+// and the matrices are brought into L1 before the wait for the kernel before this one.
 
-constexpr int HT_THREADS = 256;
+constexpr int HT_THREADS = 512;
+constexpr int HT_PARTS = 4;  // threads per channel that add up the partial sums
+
+// mean, size-scaled mean and third statistic (maximum, or the value head's second size-scaled mean) of C channels of in
+// ([rowsPad][stride], activated and masked) into pooled [3*C]; part [2][HT_THREADS / (C/8)][C]
+template <typename T, bool VALUE>
+__device__ __forceinline__ void headPool(
+  const T* in, int stride, int C, const float* mask, float boardSum, float* part, float* pooled, size_t board, const Geom& g) {
+  const int vecs = C / 8, groups = HT_THREADS / vecs;
+  const int cv = (int)threadIdx.x % vecs, rg = (int)threadIdx.x / vecs;
+  if(rg < groups) {
+    float s[8], mx[8];
+#pragma unroll
+    for(int j = 0; j < 8; j++) { s[j] = 0.0f; mx[j] = -1.0f; }
+    // padding rows hold zeros and count as points off the board
+#pragma unroll 5
+    for(int r = rg; r < g.PB; r += groups) {
+      const uint4 v4 = *reinterpret_cast<const uint4*>(in + (board + r) * stride + cv * 8);
+      const T* ve = reinterpret_cast<const T*>(&v4);
+      const float mOff = VALUE ? 0.0f : mask[board + r] - 1.0f;
+#pragma unroll
+      for(int j = 0; j < 8; j++) {
+        const float v = toF<T>(ve[j]);
+        s[j] += v;
+        if(!VALUE) mx[j] = fmaxf(mx[j], v + mOff);
+      }
+    }
+#pragma unroll
+    for(int j = 0; j < 8; j++) {
+      part[rg * C + cv * 8 + j] = s[j];
+      if(!VALUE) part[(groups + rg) * C + cv * 8 + j] = mx[j];
+    }
+  }
+  __syncthreads();
+  // HT_PARTS neighbouring lanes share a channel
+  for(int i = threadIdx.x; i < (C * HT_PARTS + 31) / 32 * 32; i += HT_THREADS) {
+    const int c = min(i / HT_PARTS, C - 1), q = i % HT_PARTS;
+    float ss = 0.0f, mm = -1.0f;
+    for(int k = q; k < groups; k += HT_PARTS) {
+      ss += part[k * C + c];
+      if(!VALUE) mm = fmaxf(mm, part[(groups + k) * C + c]);
+    }
+#pragma unroll
+    for(int o = 1; o < HT_PARTS; o <<= 1) {
+      ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+    }
+    if(q == 0 && i < C * HT_PARTS) {
+      const float sq = sqrtf(boardSum);
+      const float mean = ss / boardSum;
+      pooled[c] = mean;
+      pooled[C + c] = mean * (sq - 14.0f) * 0.1f;
+      pooled[2 * C + c] = VALUE ? mean * ((sq - 14.0f) * (sq - 14.0f) * 0.01f - 0.1f) : mm;
+    }
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void prefetchL1(const float* p, int count) {
+  for(int i = (int)threadIdx.x * 32; i < count; i += HT_THREADS * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + i));
+}
 
 template <typename T>
 __global__ void __launch_bounds__(HT_THREADS) headsTailKernel(const HeadsTailArgs a, Geom g) {
   extern __shared__ float sm[];
   const int n = blockIdx.x;
   const int GV = a.G1 + a.V1;
-  const int vecs = GV / 8;
-  const int groups = HT_THREADS / vecs;
-  float* sPart = sm;                                  // [2][groups][GV]
-  float* sPoolG = sPart + 2 * groups * GV;            // [3*G1]
-  float* sPoolV = sPoolG + 3 * a.G1;                  // [3*V1]
-  float* sPBias = sPoolV + 3 * a.V1;                  // [P1]
-  float* sHidden = sPBias + a.P1;                     // [passH]
-  float* sV2 = sHidden + (a.passH > 0 ? a.passH : 1); // [V2]
-  float* sSmall = sV2 + a.V2;                         // pass [Pc], value [Vc], score [Sv]
-  float* sW2 = sSmall + a.Pc + a.Vc + a.Sv;           // [P1][Pc]
-  float* sWOwn = sW2 + a.P1 * a.Pc;                   // [V1]
-  float* sScale = sWOwn + a.V1;                       // [P1] then bias [P1]
-  for(int i = threadIdx.x; i < a.P1 * a.Pc; i += blockDim.x) sW2[i] = a.w2[i];
-  for(int i = threadIdx.x; i < a.V1; i += blockDim.x) sWOwn[i] = a.wOwn[i];
-  for(int i = threadIdx.x; i < a.P1; i += blockDim.x) { sScale[i] = a.pScale[i]; sScale[a.P1 + i] = a.pBias[i]; }
   const T* gv = static_cast<const T*>(a.gv);
-  const T* praw = static_cast<const T*>(a.pRaw);
-  {
-    const int cv = threadIdx.x % vecs, rg = threadIdx.x / vecs;
-    float s[8], mx[8];
-#pragma unroll
-    for(int j = 0; j < 8; j++) { s[j] = 0.0f; mx[j] = -1.0f; }
-    if(rg < groups) {
+  const size_t board = (size_t)n * g.PB;
+  gridDepLaunch();
+  if(blockIdx.y == 0) {
+    // ---- policy head ----
+    float* sPart = sm;                                               // [2][groups][G1]
+    float* sPool = sPart + 2 * (HT_THREADS / (a.G1 / 8)) * a.G1;     // [3*G1]
+    float* sPBias = sPool + 3 * a.G1;                                // [P1]
+    float* sHidden = sPBias + a.P1;                                  // [passH]
+    float* sPass = sHidden + (a.passH > 0 ? a.passH : 1);            // [Pc]
+    float* sW2 = sPass + a.Pc;                                       // [P1][Pc]
+    float* sScale = sW2 + a.P1 * a.Pc;                               // [P1] then bias [P1]
+    for(int i = threadIdx.x; i < a.P1 * a.Pc; i += blockDim.x) sW2[i] = a.w2[i];
+    for(int i = threadIdx.x; i < a.P1; i += blockDim.x) { sScale[i] = a.pScale[i]; sScale[a.P1 + i] = a.pBias[i]; }
+    prefetchL1(a.wGB, 3 * a.G1 * a.P1);
+    prefetchL1(a.wPass, 3 * a.G1 * (a.passH > 0 ? a.passH : a.Pc));
+    if(a.passH > 0) prefetchL1(a.wPass2, a.passH * a.Pc);
+    gridDepWait();
+    headPool<T, false>(gv, GV, a.G1, a.mask, a.maskSum[n], sPart, sPool, board, g);
+    blockMatVecT(sPool, 3 * a.G1, a.wGB, a.P1, nullptr, KB_ACT_IDENTITY, sPBias);
+    if(a.passH > 0) blockMatVecT(sPool, 3 * a.G1, a.wPass, a.passH, a.bPass, a.passAct, sHidden);
+    else blockMatVecT(sPool, 3 * a.G1, a.wPass, a.Pc, nullptr, KB_ACT_IDENTITY, sPass);
+    __syncthreads();
+    if(a.passH > 0) {
+      blockMatVecT(sHidden, a.passH, a.wPass2, a.Pc, nullptr, KB_ACT_IDENTITY, sPass);
+      __syncthreads();
+    }
+    for(int i = threadIdx.x; i < a.Pc; i += blockDim.x) a.outPass[(size_t)n * a.Pc + i] = sPass[i];
+    const int sym = a.symmetry ? a.symmetry[n] : 0;
+    const T* praw = static_cast<const T*>(a.pRaw);
+    for(int p = threadIdx.x; p < g.S; p += blockDim.x) {
+      const int h = p / g.X, w = p - h * g.X;
+      const size_t row = board + (size_t)h * g.RW + w;
+      int h2, w2p;
+      symMap(sym, true, g.Y, g.X, h, w, h2, w2p);
+      const size_t outPos = (size_t)n * g.S + (size_t)h2 * g.X + w2p;
+      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if(a.mask[row] == 1.0f) {
+        const T* pr = praw + row * a.P1;
 #pragma unroll 2
-      for(int p = rg; p < g.S; p += groups) {
-        const int y = p / g.X, x = p - y * g.X;
-        const size_t row = (size_t)n * g.PB + (size_t)y * g.RW + x;
-        const uint4 v4 = *reinterpret_cast<const uint4*>(gv + row * GV + cv * 8);
-        const T* ve = reinterpret_cast<const T*>(&v4);
-        const float mOff = a.mask[row] - 1.0f;
+        for(int c8 = 0; c8 < a.P1; c8 += 8) {
+          const uint4 x = *reinterpret_cast<const uint4*>(pr + c8);
+          const T* xe = reinterpret_cast<const T*>(&x);
 #pragma unroll
-        for(int j = 0; j < 8; j++) {
-          const float v = toF<T>(ve[j]);
-          s[j] += v;
-          mx[j] = fmaxf(mx[j], v + mOff);
+          for(int j = 0; j < 8; j++) {
+            const int c = c8 + j;
+            // the activated value passes through the storage type, as it does where this tensor is written out
+            const float v = toF<T>(fromF<T>(fastAct(fmaf(toF<T>(xe[j]) + sPBias[c], sScale[c], sScale[a.P1 + c]), a.pAct)));
+            for(int k = 0; k < a.Pc && k < 4; k++) acc[k] = fmaf(v, sW2[c * a.Pc + k], acc[k]);
+          }
         }
       }
-#pragma unroll
-      for(int j = 0; j < 8; j++) { sPart[rg * GV + cv * 8 + j] = s[j]; sPart[(groups + rg) * GV + cv * 8 + j] = mx[j]; }
+      for(int k = 0; k < a.Pc && k < 4; k++) a.outPolicy[outPos * a.Pc + k] = acc[k];
     }
   }
-  __syncthreads();
-  for(int c = threadIdx.x; c < GV; c += blockDim.x) {
-    float ss = 0.0f, mm = -1.0f;
-    for(int k = 0; k < groups; k++) { ss += sPart[k * GV + c]; mm = fmaxf(mm, sPart[(groups + k) * GV + c]); }
-    const float div = a.maskSum[n];
-    const float sq = sqrtf(div);
-    const float mean = ss / div;
-    if(c < a.G1) {
-      sPoolG[c] = mean; sPoolG[a.G1 + c] = mean * (sq - 14.0f) * 0.1f; sPoolG[2 * a.G1 + c] = mm;
-    }
-    else {
-      const int cc = c - a.G1;
-      sPoolV[cc] = mean; sPoolV[a.V1 + cc] = mean * (sq - 14.0f) * 0.1f; sPoolV[2 * a.V1 + cc] = mean * ((sq - 14.0f) * (sq - 14.0f) * 0.01f - 0.1f);
-    }
-  }
-  __syncthreads();
-  blockMatVecT(sPoolG, 3 * a.G1, a.wGB, a.P1, nullptr, KB_ACT_IDENTITY, sPBias);
-  if(a.passH > 0) blockMatVecT(sPoolG, 3 * a.G1, a.wPass, a.passH, a.bPass, a.passAct, sHidden);
-  else blockMatVecT(sPoolG, 3 * a.G1, a.wPass, a.Pc, nullptr, KB_ACT_IDENTITY, sSmall);
-  blockMatVecT(sPoolV, 3 * a.V1, a.wV2, a.V2, a.bV2, a.v2Act, sV2);
-  __syncthreads();
-  if(a.passH > 0) blockMatVecT(sHidden, a.passH, a.wPass2, a.Pc, nullptr, KB_ACT_IDENTITY, sSmall);
-  blockMatVecT(sV2, a.V2, a.wV3, a.Vc, a.bV3, KB_ACT_IDENTITY, sSmall + a.Pc);
-  blockMatVecT(sV2, a.V2, a.wSV, a.Sv, a.bSV, KB_ACT_IDENTITY, sSmall + a.Pc + a.Vc);
-  __syncthreads();
-  for(int i = threadIdx.x; i < a.Pc; i += blockDim.x) a.outPass[(size_t)n * a.Pc + i] = sSmall[i];
-  for(int i = threadIdx.x; i < a.Vc; i += blockDim.x) a.outValue[(size_t)n * a.Vc + i] = sSmall[a.Pc + i];
-  for(int i = threadIdx.x; i < a.Sv; i += blockDim.x) a.outScore[(size_t)n * a.Sv + i] = sSmall[a.Pc + a.Vc + i];
-  const int sym = a.symmetry ? a.symmetry[n] : 0;
-  for(int p = threadIdx.x; p < g.S; p += blockDim.x) {
-    const int h = p / g.X, w = p - h * g.X;
-    const size_t row = (size_t)n * g.PB + (size_t)h * g.RW + w;
-    int h2, w2p;
-    symMap(sym, true, g.Y, g.X, h, w, h2, w2p);
-    const size_t outPos = (size_t)n * g.S + (size_t)h2 * g.X + w2p;
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if(a.mask[row] == 1.0f) {
-      const T* pr = praw + row * a.P1;
-      for(int c8 = 0; c8 < a.P1; c8 += 8) {
-        const uint4 x = *reinterpret_cast<const uint4*>(pr + c8);
+  else {
+    // ---- value head ----
+    float* sPart = sm;                                            // [groups][V1]
+    float* sPool = sPart + (HT_THREADS / (a.V1 / 8)) * a.V1;      // [3*V1]
+    float* sV2 = sPool + 3 * a.V1;                                // [V2]
+    float* sOut = sV2 + a.V2;                                     // value [Vc], score [Sv]
+    float* sWOwn = sOut + a.Vc + a.Sv;                            // [V1]
+    for(int i = threadIdx.x; i < a.V1; i += blockDim.x) sWOwn[i] = a.wOwn[i];
+    prefetchL1(a.wV2, 3 * a.V1 * a.V2);
+    prefetchL1(a.wV3, a.V2 * a.Vc);
+    prefetchL1(a.wSV, a.V2 * a.Sv);
+    gridDepWait();
+    headPool<T, true>(gv + a.G1, GV, a.V1, a.mask, a.maskSum[n], sPart, sPool, board, g);
+    blockMatVecT(sPool, 3 * a.V1, a.wV2, a.V2, a.bV2, a.v2Act, sV2);
+    const int sym = a.symmetry ? a.symmetry[n] : 0;
+    for(int p = threadIdx.x; p < g.S; p += blockDim.x) {
+      const int h = p / g.X, w = p - h * g.X;
+      const size_t row = board + (size_t)h * g.RW + w;
+      int h2, w2p;
+      symMap(sym, true, g.Y, g.X, h, w, h2, w2p);
+      float o = 0.0f;
+      const T* vr = gv + row * GV + a.G1;
+#pragma unroll 4
+      for(int c8 = 0; c8 < a.V1; c8 += 8) {
+        const uint4 x = *reinterpret_cast<const uint4*>(vr + c8);
         const T* xe = reinterpret_cast<const T*>(&x);
 #pragma unroll
-        for(int j = 0; j < 8; j++) {
-          const int c = c8 + j;
-          // the activated value passes through the storage type, as it does where this tensor is written out
-          const float v = toF<T>(fromF<T>(fastAct(fmaf(toF<T>(xe[j]) + sPBias[c], sScale[c], sScale[a.P1 + c]), a.pAct)));
-          for(int k = 0; k < a.Pc && k < 4; k++) acc[k] = fmaf(v, sW2[c * a.Pc + k], acc[k]);
-        }
+        for(int j = 0; j < 8; j++) o = fmaf(toF<T>(xe[j]), sWOwn[c8 + j], o);
       }
+      a.outOwnership[(size_t)n * g.S + (size_t)h2 * g.X + w2p] = o;
     }
-    for(int k = 0; k < a.Pc && k < 4; k++) a.outPolicy[outPos * a.Pc + k] = acc[k];
-    float o = 0.0f;
-    const T* vr = gv + row * GV + a.G1;
-    for(int c8 = 0; c8 < a.V1; c8 += 8) {
-      const uint4 x = *reinterpret_cast<const uint4*>(vr + c8);
-      const T* xe = reinterpret_cast<const T*>(&x);
-#pragma unroll
-      for(int j = 0; j < 8; j++) o = fmaf(toF<T>(xe[j]), sWOwn[c8 + j], o);
-    }
-    a.outOwnership[outPos] = o;
+    __syncthreads();
+    blockMatVecT(sV2, a.V2, a.wV3, a.Vc, a.bV3, KB_ACT_IDENTITY, sOut);
+    blockMatVecT(sV2, a.V2, a.wSV, a.Sv, a.bSV, KB_ACT_IDENTITY, sOut + a.Vc);
+    __syncthreads();
+    for(int i = threadIdx.x; i < a.Vc; i += blockDim.x) a.outValue[(size_t)n * a.Vc + i] = sOut[i];
+    for(int i = threadIdx.x; i < a.Sv; i += blockDim.x) a.outScore[(size_t)n * a.Sv + i] = sOut[a.Vc + i];
   }
 }
 
+static size_t headsTailSmem(const HeadsTailArgs& a) {
+  const size_t policy = (size_t)2 * (HT_THREADS / (a.G1 / 8)) * a.G1 + 3 * a.G1 + a.P1 + (a.passH > 0 ? a.passH : 1) + a.Pc + (size_t)a.P1 * a.Pc + 2 * a.P1;
+  const size_t value = (size_t)(HT_THREADS / (a.V1 / 8)) * a.V1 + 3 * a.V1 + a.V2 + a.Vc + a.Sv + a.V1;
+  return (policy > value ? policy : value) * sizeof(float);
+}
+
 bool headsTailEligible(int dt, const HeadsTailArgs& a) {
-  const int GV = a.G1 + a.V1;
-  return dt != DT_F32 && (a.P1 % 8) == 0 && (a.G1 % 8) == 0 && (a.V1 % 8) == 0 && a.Pc >= 1 && a.Pc <= 4 && GV / 8 <= HT_THREADS &&
-         a.P1 <= 512 && a.V2 <= 4096 && a.passH <= 4096;
+  return dt != DT_F32 && (a.P1 % 8) == 0 && a.G1 >= 8 && (a.G1 % 8) == 0 && a.V1 >= 8 && (a.V1 % 8) == 0 && a.Pc >= 1 && a.Pc <= 4 &&
+         a.G1 / 8 <= HT_THREADS && a.V1 / 8 <= HT_THREADS && a.P1 <= 512 && a.V2 <= 4096 && a.passH <= 4096;
 }
 
 cudaError_t launchHeadsTail(cudaStream_t st, int dt, const HeadsTailArgs& a, Geom g) {
   if(!headsTailEligible(dt, a)) return cudaErrorInvalidValue;
-  const int GV = a.G1 + a.V1;
-  const int groups = HT_THREADS / (GV / 8);
-  const size_t floats = (size_t)2 * groups * GV + 3 * a.G1 + 3 * a.V1 + a.P1 + (a.passH > 0 ? a.passH : 1) + a.V2 + a.Pc + a.Vc + a.Sv +
-                        (size_t)a.P1 * a.Pc + a.V1 + 2 * a.P1;
-  const size_t smem = floats * sizeof(float);
+  const size_t smem = headsTailSmem(a);
   if(smem > 200 * 1024) return cudaErrorInvalidValue;
-  if(dt == DT_F16) {
-    if(smem > 48 * 1024) cudaFuncSetAttribute(headsTailKernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    headsTailKernel<__half><<<g.n, HT_THREADS, smem, st>>>(a, g);
+  void (*fn)(HeadsTailArgs, Geom) = dt == DT_F16 ? headsTailKernel<__half> : headsTailKernel<__nv_bfloat16>;
+  if(smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if(e != cudaSuccess) return e;
   }
-  else {
-    if(smem > 48 * 1024) cudaFuncSetAttribute(headsTailKernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    headsTailKernel<__nv_bfloat16><<<g.n, HT_THREADS, smem, st>>>(a, g);
-  }
-  return cudaGetLastError();
+  return launchDependent(fn, dim3(g.n, 2), dim3(HT_THREADS), smem, st, a, g);
 }
 
 // ---------------------------------------------------------------------------------------------
