@@ -2,13 +2,14 @@
 //
 // convSimtKernel (kb_kernels.cu) takes any shape, one 16-channel slice of one tap at a time with two block barriers each and
 // scalar loads; a 3x3 96->96 layer of eight boards ran at 6.5 of the 72 TFLOP/s the FMA units give, its 100 blocks spending
-// their time on the load latency between the barriers.  Here a block stages ALL taps of a 16-channel slice at once: the 64
+// their time on the load latency between the barriers.  Here a block stages ALL taps of a 16-channel slice at once: its
 // output rows with their halo (every tap reads the same staged rows at another offset, the padded-rows layout makes that a
 // constant) and the nine weight slices, double-buffered with cp.async, so that there are inC/16 steps per tile instead of
-// 9*inC/16.  Tiles of 64 x 32 keep small batches on many SMs (eight boards: 150 blocks).  Each of the eight warps computes
-// the whole tile over two channels of every slice, 8 x 8 outputs per thread, and the eight sums are added in warp order at
-// the end: with 4 x 4 outputs per thread and two halves of a slice the shared-memory loads took twice the time of the FMAs
-// (32 us per layer).  The order of the additions is the same in every batch size.
+// 9*inC/16.  A tile is 32 to 80 rows x 32 channels; eight warps share each half of its rows, each computes all of them over two
+// channels of every slice, up to 5 x 8 outputs per thread, and the eight sums are added in warp order at the end.  Measured
+// per 96->96 layer of eight boards (event overhead of 4.5 us included): 72 us before; 37 us with 4 x 4 outputs per thread, whose
+// shared-memory loads took twice the time of the FMAs; 35 us with 8 x 8 from eight warps (two per scheduler, 41 % FMA
+// utilisation, and 156 tiles of 64 rows on 148 SMs); 27 us as it is.  The order of the additions is the same in every batch size.
 #include "kb_kernels.cuh"
 #include "kb_act.cuh"
 #include "kb_tc_ptx.cuh"
@@ -16,32 +17,38 @@
 #include <mutex>
 #include <vector>
 #include <algorithm>
+#include <utility>
 
 namespace kb {
 
 namespace {
 
-constexpr int CF_BM = 64, CF_BN = 32, CF_BK = 16;
+constexpr int CF_BN = 32, CF_BK = 16;
 constexpr int CF_AS = CF_BK + 4;      // floats per staged row: 16-byte loads of rows 20 floats apart meet no bank twice
-constexpr int CF_THREADS = 256;
+constexpr int CF_KG = 8;               // warps that share a tile's channels
+constexpr int CF_THREADS = 512;        // two halves of a tile's rows, CF_KG warps each
+constexpr int cfRows(int nr) { return 16 * nr; }  // rows of a tile whose threads hold nr x 8 outputs
 
 __device__ __forceinline__ void cpAsync16(float* dst, const float* src, bool valid) {
   // zero-filled where there is nothing to read
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smemU32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-template <int TAPS>
+template <int TAPS, int NR>
 __global__ void __launch_bounds__(CF_THREADS) convF32Kernel(
   const float* __restrict__ in, int inStride, int inC, const float* __restrict__ w, int outC, int halo, Geom g, Epilogue ep) {
   extern __shared__ float4 smem4[];
   float* sm = reinterpret_cast<float*>(smem4);
-  const int aRows = CF_BM + 2 * halo;
+  constexpr int BM = cfRows(NR);
+  const int aRows = BM + 2 * halo;
   const int aFloats = aRows * CF_AS, bFloats = TAPS * CF_BK * CF_BN;
   const int stage = aFloats + bFloats;
   const int tid = threadIdx.x;
-  const int kg = tid >> 5, lane = tid & 31;  // this warp takes channels 2*kg, 2*kg+1 of every slice
-  const int tx = lane & 3, ty = lane >> 2;   // 8 channels (4 from tx*4, 4 from 16+tx*4); rows ty, ty+8, ..., ty+56
-  const int m0 = (int)blockIdx.x * CF_BM, n0 = (int)blockIdx.y * CF_BN;
+  const int warp = tid >> 5, lane = tid & 31;
+  const int kg = warp & (CF_KG - 1);         // this warp takes channels 2*kg, 2*kg+1 of every slice
+  const int r0 = (warp / CF_KG) * (BM / 2);  // of this half of the rows
+  const int tx = lane & 3, ty = lane >> 2;   // 8 channels (4 from tx*4, 4 from 16+tx*4); rows r0 + ty, r0 + ty+8, ...
+  const int m0 = (int)blockIdx.x * BM, n0 = (int)blockIdx.y * CF_BN;
   const int slices = (inC + CF_BK - 1) / CF_BK;
 
   auto loadB = [&](int s) {
@@ -69,9 +76,9 @@ __global__ void __launch_bounds__(CF_THREADS) convF32Kernel(
   loadA(0);
   asm volatile("cp.async.commit_group;" ::: "memory");
 
-  float acc[8][8];
+  float acc[NR][8];
 #pragma unroll
-  for(int i = 0; i < 8; i++)
+  for(int i = 0; i < NR; i++)
 #pragma unroll
     for(int j = 0; j < 8; j++) acc[i][j] = 0.0f;
 
@@ -85,16 +92,16 @@ __global__ void __launch_bounds__(CF_THREADS) convF32Kernel(
 #pragma unroll(TAPS == 9 ? 3 : 1)
     for(int tap = 0; tap < TAPS; tap++) {
       const int shift = TAPS == 9 ? (tap / 3 - 1) * g.RW + tap % 3 - 1 : 0;
-      const float* a = sA + (ty + halo + shift) * CF_AS;
+      const float* a = sA + (r0 + ty + halo + shift) * CF_AS;
       const float* b = sB + tap * CF_BK * CF_BN;
-      float2 av[8];
+      float2 av[NR];
 #pragma unroll
-      for(int i = 0; i < 8; i++) av[i] = *reinterpret_cast<const float2*>(a + 8 * i * CF_AS);
+      for(int i = 0; i < NR; i++) av[i] = *reinterpret_cast<const float2*>(a + 8 * i * CF_AS);
 #pragma unroll
       for(int k = 0; k < 2; k++) {
         const float4 b0 = *reinterpret_cast<const float4*>(b + k * CF_BN), b1 = *reinterpret_cast<const float4*>(b + k * CF_BN + 16);
 #pragma unroll
-        for(int i = 0; i < 8; i++) {
+        for(int i = 0; i < NR; i++) {
           const float x = k == 0 ? av[i].x : av[i].y;
           acc[i][0] = fmaf(x, b0.x, acc[i][0]); acc[i][1] = fmaf(x, b0.y, acc[i][1]);
           acc[i][2] = fmaf(x, b0.z, acc[i][2]); acc[i][3] = fmaf(x, b0.w, acc[i][3]);
@@ -106,29 +113,27 @@ __global__ void __launch_bounds__(CF_THREADS) convF32Kernel(
     __syncthreads();  // the buffer is free for the slice after next
   }
 
-  // The warps' partial sums of the 64 x 32 tile, added in warp order by the thread that finishes 8 channels of a row.
+  // The warps' partial sums of the tile, added in warp order by the thread that finishes 4 channels of a row.
 #pragma unroll
-  for(int i = 0; i < 8; i++) {
-    float4* o = reinterpret_cast<float4*>(sm + kg * CF_BM * CF_BN + (ty + 8 * i) * CF_BN);
+  for(int i = 0; i < NR; i++) {
+    float4* o = reinterpret_cast<float4*>(sm + (kg * BM + r0 + ty + 8 * i) * CF_BN);
     o[tx] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
     o[4 + tx] = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
   }
   __syncthreads();
-  const int r = tid >> 2, m = m0 + r;
-  if(m >= g.rowsPad) return;
-  const int br = m % g.PB, y = br / g.RW, x = br - y * g.RW;
-  const bool point = m < g.rows && y < g.Y && x < g.X;
-  const float mk = ep.mask ? ep.mask[m] : 1.0f;
-  const int bIdx = min(m / g.PB, g.n - 1);
-#pragma unroll
-  for(int h = 0; h < 2; h++) {
-    const int cl = h * 16 + (tid & 3) * 4, c = n0 + cl;
-    if(c >= outC) continue;
+  for(int i = tid; i < BM * (CF_BN / 4); i += CF_THREADS) {
+    const int r = i >> 3, cl = (i & 7) * 4, c = n0 + cl;
+    const int m = m0 + r;
+    if(m >= g.rowsPad || c >= outC) continue;
+    const int br = m % g.PB, y = br / g.RW, x = br - y * g.RW;
+    const bool point = m < g.rows && y < g.Y && x < g.X;
+    const float mk = ep.mask ? ep.mask[m] : 1.0f;
+    const int bIdx = min(m / g.PB, g.n - 1);
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // stays 0 on rows of the layout that are not board points, as in the general kernel
     if(point) {
 #pragma unroll
-      for(int k = 0; k < CF_THREADS / 32; k++) {
-        const float4 t = *reinterpret_cast<const float4*>(sm + k * CF_BM * CF_BN + r * CF_BN + cl);
+      for(int k = 0; k < CF_KG; k++) {
+        const float4 t = *reinterpret_cast<const float4*>(sm + (k * BM + r) * CF_BN + cl);
         v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
       }
     }
@@ -165,9 +170,17 @@ __global__ void __launch_bounds__(CF_THREADS) convF32Kernel(
   }
 }
 
-size_t smemBytes(int taps, int halo) {
-  const size_t stages = 2 * ((size_t)(CF_BM + 2 * halo) * CF_AS + (size_t)taps * CF_BK * CF_BN);
-  return std::max(stages, (size_t)(CF_THREADS / 32) * CF_BM * CF_BN) * sizeof(float);
+size_t smemBytes(int taps, int nr, int halo) {
+  const size_t stages = 2 * ((size_t)(cfRows(nr) + 2 * halo) * CF_AS + (size_t)taps * CF_BK * CF_BN);
+  return std::max(stages, (size_t)CF_KG * cfRows(nr) * CF_BN) * sizeof(float);
+}
+
+typedef void (*ConvF32Fn)(const float*, int, int, const float*, int, int, Geom, Epilogue);
+constexpr int CF_MAX_NR = 5;
+ConvF32Fn kernelOf(int taps, int nr) {
+  static const ConvF32Fn k1[] = {convF32Kernel<1, 2>, convF32Kernel<1, 3>, convF32Kernel<1, 4>, convF32Kernel<1, 5>};
+  static const ConvF32Fn k9[] = {convF32Kernel<9, 2>, convF32Kernel<9, 3>, convF32Kernel<9, 4>, convF32Kernel<9, 5>};
+  return (taps == 9 ? k9 : k1)[nr - 2];
 }
 
 }  // namespace
@@ -176,30 +189,39 @@ size_t smemBytes(int taps, int halo) {
 bool convF32Eligible(const void* in, int inStride, int inC, const void* w, int outC, int kY, int kX, const Geom& g) {
   return ((kY == 1 && kX == 1) || (kY == 3 && kX == 3)) && (inC % 4) == 0 && (outC % 4) == 0 && (inStride % 4) == 0 &&
          (reinterpret_cast<uintptr_t>(in) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
-         smemBytes(kY * kX, kY == 3 ? g.RW + 1 : 0) <= 200 * 1024;
+         smemBytes(kY * kX, CF_MAX_NR, kY == 3 ? g.RW + 1 : 0) <= 200 * 1024;
 }
 
 cudaError_t launchConvF32(
   cudaStream_t st, const void* in, int inStride, int inC, const void* w, int outC, int kY, Geom g, const Epilogue& ep) {
   const int halo = kY == 3 ? g.RW + 1 : 0;
-  const size_t smem = smemBytes(kY * kY, halo);
-  void (*fn)(const float*, int, int, const float*, int, int, Geom, Epilogue) = kY == 3 ? convF32Kernel<9> : convF32Kernel<1>;
+  int dev = 0, sms = 148;
+  if(cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // Rows per tile: what counts is the SM with the most tiles, times their height (b6c96, eight boards: 150 tiles of 64 rows are
+  // two on some SM, 120 of 80 rows one everywhere).
+  const int nTiles = (outC + CF_BN - 1) / CF_BN;
+  int nr = 2;
+  long long best = 0;
+  for(int c = 2; c <= CF_MAX_NR; c++) {
+    const long long tiles = (long long)((g.rows + cfRows(c) - 1) / cfRows(c)) * nTiles;
+    const long long cost = (tiles + sms - 1) / sms * c;
+    if(c == 2 || cost <= best) { best = cost; nr = c; }
+  }
+  const ConvF32Fn fn = kernelOf(kY * kY, nr);
   {
-    // opt in to the large dynamic shared memory once per device
+    // opt in to the large dynamic shared memory once per variant and device
     static std::mutex mu;
-    static std::vector<int> done;
-    int dev = 0;
-    cudaGetDevice(&dev);
+    static std::vector<std::pair<ConvF32Fn, int>> done;
     std::lock_guard<std::mutex> lock(mu);
-    if(std::find(done.begin(), done.end(), dev) == done.end()) {
-      cudaError_t e = cudaFuncSetAttribute((const void*)convF32Kernel<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      if(e == cudaSuccess) e = cudaFuncSetAttribute((const void*)convF32Kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    const std::pair<ConvF32Fn, int> key(fn, dev);
+    if(std::find(done.begin(), done.end(), key) == done.end()) {
+      cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       if(e != cudaSuccess) return e;
-      done.push_back(dev);
+      done.push_back(key);
     }
   }
-  return launchDependent(fn, dim3(g.rowsPad / CF_BM, (outC + CF_BN - 1) / CF_BN), dim3(CF_THREADS), smem, st, (const float*)in, inStride, inC,
-                         (const float*)w, outC, halo, g, ep);
+  return launchDependent(fn, dim3((g.rows + cfRows(nr) - 1) / cfRows(nr), nTiles), dim3(CF_THREADS), smemBytes(kY * kY, nr, halo), st, (const float*)in,
+                         inStride, inC, (const float*)w, outC, halo, g, ep);
 }
 
 }  // namespace kb
