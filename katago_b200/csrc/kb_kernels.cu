@@ -226,8 +226,6 @@ __global__ void __launch_bounds__(256) convSimtKernel(
 cudaError_t launchConvSimt(
   cudaStream_t st, int dt, const void* in, int inStride, int inC, const void* w, int outC, int kY, int kX,
   Geom g, const Epilogue& ep) {
-  // b6c96, eight boards: 3x3 96->96 72 us in convSimtKernel, 27 us in convF32Kernel (events around each launch)
-  if(dt == DT_F32 && convF32Eligible(in, inStride, inC, w, outC, kY, kX, g)) return launchConvF32(st, in, inStride, inC, w, outC, kY, g, ep);
   dim3 grid(g.rowsPad / SC_BM, (outC + SC_BN - 1) / SC_BN);
   KB_DISPATCH_DT(dt, (convSimtKernel<T><<<grid, 256, 0, st>>>((const T*)in, inStride, inC, (const T*)w, outC, kY, kX, g, ep)));
   return cudaGetLastError();
