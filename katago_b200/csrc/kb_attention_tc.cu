@@ -447,6 +447,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1) attentionPipeKernel(const __gri
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  gridDepLaunch();
   AT_TRACE(0);
   if(tid == 0) {
     for(int i = 0; i < AP_NUM_BARS; i++) mbarInit(smemU32(&bars[i]), (i == AP_SM_DONE || (i >= AP_O_FREE && i < AP_P_FREE)) ? 8 : 1);
@@ -465,6 +466,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1) attentionPipeKernel(const __gri
   tcFenceBefore();
   __syncthreads();
   tcFenceAfter();
+  gridDepWait();  // Q, K, V and the output buffer belong to the kernels before this one
   const uint32_t tmemBase = *tmemSlot;
   const uint32_t tmemS = tmemBase, tmemO = tmemBase + AT_SK;  // O buffer b at tmemO + 64 b
 
@@ -907,14 +909,11 @@ cudaError_t launchAttentionTc(
     if(units <= 0) return cudaSuccess;
     dim3 pgrid(units < p->numSMs ? units : p->numSMs);
     if(relBias) {
-      if(p->dt == DT_F16) attentionPipeKernel<__half, true><<<pgrid, AP_THREADS, p->smemBytesPipe, st>>>(p->tmQKV, a);
-      else attentionPipeKernel<__nv_bfloat16, true><<<pgrid, AP_THREADS, p->smemBytesPipe, st>>>(p->tmQKV, a);
+      if(p->dt == DT_F16) return launchDependent(attentionPipeKernel<__half, true>, pgrid, dim3(AP_THREADS), p->smemBytesPipe, st, p->tmQKV, a);
+      return launchDependent(attentionPipeKernel<__nv_bfloat16, true>, pgrid, dim3(AP_THREADS), p->smemBytesPipe, st, p->tmQKV, a);
     }
-    else {
-      if(p->dt == DT_F16) attentionPipeKernel<__half, false><<<pgrid, AP_THREADS, p->smemBytesPipe, st>>>(p->tmQKV, a);
-      else attentionPipeKernel<__nv_bfloat16, false><<<pgrid, AP_THREADS, p->smemBytesPipe, st>>>(p->tmQKV, a);
-    }
-    return cudaGetLastError();
+    if(p->dt == DT_F16) return launchDependent(attentionPipeKernel<__half, false>, pgrid, dim3(AP_THREADS), p->smemBytesPipe, st, p->tmQKV, a);
+    return launchDependent(attentionPipeKernel<__nv_bfloat16, false>, pgrid, dim3(AP_THREADS), p->smemBytesPipe, st, p->tmQKV, a);
   }
   dim3 grid(g.n * heads);
   if(relBias) {
