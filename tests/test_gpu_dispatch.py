@@ -85,3 +85,15 @@ def test_gpool_widths(reg, gp, n, edge, oracle):
     ref = oracle.eval_layer(blob, x, mask, C)
     out = capi.eval_layer(blob, x, mask, C, precision=capi.PRECISION_FP16)
     assert np.all(np.abs(out - ref) <= 0.03 * np.maximum(np.maximum(np.abs(out), np.abs(ref)), 3.0))
+
+
+def test_noalloc_convolution_after_another_geometry(oracle):
+    """kb_conv_noalloc keeps one buffer for all geometries: a call's padding rows may hold an earlier call's board points, in
+    widths that the engine's staged fp32 kernel would take."""
+    pytest.importorskip("torch")
+    from tests.test_zz_no_alloc import _run_pair
+    import torch
+    g = mf._Gen(77)
+    rng = np.random.default_rng(3)
+    for n, ylen, xlen in [(3, 19, 19), (2, 7, 30), (4, 9, 9), (1, 19, 19)]:
+        _run_pair(torch, g.conv(3, 64, 32), rng.standard_normal((n, ylen, xlen, 64)).astype(np.float32), oracle)
