@@ -5,7 +5,7 @@
 // takes as long as ONE tile, i.e. 108 MMAs in a row (3x3 192->192), a weight stream of 663 KB into one SM, an epilogue of
 // six 32-channel units and the start-up of a kernel.  Everything here shortens that chain:
 //
-// * narrow tiles: the same MMAs per tile, but about 50 cycles each (M=128, N=16 to 64, issue included) instead of 96, a half
+// * narrow tiles: the same MMAs per tile, but about 50 cycles each (M=128, N=32, issued by this loop in isolation) instead of 96, a half
 //   to a twelfth of the weights per SM, and an epilogue of one or two 8-channel pieces per warp.  The order of the additions
 //   inside an accumulator does not depend on N, so a position's results stay the same bit for bit in every batch size;
 // * all weights of a tile in shared memory where they fit, behind one barrier, else a ring whose slots hold three taps: a
@@ -14,8 +14,10 @@
 //   (programmatic dependent launch); what is left after it is the activations, the MMAs and the epilogue;
 // * the epilogue goes straight from registers to global memory.
 //
-// Where the time of a 3x3 192->192 launch of one position goes (6.0 us from exit to exit; 15 us before): 0.85 us until the
-// wait for the previous launch returns, 0.75 us until the first activations arrive, 2.9 us of MMAs, 0.7 us epilogue, 0.3 us exit.
+// A 3x3 192->192 launch of one position takes 6.5 us (15 us per layer in the wide-tile chain).  Where it goes was measured with
+// the issuing loop still inside one thread and an epilogue of half as many warps (7.1 us from exit to exit): 0.85 us until
+// the wait for the previous launch returns, 0.75 us until the first activations arrive, 3.8 us of MMAs (108 in a row at 69
+// cycles, issue-bound), 0.9 us epilogue, 0.4 us exit.
 //
 // Each CTA computes one tile and leaves.  Every wait is bounded; see kb_conv_tc.cu.
 #include "kb_conv_dev.cuh"
