@@ -447,7 +447,6 @@ __global__ void __launch_bounds__(AP_THREADS, 1) attentionPipeKernel(const __gri
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  gridDepLaunch();
   AT_TRACE(0);
   if(tid == 0) {
     for(int i = 0; i < AP_NUM_BARS; i++) mbarInit(smemU32(&bars[i]), (i == AP_SM_DONE || (i >= AP_O_FREE && i < AP_P_FREE)) ? 8 : 1);
@@ -466,6 +465,7 @@ __global__ void __launch_bounds__(AP_THREADS, 1) attentionPipeKernel(const __gri
   tcFenceBefore();
   __syncthreads();
   tcFenceAfter();
+  gridDepLaunch();
   gridDepWait();  // Q, K, V and the output buffer belong to the kernels before this one
   const uint32_t tmemBase = *tmemSlot;
   const uint32_t tmemS = tmemBase, tmemO = tmemBase + AT_SK;  // O buffer b at tmemO + 64 b

@@ -106,7 +106,6 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
   const int cpp = a.NP / 64;   // K chunks of GEMM2 per part
   const int UP = a.NP / 32;    // 32-channel units per part
 
-  gridDepLaunch();
   if(threadIdx.x == 0) {
     mbarInit(smemU32(a1Full), 1); mbarInit(smemU32(a1Empty), 1);
     for(int s = 0; s < a.numB1; s++) { mbarInit(smemU32(&b1Full[s]), 1); mbarInit(smemU32(&b1Empty[s]), 1); }
@@ -125,6 +124,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
   tcFenceBefore();
   __syncthreads();
   tcFenceAfter();
+  gridDepLaunch();
   const uint32_t tmemBase = *tmemSlot;
   const uint32_t d1Col = 0u, d2Col = (uint32_t)a.NP;
   const bool bad = *abortFlag != 0;

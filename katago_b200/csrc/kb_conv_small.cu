@@ -84,7 +84,6 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
   const int totalB = a.kChunks * groupsPerChunk;
   const bool residentB = a.numB >= totalB;  // all weights of the tile fit: one barrier for all of them
 
-  gridDepLaunch();
   if(warp == 0 && electOne()) {
     for(int s = 0; s < a.numA; s++) { mbarInit(smemU32(&fullA[s]), 1); mbarInit(smemU32(&emptyA[s]), 1); }
     for(int s = 0; s < a.numB; s++) { mbarInit(smemU32(&fullB[s]), 1); mbarInit(smemU32(&emptyB[s]), 1); }
@@ -115,6 +114,7 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
   tcFenceBefore();
   __syncthreads();
   tcFenceAfter();
+  gridDepLaunch();  // only now that this CTA holds its tensor memory (see gridDepLaunch)
   const uint32_t tmemBase = *tmemSlot;
 
   if(warp == 0) {

@@ -477,7 +477,6 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
   tm.rowBase = (int)rank * TC_BM;
   const int numTiles = tm.numTiles;
 
-  gridDepLaunch();
   if(threadIdx.x == 0) {
     TLT(0);
 #ifdef KB_TC_TRACE
@@ -511,6 +510,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
   __syncthreads();
   if(PAIR) clusterSync();  // the other CTA's barriers are initialised before anything here signals them
   tcFenceAfter();
+  gridDepLaunch();
   const uint32_t tmemBase = *tmemSlot;
 
   // The feeding and the issuing warp of a CTA pair run their loops with all lanes and elect a thread for each batch of
@@ -897,7 +897,6 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
   struct { int trace, tlSlot; } a = {0, c.tlSlot};  // what the timeline macros look at
 #endif
 
-  gridDepLaunch();
   // every layer's arguments into shared memory (the roles read them in their inner loops)
   for(int i = threadIdx.x; i < c.numLayers * (int)(sizeof(ConvTcArgs) / 4); i += blockDim.x)
     reinterpret_cast<uint32_t*>(sArgs)[i] = reinterpret_cast<const uint32_t*>(&layers[i / (int)(sizeof(ConvTcArgs) / 4)].a)[i % (int)(sizeof(ConvTcArgs) / 4)];
@@ -919,6 +918,7 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
   tcFenceBefore();
   __syncthreads();
   tcFenceAfter();
+  gridDepLaunch();
   const uint32_t tmemBase = *tmemSlot;
 
   // The list of this CTA's tiles: for L in layers, t = first(L), first(L) + grid, ... with first(L) chosen so that the

@@ -85,6 +85,12 @@ __device__ __forceinline__ void mbarWaitWarp(uint32_t bar, uint32_t parity, vola
 // Programmatic dependent launch: a kernel launched with the programmatic-stream-serialization attribute may start
 // while the kernel before it in the stream still runs; it must not touch memory that kernel produces (or still
 // reads) before gridDepWait() returns.  gridDepLaunch() lets the next such kernel begin its own preamble.
+//
+// A kernel that allocates tensor memory calls gridDepLaunch() only after the block barrier behind its allocation.  An
+// allocation blocks without a limit, and two kernels fit one SM where registers and shared memory allow it: 96 registers x
+// 320 threads of a convTcKernel with the direct epilogue and 56 x 576 of convSmallKernel are 62 976 of 65 536.  If the later
+// of the two could start before the earlier one's CTA holds its columns, it could take the ones that are left (a 192-wide
+// tile's accumulators are all 512), and then wait for a kernel that waits for it.
 __device__ __forceinline__ void gridDepWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void gridDepLaunch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -1,0 +1,48 @@
+"""Rules of the kernels' sources that a run on a GPU cannot show to be broken (a race that is rarely lost), checked on the text."""
+import os
+import re
+
+import pytest
+
+_CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "katago_b200", "csrc")
+
+
+def _kernels():
+    """(name, parameter list, body) of every __global__ function."""
+    found = []
+    for f in sorted(os.listdir(_CSRC)):
+        if not f.endswith((".cu", ".cuh")):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(_CSRC, f)).read())
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(", text):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"(": 1, ")": -1}.get(text[i], 0)
+                i += 1
+            params = text[m.end():i - 1]
+            start = text.index("{", i)
+            depth, j = 1, start + 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[j], 0)
+                j += 1
+            found.append((m.group(1), params, text[start:j]))
+    return found
+
+
+KERNELS = _kernels()
+
+
+def test_the_sources_are_read():
+    names = [k[0] for k in KERNELS]
+    assert len(names) >= 30 and {"convTcKernel", "convSmallKernel", "convChainKernel", "gpoolMidKernel"} <= set(names)
+
+
+@pytest.mark.parametrize("name", [n for n, _, b in KERNELS if "tmemAlloc" in b and "gridDepLaunch" in b])
+def test_dependents_start_after_the_tensor_memory_is_allocated(name):
+    """A tcgen05 allocation blocks without a limit; a dependent kernel that got onto the SM first could hold the columns it
+    waits for while itself waiting for this kernel."""
+    body = next(b for n, _, b in KERNELS if n == name)
+    last_alloc = max(m.start() for m in re.finditer(r"tmemAlloc(?:Pair)?\(", body))
+    launch = [m.start() for m in re.finditer(r"gridDepLaunch\(\)", body)]
+    assert len(launch) == 1
+    assert "__syncthreads();" in body[last_alloc:launch[0]]
