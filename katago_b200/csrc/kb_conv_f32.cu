@@ -36,7 +36,7 @@ __device__ __forceinline__ void cpAsync16(float* dst, const float* src, bool val
 
 template <int TAPS, int NR>
 __global__ void __launch_bounds__(CF_THREADS) convF32Kernel(
-  const float* __restrict__ in, int inStride, int inC, const float* __restrict__ w, int outC, int halo, Geom g, Epilogue ep) {
+  const float* in, int inStride, int inC, const float* __restrict__ w, int outC, int halo, Geom g, Epilogue ep) {
   extern __shared__ float4 smem4[];
   float* sm = reinterpret_cast<float*>(smem4);
   constexpr int BM = cfRows(NR);

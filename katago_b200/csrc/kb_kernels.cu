@@ -238,8 +238,8 @@ constexpr int MM_ROWS = 4;
 constexpr int MM_KSPLIT = 4;  // the input channels are split over threadIdx.y so that each thread's dependent chain is short
 
 __global__ void matMulSmallKernel(
-  const float* __restrict__ in, int inC, const float* __restrict__ w, int outC, const float* __restrict__ bias, int act,
-  float* __restrict__ out, int rows, int accumulate) {
+  const float* in, int inC, const float* __restrict__ w, int outC, const float* __restrict__ bias, int act, float* out, int rows,
+  int accumulate) {
   extern __shared__ float sIn[];  // [MM_ROWS][inC], then partial sums [MM_KSPLIT][MM_ROWS][blockDim.x]
   float* sPart = sIn + MM_ROWS * inC;
   const int r0 = blockIdx.x * MM_ROWS;
@@ -303,8 +303,7 @@ constexpr int GP_GROUPS = 32;
 
 template <typename T>
 __global__ void __launch_bounds__(32 * GP_GROUPS) gpoolKernel(
-  const T* __restrict__ in, int inStride, int c0, int C, const float* __restrict__ mask, const float* __restrict__ maskSum,
-  float* __restrict__ out, int valueHead, Geom g) {
+  const T* in, int inStride, int c0, int C, const float* mask, const float* maskSum, float* out, int valueHead, Geom g) {
   const int n = blockIdx.x;
   const int c = blockIdx.y * 32 + threadIdx.x;
   float s = 0.0f, mx = -1.0f;
@@ -544,9 +543,9 @@ constexpr int GPM_THREADS = 512;
 // Cg / 8, the 16-byte pieces of a gpool row, is a power of two up to 32; cPer is a multiple of 8.
 template <typename T>
 __global__ void __launch_bounds__(GPM_THREADS) gpoolMidKernel(
-  const T* __restrict__ gIn, int gStride, int Cg, const T* __restrict__ rIn, int rStride, int cPer, const float* __restrict__ wT,
-  const float* __restrict__ scale, const float* __restrict__ bias, int act, const float* __restrict__ mask,
-  const float* __restrict__ maskSum, T* __restrict__ out, int outStride, Geom g) {
+  const T* gIn, int gStride, int Cg, const T* rIn, int rStride, int cPer, const float* __restrict__ wT,
+  const float* __restrict__ scale, const float* __restrict__ bias, int act, const float* mask, const float* maskSum, T* out,
+  int outStride, Geom g) {
   extern __shared__ float sm[];  // [2][warps][Cg] partial sums / maxima, then pooled [3*Cg], then board bias [cPer]
   constexpr int WARPS = GPM_THREADS / 32;
   const int n = blockIdx.x, c0 = blockIdx.y * cPer;

@@ -110,7 +110,9 @@ cudaError_t launchConvF32(
   cudaStream_t st, const void* in, int inStride, int inC, const void* w, int outC, int kY, Geom g, const Epilogue& ep);
 
 // Launches a kernel that may become resident while the kernel before it in the stream still runs (programmatic dependent
-// launch).  It has to call gridDepWait() before it touches anything that other kernels of the stream read or write.
+// launch).  It has to call gridDepWait() before it touches anything that other kernels of the stream read or write, and may
+// declare const __restrict__ only what none of them writes (weights): the qualifier promises data that does not change while
+// the kernel runs, and a kernel that is resident early runs while its inputs are written.
 inline bool dependentLaunches() {
   static const bool on = getenv("KB_NO_PDL") == nullptr;
   return on;

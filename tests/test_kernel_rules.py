@@ -46,3 +46,11 @@ def test_dependents_start_after_the_tensor_memory_is_allocated(name):
     launch = [m.start() for m in re.finditer(r"gridDepLaunch\(\)", body)]
     assert len(launch) == 1
     assert "__syncthreads();" in body[last_alloc:launch[0]]
+
+
+@pytest.mark.parametrize("name", [n for n, _, b in KERNELS if "gridDepWait" in b])
+def test_early_kernels_promise_constant_data_for_weights_only(name):
+    """const __restrict__ allows loads that are not coherent with, or not ordered after, what the kernel before still writes."""
+    params = next(p for n, p, _ in KERNELS if n == name)
+    constant = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", params))
+    assert constant <= {"w", "wT", "scale", "bias", "layers"}
