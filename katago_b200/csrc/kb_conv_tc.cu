@@ -448,8 +448,8 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
   uint8_t* smemB = smemA + (size_t)a.numA * a.aSlotBytes;
   uint8_t* smemR = smemB + (size_t)a.numB * a.bSlotBytes;  // epilogue staging (TMA epilogue only)
   float* sScale = reinterpret_cast<float*>(smemR + (TMA_EPI ? (size_t)TC_EPI_WARPS * a.epiWarpBytes : 0));
-  float* sBias = sScale + 512;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sBias + 512);
+  float* sBias = sScale + CONV_TC_MAX_ACT;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sBias + CONV_TC_MAX_ACT);
   // barrier layout: fullA[numA] emptyA[numA] fullB[numB] emptyB[numB] accFull[2] accEmpty[2]
   uint64_t* fullA = bars;
   uint64_t* emptyA = fullA + a.numA;
@@ -1345,7 +1345,7 @@ static bool encodeWeights3d(CUtensorMap* tm, int dt, const void* base, int inC, 
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr int TC_FIXED_SMEM = 2 * 512 * 4 + 96 * 8 + 64 + 1024;  // norm parameters, barriers, TMEM slot, alignment slack
+constexpr int TC_FIXED_SMEM = 2 * CONV_TC_MAX_ACT * 4 + 96 * 8 + 64 + 1024;  // norm parameters, barriers, TMEM slot, alignment slack
 
 // Splits the shared memory between the weight ring and (optionally) the epilogue staging blocks.
 static bool sizeRings(ConvTcPlan* p, int epiBytes) {
@@ -1529,7 +1529,7 @@ int convTcGridSize(const ConvTcPlan* p, const Geom& g) {
 cudaError_t launchConvTc(cudaStream_t st, const ConvTcPlan* p, Geom g, const Epilogue& ep, int* statusWord, const ConvTcDeps* deps) {
   // vector accesses in the epilogue need 16-byte aligned rows and 16-channel aligned ranges
   if(ep.outRaw && ((ep.rawStride % 8) || (ep.rawC0 % 16) || (ep.rawC1 % 16))) return cudaErrorInvalidValue;
-  if(ep.outAct && ((ep.actStride % 8) || (ep.actC0 % 16) || (ep.actC1 % 16) || ((ep.actC1 - ep.actC0) > 512 && ep.act != KB_ACT_SWIGLU_PAIRS))) return cudaErrorInvalidValue;
+  if(ep.outAct && ((ep.actStride % 8) || (ep.actC0 % 16) || (ep.actC1 % 16) || ((ep.actC1 - ep.actC0) > CONV_TC_MAX_ACT && ep.act != KB_ACT_SWIGLU_PAIRS))) return cudaErrorInvalidValue;
   if(ep.residual && (ep.resStride % 8)) return cudaErrorInvalidValue;
   if(!(deps && (deps->done || deps->wait))) {
     if(const int bn = smallWidth(p, g)) return launchConvSmall(st, p->smallShape, bn, p->numSMs, g, ep, statusWord);

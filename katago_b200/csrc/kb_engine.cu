@@ -178,14 +178,16 @@ void* Engine::uploadConvWeights(const std::vector<const ConvW*>& parts, int inCd
   return uploadShared(bytes.data(), bytes.size());
 }
 
-Engine::ConvDev Engine::makeConv(const std::vector<const ConvW*>& parts, const void* in, int inStride, int inCdev) {
+// actC: channels of the activated output (0: none).  A convolution whose norm parameters do not fit the tensor-core kernel
+// runs on the CUDA cores.
+Engine::ConvDev Engine::makeConv(const std::vector<const ConvW*>& parts, const void* in, int inStride, int inCdev, int actC) {
   ConvDev c;
   c.kY = parts[0]->kY; c.kX = parts[0]->kX; c.inC = inCdev; c.inCReal = parts[0]->inC;
   c.outC = 0;
   bool aligned = true;
   for(const ConvW* p : parts) { c.outC += p->outC; if(p->outC % 16) aligned = false; }
   c.in = in; c.inStride = inStride;
-  c.tc = !forceSimt_ && aligned && convTcEligible(dt_, inCdev, c.outC, c.kY, c.kX) && (inStride % 8) == 0;
+  c.tc = !forceSimt_ && aligned && actC <= CONV_TC_MAX_ACT && convTcEligible(dt_, inCdev, c.outC, c.kY, c.kX) && (inStride % 8) == 0;
   c.w = uploadConvWeights(parts, inCdev, c.tc);
   if(c.tc) {
     c.plan = convTcCreate(dt_, in, inStride, inCdev, c.w, c.outC, c.kY, c.kX, X_, Y_, rowsPadMax_);
@@ -429,6 +431,7 @@ void Engine::emitStack(const std::vector<BlockW>& blocks, int C, void* raw, void
 void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* next, int depth) {
   const size_t es = dtypeSize(dt_);
   const std::string d = "_d" + std::to_string(depth);
+  const int nextC = next ? C : 0;  // activated channels of the convolution that ends the block
   auto finishEp = [&](Epilogue& ep) {
     // residual add into the stream + (optionally) the next block's norm/activation
     ep.residual = raw; ep.resStride = C;
@@ -443,12 +446,12 @@ void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* 
   if(b.kind == BLOCK_ORDINARY) {
     const int mid = b.conv1.outC;
     void* tmp = scratch("tmp" + d + "_c" + std::to_string(mid), (size_t)rowsPadMax_ * mid * es);
-    ConvDev c1 = makeConv({&b.conv1}, act, C, C);
+    ConvDev c1 = makeConv({&b.conv1}, act, C, C, mid);
     BNDev mb = makeBN({&b.midBN});
     Epilogue e1;
     e1.outAct = tmp; e1.actStride = mid; e1.actC0 = 0; e1.actC1 = mid; e1.scale = mb.scale; e1.bias = mb.bias; e1.act = mb.act;
     addConvOp(c1, e1, "");
-    ConvDev c2 = makeConv({&b.conv2}, tmp, mid, mid);
+    ConvDev c2 = makeConv({&b.conv2}, tmp, mid, mid, nextC);
     Epilogue e2;
     finishEp(e2);
     addConvOp(c2, e2, "+res");
@@ -463,7 +466,7 @@ void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* 
     BNDev gb = makeBN({&b.gpoolBN});
     if(b.conv1.kY == b.gpoolConv.kY && b.conv1.kX == b.gpoolConv.kX) {
       // regular and gpool convolutions read the same tensor: one launch, outputs split by channel range
-      ConvDev c1 = makeConv({&b.conv1, &b.gpoolConv}, act, C, C);
+      ConvDev c1 = makeConv({&b.conv1, &b.gpoolConv}, act, C, C, gp);
       Epilogue e1;
       e1.outRaw = R; e1.rawStride = reg; e1.rawC0 = 0; e1.rawC1 = reg;
       e1.outAct = G; e1.actStride = gp; e1.actC0 = reg; e1.actC1 = reg + gp; e1.scale = gb.scale; e1.bias = gb.bias; e1.act = gb.act;
@@ -474,7 +477,7 @@ void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* 
       Epilogue er;
       er.outRaw = R; er.rawStride = reg; er.rawC0 = 0; er.rawC1 = reg;
       addConvOp(cr, er, "reg");
-      ConvDev cg = makeConv({&b.gpoolConv}, act, C, C);
+      ConvDev cg = makeConv({&b.gpoolConv}, act, C, C, gp);
       Epilogue eg;
       eg.outAct = G; eg.actStride = gp; eg.actC0 = 0; eg.actC1 = gp; eg.scale = gb.scale; eg.bias = gb.bias; eg.act = gb.act;
       addConvOp(cg, eg, "gpool");
@@ -503,7 +506,7 @@ void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* 
         return launchBiasBnAct(st, dt, R, reg, gbias, mb.scale, mb.bias, mb.act, mask, Ract, reg, reg, g);
       });
     }
-    ConvDev c2 = makeConv({&b.conv2}, Ract, reg, reg);
+    ConvDev c2 = makeConv({&b.conv2}, Ract, reg, reg, nextC);
     Epilogue e2;
     finishEp(e2);
     addConvOp(c2, e2, "+res");
@@ -513,17 +516,17 @@ void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* 
     const std::string d1 = "_d" + std::to_string(depth + 1);
     void* midRaw = scratch("nRaw" + d1 + "_c" + std::to_string(mid), (size_t)rowsPadMax_ * mid * es);
     void* midAct = scratch("nAct" + d1 + "_c" + std::to_string(mid), (size_t)rowsPadMax_ * mid * es);
-    ConvDev c1 = makeConv({&b.conv1}, act, C, C);
+    const bool innerConv = isConvBlock(b.inner[0]);
+    ConvDev c1 = makeConv({&b.conv1}, act, C, C, innerConv ? mid : 0);
     Epilogue e1;
     e1.outRaw = midRaw; e1.rawStride = mid; e1.rawC0 = 0; e1.rawC1 = mid;
-    const bool innerConv = isConvBlock(b.inner[0]);
     if(innerConv) {
       BNDev ib = makeBN({&b.inner[0].preBN});
       e1.outAct = midAct; e1.actStride = mid; e1.actC0 = 0; e1.actC1 = mid; e1.scale = ib.scale; e1.bias = ib.bias; e1.act = ib.act;
     }
     addConvOp(c1, e1, "");
     emitStack(b.inner, mid, midRaw, midAct, &b.midBN, depth + 1, innerConv);
-    ConvDev c2 = makeConv({&b.conv2}, midAct, mid, mid);
+    ConvDev c2 = makeConv({&b.conv2}, midAct, mid, mid, nextC);
     Epilogue e2;
     finishEp(e2);
     addConvOp(c2, e2, "+res");
@@ -624,11 +627,12 @@ void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* 
       });
     }
     ConvW outW = matmulsAsConv({&b.out});
-    ConvDev co = makeConv({&outW}, attn, oC, oC);
+    ConvDev co = makeConv({&outW}, attn, oC, oC, nextC);
     Epilogue eo;
     finishEp(eo);
     eo.resMask = 1;
-    produceRowSums(eo, 1, oC, C);
+    if(co.tc) produceRowSums(eo, 1, oC, C);
+    else rowSumsCur_ = -1;
     addConvOp(co, eo, "attn out +res");
   }
   else if(b.kind == BLOCK_FFN) {
@@ -668,11 +672,12 @@ void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* 
       addOp("swiglu", 0.0, 3.0 * S * F * es, [=](cudaStream_t st, const Geom& g) { return launchSwiGLU(st, dt, up, 2 * F, hid, F, F, g); });
     }
     ConvW downW = matmulsAsConv({&b.linear2});
-    ConvDev cd = makeConv({&downW}, hid, F, F);
+    ConvDev cd = makeConv({&downW}, hid, F, F, nextC);
     Epilogue ed;
     finishEp(ed);
     ed.resMask = 1;
-    produceRowSums(ed, 1, F, C);
+    if(cd.tc) produceRowSums(ed, 1, F, C);
+    else rowSumsCur_ = -1;
     addConvOp(cd, ed, "ffn down +res");
   }
   else {
@@ -696,7 +701,7 @@ void Engine::emitHeads(const Model& m, const void* trunkAct) {
   if(m.g1BN.act == m.v1BN.act) {
     // the three 1x1 convolutions that read the trunk run as one GEMM (reference: three cuDNN calls,
     // cudabackend.cpp:2603-2692, 2788-2846)
-    ConvDev hc = makeConv({&m.p1Conv, &m.g1Conv, &m.v1Conv}, trunkAct, C, C);
+    ConvDev hc = makeConv({&m.p1Conv, &m.g1Conv, &m.v1Conv}, trunkAct, C, C, G1 + V1);
     BNDev gv = makeBN({&m.g1BN, &m.v1BN});
     Epilogue e;
     e.outRaw = Praw; e.rawStride = P1; e.rawC0 = 0; e.rawC1 = P1;
@@ -708,12 +713,12 @@ void Engine::emitHeads(const Model& m, const void* trunkAct) {
     Epilogue ep;
     ep.outRaw = Praw; ep.rawStride = P1; ep.rawC0 = 0; ep.rawC1 = P1;
     addConvOp(pc, ep, "head p1");
-    ConvDev gc = makeConv({&m.g1Conv}, trunkAct, C, C);
+    ConvDev gc = makeConv({&m.g1Conv}, trunkAct, C, C, G1);
     BNDev gb = makeBN({&m.g1BN});
     Epilogue eg;
     eg.outAct = GV; eg.actStride = G1 + V1; eg.actC0 = 0; eg.actC1 = G1; eg.scale = gb.scale; eg.bias = gb.bias; eg.act = gb.act;
     addConvOp(gc, eg, "head g1");
-    ConvDev vc = makeConv({&m.v1Conv}, trunkAct, C, C);
+    ConvDev vc = makeConv({&m.v1Conv}, trunkAct, C, C, V1);
     BNDev vb = makeBN({&m.v1BN});
     Epilogue ev;
     ev.outAct = static_cast<uint8_t*>(GV) + (size_t)G1 * es; ev.actStride = G1 + V1; ev.actC0 = 0; ev.actC1 = V1;
@@ -921,7 +926,7 @@ Engine::Engine(const Model& m, int device, int maxBatch, int X, int Y, int preci
   }
   // initial convolution + global bias, producing the stream and the first block's activated input
   {
-    ConvDev c0 = makeConv({&m.initialConv}, inputBuf_, inCdev_, inCdev_);
+    ConvDev c0 = makeConv({&m.initialConv}, inputBuf_, inCdev_, inCdev_, isConvBlock(m.blocks[0]) ? m.trunkC : 0);
     Epilogue e;
     e.biasNC = gbias;
     e.outRaw = trunkRaw; e.rawStride = m.trunkC; e.rawC0 = 0; e.rawC1 = m.trunkC;

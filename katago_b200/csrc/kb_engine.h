@@ -136,7 +136,7 @@ class Engine {
   float* uploadF32(const std::vector<float>& v);
   float* uploadF32Transposed(const std::vector<float>& w, int inC, int outC);
   void* uploadConvWeights(const std::vector<const ConvW*>& parts, int inCdev, bool tcLayout);
-  ConvDev makeConv(const std::vector<const ConvW*>& parts, const void* in, int inStride, int inCdev);
+  ConvDev makeConv(const std::vector<const ConvW*>& parts, const void* in, int inStride, int inCdev, int actC = 0);
   BNDev makeBN(const std::vector<const BNW*>& parts);
   int classId(const std::string& name);
   void addConvOp(const ConvDev& c, Epilogue ep, const std::string& tag);

@@ -195,6 +195,8 @@ cudaError_t launchMaskToPadded(cudaStream_t st, const float* src, float* mask, f
 // --- Tensor-core convolution (fp16 / bf16, sm_100a tcgen05) ------------------------------------------
 
 struct ConvTcPlan;  // opaque: tensor maps + tile configuration for one convolution
+// Norm parameters (channels of the activated output) a convolution keeps in shared memory.
+constexpr int CONV_TC_MAX_ACT = 512;
 // True if the tensor-core kernel can run this convolution shape.
 bool convTcEligible(int dt, int inC, int outC, int kY, int kX);
 // True if a 1x1 convolution inC -> outC takes the staged epilogue that supports sumsqOut / rowSumsq.

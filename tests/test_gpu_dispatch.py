@@ -27,6 +27,31 @@ def test_input_widths_between_chunks(prec, tol, trunk, mid, oracle):
     assert np.all(np.abs(out - ref) <= tol * np.maximum(np.maximum(np.abs(out), np.abs(ref)), 3.0))
 
 
+@pytest.mark.parametrize("trunk,mid", [(96, 528), (72, 640), (528, 96), (64, 576)])
+def test_more_activated_channels_than_the_tensor_core_kernel_holds(trunk, mid, oracle):
+    """The norm parameters of more than 512 channels do not fit that kernel: such a layer runs on the CUDA cores, at any input
+    width.  Tolerance as above; once as a block and once in a net, whose first convolution and block ends are as wide."""
+    g = mf._Gen(450 + trunk + mid)
+    rng = np.random.default_rng(trunk + mid)
+    mask = np.ones((2, 9, 9), np.float32)
+    mask[1, 7:] = 0
+    layer = mf._gen_ordinary(g, trunk, mid, mf.ACT_MISH)
+    x = rng.standard_normal((2, 9, 9, trunk)).astype(np.float32) * mask[..., None]
+    blob = mf.layer_blob(layer)
+    ref = oracle.eval_layer(blob, x, mask, trunk)
+    out = capi.eval_layer(blob, x, mask, trunk, precision=capi.PRECISION_FP16)
+    assert np.all(np.abs(out - ref) <= 0.03 * np.maximum(np.maximum(np.abs(out), np.abs(ref)), 3.0))
+    blob = mf.to_blob(mf.make_convnet("wide", 451, 15, trunk, ["plain", "plain"], (32, 32, 32, 64), mf.ACT_MISH, mid_c=mid, regular_c=64, gpool_c=32))
+    sp, gl = mf.random_positions(2, seed=9, nn_len=9)
+    ref = oracle.OracleModel(blob, 9, 9).forward(sp, gl)
+    h = capi.Handle(capi.Model(blob), 2, nn_x=9, nn_y=9, precision=capi.PRECISION_FP16)
+    for _ in range(2):  # the eager run and the graph
+        out = h.forward(sp, gl)
+        for k in ref:
+            assert np.all(np.abs(out[k] - ref[k]) <= 0.03 * np.maximum(np.maximum(np.abs(out[k]), np.abs(ref[k])), 3.0)), k
+    h.close()
+
+
 @pytest.mark.parametrize("factory,prec,full,edge", [
     (lambda: mf.make_b18c384nbt(num_blocks=3), capi.PRECISION_FP16, 128, 19),
     (lambda: mf.make_b18c384nbt(num_blocks=3), capi.PRECISION_BF16, 128, 9),
