@@ -8,7 +8,26 @@
 #include "kb_tc_ptx.cuh"
 #include "../../include/kb_modelblob.h"
 
+#include <algorithm>
+#include <mutex>
+#include <utility>
+#include <vector>
+
 namespace kb {
+
+cudaError_t allowSharedMemory(const void* fn, int bytes) {
+  static std::mutex mu;
+  static std::vector<std::pair<const void*, int>> done;  // (kernel, device)
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if(e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  const std::pair<const void*, int> key(fn, dev);
+  if(std::find(done.begin(), done.end(), key) != done.end()) return cudaSuccess;
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if(e == cudaSuccess) done.push_back(key);
+  return e;
+}
 
 // ---------------------------------------------------------------------------------------------
 // dtype helpers
@@ -751,6 +770,7 @@ cudaError_t launchHeadFinal(
 // and the matrices are brought into L1 before the wait for the kernel before this one.
 
 constexpr int HT_THREADS = 512;
+constexpr int HT_MAX_SMEM = 200 * 1024;
 constexpr int HT_PARTS = 4;  // threads per channel that add up the partial sums
 
 // mean, size-scaled mean and third statistic (maximum, or the value head's second size-scaled mean) of C channels of in
@@ -926,10 +946,10 @@ bool headsTailEligible(int dt, const HeadsTailArgs& a) {
 cudaError_t launchHeadsTail(cudaStream_t st, int dt, const HeadsTailArgs& a, Geom g) {
   if(!headsTailEligible(dt, a)) return cudaErrorInvalidValue;
   const size_t smem = headsTailSmem(a);
-  if(smem > 200 * 1024) return cudaErrorInvalidValue;
+  if(smem > HT_MAX_SMEM) return cudaErrorInvalidValue;
   void (*fn)(HeadsTailArgs, Geom) = dt == DT_F16 ? headsTailKernel<__half> : headsTailKernel<__nv_bfloat16>;
   if(smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allowSharedMemory((const void*)fn, HT_MAX_SMEM);
     if(e != cudaSuccess) return e;
   }
   return launchDependent(fn, dim3(g.n, 2), dim3(HT_THREADS), smem, st, a, g);

@@ -109,6 +109,11 @@ bool convF32Eligible(const void* in, int inStride, int inC, const void* w, int o
 cudaError_t launchConvF32(
   cudaStream_t st, const void* in, int inStride, int inC, const void* w, int outC, int kY, Geom g, const Epilogue& ep);
 
+// Lets a kernel be launched with up to `bytes` of dynamic shared memory on the current device.  `bytes` is the most the kernel
+// ever asks for, not what one launch needs: the limit belongs to the function, and a launch that needs less, perhaps from
+// another thread, must not lower it between another launch's opt-in and that launch.
+cudaError_t allowSharedMemory(const void* fn, int bytes);
+
 // Launches a kernel that may become resident while the kernel before it in the stream still runs (programmatic dependent
 // launch).  It has to call gridDepWait() before it touches anything that other kernels of the stream read or write, and may
 // declare const __restrict__ only what none of them writes (weights): the qualifier promises data that does not change while

@@ -1,5 +1,7 @@
 """Dispatch rules of the tensor-core convolutions at the sizes where they change: input widths that do not fill the last
 64-channel chunk, and batches on either side of the small-batch kernel's limit."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -110,6 +112,35 @@ def test_gpool_widths(reg, gp, n, edge, oracle):
     ref = oracle.eval_layer(blob, x, mask, C)
     out = capi.eval_layer(blob, x, mask, C, precision=capi.PRECISION_FP16)
     assert np.all(np.abs(out - ref) <= 0.03 * np.maximum(np.maximum(np.abs(out), np.abs(ref)), 3.0))
+
+
+def test_head_kernels_of_different_sizes_from_two_threads(monkeypatch):
+    """The fused heads need more shared memory than a kernel has by default for wide heads, and how much depends on the net: two
+    nets that are run from two threads must not take the larger limit away from each other."""
+    monkeypatch.setenv("KB_NO_GRAPH", "1")  # read when a handle is created: every pass launches its kernels anew
+    sp, gl = mf.random_positions(1, seed=12, nn_len=5)
+    handles, refs, errors = [], [], []
+    for seed, g1 in ((900, 408), (901, 448)):
+        tree = mf.make_convnet("heads", seed, 15, 64, ["plain"], (512, g1, 64, 64), mf.ACT_RELU, regular_c=32, gpool_c=32)
+        handles.append(capi.Handle(capi.Model(mf.to_blob(tree)), 1, nn_x=5, nn_y=5, precision=capi.PRECISION_FP16))
+        refs.append(handles[-1].forward(sp, gl))
+
+    def work(h, ref):
+        try:
+            for _ in range(3000):
+                out = h.forward(sp, gl)
+                assert all(np.array_equal(out[k], ref[k]) for k in ref)
+        except Exception as e:  # handed to the test's own thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in zip(handles, refs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for h in handles:
+        h.close()
 
 
 def test_noalloc_convolution_after_another_geometry(oracle):
