@@ -15,6 +15,12 @@
 
 namespace kb {
 
+int smCount() {
+  int dev = 0, sms = 148;
+  if(cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 cudaError_t allowSharedMemory(const void* fn, int bytes) {
   static std::mutex mu;
   static std::vector<std::pair<const void*, int>> done;  // (kernel, device)
@@ -557,19 +563,82 @@ __device__ __forceinline__ void blockMatVecT(const float* in, int K, const float
   }
 }
 
-constexpr int GPM_THREADS = 512;
+constexpr int BP_THREADS = 512;  // of a block that pools a board
+constexpr int BP_PARTS = 4;      // threads per channel that add up the partial sums
 
-// Cg / 8, the 16-byte pieces of a gpool row, is a power of two up to 32; cPer is a multiple of 8.
-template <typename T>
+// mean, size-scaled mean and third statistic (maximum, or the value head's second size-scaled mean) of C channels of in
+// ([rowsPad][stride], activated and masked) into pooled [3*C]; part [2][BP_THREADS / (C/8)][C]
+template <typename T, bool VALUE>
+__device__ __forceinline__ void boardPool(
+  const T* in, int stride, int C, const float* mask, float boardSum, float* part, float* pooled, size_t board, const Geom& g) {
+  const int vecs = C / 8, groups = BP_THREADS / vecs;
+  const int cv = (int)threadIdx.x % vecs, rg = (int)threadIdx.x / vecs;
+  if(rg < groups) {
+    float s[8], mx[8];
+#pragma unroll
+    for(int j = 0; j < 8; j++) { s[j] = 0.0f; mx[j] = -1.0f; }
+    // padding rows hold zeros and count as points off the board
+#pragma unroll 5
+    for(int r = rg; r < g.PB; r += groups) {
+      const uint4 v4 = *reinterpret_cast<const uint4*>(in + (board + r) * stride + cv * 8);
+      const T* ve = reinterpret_cast<const T*>(&v4);
+      const float mOff = VALUE ? 0.0f : mask[board + r] - 1.0f;
+#pragma unroll
+      for(int j = 0; j < 8; j++) {
+        const float v = toF<T>(ve[j]);
+        s[j] += v;
+        if(!VALUE) mx[j] = fmaxf(mx[j], v + mOff);
+      }
+    }
+#pragma unroll
+    for(int j = 0; j < 8; j++) {
+      part[rg * C + cv * 8 + j] = s[j];
+      if(!VALUE) part[(groups + rg) * C + cv * 8 + j] = mx[j];
+    }
+  }
+  __syncthreads();
+  // BP_PARTS neighbouring lanes share a channel
+  for(int i = threadIdx.x; i < (C * BP_PARTS + 31) / 32 * 32; i += BP_THREADS) {
+    const int c = min(i / BP_PARTS, C - 1), q = i % BP_PARTS;
+    float ss = 0.0f, mm = -1.0f;
+    for(int k = q; k < groups; k += BP_PARTS) {
+      ss += part[k * C + c];
+      if(!VALUE) mm = fmaxf(mm, part[(groups + k) * C + c]);
+    }
+#pragma unroll
+    for(int o = 1; o < BP_PARTS; o <<= 1) {
+      ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+    }
+    if(q == 0 && i < C * BP_PARTS) {
+      const float sq = sqrtf(boardSum);
+      const float mean = ss / boardSum;
+      pooled[c] = mean;
+      pooled[C + c] = mean * (sq - 14.0f) * 0.1f;
+      pooled[2 * C + c] = VALUE ? mean * ((sq - 14.0f) * (sq - 14.0f) * 0.01f - 0.1f) : mm;
+    }
+  }
+  __syncthreads();
+}
+
+constexpr int GPM_THREADS = BP_THREADS;
+constexpr int GPM_MAX_SMEM = 100 * 1024;
+
+// Rows of partial sums in shared memory: one per warp, or one per group of threads that reads the same rows of the board.
+__host__ __device__ constexpr int gpmPartRows(bool shuffle, int Cg) { return shuffle ? GPM_THREADS / 32 : GPM_THREADS / (Cg / 8); }
+
+// SHUFFLE: the lanes of a warp that hold the same channels add up by shuffles, for which Cg / 8, the 16-byte pieces of a gpool
+// row, has to be a power of two up to 32.  Any other multiple of 8 channels goes through shared memory (boardPool).
+template <typename T, bool SHUFFLE>
 __global__ void __launch_bounds__(GPM_THREADS) gpoolMidKernel(
   const T* gIn, int gStride, int Cg, const T* rIn, int rStride, int cPer, const float* __restrict__ wT,
   const float* __restrict__ scale, const float* __restrict__ bias, int act, const float* mask, const float* maskSum, T* out,
   int outStride, Geom g) {
-  extern __shared__ float sm[];  // [2][warps][Cg] partial sums / maxima, then pooled [3*Cg], then board bias [cPer]
+  extern __shared__ float sm[];  // [2][gpmPartRows][Cg] partial sums / maxima, then pooled [3*Cg], then board bias [cPer]
   constexpr int WARPS = GPM_THREADS / 32;
   const int n = blockIdx.x, c0 = blockIdx.y * cPer;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* sPooled = sm + 2 * WARPS * Cg;
+  float* sPooled = sm + 2 * gpmPartRows(SHUFFLE, Cg) * Cg;
   float* sBias = sPooled + 3 * Cg;
   // (no early start for the launch after this one: it would take SMs from boards that have not started; batch 256 1 % slower)
   gridDepWait();
@@ -583,7 +652,7 @@ __global__ void __launch_bounds__(GPM_THREADS) gpoolMidKernel(
     first = *reinterpret_cast<const uint4*>(rIn + (board + row0) * rStride + c0 + cv0 * 8);
     firstMask = mask[board + row0];
   }
-  {
+  if(SHUFFLE) {
     const int vecs = Cg / 8, groups = GPM_THREADS / vecs;
     const int cv = (int)threadIdx.x % vecs, rg = (int)threadIdx.x / vecs;
     float s[8], mx[8];
@@ -613,20 +682,23 @@ __global__ void __launch_bounds__(GPM_THREADS) gpoolMidKernel(
 #pragma unroll
       for(int j = 0; j < 8; j++) { sm[warp * Cg + lane * 8 + j] = s[j]; sm[(WARPS + warp) * Cg + lane * 8 + j] = mx[j]; }
     }
-  }
-  __syncthreads();
-  for(int c = threadIdx.x; c < Cg; c += blockDim.x) {
-    float ss = 0.0f, mm = -1.0f;
+    __syncthreads();
+    for(int c = threadIdx.x; c < Cg; c += blockDim.x) {
+      float ss = 0.0f, mm = -1.0f;
 #pragma unroll
-    for(int k = 0; k < WARPS; k++) { ss += sm[k * Cg + c]; mm = fmaxf(mm, sm[(WARPS + k) * Cg + c]); }
-    const float div = maskSum[n];
-    const float sq = sqrtf(div);
-    const float mean = ss / div;
-    sPooled[c] = mean;
-    sPooled[Cg + c] = mean * (sq - 14.0f) * 0.1f;
-    sPooled[2 * Cg + c] = mm;
+      for(int k = 0; k < WARPS; k++) { ss += sm[k * Cg + c]; mm = fmaxf(mm, sm[(WARPS + k) * Cg + c]); }
+      const float div = maskSum[n];
+      const float sq = sqrtf(div);
+      const float mean = ss / div;
+      sPooled[c] = mean;
+      sPooled[Cg + c] = mean * (sq - 14.0f) * 0.1f;
+      sPooled[2 * Cg + c] = mm;
+    }
+    __syncthreads();
   }
-  __syncthreads();
+  else {
+    boardPool<T, false>(gIn, gStride, Cg, mask, maskSum[n], sm, sPooled, board, g);
+  }
   blockMatVecT(sPooled, 3 * Cg, wT + (size_t)c0 * 3 * Cg, cPer, nullptr, KB_ACT_IDENTITY, sBias);
   __syncthreads();
   // all rows of the board (padding rows included: they are written as zeros)
@@ -666,10 +738,24 @@ __global__ void __launch_bounds__(GPM_THREADS) gpoolMidKernel(
   }
 }
 
+static bool gpmShuffle(int Cg) { const int vecs = Cg / 8; return vecs <= 32 && (vecs & (vecs - 1)) == 0; }
+static size_t gpmSmem(int Cg, int cPer) { return (size_t)(2 * gpmPartRows(gpmShuffle(Cg), Cg) * Cg + 3 * Cg + cPer) * sizeof(float); }
+
 bool gpoolMidEligible(int dt, int Cg, int gStride, int Cr, int rStride, int outStride) {
-  const int vecs = Cg / 8;
   return dt != DT_F32 && (Cg % 8) == 0 && (Cr % 8) == 0 && (gStride % 8) == 0 && (rStride % 8) == 0 && (outStride % 8) == 0 &&
-         vecs >= 1 && vecs <= 32 && (vecs & (vecs - 1)) == 0 && Cr / 8 <= GPM_THREADS;
+         Cg >= 8 && Cg / 8 <= GPM_THREADS && Cr / 8 <= GPM_THREADS && gpmSmem(Cg, Cr) <= GPM_MAX_SMEM;
+}
+
+template <typename T>
+static cudaError_t launchGPoolMidT(
+  cudaStream_t st, bool shuffle, dim3 grid, size_t smem, const void* gIn, int gStride, int Cg, const void* rIn, int rStride, int cPer,
+  const float* w, const float* scale, const float* bias, int act, const float* mask, const float* maskSum, void* out, int outStride, Geom g) {
+  auto fn = shuffle ? gpoolMidKernel<T, true> : gpoolMidKernel<T, false>;
+  if(smem > 48 * 1024) {
+    cudaError_t e = allowSharedMemory((const void*)fn, GPM_MAX_SMEM);
+    if(e != cudaSuccess) return e;
+  }
+  return launchDependent(fn, grid, dim3(GPM_THREADS), smem, st, (const T*)gIn, gStride, Cg, (const T*)rIn, rStride, cPer, w, scale, bias, act, mask, maskSum, (T*)out, outStride, g);
 }
 
 cudaError_t launchGPoolMid(
@@ -677,14 +763,15 @@ cudaError_t launchGPoolMid(
   const float* scale, const float* bias, int act, const float* mask, const float* maskSum, void* out, int outStride, Geom g) {
   if(!gpoolMidEligible(dt, Cg, gStride, Cr, rStride, outStride)) return cudaErrorInvalidValue;
   // channels per CTA: 32 (a row's 64 bytes are then written whole) while two CTAs per SM are not reached, else twice as many and so on
+  const long long full = 2LL * smCount();
   int cPer = Cr % 32 == 0 ? 32 : Cr;
-  while(cPer < Cr && (Cr % (2 * cPer)) == 0 && (long long)g.n * (Cr / cPer) > 296) cPer *= 2;
-  if(cPer < Cr && (long long)g.n * (Cr / cPer) > 296) cPer = Cr;
-  const size_t smem = (size_t)(2 * (GPM_THREADS / 32) * Cg + 3 * Cg + cPer) * sizeof(float);
+  while(cPer < Cr && (Cr % (2 * cPer)) == 0 && (long long)g.n * (Cr / cPer) > full) cPer *= 2;
+  if(cPer < Cr && (long long)g.n * (Cr / cPer) > full) cPer = Cr;
   const dim3 grid(g.n, Cr / cPer);
-  if(dt == DT_F16)
-    return launchDependent(gpoolMidKernel<__half>, grid, dim3(GPM_THREADS), smem, st, (const __half*)gIn, gStride, Cg, (const __half*)rIn, rStride, cPer, w, scale, bias, act, mask, maskSum, (__half*)out, outStride, g);
-  return launchDependent(gpoolMidKernel<__nv_bfloat16>, grid, dim3(GPM_THREADS), smem, st, (const __nv_bfloat16*)gIn, gStride, Cg, (const __nv_bfloat16*)rIn, rStride, cPer, w, scale, bias, act, mask, maskSum, (__nv_bfloat16*)out, outStride, g);
+  const bool shuffle = gpmShuffle(Cg);
+  const size_t smem = gpmSmem(Cg, cPer);
+  if(dt == DT_F16) return launchGPoolMidT<__half>(st, shuffle, grid, smem, gIn, gStride, Cg, rIn, rStride, cPer, w, scale, bias, act, mask, maskSum, out, outStride, g);
+  return launchGPoolMidT<__nv_bfloat16>(st, shuffle, grid, smem, gIn, gStride, Cg, rIn, rStride, cPer, w, scale, bias, act, mask, maskSum, out, outStride, g);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -769,64 +856,8 @@ cudaError_t launchHeadFinal(
 // Like gpoolMidKernel the launch is a dependent chain for a few boards; 512 threads take a board in one or two rounds of loads
 // and the matrices are brought into L1 before the wait for the kernel before this one.
 
-constexpr int HT_THREADS = 512;
+constexpr int HT_THREADS = BP_THREADS;
 constexpr int HT_MAX_SMEM = 200 * 1024;
-constexpr int HT_PARTS = 4;  // threads per channel that add up the partial sums
-
-// mean, size-scaled mean and third statistic (maximum, or the value head's second size-scaled mean) of C channels of in
-// ([rowsPad][stride], activated and masked) into pooled [3*C]; part [2][HT_THREADS / (C/8)][C]
-template <typename T, bool VALUE>
-__device__ __forceinline__ void headPool(
-  const T* in, int stride, int C, const float* mask, float boardSum, float* part, float* pooled, size_t board, const Geom& g) {
-  const int vecs = C / 8, groups = HT_THREADS / vecs;
-  const int cv = (int)threadIdx.x % vecs, rg = (int)threadIdx.x / vecs;
-  if(rg < groups) {
-    float s[8], mx[8];
-#pragma unroll
-    for(int j = 0; j < 8; j++) { s[j] = 0.0f; mx[j] = -1.0f; }
-    // padding rows hold zeros and count as points off the board
-#pragma unroll 5
-    for(int r = rg; r < g.PB; r += groups) {
-      const uint4 v4 = *reinterpret_cast<const uint4*>(in + (board + r) * stride + cv * 8);
-      const T* ve = reinterpret_cast<const T*>(&v4);
-      const float mOff = VALUE ? 0.0f : mask[board + r] - 1.0f;
-#pragma unroll
-      for(int j = 0; j < 8; j++) {
-        const float v = toF<T>(ve[j]);
-        s[j] += v;
-        if(!VALUE) mx[j] = fmaxf(mx[j], v + mOff);
-      }
-    }
-#pragma unroll
-    for(int j = 0; j < 8; j++) {
-      part[rg * C + cv * 8 + j] = s[j];
-      if(!VALUE) part[(groups + rg) * C + cv * 8 + j] = mx[j];
-    }
-  }
-  __syncthreads();
-  // HT_PARTS neighbouring lanes share a channel
-  for(int i = threadIdx.x; i < (C * HT_PARTS + 31) / 32 * 32; i += HT_THREADS) {
-    const int c = min(i / HT_PARTS, C - 1), q = i % HT_PARTS;
-    float ss = 0.0f, mm = -1.0f;
-    for(int k = q; k < groups; k += HT_PARTS) {
-      ss += part[k * C + c];
-      if(!VALUE) mm = fmaxf(mm, part[(groups + k) * C + c]);
-    }
-#pragma unroll
-    for(int o = 1; o < HT_PARTS; o <<= 1) {
-      ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-    }
-    if(q == 0 && i < C * HT_PARTS) {
-      const float sq = sqrtf(boardSum);
-      const float mean = ss / boardSum;
-      pooled[c] = mean;
-      pooled[C + c] = mean * (sq - 14.0f) * 0.1f;
-      pooled[2 * C + c] = VALUE ? mean * ((sq - 14.0f) * (sq - 14.0f) * 0.01f - 0.1f) : mm;
-    }
-  }
-  __syncthreads();
-}
 
 __device__ __forceinline__ void prefetchL1(const float* p, int count) {
   for(int i = (int)threadIdx.x * 32; i < count; i += HT_THREADS * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + i));
@@ -855,7 +886,7 @@ __global__ void __launch_bounds__(HT_THREADS) headsTailKernel(const HeadsTailArg
     prefetchL1(a.wPass, 3 * a.G1 * (a.passH > 0 ? a.passH : a.Pc));
     if(a.passH > 0) prefetchL1(a.wPass2, a.passH * a.Pc);
     gridDepWait();
-    headPool<T, false>(gv, GV, a.G1, a.mask, a.maskSum[n], sPart, sPool, board, g);
+    boardPool<T, false>(gv, GV, a.G1, a.mask, a.maskSum[n], sPart, sPool, board, g);
     blockMatVecT(sPool, 3 * a.G1, a.wGB, a.P1, nullptr, KB_ACT_IDENTITY, sPBias);
     if(a.passH > 0) blockMatVecT(sPool, 3 * a.G1, a.wPass, a.passH, a.bPass, a.passAct, sHidden);
     else blockMatVecT(sPool, 3 * a.G1, a.wPass, a.Pc, nullptr, KB_ACT_IDENTITY, sPass);
@@ -904,7 +935,7 @@ __global__ void __launch_bounds__(HT_THREADS) headsTailKernel(const HeadsTailArg
     prefetchL1(a.wV3, a.V2 * a.Vc);
     prefetchL1(a.wSV, a.V2 * a.Sv);
     gridDepWait();
-    headPool<T, true>(gv + a.G1, GV, a.V1, a.mask, a.maskSum[n], sPart, sPool, board, g);
+    boardPool<T, true>(gv + a.G1, GV, a.V1, a.mask, a.maskSum[n], sPart, sPool, board, g);
     blockMatVecT(sPool, 3 * a.V1, a.wV2, a.V2, a.bV2, a.v2Act, sV2);
     const int sym = a.symmetry ? a.symmetry[n] : 0;
     for(int p = threadIdx.x; p < g.S; p += blockDim.x) {

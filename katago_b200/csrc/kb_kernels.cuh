@@ -114,6 +114,9 @@ cudaError_t launchConvF32(
 // another thread, must not lower it between another launch's opt-in and that launch.
 cudaError_t allowSharedMemory(const void* fn, int bytes);
 
+// Multiprocessors of the current device.
+int smCount();
+
 // Launches a kernel that may become resident while the kernel before it in the stream still runs (programmatic dependent
 // launch).  It has to call gridDepWait() before it touches anything that other kernels of the stream read or write, and may
 // declare const __restrict__ only what none of them writes (weights): the qualifier promises data that does not change while

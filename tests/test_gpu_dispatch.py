@@ -95,11 +95,11 @@ def test_fp32_block_widths(trunk, mid, n, ylen, xlen, oracle):
     assert np.abs(out - ref).max() <= 1e-4 * max(1.0, np.abs(ref).max())
 
 
-@pytest.mark.parametrize("reg,gp", [(32, 8), (64, 16), (96, 64), (160, 32), (40, 128), (64, 24)])
+@pytest.mark.parametrize("reg,gp", [(32, 8), (64, 16), (96, 64), (160, 32), (40, 128), (64, 24), (80, 48), (64, 192), (48, 320), (32, 1024)])
 @pytest.mark.parametrize("n,edge", [(1, 19), (11, 9), (80, 13)])
 def test_gpool_widths(reg, gp, n, edge, oracle):
     """Global-pooling blocks at the widths where the fused middle changes its split (channels per CTA, lanes per pooled
-    channel) or is left to the separate kernels (24 pooled channels), for few and for many boards; the tolerance is the
+    channel) or adds up in another way (a number of 8-channel pieces that does not divide a warp), for few and for many boards; the tolerance is the
     reference's reduced-precision layer tolerance (cpp/tests/testnn.cpp:8-15)."""
     C = 64
     g = mf._Gen(600 + reg + gp)
@@ -108,6 +108,35 @@ def test_gpool_widths(reg, gp, n, edge, oracle):
     mask[0, :, edge // 2:] = 0
     layer = mf._gen_gpool(g, C, reg, gp, mf.ACT_MISH)
     x = rng.standard_normal((n, edge, edge, C)).astype(np.float32) * mask[..., None]
+    blob = mf.layer_blob(layer)
+    ref = oracle.eval_layer(blob, x, mask, C)
+    out = capi.eval_layer(blob, x, mask, C, precision=capi.PRECISION_FP16)
+    assert np.all(np.abs(out - ref) <= 0.03 * np.maximum(np.maximum(np.abs(out), np.abs(ref)), 3.0))
+
+
+@pytest.mark.parametrize("gp", [24, 40, 48, 96, 192, 512])
+def test_gpool_middle_is_one_launch(gp):
+    """Every pooled width that is a multiple of 8 takes the fused middle."""
+    def launches(gp):
+        tree = mf.make_convnet("gp", 610, 15, 64, ["gpool"], (32, 32, 32, 64), mf.ACT_RELU, regular_c=64, gpool_c=gp)
+        h = capi.Handle(capi.Model(mf.to_blob(tree)), 4, nn_x=9, nn_y=9, precision=capi.PRECISION_FP16)
+        n = h.launches_per_forward(4)
+        h.close()
+        return n
+    assert launches(gp) == launches(32)
+
+
+@pytest.mark.parametrize("n", [3, 44])
+def test_gpool_middle_with_more_than_48_kb(n, oracle):
+    """How many channels a CTA of the fused middle takes, and with them its shared memory, grows with the number of boards: past
+    42 boards these widths need 49 KB.  Tolerance as above."""
+    C, reg, gp = 16, 3584, 256
+    g = mf._Gen(620)
+    rng = np.random.default_rng(n)
+    mask = np.ones((n, 5, 5), np.float32)
+    mask[0, 3:] = 0
+    layer = mf._gen_gpool(g, C, reg, gp, mf.ACT_MISH)
+    x = rng.standard_normal((n, 5, 5, C)).astype(np.float32) * mask[..., None]
     blob = mf.layer_blob(layer)
     ref = oracle.eval_layer(blob, x, mask, C)
     out = capi.eval_layer(blob, x, mask, C, precision=capi.PRECISION_FP16)
