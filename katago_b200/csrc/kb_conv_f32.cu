@@ -14,10 +14,7 @@
 #include "kb_act.cuh"
 #include "kb_tc_ptx.cuh"
 
-#include <mutex>
-#include <vector>
 #include <algorithm>
-#include <utility>
 
 namespace kb {
 
@@ -177,6 +174,7 @@ size_t smemBytes(int taps, int nr, int halo) {
 
 typedef void (*ConvF32Fn)(const float*, int, int, const float*, int, int, Geom, Epilogue);
 constexpr int CF_MAX_NR = 5;
+constexpr int CF_MAX_SMEM = 200 * 1024;
 ConvF32Fn kernelOf(int taps, int nr) {
   static const ConvF32Fn k1[] = {convF32Kernel<1, 2>, convF32Kernel<1, 3>, convF32Kernel<1, 4>, convF32Kernel<1, 5>};
   static const ConvF32Fn k9[] = {convF32Kernel<9, 2>, convF32Kernel<9, 3>, convF32Kernel<9, 4>, convF32Kernel<9, 5>};
@@ -189,14 +187,13 @@ ConvF32Fn kernelOf(int taps, int nr) {
 bool convF32Eligible(const void* in, int inStride, int inC, const void* w, int outC, int kY, int kX, const Geom& g) {
   return ((kY == 1 && kX == 1) || (kY == 3 && kX == 3)) && (inC % 4) == 0 && (outC % 4) == 0 && (inStride % 4) == 0 &&
          (reinterpret_cast<uintptr_t>(in) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
-         smemBytes(kY * kX, CF_MAX_NR, kY == 3 ? g.RW + 1 : 0) <= 200 * 1024;
+         smemBytes(kY * kX, CF_MAX_NR, kY == 3 ? g.RW + 1 : 0) <= CF_MAX_SMEM;
 }
 
 cudaError_t launchConvF32(
   cudaStream_t st, const void* in, int inStride, int inC, const void* w, int outC, int kY, Geom g, const Epilogue& ep) {
   const int halo = kY == 3 ? g.RW + 1 : 0;
-  int dev = 0, sms = 148;
-  if(cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = smCount();
   // Rows per tile: what counts is the SM with the most tiles, times their height (b6c96, eight boards: 150 tiles of 64 rows are
   // two on some SM, 120 of 80 rows one everywhere).
   const int nTiles = (outC + CF_BN - 1) / CF_BN;
@@ -208,18 +205,7 @@ cudaError_t launchConvF32(
     if(c == 2 || cost <= best) { best = cost; nr = c; }
   }
   const ConvF32Fn fn = kernelOf(kY * kY, nr);
-  {
-    // opt in to the large dynamic shared memory once per variant and device
-    static std::mutex mu;
-    static std::vector<std::pair<ConvF32Fn, int>> done;
-    std::lock_guard<std::mutex> lock(mu);
-    const std::pair<ConvF32Fn, int> key(fn, dev);
-    if(std::find(done.begin(), done.end(), key) == done.end()) {
-      cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      if(e != cudaSuccess) return e;
-      done.push_back(key);
-    }
-  }
+  if(const cudaError_t e = allowSharedMemory((const void*)fn, CF_MAX_SMEM)) return e;
   return launchDependent(fn, dim3((g.rows + cfRows(nr) - 1) / cfRows(nr), nTiles), dim3(CF_THREADS), smemBytes(kY * kY, nr, halo), st, (const float*)in,
                          inStride, inC, (const float*)w, outC, halo, g, ep);
 }

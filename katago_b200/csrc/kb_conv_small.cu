@@ -24,10 +24,6 @@
 #include "kb_conv_small.cuh"
 
 #include <algorithm>
-#include <cstdlib>
-#include <mutex>
-#include <vector>
-#include <utility>
 
 namespace kb {
 
@@ -369,31 +365,8 @@ cudaError_t launchConvSmall(cudaStream_t st, const ConvSmallShape& s, int BN, in
   const int act = ep.outAct ? ep.act : KB_ACT_IDENTITY;
   ConvSmallKernelFn fn = s.dt == DT_F16 ? smallKernelForT<__half>(act) : smallKernelForT<__nv_bfloat16>(act);
   if(!fn) return cudaErrorInvalidValue;
-  {
-    // opt in to the large dynamic shared memory once per variant and device
-    static std::mutex mu;
-    static std::vector<std::pair<const void*, int>> done;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lock(mu);
-    const std::pair<const void*, int> key((const void*)fn, dev);
-    if(std::find(done.begin(), done.end(), key) == done.end()) {
-      cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, CS_SMEM_FULL);
-      if(e != cudaSuccess) return e;
-      done.push_back(key);
-    }
-  }
-  static const bool usePdl = getenv("KB_NO_PDL") == nullptr;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(CS_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  if(usePdl) {
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-  }
-  return cudaLaunchKernelEx(&cfg, fn, *s.tmA, s.tmB[convSmallMapIndex(BN)], a);
+  if(const cudaError_t e = allowSharedMemory((const void*)fn, CS_SMEM_FULL)) return e;
+  return launchDependent(fn, grid, dim3(CS_THREADS), smem, st, *s.tmA, s.tmB[convSmallMapIndex(BN)], a);
 }
 
 }  // namespace kb
