@@ -1167,6 +1167,16 @@ void Engine::selfTestWaitTimeout(unsigned long long limitNs) {
   sync();
 }
 
+std::vector<const Op*> Engine::launchList(const Geom& g) const {
+  std::vector<const Op*> list;
+  for(const Op& op : ops_) {
+    if(!op.runsSingly(g)) list.push_back(&op);
+    else
+      for(const Op& m : op.members) list.push_back(&m);
+  }
+  return list;
+}
+
 void Engine::launchOpsEager(int n) {
   // Optionally (KB_CHUNK_BOARDS) the batch runs through the launch list in chunks of boards that reuse the same
   // activation buffers, so that tensors handed from kernel to kernel stay in the 126 MB L2.
@@ -1176,30 +1186,31 @@ void Engine::launchOpsEager(int n) {
     boardOffset_ = c0;
     const Geom g = makeGeom(X_, Y_, nc);
     // the tile counters are read by multi-layer launches (small batches have none) and by per-tile dependencies
+    const std::vector<const Op*> list = launchList(g);
     bool counters = tileDeps_;
-    for(const Op& op : ops_) counters = counters || (op.tileCounters && !op.runsSingly(g));
+    for(const Op* op : list) counters = counters || op->tileCounters;
     if(tileCtr_ && counters) cudaCheck(cudaMemsetAsync(tileCtr_, 0, tileCtrBytes_, stream_), "reset of the tile counters");
-    for(size_t i = 0; i < ops_.size(); i++) {
+    while(profiling_ && events_.size() < 2 * list.size()) {
+      cudaEvent_t ev;
+      cudaCheck(cudaEventCreate(&ev), "cudaEventCreate");
+      events_.push_back(ev);
+    }
+    for(size_t i = 0; i < list.size(); i++) {
       if(profiling_) cudaCheck(cudaEventRecord(events_[2 * i], stream_), "event record");
-      cudaError_t e = cudaSuccess;
-      if(ops_[i].runsSingly(g)) {
-        for(const Op& m : ops_[i].members)
-          if(e == cudaSuccess) e = m.run(stream_, g);
-      }
-      else e = ops_[i].run(stream_, g);
-      if(e != cudaSuccess) throw CudaError("launch of '" + classes_[ops_[i].cls].name + "' failed: " + cudaGetErrorString(e));
+      const cudaError_t e = list[i]->run(stream_, g);
+      if(e != cudaSuccess) throw CudaError("launch of '" + classes_[list[i]->cls].name + "' failed: " + cudaGetErrorString(e));
       if(profiling_) cudaCheck(cudaEventRecord(events_[2 * i + 1], stream_), "event record");
     }
     if(profiling_) {
       cudaCheck(cudaStreamSynchronize(stream_), "stream synchronize");
-      for(size_t i = 0; i < ops_.size(); i++) {
+      for(size_t i = 0; i < list.size(); i++) {
         float ms = 0.0f;
         cudaCheck(cudaEventElapsedTime(&ms, events_[2 * i], events_[2 * i + 1]), "event elapsed");
-        OpClass& c = classes_[ops_[i].cls];
+        OpClass& c = classes_[list[i]->cls];
         c.launches += 1;
         c.ms += ms;
-        c.flops += ops_[i].flops * nc;
-        c.bytes += ops_[i].bytes * nc;
+        c.flops += list[i]->flops * nc;
+        c.bytes += list[i]->bytes * nc;
       }
     }
   }
@@ -1208,11 +1219,6 @@ void Engine::launchOpsEager(int n) {
 
 void Engine::runOps(int n) {
   if(n < 1 || n > maxBatch_) throw std::runtime_error("batch size out of range for this handle");
-  if(profiling_ && events_.size() < 2 * ops_.size()) {
-    size_t old = events_.size();
-    events_.resize(2 * ops_.size());
-    for(size_t i = old; i < events_.size(); i++) cudaCheck(cudaEventCreate(&events_[i]), "cudaEventCreate");
-  }
   // Whole-network runs replay a CUDA graph of the launch list from the second run of a batch size on: the kernels'
   // arguments depend only on the batch size and on whether symmetries were uploaded.
   const bool graphable = graphsEnabled_ && !profiling_ && layerN_ == 0 && chunkBoards_ == 0;

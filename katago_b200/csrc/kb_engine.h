@@ -70,10 +70,7 @@ class Engine {
   int precision() const { return dt_; }
   int launchesPerForward(int n) const {
     const int chunk = chunkBoards_ > 0 ? chunkBoards_ : n;
-    const Geom g = makeGeom(X_, Y_, std::min(chunk, n));
-    int perChunk = 0;
-    for(const Op& op : ops_) perChunk += op.runsSingly(g) ? (int)op.members.size() : 1;
-    return perChunk * ((n + chunk - 1) / chunk);
+    return (int)launchList(makeGeom(X_, Y_, std::min(chunk, n))).size() * ((n + chunk - 1) / chunk);
   }
 
   // meta: [n][inMetaC] rows for nets with an SGF metadata encoder (must be non-NULL exactly for those nets)
@@ -113,6 +110,8 @@ class Engine {
   std::map<int, GraphEntry> graphs_;
   bool graphsEnabled_ = true;
   int graphsInstantiated_ = 0;  // instantiated graphs (at most 64 batch sizes are captured; the others stay eager)
+  // what a pass over these boards launches: the operations, merged ones replaced by their members where those run singly
+  std::vector<const Op*> launchList(const Geom& g) const;
   void launchOpsEager(int n);
 
   // RMS norms of pre-norm transformer blocks folded into the convolutions around them: the producer of the residual

@@ -172,6 +172,26 @@ def test_head_kernels_of_different_sizes_from_two_threads(monkeypatch):
         h.close()
 
 
+def test_profile_counts_what_a_small_batch_launches():
+    """A small batch runs the members of merged launches one by one: the profile has them under their own names, with their own
+    bytes, and as many as the launch count says; a full batch has the merged launches."""
+    h = capi.Handle(capi.Model(mf.to_blob(mf.make_b18c384nbt(num_blocks=3))), 128, precision=capi.PRECISION_FP16)
+    sp, gl = mf.random_positions(128, seed=13)
+    h.upload(sp, gl)
+    h.profile_enable(True)
+    totals = {}
+    for n in (2, 128):
+        h.profile_reset()
+        h.forward_resident(n)
+        ran = [e for e in h.profile_read() if e["launches"]]
+        assert sum(e["launches"] for e in ran) == h.launches_per_forward(n)
+        assert any("chain" in e["name"] or "fused" in e["name"] for e in ran) == (n == 128)
+        totals[n] = (sum(e["flops"] for e in ran) / n, sum(e["bytes"] for e in ran) / n)
+    h.close()
+    assert totals[2][0] == pytest.approx(totals[128][0])
+    assert totals[2][1] > totals[128][1]  # the activated trunk tensor, which the fused 1x1 launches do not write
+
+
 def test_noalloc_convolution_after_another_geometry(oracle):
     """kb_conv_noalloc keeps one buffer for all geometries: a call's padding rows may hold an earlier call's board points, in
     widths that the engine's staged fp32 kernel would take."""
