@@ -115,7 +115,8 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
 
   if(warp == 0) {
     // ---------------- TMA producer: all lanes wait, an elected one issues ----------------
-    auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_PRODUCER_TIMEOUT); };
+    bool live = true;  // (what counts is the flag: see mbarWaitWarp)
+    auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_PRODUCER_TIMEOUT, live); };
     int ib = residentB ? totalB : a.numB;  // next weight slot to request
     gridDepWait();  // activations belong to the kernels before this one
     // they may have been written with ordinary stores
@@ -123,31 +124,35 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
     auto loadB = [&]() {
       const uint32_t s = (uint32_t)(ib % a.numB);
       wait(&emptyB[s], (uint32_t)(ib / a.numB - 1) & 1u);
-      if(electOne()) {
+      if(electOne() && !*abortFlag) {
         const uint32_t bar = smemU32(&fullB[s]);
         mbarExpectTx(bar, (uint32_t)a.bSlotBytes);
         tmaLoad3d(smemU32(smemB + (size_t)s * a.bSlotBytes), &tmB, (ib / groupsPerChunk) * CS_BK, n0, (ib % groupsPerChunk) * a.tapGroup, bar);
       }
       ib++;
     };
-    for(int kc = 0; kc < a.kChunks; kc++) {
+    auto loadA = [&](int kc, uint32_t s) {
+      const uint32_t bar = smemU32(&fullA[s]);
+      mbarExpectTx(bar, (uint32_t)a.aSlotBytes);
+      tmaLoad2d(smemU32(smemA + (size_t)s * a.aSlotBytes), &tmA, kc * CS_BK, m0 - a.haloPad, bar);
+    };
+    const int first = min(a.numA, a.kChunks);
+    if(electOne()) {
+      for(int kc = 0; kc < first; kc++) loadA(kc, (uint32_t)kc);
+    }
+    for(int kc = first; kc < a.kChunks; kc++) {
       const uint32_t s = (uint32_t)(kc % a.numA);
-      if(kc >= a.numA) {
-        // weight slots that come free before this activation slot does are refilled first
-        while(ib < totalB && ib < a.numB + (kc - a.numA + 1) * groupsPerChunk) loadB();
-        wait(&emptyA[s], (uint32_t)(kc / a.numA - 1) & 1u);
-      }
-      if(electOne()) {
-        const uint32_t bar = smemU32(&fullA[s]);
-        mbarExpectTx(bar, (uint32_t)a.aSlotBytes);
-        tmaLoad2d(smemU32(smemA + (size_t)s * a.aSlotBytes), &tmA, kc * CS_BK, m0 - a.haloPad, bar);
-      }
+      // weight slots that come free before this activation slot does are refilled first
+      while(ib < totalB && ib < a.numB + (kc - a.numA + 1) * groupsPerChunk) loadB();
+      wait(&emptyA[s], (uint32_t)(kc / a.numA - 1) & 1u);
+      if(electOne() && !*abortFlag) loadA(kc, s);
     }
     while(ib < totalB) loadB();
   }
   else if(warp == 1) {
     // ---------------- MMA issuer: all lanes wait, an elected one issues ----------------
-    auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_MMA_TIMEOUT); };
+    bool live = true;  // (goes on after a time-out: see mbarWaitWarp)
+    auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_MMA_TIMEOUT, live); };
     const uint32_t descHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);  // stride offset | version | SWIZZLE_128B
     const uint32_t aLoBase = ((smemU32(smemA) & 0x3FFFFu) >> 4) | (1u << 16);
     const uint32_t bLoBase = ((smemU32(smemB) & 0x3FFFFu) >> 4) | (1u << 16);

@@ -527,7 +527,9 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
       // leader's barrier, on which the leader alone has announced the bytes of both CTAs.
       const uint32_t aBytes = (PAIR ? 2u : 1u) * (uint32_t)a.aSlotBytes, bBytes = (PAIR ? 2u : 1u) * (uint32_t)a.bSlotBytes;
       const int bRow0 = PAIR ? (int)rank * (a.BN / 2) : 0;
-      auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_PRODUCER_TIMEOUT); };
+      bool live = true;  // this lane's waits have all been met
+      auto go = [&]() { return PAIR ? live : !*abortFlag; };  // see mbarWaitWarp
+      auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_PRODUCER_TIMEOUT, live); };
       auto loadA = [&](uint32_t slot, int kc, int m0) {
         const uint32_t bar = smemU32(&fullA[slot]), dst = smemU32(smemA + (size_t)slot * a.aSlotBytes);
         if(leader) mbarExpectTx(bar, aBytes);
@@ -580,7 +582,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
           TRACE(true, ((t - tm.first) / tm.step) * 16 + kc);
           if(!PAIR && a.jointAB) {
             // both operands of the step on the activation slot's barrier; the weight slot has the same index
-            if(one()) {
+            if(one() && go()) {
               const uint32_t bar = smemU32(&fullA[sa]);
               mbarExpectTx(bar, aBytes + bBytes);
               tmaLoad2d(smemU32(smemA + (size_t)sa * a.aSlotBytes), &tmA, kc * TC_BK, m0 - a.haloPad, bar);
@@ -589,13 +591,13 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
             if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
             continue;
           }
-          if(one()) loadA(sa, kc, m0);
+          if(one() && go()) loadA(sa, kc, m0);
           if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
           if(a.residentB) continue;
           for(int tap = 0; tap < taps; tap++, issuedB++) {
             if(issuedB >= prefilled) {
               wait(&emptyB[sb], phB ^ 1u);
-              if(one()) loadB(sb, kc, tap * a.outC + n0);
+              if(one() && go()) loadB(sb, kc, tap * a.outC + n0);
             }
             if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
           }
@@ -610,7 +612,9 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
     // In a pair only the leader issues; its MMAs read both CTAs' shared memory and write both CTAs' TMEM, and every
     // completion is signalled to the same barrier of both CTAs.
     if(leader && (PAIR || electOne())) {
-      auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_MMA_TIMEOUT); };
+      bool live = true;  // this lane's waits have all been met
+      auto go = [&]() { return PAIR ? live : true; };
+      auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_MMA_TIMEOUT, live); };
       auto commit = [&](uint64_t* bar) {
         const uint32_t b = smemU32(bar);
         if(PAIR) { ummaCommitPair(b); ummaCommitPair(clusterMapAddr(b, 1u)); }
@@ -653,7 +657,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
             for(int tap = 0; tap < 9; tap++) {
               wait(&fullB[sb], phB);
               tcFenceAfter();
-              if(one()) {
+              if(one() && go()) {
                 mma4(dTmem, aLo + tapOff[tap], bLoBase + sb * bSlot16, tap == 0 ? accumulate : 1u);
                 commit(&emptyB[sb]);  // frees the weight slot once these MMAs have read it
                 if(tap == 8) commit(&emptyA[sa]);
@@ -665,7 +669,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
             // weights were loaded once; the barrier of chunk kc completed its only phase during the first tile
             if(it == 0) wait(&fullB[kc], 0u);
             tcFenceAfter();
-            if(one()) {
+            if(one() && go()) {
               mma4(dTmem, aLo, bLoBase + (uint32_t)kc * bSlot16, accumulate);
               commit(&emptyA[sa]);
             }
@@ -673,7 +677,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
           else if(!PAIR && a.jointAB) {
             // the weight chunk arrived on the same barrier as the activation chunk and is released with it
             tcFenceAfter();
-            if(one()) {
+            if(one() && go()) {
               mma4(dTmem, aLo, bLoBase + sa * bSlot16, accumulate);
               commit(&emptyA[sa]);
             }
@@ -681,7 +685,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
           else {
             wait(&fullB[sb], phB);
             tcFenceAfter();
-            if(one()) {
+            if(one() && go()) {
               mma4(dTmem, aLo, bLoBase + sb * bSlot16, accumulate);
               commit(&emptyB[sb]);
               commit(&emptyA[sa]);
@@ -690,7 +694,7 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
           }
           if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
         }
-        if(one()) commit(&accFull[buf]);
+        if(one() && go()) commit(&accFull[buf]);
         { TLT(3); TL(9, (unsigned long long)clock64()); }
         TRACE(true, 256 + it * 16 + 15);
       }
@@ -1773,22 +1777,32 @@ cudaError_t launchConvChain(cudaStream_t st, const ConvChainPlan* c, Geom g, int
 }
 
 // ---------------------------------------------------------------------------------------------
-// Self-test of the bounded waits: a one-thread kernel waits, with the given limit, on a barrier that nothing ever arrives
-// at.  The wait gives up, the kernel records its code in the status word exactly as the convolution kernels do on a
-// time-out, and returns; the context stays usable.
+// Self-test of the bounded waits: one warp waits, half of the given limit in each of the two forms, on a barrier that nothing
+// ever arrives at.  The waits give up, the kernel records its code in the status word exactly as the convolution kernels do
+// on a time-out, and returns; the context stays usable.  The second form is used as a feeding warp uses it, on a slot that
+// is never given back: a slot armed again behind the failed wait, or a wait that reports success, is recorded as 198.
 
-enum { TC_ERR_SELFTEST_TIMEOUT = 199 };
+enum { TC_ERR_SELFTEST_FAILED = 198, TC_ERR_SELFTEST_TIMEOUT = 199 };
 
 __global__ void waitTimeoutSelfTestKernel(int* status, unsigned long long limitNs) {
-  __shared__ uint64_t bar;
+  __shared__ uint64_t empty, full;
   __shared__ int abortFlag;
+  bool ok = true;
   if(threadIdx.x == 0) {
     abortFlag = 0;
-    mbarInit(smemU32(&bar), 1);
+    mbarInit(smemU32(&empty), 1); mbarInit(smemU32(&full), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    const bool arrived = mbarWait(smemU32(&bar), 0u, &abortFlag, (uint64_t)limitNs);
-    if(!arrived) atomicCAS(status, 0, TC_ERR_SELFTEST_TIMEOUT);
+    ok = !mbarWait(smemU32(&empty), 0u, &abortFlag, (uint64_t)limitNs / 2);
   }
+  __syncwarp();
+  bool live = true;
+  for(int use = 0; use < 2; use++) {
+    if(use > 0) mbarWaitWarp(smemU32(&empty), 0u, &abortFlag, status, TC_ERR_SELFTEST_TIMEOUT, live, (uint64_t)limitNs / 2);
+    if(electOne() && live) mbarArrive(smemU32(&full));
+  }
+  __syncwarp();
+  // armed once: its first phase is over, its second is not
+  if(threadIdx.x == 0 && !(ok && mbarTryWait(smemU32(&full), 0u) && !mbarTryWait(smemU32(&full), 1u))) atomicExch(status, TC_ERR_SELFTEST_FAILED);
 }
 
 cudaError_t launchWaitTimeoutSelfTest(cudaStream_t st, int* statusWord, unsigned long long limitNs) {

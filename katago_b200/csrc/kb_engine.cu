@@ -996,7 +996,7 @@ void Engine::sync() {
     int code = *statusHost_;
     *statusHost_ = 0;
     cudaMemsetAsync(statusWord_, 0, sizeof(int), stream_);
-    throw CudaError("a device-side wait timed out (status " + std::to_string(code) + ": 101 producer, 102 MMA issuer, 103 epilogue of a tensor-core kernel, 121 to 123 the same of the small-batch kernel, 199 wait self-test)");
+    throw CudaError("a device-side wait timed out (status " + std::to_string(code) + ": 101 producer, 102 MMA issuer, 103 epilogue of a tensor-core kernel, 121 to 123 the same of the small-batch kernel, 199 wait self-test, 198 that self-test failed)");
   }
 }
 

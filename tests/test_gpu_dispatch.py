@@ -192,6 +192,14 @@ def test_profile_counts_what_a_small_batch_launches():
     assert totals[2][1] > totals[128][1]  # the activated trunk tensor, which the fused 1x1 launches do not write
 
 
+def test_both_forms_of_the_bounded_wait_give_up():
+    """199 is the time-out itself; 198 would be a wait that reported success, or a slot armed again behind a failed one."""
+    h = capi.Handle(capi.Model(mf.to_blob(mf.make_b18c384nbt(num_blocks=1))), 1, precision=capi.PRECISION_FP16)
+    with pytest.raises(capi.KBError, match="status 199:"):
+        h.selftest_wait_timeout(1_000_000)
+    h.close()
+
+
 def test_noalloc_convolution_after_another_geometry(oracle):
     """kb_conv_noalloc keeps one buffer for all geometries: a call's padding rows may hold an earlier call's board points, in
     widths that the engine's staged fp32 kernel would take."""

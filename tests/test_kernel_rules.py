@@ -54,3 +54,15 @@ def test_early_kernels_promise_constant_data_for_weights_only(name):
     params = next(p for n, p, _ in KERNELS if n == name)
     constant = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", params))
     assert constant <= {"w", "wT", "scale", "bias", "layers"}
+
+
+@pytest.mark.parametrize("name", [n for n, _, b in KERNELS if "mbarWaitWarp" in b])
+def test_nothing_is_issued_behind_a_wait_that_ran_out(name):
+    """A slot whose wait ran out may still be armed: arming it again in the same phase is past what its barrier can count.  Every
+    arming behind a wait therefore asks whether the waits have been met."""
+    body = next(b for n, _, b in KERNELS if n == name)
+    body = body.split("else if(warp == 1)")[0]  # the feeding warp's part
+    issues = list(re.finditer(r"if\((?:one|electOne)\(\)([^{;]*)", body))
+    for w in re.finditer(r"\bwait\(&|mbarWaitWarp\(smemU32\(&", body):
+        behind = next((i for i in issues if i.start() > w.start()), None)
+        assert behind is not None and re.match(r" && (?:go\(\)|live|!\*abortFlag)\)", behind.group(1)), body[w.start():w.start() + 200]
