@@ -21,7 +21,7 @@ namespace kb {
 namespace {
 
 constexpr int CF_BN = 32, CF_BK = 16;
-constexpr int CF_AS = CF_BK + 4;      // floats per staged row: 16-byte loads of rows 20 floats apart meet no bank twice
+constexpr int CF_AS = CF_BK + 4;      // floats per staged row: cp.async writes 16-byte pieces; the 8-byte loads of the eight rows a warp reads start 20 floats apart
 constexpr int CF_KG = 8;               // warps that share a tile's channels
 constexpr int CF_THREADS = 512;        // two halves of a tile's rows, CF_KG warps each
 constexpr int cfRows(int nr) { return 16 * nr; }  // rows of a tile whose threads hold nr x 8 outputs

@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
     // the sequence of this warp's residual units: (tile, part, unit in part) with unit % PP_CG == cg
     int nt = (int)blockIdx.x, np = 0, nj = cg - PP_CG;   // the unit before the first one
     auto fetchNext = [&](uint32_t slotSeq) {
-      // lane 0: request the residual of the next unit of this warp's sequence into ring slot slotSeq % 2
+      // an elected thread: request the residual of the next unit of this warp's sequence into ring slot slotSeq % 2
       nj += PP_CG;
       if(nj >= UP) { nj = cg; if(++np >= a.parts) { np = 0; nt += grid; } }
       if(nt >= numTiles) return;

@@ -220,7 +220,7 @@ struct EpiWarp {
 };
 
 // Fetches the residual of this warp's unit number `seq` (counted over all of the CTA's tiles, nU per tile) into its
-// ring slot, if that tile exists (lane 0 only).
+// ring slot, if that tile exists (an elected thread only).
 // Which tiles a CTA works on: tile t covers rows (t / numNTiles) * rowsPerUnit + rowBase and channel tile t % numNTiles;
 // a CTA takes t = first, first + step, ...  (a CTA pair shares t; rowBase selects the half).
 struct TileMap {
@@ -419,7 +419,7 @@ __device__ __forceinline__ bool epilogueTileTma(
       for(int jj = 0; jj < 4; jj++)
         *reinterpret_cast<uint4*>(oRow + ((jj ^ sw) << 4)) = make_uint4(actP[4 * jj], actP[4 * jj + 1], actP[4 * jj + 2], actP[4 * jj + 3]);
     }
-    // make the generic-proxy writes visible to the TMA engine, then let lane 0 send the unit out
+    // make the generic-proxy writes visible to the TMA engine, then let an elected thread send the unit out
     fenceProxyAsync();
     __syncwarp();
     if(electOne()) {

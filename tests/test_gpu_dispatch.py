@@ -1,5 +1,8 @@
 """Dispatch rules of the tensor-core convolutions at the sizes where they change: input widths that do not fill the last
 64-channel chunk, and batches on either side of the small-batch kernel's limit."""
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -27,6 +30,58 @@ def test_input_widths_between_chunks(prec, tol, trunk, mid, oracle):
     ref = oracle.eval_layer(blob, x, mask, trunk)
     out = capi.eval_layer(blob, x, mask, trunk, precision=prec)
     assert np.all(np.abs(out - ref) <= tol * np.maximum(np.maximum(np.abs(out), np.abs(ref)), 3.0))
+
+
+def _wide_tiles(test_file, keyword):
+    """Runs tests in a process of their own in which no batch is small (the switch is read once per process): their few boards
+    then go through the wide-tile kernels and the merged launches."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-m", "pytest", "-x", "-q", "-m", "gpu", os.path.join("tests", test_file), "-k", keyword], cwd=root,
+                       env=dict(os.environ, KB_NO_SMALL="1"), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=600)
+    assert r.returncode == 0 and " passed" in r.stdout, r.stdout[-3000:]
+
+
+def test_input_widths_between_chunks_in_wide_tiles():
+    _wide_tiles("test_gpu_dispatch.py", "(between_chunks or gpool_widths) and not wide_tiles")
+
+
+def test_layers_and_nets_in_wide_tiles():
+    _wide_tiles("test_gpu_parity.py", "conv_layer_tensor_core or blocks_and_norm_with_masks or nbt_reduced_precision or every_block_at_full_depth")
+
+
+def test_chains_and_pairs_with_partial_chunks(oracle):
+    """Full batches of nets whose widths end inside a 64-channel chunk, a few rows against the oracle: 96 input channels in the
+    multi-layer launches, 96 and 160 into 256-wide tiles in CTA pairs.  Tolerance as above."""
+    for trunk, mid, n, edge in ((96, 96, 128, 19), (96, 256, 200, 13), (256, 160, 200, 13)):
+        blob = mf.to_blob(mf.make_convnet("partial", 460 + mid, 15, trunk, ["plain", "gpool", "plain"], (32, 32, 32, 64), mf.ACT_MISH, mid_c=mid,
+                                          regular_c=64, gpool_c=32))
+        sizes = ([edge, 9, 7, edge] * n)[:n]
+        sp, gl = mf.random_positions(n, seed=14, nn_len=edge, board_sizes=sizes)
+        h = capi.Handle(capi.Model(blob), n, nn_x=edge, nn_y=edge, precision=capi.PRECISION_FP16)
+        out = h.forward(sp, gl)
+        h.close()
+        rows = [0, 1, n // 2, n - 2, n - 1]
+        ref = oracle.OracleModel(blob, edge, edge).forward(sp[rows], gl[rows])
+        for k in ref:
+            got = out[k][rows]
+            assert np.all(np.abs(got - ref[k]) <= 0.03 * np.maximum(np.maximum(np.abs(got), np.abs(ref[k])), 3.0)), (trunk, mid, k)
+
+
+@pytest.mark.parametrize("d,heads,head_dim,ffn,rope", [(96, 3, 32, 160, "learnable"), (96, 2, 64, 96, "fixed"), (160, 5, 64, 416, "learnable"),
+                                                        (224, 4, 64, 320, "none")])
+@pytest.mark.parametrize("n", [3, 40])
+def test_transformers_with_partial_chunks(d, heads, head_dim, ffn, rope, n, oracle):
+    """Trunk and FFN widths that end inside a 64-channel chunk: the folded RMS norms, the rotary and the SwiGLU epilogues then run
+    on the tensor-core path too.  Bounds as for the other transformers in reduced precision."""
+    from tests.test_gpu_parity import _assert_reduced_close  # (not at the top: its tests would be collected here again)
+    blob = mf.to_blob(mf.make_transformer(seed=470 + d, layers=2, d=d, heads=heads, head_dim=head_dim, ffn=ffn, rope=rope, rel_bias=rope == "none"))
+    sp, gl = mf.random_positions(n, seed=15, board_sizes=([19, 13, 9] * n)[:n])
+    h = capi.Handle(capi.Model(blob), n, precision=capi.PRECISION_FP16)
+    out = h.forward(sp, gl)
+    h.close()
+    rows = list(range(3)) if n == 3 else [0, 1, 20, n - 2, n - 1]
+    ref = oracle.OracleModel(blob).forward(sp[rows], gl[rows])
+    _assert_reduced_close({k: v[rows] for k, v in out.items()}, ref, sp[rows][..., 0].reshape(len(rows), -1))
 
 
 @pytest.mark.parametrize("trunk,mid", [(96, 528), (72, 640), (528, 96), (64, 576)])
@@ -60,6 +115,8 @@ def test_more_activated_channels_than_the_tensor_core_kernel_holds(trunk, mid, o
     (lambda: mf.make_b28c512nbt(num_blocks=3), capi.PRECISION_BF16, 128, 19),
     (lambda: mf.make_b28c512nbt(num_blocks=3), capi.PRECISION_FP16, 64, 13),
     (lambda: mf.make_b6c96(), capi.PRECISION_FP16, 256, 19),
+    (lambda: mf.make_transformer(layers=2), capi.PRECISION_FP16, 64, 19),
+    (lambda: mf.make_transformer_relbias(layers=2), capi.PRECISION_FP16, 64, 19),
 ])
 def test_small_batches_give_the_rows_of_a_full_batch(factory, prec, full, edge):
     """Small batches run in narrow tiles (kb_conv_small.cu), full ones in wide tiles and merged launches.  The order of an
@@ -80,7 +137,7 @@ def test_small_batches_give_the_rows_of_a_full_batch(factory, prec, full, edge):
 @pytest.mark.parametrize("trunk,mid", [(4, 8), (20, 36), (96, 96), (64, 100), (132, 48)])
 @pytest.mark.parametrize("n,ylen,xlen", [(1, 19, 19), (5, 9, 13), (2, 5, 30)])
 def test_fp32_block_widths(trunk, mid, n, ylen, xlen, oracle):
-    """fp32 residual blocks at the edges of the staged kernel's tiles (16-channel slices, 32-channel and 64-row tiles, wide
+    """fp32 residual blocks at the edges of the staged kernel's tiles (16-channel slices, tiles of 32 channels and 32 to 80 rows, wide
     boards with their larger halo).  A sum of K products of order one in fp32 is off by at most about K * 2^-24 of their
     magnitude: 2 * 9 * 132 * 6e-8 = 1.4e-4 in the worst case and two orders less in practice; 1e-4 as for the other fp32 tests."""
     g = mf._Gen(500 + trunk + mid)
