@@ -115,8 +115,10 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
 
   if(warp == 0) {
     // ---------------- TMA producer: all lanes wait, an elected one issues ----------------
-    bool live = true;  // (what counts is the flag: see mbarWaitWarp)
-    auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_PRODUCER_TIMEOUT, live); };
+    // Behind a wait it asks the abort flag before it arms a slot.  The flag is raised before any slot can be given back
+    // wrongly: by its own wait, or by one of the MMA issuer, which goes on after a time-out (its MMAs stay inside the CTA's
+    // buffers, and each of its arrivals ends a phase of a barrier that counts one).
+    auto wait = [&](uint64_t* bar, uint32_t parity) { (void)mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_PRODUCER_TIMEOUT); };
     int ib = residentB ? totalB : a.numB;  // next weight slot to request
     gridDepWait();  // activations belong to the kernels before this one
     // they may have been written with ordinary stores
@@ -151,8 +153,7 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
   }
   else if(warp == 1) {
     // ---------------- MMA issuer: all lanes wait, an elected one issues ----------------
-    bool live = true;  // (goes on after a time-out: see mbarWaitWarp)
-    auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_MMA_TIMEOUT, live); };
+    auto wait = [&](uint64_t* bar, uint32_t parity) { (void)mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_MMA_TIMEOUT); };
     const uint32_t descHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);  // stride offset | version | SWIZZLE_128B
     const uint32_t aLoBase = ((smemU32(smemA) & 0x3FFFFu) >> 4) | (1u << 16);
     const uint32_t bLoBase = ((smemU32(smemB) & 0x3FFFFu) >> 4) | (1u << 16);

@@ -528,8 +528,12 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
       const uint32_t aBytes = (PAIR ? 2u : 1u) * (uint32_t)a.aSlotBytes, bBytes = (PAIR ? 2u : 1u) * (uint32_t)a.bSlotBytes;
       const int bRow0 = PAIR ? (int)rank * (a.BN / 2) : 0;
       bool live = true;  // this lane's waits have all been met
-      auto go = [&]() { return PAIR ? live : !*abortFlag; };  // see mbarWaitWarp
-      auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_PRODUCER_TIMEOUT, live); };
+      // false: this thread leaves its role (single CTAs); in a pair the warp stays together and issues nothing more
+      auto wait = [&](uint64_t* bar, uint32_t parity) {
+        const bool met = mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_PRODUCER_TIMEOUT);
+        if(PAIR && !met) live = false;
+        return PAIR || met;
+      };
       auto loadA = [&](uint32_t slot, int kc, int m0) {
         const uint32_t bar = smemU32(&fullA[slot]), dst = smemU32(smemA + (size_t)slot * a.aSlotBytes);
         if(leader) mbarExpectTx(bar, aBytes);
@@ -578,11 +582,11 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
         }
         if(t == tm.first) TLT(1);
         for(int kc = 0; kc < a.kChunks; kc++) {
-          wait(&emptyA[sa], phA ^ 1u);
+          if(!wait(&emptyA[sa], phA ^ 1u)) goto fed;
           TRACE(true, ((t - tm.first) / tm.step) * 16 + kc);
           if(!PAIR && a.jointAB) {
             // both operands of the step on the activation slot's barrier; the weight slot has the same index
-            if(one() && go()) {
+            if(one() && live) {
               const uint32_t bar = smemU32(&fullA[sa]);
               mbarExpectTx(bar, aBytes + bBytes);
               tmaLoad2d(smemU32(smemA + (size_t)sa * a.aSlotBytes), &tmA, kc * TC_BK, m0 - a.haloPad, bar);
@@ -591,18 +595,19 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
             if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
             continue;
           }
-          if(one() && go()) loadA(sa, kc, m0);
+          if(one() && live) loadA(sa, kc, m0);
           if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
           if(a.residentB) continue;
           for(int tap = 0; tap < taps; tap++, issuedB++) {
             if(issuedB >= prefilled) {
-              wait(&emptyB[sb], phB ^ 1u);
-              if(one() && go()) loadB(sb, kc, tap * a.outC + n0);
+              if(!wait(&emptyB[sb], phB ^ 1u)) goto fed;
+              if(one() && live) loadB(sb, kc, tap * a.outC + n0);
             }
             if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
           }
         }
       }
+    fed:;
     }
   }
   else if(warp == 1) {
@@ -613,8 +618,12 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
     // completion is signalled to the same barrier of both CTAs.
     if(leader && (PAIR || electOne())) {
       bool live = true;  // this lane's waits have all been met
-      auto go = [&]() { return PAIR ? live : true; };
-      auto wait = [&](uint64_t* bar, uint32_t parity) { mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_MMA_TIMEOUT, live); };
+      // false: this thread leaves its role (single CTAs); in a pair the warp stays together and issues nothing more
+      auto wait = [&](uint64_t* bar, uint32_t parity) {
+        const bool met = mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_MMA_TIMEOUT);
+        if(PAIR && !met) live = false;
+        return PAIR || met;
+      };
       auto commit = [&](uint64_t* bar) {
         const uint32_t b = smemU32(bar);
         if(PAIR) { ummaCommitPair(b); ummaCommitPair(clusterMapAddr(b, 1u)); }
@@ -643,21 +652,21 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
       for(int t = tm.first; t < numTiles && !aborted(); t += tm.step, it++) {
         const uint32_t buf = it & 1u;
         // wait until the epilogue has drained this accumulator (two tiles ago)
-        wait(&accEmpty[buf], ((it >> 1) & 1u) ^ 1u);
+        if(!wait(&accEmpty[buf], ((it >> 1) & 1u) ^ 1u)) goto issued;
         tcFenceAfter();
         TRACE(true, 256 + it * 16);
         const uint32_t dTmem = tmemBase + buf * (uint32_t)a.BN;
         for(int kc = 0; kc < a.kChunks; kc++) {
-          wait(&fullA[sa], phA);
+          if(!wait(&fullA[sa], phA)) goto issued;
           if(it == 0 && kc == 0) { TLT(2); TL(8, (unsigned long long)clock64()); }
           TRACE(true, 256 + it * 16 + 1 + kc);
           const uint32_t aLo = aLoBase + sa * aSlot16, accumulate = kc > 0 ? 1u : 0u;
           if(taps == 9) {
 #pragma unroll
             for(int tap = 0; tap < 9; tap++) {
-              wait(&fullB[sb], phB);
+              if(!wait(&fullB[sb], phB)) goto issued;
               tcFenceAfter();
-              if(one() && go()) {
+              if(one() && live) {
                 mma4(dTmem, aLo + tapOff[tap], bLoBase + sb * bSlot16, tap == 0 ? accumulate : 1u);
                 commit(&emptyB[sb]);  // frees the weight slot once these MMAs have read it
                 if(tap == 8) commit(&emptyA[sa]);
@@ -667,9 +676,9 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
           }
           else if(a.residentB) {
             // weights were loaded once; the barrier of chunk kc completed its only phase during the first tile
-            if(it == 0) wait(&fullB[kc], 0u);
+            if(it == 0 && !wait(&fullB[kc], 0u)) goto issued;
             tcFenceAfter();
-            if(one() && go()) {
+            if(one() && live) {
               mma4(dTmem, aLo, bLoBase + (uint32_t)kc * bSlot16, accumulate);
               commit(&emptyA[sa]);
             }
@@ -677,15 +686,15 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
           else if(!PAIR && a.jointAB) {
             // the weight chunk arrived on the same barrier as the activation chunk and is released with it
             tcFenceAfter();
-            if(one() && go()) {
+            if(one() && live) {
               mma4(dTmem, aLo, bLoBase + sa * bSlot16, accumulate);
               commit(&emptyA[sa]);
             }
           }
           else {
-            wait(&fullB[sb], phB);
+            if(!wait(&fullB[sb], phB)) goto issued;
             tcFenceAfter();
-            if(one() && go()) {
+            if(one() && live) {
               mma4(dTmem, aLo, bLoBase + sb * bSlot16, accumulate);
               commit(&emptyB[sb]);
               commit(&emptyA[sa]);
@@ -694,10 +703,11 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
           }
           if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
         }
-        if(one() && go()) commit(&accFull[buf]);
+        if(one() && live) commit(&accFull[buf]);
         { TLT(3); TL(9, (unsigned long long)clock64()); }
         TRACE(true, 256 + it * 16 + 15);
       }
+    issued:;
     }
   }
   else if(warp < 2 + TC_EPI_WARPS) {
@@ -1797,7 +1807,7 @@ __global__ void waitTimeoutSelfTestKernel(int* status, unsigned long long limitN
   __syncwarp();
   bool live = true;
   for(int use = 0; use < 2; use++) {
-    if(use > 0) mbarWaitWarp(smemU32(&empty), 0u, &abortFlag, status, TC_ERR_SELFTEST_TIMEOUT, live, (uint64_t)limitNs / 2);
+    if(use > 0) live = mbarWaitWarp(smemU32(&empty), 0u, &abortFlag, status, TC_ERR_SELFTEST_TIMEOUT, (uint64_t)limitNs / 2);
     if(electOne() && live) mbarArrive(smemU32(&full));
   }
   __syncwarp();

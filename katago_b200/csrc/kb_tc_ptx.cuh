@@ -58,36 +58,33 @@ __device__ __forceinline__ bool mbarWait(uint32_t bar, uint32_t parity, volatile
 __device__ __forceinline__ bool warpAny(int flag) { return __any_sync(0xffffffffu, flag != 0); }
 
 // The same for a warp that feeds or issues MMAs: all lanes wait, and there is next to no code between a completed barrier and
-// what follows it.  A wait that runs out records `code`, raises the abort flag and clears `live`, as does one that finds the
-// flag raised.  The warp then runs through the rest of its loop: every further wait ends soon, and the launch's result is
-// discarded with the status.  A FEEDING warp must not arm a slot's barrier any more: the slot may still be armed, and a second
-// time in one phase is past the arrivals and bytes a barrier can count.  It asks the abort flag, which is raised before any
-// slot can be given back wrongly, after each wait; an issuing warp may go on (its MMAs stay inside the CTA's buffers, and its
-// arrivals at barriers of one arrival count each end a phase).  In a CTA pair, whose two CTAs have a flag each and fill
-// barriers of the leader, both roles ask `live`.  Asking `live` in the issuing warps of single CTAs as well made the
-// transformer's net 1.5 to 2 % slower at one to four positions, b18's 1 % at one to twenty.
+// what follows it.  A wait that runs out records `code`, raises the abort flag and returns false, as does one that finds the
+// flag raised; the launch's result is then discarded with the status.  Behind such a wait a FEEDING warp must not arm a
+// slot's barrier any more: the slot may still be armed, and a second time in one phase is past the arrivals and bytes a
+// barrier can count.  A role inside one thread leaves.  A warp that elects threads cannot, as its lanes may see different
+// results: it runs through the rest of its loop, in which every further wait ends soon, and asks before it arms.
 //
 // Such a warp runs its loop with all lanes and elects a thread for each batch of TMA or MMA instructions.  Measured on
 // barriers that have completed, six steps of two waits, four MMAs (M=128, N=32) and a commit: 740 cycles per step with the loop
 // inside the elected thread, 520 in this form, 420 with one barrier per step.
-__device__ __forceinline__ void mbarWaitWarp(
-  uint32_t bar, uint32_t parity, volatile int* abortFlag, int* status, int code, bool& live, uint64_t limitNs = 2000000000ull) {
+__device__ __forceinline__ bool mbarWaitWarp(
+  uint32_t bar, uint32_t parity, volatile int* abortFlag, int* status, int code, uint64_t limitNs = 2000000000ull) {
   uint32_t spins = 0;
   uint64_t t0 = 0;
   while(!mbarTryWait(bar, parity)) {
     if((++spins & 63u) == 0u) {
-      if(*abortFlag) { live = false; break; }
+      if(*abortFlag) return false;
       const uint64_t now = globalTimerNs();
       if(spins == 64u) t0 = now;
       else if(now - t0 > limitNs) {
         *abortFlag = 1;
         __threadfence_block();
         atomicCAS(status, 0, code);
-        live = false;
-        break;
+        return false;
       }
     }
   }
+  return true;
 }
 
 // Programmatic dependent launch: a kernel launched with the programmatic-stream-serialization attribute may start
