@@ -6,7 +6,7 @@
 // six 32-channel units and the start-up of a kernel.  Everything here shortens that chain:
 //
 // * narrow tiles: the same MMAs per tile, but about 50 cycles each (M=128, N=32, issued by this loop in isolation) instead of 96, a half
-//   to a twelfth of the weights per SM, and an epilogue of one or two 8-channel pieces per warp.  The order of the additions
+//   to a twelfth of the weights per SM, and an epilogue of one to three 8-channel pieces per warp.  The order of the additions
 //   inside an accumulator does not depend on N, so a position's results stay the same bit for bit in every batch size;
 // * all weights of a tile in shared memory where they fit, behind one barrier, else a ring whose slots hold three taps: a
 //   wait costs the issuing warp as much as two narrow MMAs;
@@ -14,10 +14,9 @@
 //   (programmatic dependent launch); what is left after it is the activations, the MMAs and the epilogue;
 // * the epilogue goes straight from registers to global memory.
 //
-// A 3x3 192->192 launch of one position takes 6.5 us (15 us per layer in the wide-tile chain).  Where it goes was measured with
-// the issuing loop still inside one thread and an epilogue of half as many warps (7.1 us from exit to exit): 0.85 us until
-// the wait for the previous launch returns, 0.75 us until the first activations arrive, 3.8 us of MMAs (108 in a row at 69
-// cycles, issue-bound), 0.9 us epilogue, 0.4 us exit.
+// A 3x3 192->192 launch of one position takes 6.5 us (15 us per layer in the wide-tile chain), and nothing in it is busy: on the
+// 48 SMs that have a tile the tensor pipe works 7 % of the cycles and 12 % of the issue slots are taken.  It is a chain of the
+// launch boundary, the first activations, 108 MMAs in a row and the epilogue.
 //
 // Each CTA computes one tile and leaves.  Every wait is bounded; see kb_conv_tc.cu.
 #include "kb_conv_dev.cuh"
@@ -201,7 +200,7 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
   }
   else {
     // ---------------- Epilogue: TMEM lane quarter = warp % 4; four warps per quarter take the 8-channel groups in turn ----------------
-    // Little code per thread on purpose: it runs once or twice per launch, so fetching it counts.
+    // Little code per thread on purpose: it runs one to three times per launch, so fetching it counts.
     const int q = warp & 3, part = (warp - 2) >> 2;
     const int m = m0 + q * 32 + lane;
     const int groups = a.BN / 8;
@@ -325,7 +324,9 @@ bool convSmallSupports(const Epilogue& ep) {
 // twenty - / - / 1954 / 1328; the figures left of the smallest are past one CTA per SM with a full SM's memory each.)
 // Past that, two CTAs share an SM with half of its memory each: with 152 64-wide tiles b28's twelve positions take 2411 us
 // against 2536 in 128-wide tiles with an SM each and 3049 in the wide-tile kernels; with 228 32-wide ones b18's twelve
-// take 1143 us against 1106 in 114 64-wide ones.
+// take 1143 us against 1106 in 114 64-wide ones.  Over the whole range of this rule, against the wide-tile kernels: b18 with
+// 24 to 31 boards (225 to 291 64-wide tiles) 1278 to 1299 us against 1426 to 1439, with 96 to 120 boards of 9x9 1290 to 1301
+// against 1437 to 1441, b28 with 12 to 23 boards 2261 to 2359 against 2836 to 2947; one board past it both are the same.
 int convSmallTileWidth(int outC, int rowTiles, int numSMs) {
   for(int bn : {16, 32, 64, 96})
     if(outC % bn == 0 && (long long)rowTiles * (outC / bn) <= numSMs) return bn;
