@@ -1,43 +1,50 @@
-// Tensor-core convolution for small batches: one CTA per tile of 128 rows x 16 to 96 output channels.
+// Tensor-core convolution for small batches: one CTA per tile of 64 or 128 rows x 16 to 192 output channels.
 //
 // convTcKernel (kb_conv_tc.cu) gives every CTA a wide tile and a deep pipeline, which is right when there are more tiles
 // than SMs.  A batch of a few positions has 4 to 40 row tiles: with 192- or 256-wide tiles most SMs idle, and a layer
 // takes as long as ONE tile, i.e. 108 MMAs in a row (3x3 192->192), a weight stream of 663 KB into one SM, an epilogue of
 // six 32-channel units and the start-up of a kernel.  Everything here shortens that chain:
 //
-// * narrow tiles: the same MMAs per tile, but about 50 cycles each (M=128, N=32, issued by this loop in isolation) instead of 96, a half
-//   to a twelfth of the weights per SM, and an epilogue of one to three 8-channel pieces per warp.  The order of the additions
-//   inside an accumulator does not depend on N, so a position's results stay the same bit for bit in every batch size;
-// * all weights of a tile in shared memory where they fit, behind one barrier, else a ring whose slots hold three taps: a
-//   wait costs the issuing warp as much as two narrow MMAs;
+// * small tiles: the same MMAs per tile, but cheaper ones, a part of the weights per SM and a short epilogue.  Cycles per MMA
+//   (K=16, issued back to back): 128 rows 41 / 42 / 46 / 50 / 58 / 66 / 98 for N = 16 / 32 / 48 / 64 / 96 / 128 / 192, 64 rows
+//   28 / 28 / 31 / 34 / 50 / 66 / 98: up to N = 64 the operand rows read from shared memory set the pace, so half the rows cost
+//   two thirds.  The order of the additions inside an accumulator depends on neither, so a position's results stay the same
+//   bit for bit in every batch size;
+// * all weights of a tile in shared memory where they fit, behind one barrier, else a ring;
 // * barriers, TMEM, weights and tensor maps are on their way before the wait for the launch before this one
 //   (programmatic dependent launch); what is left after it is the activations, the MMAs and the epilogue;
-// * the epilogue goes straight from registers to global memory.
+// * the MMAs come from one elected thread whose loops are chosen once per launch and whose waits cost a single try: with a run-time
+//   choice of the loop's form and a bounded wait spelled out inside it, every step cost 470 cycles beyond its MMAs
+//   (3x3 192->192 of one position: 6.2 k cycles from the first MMA to the last, 1x1 384->192 3.7 k; now 3.1 k and 1.1 k);
+// * the epilogue goes straight from registers to global memory, 32 bytes (a sector) per thread and access: with 16-byte accesses
+//   the closing 1x1 of five positions took 1.5 to 4.5 us for its epilogue alone, every sector being written twice.
 //
-// A 3x3 192->192 launch of one position takes 6.5 us (15 us per layer in the wide-tile chain), and nothing in it is busy: on the
-// 48 SMs that have a tile the tensor pipe works 7 % of the cycles and 12 % of the issue slots are taken.  It is a chain of the
-// launch boundary, the first activations, 108 MMAs in a row and the epilogue.
+// What is left of a launch (5 us for a 3x3 layer of one position before these changes, 3.7 us now) is the launch boundary (about 1 us),
+// the first activations (0.6 us), the MMAs and the epilogue (0.5 us).
 //
 // Each CTA computes one tile and leaves.  Every wait is bounded; see kb_conv_tc.cu.
 #include "kb_conv_dev.cuh"
 #include "kb_conv_small.cuh"
 
 #include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+#include <type_traits>
 
 namespace kb {
 
 namespace {
 
-constexpr int CS_BM = 128;
 constexpr int CS_BK = 64;
-constexpr int CS_EPI_WARPS = 16;                   // four per TMEM lane quarter
+constexpr int CS_EPI_WARPS = 12;                    // three per TMEM lane quarter
+constexpr int CS_PARTS = CS_EPI_WARPS / 4;
 constexpr int CS_THREADS = 64 + 32 * CS_EPI_WARPS;  // producer warp, MMA warp, epilogue warps
 constexpr int CS_MAX_SLOTS = 32;
-constexpr int CS_MAX_BN = 96;
+constexpr int CS_MAX_BN = 192;
 // barriers (full and empty of both rings, accumulator), the TMEM slot and flags, the norm parameters of the tile, and the
 // slack of the 1024-byte alignment
 constexpr int CS_FIXED_SMEM = (4 * CS_MAX_SLOTS + 1) * 8 + 64 + 2 * CS_MAX_BN * 4 + 1024;
-// Shared memory of a CTA: all of an SM where the tiles are no more than the SMs, else half of one (228 KB, 1 KB reserved per CTA)
+// Shared memory of a CTA: half of an SM's (228 KB, 1 KB reserved per CTA) or all of it
 constexpr int CS_SMEM_HALF = 113 * 1024, CS_SMEM_FULL = 226 * 1024;
 
 enum { CS_ERR_PRODUCER_TIMEOUT = 121, CS_ERR_MMA_TIMEOUT = 122, CS_ERR_EPILOGUE_TIMEOUT = 123 };
@@ -47,7 +54,7 @@ struct ConvSmallArgs {
   Epilogue ep;
   int outC, BN;
   int taps;        // 1 or 9
-  int tapGroup;    // taps per weight slot: 1 (1x1) or 3 (3x3)
+  int tapGroup;    // taps per weight slot: 1 or 3 (3x3)
   int kChunks;     // 64-channel chunks of the input; the last one may reach past the last channel (zeros)
   int haloPad;     // rows loaded above the tile
   int aSlotBytes, bSlotBytes;
@@ -56,43 +63,41 @@ struct ConvSmallArgs {
   int* status;
 };
 
-template <typename T, int ACT>
+template <typename T, int ACT, int BM>
 __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
-  const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const ConvSmallArgs a) {
+  const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ ConvSmallArgs a) {
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smemA = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~(uintptr_t)1023);
   uint8_t* smemB = smemA + (size_t)a.numA * a.aSlotBytes;
   float* sScale = reinterpret_cast<float*>(smemB + (size_t)a.numB * a.bSlotBytes);
   float* sBias = sScale + CS_MAX_BN;
-  uint64_t* fullA = reinterpret_cast<uint64_t*>(sBias + CS_MAX_BN);
-  uint64_t* emptyA = fullA + a.numA;
-  uint64_t* fullB = emptyA + a.numA;
-  uint64_t* emptyB = fullB + a.numB;
-  uint64_t* accFull = emptyB + a.numB;
-  uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(accFull + 1);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sBias + CS_MAX_BN);
+  uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bars + 2 * (a.numA + a.numB) + 1);
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
+  // barriers by shared-memory address: full and empty of the activation ring, full and empty of the weight ring, accumulator
+  const uint32_t fullA = smemU32(bars), emptyA = fullA + 8u * (uint32_t)a.numA;
+  const uint32_t fullB = emptyA + 8u * (uint32_t)a.numA, emptyB = fullB + 8u * (uint32_t)a.numB, accFull = emptyB + 8u * (uint32_t)a.numB;
+  const uint32_t sA = smemU32(smemA), sB = smemU32(smemB);
 
   const int warp = warpIndex(), lane = threadIdx.x & 31;
-  const int n0 = (int)blockIdx.x * a.BN, m0 = (int)blockIdx.y * CS_BM;
+  const int n0 = (int)blockIdx.x * a.BN, m0 = (int)blockIdx.y * BM;
   const Epilogue& ep = a.ep;
   const int groupsPerChunk = a.taps / a.tapGroup;
   const int totalB = a.kChunks * groupsPerChunk;
   const bool residentB = a.numB >= totalB;  // all weights of the tile fit: one barrier for all of them
 
   if(warp == 0 && electOne()) {
-    for(int s = 0; s < a.numA; s++) { mbarInit(smemU32(&fullA[s]), 1); mbarInit(smemU32(&emptyA[s]), 1); }
-    for(int s = 0; s < a.numB; s++) { mbarInit(smemU32(&fullB[s]), 1); mbarInit(smemU32(&emptyB[s]), 1); }
-    mbarInit(smemU32(accFull), 1);
+    for(int s = 0; s < 2 * (a.numA + a.numB) + 1; s++) mbarInit(fullA + 8u * (uint32_t)s, 1);
     *abortFlag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fenceProxyAsync();
     // The first weights: nothing before this launch produces them, and the ring is empty.
-    if(residentB) mbarExpectTx(smemU32(&fullB[0]), (uint32_t)(totalB * a.bSlotBytes));
+    if(residentB) mbarExpectTx(fullB, (uint32_t)(totalB * a.bSlotBytes));
     const int pre = residentB ? totalB : a.numB;
     for(int i = 0; i < pre; i++) {
-      const uint32_t bar = smemU32(&fullB[residentB ? 0 : i]);
+      const uint32_t bar = residentB ? fullB : fullB + 8u * (uint32_t)i;
       if(!residentB) mbarExpectTx(bar, (uint32_t)a.bSlotBytes);
-      tmaLoad3d(smemU32(smemB + (size_t)i * a.bSlotBytes), &tmB, (i / groupsPerChunk) * CS_BK, n0, (i % groupsPerChunk) * a.tapGroup, bar);
+      tmaLoad3d(sB + (uint32_t)(i * a.bSlotBytes), &tmB, (i / groupsPerChunk) * CS_BK, n0, (i % groupsPerChunk) * a.tapGroup, bar);
     }
     prefetchTensorMap(&tmA);
   }
@@ -113,112 +118,114 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
   const uint32_t tmemBase = *tmemSlot;
 
   if(warp == 0) {
-    // ---------------- TMA producer: all lanes wait, an elected one issues ----------------
-    // Behind a wait it asks the abort flag before it arms a slot.  The flag is raised before any slot can be given back
-    // wrongly: by its own wait, or by one of the MMA issuer, which goes on after a time-out (its MMAs stay inside the CTA's
-    // buffers, and each of its arrivals ends a phase of a barrier that counts one).
-    auto wait = [&](uint64_t* bar, uint32_t parity) { (void)mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_PRODUCER_TIMEOUT); };
-    int ib = residentB ? totalB : a.numB;  // next weight slot to request
-    gridDepWait();  // activations belong to the kernels before this one
-    // they may have been written with ordinary stores
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    auto loadB = [&]() {
-      const uint32_t s = (uint32_t)(ib % a.numB);
-      wait(&emptyB[s], (uint32_t)(ib / a.numB - 1) & 1u);
-      if(electOne() && !*abortFlag) {
-        const uint32_t bar = smemU32(&fullB[s]);
-        mbarExpectTx(bar, (uint32_t)a.bSlotBytes);
-        tmaLoad3d(smemU32(smemB + (size_t)s * a.bSlotBytes), &tmB, (ib / groupsPerChunk) * CS_BK, n0, (ib % groupsPerChunk) * a.tapGroup, bar);
-      }
-      ib++;
-    };
-    auto loadA = [&](int kc, uint32_t s) {
-      const uint32_t bar = smemU32(&fullA[s]);
-      mbarExpectTx(bar, (uint32_t)a.aSlotBytes);
-      tmaLoad2d(smemU32(smemA + (size_t)s * a.aSlotBytes), &tmA, kc * CS_BK, m0 - a.haloPad, bar);
-    };
-    const int first = min(a.numA, a.kChunks);
+    // ---------------- TMA producer: one thread, which leaves behind a wait that ran out ----------------
     if(electOne()) {
+      auto wait = [&](uint32_t bar, uint32_t parity) { return mbarWaitThread(bar, parity, abortFlag, a.status, CS_ERR_PRODUCER_TIMEOUT); };
+      gridDepWait();  // activations belong to the kernels before this one
+      // they may have been written with ordinary stores
+      asm volatile("fence.proxy.async.global;" ::: "memory");
+      auto loadA = [&](int kc, uint32_t s) {
+        mbarExpectTx(fullA + 8u * s, (uint32_t)a.aSlotBytes);
+        tmaLoad2d(sA + s * (uint32_t)a.aSlotBytes, &tmA, kc * CS_BK, m0 - a.haloPad, fullA + 8u * s);
+      };
+      const int first = min(a.numA, a.kChunks);
       for(int kc = 0; kc < first; kc++) loadA(kc, (uint32_t)kc);
-    }
-    for(int kc = first; kc < a.kChunks; kc++) {
-      const uint32_t s = (uint32_t)(kc % a.numA);
-      // weight slots that come free before this activation slot does are refilled first
-      while(ib < totalB && ib < a.numB + (kc - a.numA + 1) * groupsPerChunk) loadB();
-      wait(&emptyA[s], (uint32_t)(kc / a.numA - 1) & 1u);
-      if(electOne() && !*abortFlag) loadA(kc, s);
-    }
-    while(ib < totalB) loadB();
-  }
-  else if(warp == 1) {
-    // ---------------- MMA issuer: all lanes wait, an elected one issues ----------------
-    auto wait = [&](uint64_t* bar, uint32_t parity) { (void)mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, CS_ERR_MMA_TIMEOUT); };
-    const uint32_t descHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);  // stride offset | version | SWIZZLE_128B
-    const uint32_t aLoBase = ((smemU32(smemA) & 0x3FFFFu) >> 4) | (1u << 16);
-    const uint32_t bLoBase = ((smemU32(smemB) & 0x3FFFFu) >> 4) | (1u << 16);
-    const uint32_t aSlot16 = (uint32_t)a.aSlotBytes >> 4, bSlot16 = (uint32_t)a.bSlotBytes >> 4, bTap16 = (uint32_t)a.BN * 8u;
-    const bool freeA = a.kChunks > a.numA;
-    uint32_t sa = 0, phA = 0, sb = 0, phB = 0;
-    if(residentB) wait(&fullB[0], 0u);
-    for(int kc = 0; kc < a.kChunks; kc++) {
-      wait(&fullA[sa], phA);
-      const uint32_t aLo = aLoBase + sa * aSlot16;
-      if(a.taps == 9) {
-        for(int grp = 0; grp < 3; grp++) {
-          if(!residentB) wait(&fullB[sb], phB);
-          tcFenceAfter();
-          if(electOne()) {
-            // the three taps of board line dy = grp - 1: one row (128 bytes, 8 units) apart in the halo tile
-            const uint32_t aT = aLo + (uint32_t)(a.haloPad + (grp - 1) * a.g.RW - 1) * 8u, bLo = bLoBase + sb * bSlot16;
-#pragma unroll
-            for(int t = 0; t < 3; t++) {
-#pragma unroll
-              for(int k = 0; k < CS_BK / 16; k++)
-                ummaLoHi(tmemBase, aT + 8u * t + 2 * k, bLo + t * bTap16 + 2 * k, descHi, a.idesc, (t == 0 && k == 0) ? (uint32_t)(kc + grp) : 1u);
-            }
-            if(!residentB) ummaCommit(smemU32(&emptyB[sb]));
-            if(freeA && grp == 2) ummaCommit(smemU32(&emptyA[sa]));
-          }
+      int ib = residentB ? totalB : a.numB;  // next weight slot to request
+      uint32_t sb = 0, phB = 0;              // its place in the ring
+      bool ok = true;
+      auto loadB = [&](int upTo) {
+        for(; ib < upTo && ok; ib++) {
+          if(!wait(emptyB + 8u * sb, phB)) { ok = false; break; }
+          mbarExpectTx(fullB + 8u * sb, (uint32_t)a.bSlotBytes);
+          tmaLoad3d(sB + sb * (uint32_t)a.bSlotBytes, &tmB, (ib / groupsPerChunk) * CS_BK, n0, (ib % groupsPerChunk) * a.tapGroup, fullB + 8u * sb);
           if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
         }
+      };
+      uint32_t s = 0, phA = 0;
+      for(int kc = first; kc < a.kChunks && ok; kc++) {
+        // weight slots that come free before this activation slot does are refilled first
+        loadB(min(totalB, a.numB + (kc - a.numA + 1) * groupsPerChunk));
+        if(!ok || !wait(emptyA + 8u * s, phA)) { ok = false; break; }
+        loadA(kc, s);
+        if(++s == (uint32_t)a.numA) { s = 0; phA ^= 1u; }
       }
-      else {
-        if(!residentB) wait(&fullB[sb], phB);
-        tcFenceAfter();
-        if(electOne()) {
-          const uint32_t bLo = bLoBase + sb * bSlot16;
-#pragma unroll
-          for(int k = 0; k < CS_BK / 16; k++) ummaLoHi(tmemBase, aLo + 2 * k, bLo + 2 * k, descHi, a.idesc, k == 0 ? (uint32_t)kc : 1u);
-          if(!residentB) ummaCommit(smemU32(&emptyB[sb]));
-          if(freeA) ummaCommit(smemU32(&emptyA[sa]));
-        }
-        if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
-      }
-      if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
+      if(ok) loadB(totalB);
     }
-    if(electOne()) ummaCommit(smemU32(accFull));
+  }
+  else if(warp == 1) {
+    // ---------------- MMA issuer: one thread; what a launch decides once is decided outside its loops ----------------
+    if(electOne()) {
+      auto wait = [&](uint32_t bar, uint32_t parity) { return mbarWaitThread(bar, parity, abortFlag, a.status, CS_ERR_MMA_TIMEOUT); };
+      const uint32_t descHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);  // stride offset | version | SWIZZLE_128B
+      const uint32_t aLoBase = ((sA & 0x3FFFFu) >> 4) | (1u << 16), bLoBase = ((sB & 0x3FFFFu) >> 4) | (1u << 16);
+      const uint32_t aSlot16 = (uint32_t)a.aSlotBytes >> 4, bSlot16 = (uint32_t)a.bSlotBytes >> 4, bTap16 = (uint32_t)a.BN * 8u;
+      const uint32_t idesc = a.idesc, RW8 = (uint32_t)a.g.RW * 8u;
+      const uint32_t tap0 = a.taps == 9 ? (uint32_t)(a.haloPad - a.g.RW - 1) * 8u : 0u;  // first row of the first tap in the halo tile
+      const int kChunks = a.kChunks, numA = a.numA, numB = a.numB;
+      const bool freeA = kChunks > numA;
+      // LINES x TAPS taps: a weight slot holds SLOT of them
+      auto issue = [&](auto lines, auto taps, auto slot, auto resident) {
+        constexpr int LINES = decltype(lines)::value, TAPS = decltype(taps)::value, SLOT = decltype(slot)::value;
+        constexpr bool RES = decltype(resident)::value;
+        uint32_t sa = 0, phA = 0, sb = 0, phB = 0, accumulate = 0;
+        if(RES && !wait(fullB, 0u)) return false;
+        for(int kc = 0; kc < kChunks; kc++) {
+          if(!wait(fullA + 8u * sa, phA)) return false;
+          uint32_t aLo = aLoBase + sa * aSlot16 + tap0;
+#pragma unroll 1
+          for(int line = 0; line < LINES; line++, aLo += RW8) {
+#pragma unroll
+            for(int t = 0; t < TAPS; t++) {
+              if(t % SLOT == 0) {
+                if(!RES && !wait(fullB + 8u * sb, phB)) return false;
+                tcFenceAfter();
+              }
+              const uint32_t bLo = bLoBase + sb * bSlot16 + (uint32_t)(t % SLOT) * bTap16;
+#pragma unroll
+              for(int k = 0; k < CS_BK / 16; k++) {
+                ummaLoHi(tmemBase, aLo + 8u * t + 2 * k, bLo + 2 * k, descHi, idesc, accumulate);
+                accumulate = 1;
+              }
+              if(t % SLOT == SLOT - 1) {
+                if(!RES) ummaCommit(emptyB + 8u * sb);
+                if(++sb == (uint32_t)numB) { sb = 0; phB ^= 1u; }
+              }
+            }
+          }
+          if(freeA) ummaCommit(emptyA + 8u * sa);
+          if(++sa == (uint32_t)numA) { sa = 0; phA ^= 1u; }
+        }
+        return true;
+      };
+      constexpr std::integral_constant<int, 1> one{};
+      constexpr std::integral_constant<int, 3> three{};
+      bool ok;
+      if(a.taps == 1) ok = residentB ? issue(one, one, one, std::true_type{}) : issue(one, one, one, std::false_type{});
+      else if(residentB) ok = issue(three, three, three, std::true_type{});
+      else if(a.tapGroup == 3) ok = issue(three, three, three, std::false_type{});
+      else ok = issue(three, three, one, std::false_type{});
+      if(ok) ummaCommit(accFull);
+    }
   }
   else {
-    // ---------------- Epilogue: TMEM lane quarter = warp % 4; four warps per quarter take the 8-channel groups in turn ----------------
-    // Little code per thread on purpose: it runs one to three times per launch, so fetching it counts.
+    // ---------------- Epilogue: TMEM lane quarter = warp % 4; three warps per quarter take the 16-channel units in turn ----------------
+    // A thread owns 16 channels of a row: 32 bytes, a whole sector, in one access per tensor.  A 64-row accumulator lies in
+    // the first 16 lanes of each quarter.
+    constexpr int QROWS = BM / 4;
     const int q = warp & 3, part = (warp - 2) >> 2;
-    const int m = m0 + q * 32 + lane;
-    const int groups = a.BN / 8;
+    const bool row = lane < QROWS;
+    const int m = m0 + q * QROWS + (lane & (QROWS - 1));
+    const int units = min(a.BN, a.outC - n0) / 16;
     gridDepWait();
     const float mk = ep.mask ? ep.mask[m] : 1.0f;
     const bool on = mk == 1.0f;
     const int bIdx = min(m / a.g.PB, a.g.n - 1);
     const float* biasRow = ep.biasNC ? ep.biasNC + (size_t)bIdx * a.outC + n0 : nullptr;
     const T* resRow = ep.residual ? reinterpret_cast<const T*>(ep.residual) + (size_t)m * ep.resStride + n0 : nullptr;
-    // The residual and the board's bias of the first group are on their way while the MMAs run.
-    uint4 res = make_uint4(0u, 0u, 0u, 0u);
-    float4 bias[2];
-    auto fetch = [&](int gi) {
-      if(resRow) res = *reinterpret_cast<const uint4*>(resRow + gi * 8);
-      if(biasRow) { bias[0] = reinterpret_cast<const float4*>(biasRow + gi * 8)[0]; bias[1] = reinterpret_cast<const float4*>(biasRow + gi * 8)[1]; }
-    };
-    if(part < groups) fetch(part);
-    bool ok = mbarWait(smemU32(accFull), 0u, abortFlag);
+    // The residual of the first unit is on its way while the MMAs run, that of the next while a unit is computed.
+    uint32_t res[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if(resRow && row && part < units) ldGlobal32(resRow + part * 16, res);
+    bool ok = mbarWait(accFull, 0u, abortFlag);
     ok = __all_sync(0xffffffffu, ok);
     if(!ok) {
       if(lane == 0 && !*abortFlag) { *abortFlag = 1; atomicCAS(a.status, 0, CS_ERR_EPILOGUE_TIMEOUT); }
@@ -226,62 +233,60 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
     else {
       tcFenceAfter();
 #pragma unroll 1
-      for(int gi = part; gi < groups; gi += CS_EPI_WARPS / 4) {
-        const int c = n0 + gi * 8;
-        uint32_t r[8];
-        tmemLd8(tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(gi * 8), r);
+      for(int u = part; u < units; u += CS_PARTS) {
+        const int c = n0 + u * 16;
+        uint32_t r[16];
+        tmemLd16(tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(u * 16), r);
         tmemLdWait();
         // from here on operation for operation what epilogueTileTma (kb_conv_tc.cu) computes
-        float2 v[4];
+        float2 v[8];
 #pragma unroll
-        for(int k = 0; k < 4; k++) v[k] = make_float2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
+        for(int k = 0; k < 8; k++) v[k] = make_float2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
         if(biasRow) {
+          const float4* bp = reinterpret_cast<const float4*>(biasRow + u * 16);
 #pragma unroll
-          for(int k = 0; k < 2; k++) {
-            v[2 * k] = __fadd2_rn(v[2 * k], make_float2(bias[k].x, bias[k].y));
-            v[2 * k + 1] = __fadd2_rn(v[2 * k + 1], make_float2(bias[k].z, bias[k].w));
+          for(int k = 0; k < 4; k++) {
+            const float4 b4 = bp[k];
+            v[2 * k] = __fadd2_rn(v[2 * k], make_float2(b4.x, b4.y));
+            v[2 * k + 1] = __fadd2_rn(v[2 * k + 1], make_float2(b4.z, b4.w));
           }
         }
         if(resRow) {
           if(ep.resMask) {
             const float2 mk2 = make_float2(mk, mk);
 #pragma unroll
-            for(int k = 0; k < 4; k++) v[k] = __fmul2_rn(v[k], mk2);
+            for(int k = 0; k < 8; k++) v[k] = __fmul2_rn(v[k], mk2);
           }
-          const uint32_t xu[4] = {res.x, res.y, res.z, res.w};
 #pragma unroll
-          for(int k = 0; k < 4; k++) v[k] = Pack2<T>::addTo(xu[k], v[k]);
+          for(int k = 0; k < 8; k++) v[k] = Pack2<T>::addTo(res[k], v[k]);
+          if(row && u + CS_PARTS < units) ldGlobal32(resRow + (u + CS_PARTS) * 16, res);
         }
-        if(gi + CS_EPI_WARPS / 4 < groups) fetch(gi + CS_EPI_WARPS / 4);
+        uint32_t o[8];
         if(ep.outRaw && c >= ep.rawC0 && c < ep.rawC1) {
-          uint4 o;
-          o.x = Pack2<T>::pack(v[0].x, v[0].y); o.y = Pack2<T>::pack(v[1].x, v[1].y);
-          o.z = Pack2<T>::pack(v[2].x, v[2].y); o.w = Pack2<T>::pack(v[3].x, v[3].y);
-          *reinterpret_cast<uint4*>(reinterpret_cast<T*>(ep.outRaw) + (size_t)m * ep.rawStride + (c - ep.rawC0)) = o;
+#pragma unroll
+          for(int k = 0; k < 8; k++) o[k] = Pack2<T>::pack(v[k].x, v[k].y);
+          if(row) stGlobal32(reinterpret_cast<T*>(ep.outRaw) + (size_t)m * ep.rawStride + (c - ep.rawC0), o);
         }
         if(ep.outAct && c >= ep.actC0 && c < ep.actC1) {
-          const float4* sp = reinterpret_cast<const float4*>(sScale + gi * 8);
-          const float4* bp = reinterpret_cast<const float4*>(sBias + gi * 8);
-          float2 x[4];
+          const float4* sp = reinterpret_cast<const float4*>(sScale + u * 16);
+          const float4* bp = reinterpret_cast<const float4*>(sBias + u * 16);
 #pragma unroll
-          for(int k = 0; k < 2; k++) {
+          for(int k = 0; k < 4; k++) {
             const float4 s4 = sp[k], b4 = bp[k];
-            x[2 * k] = __ffma2_rn(v[2 * k], make_float2(s4.x, s4.y), make_float2(b4.x, b4.y));
-            x[2 * k + 1] = __ffma2_rn(v[2 * k + 1], make_float2(s4.z, s4.w), make_float2(b4.z, b4.w));
+            v[2 * k] = __ffma2_rn(v[2 * k], make_float2(s4.x, s4.y), make_float2(b4.x, b4.y));
+            v[2 * k + 1] = __ffma2_rn(v[2 * k + 1], make_float2(s4.z, s4.w), make_float2(b4.z, b4.w));
           }
-          actStaged2<ACT, 4>(x);
-          uint4 o = make_uint4(0u, 0u, 0u, 0u);
-          if(on) {
-            o.x = Pack2<T>::pack(x[0].x, x[0].y); o.y = Pack2<T>::pack(x[1].x, x[1].y);
-            o.z = Pack2<T>::pack(x[2].x, x[2].y); o.w = Pack2<T>::pack(x[3].x, x[3].y);
-          }
-          *reinterpret_cast<uint4*>(reinterpret_cast<T*>(ep.outAct) + (size_t)m * ep.actStride + (c - ep.actC0)) = o;
+          actStaged2<ACT, 8>(v);
+#pragma unroll
+          for(int k = 0; k < 8; k++) o[k] = on ? Pack2<T>::pack(v[k].x, v[k].y) : 0u;
+          if(row) stGlobal32(reinterpret_cast<T*>(ep.outAct) + (size_t)m * ep.actStride + (c - ep.actC0), o);
         }
       }
     }
   }
 
   // ---------------- common exit ----------------
+  __syncwarp();
   tcFenceBefore();
   __syncthreads();
   if(*abortFlag) {
@@ -299,66 +304,111 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
 }
 
 typedef void (*ConvSmallKernelFn)(CUtensorMap, CUtensorMap, ConvSmallArgs);
-template <typename T>
+template <typename T, int BM>
 ConvSmallKernelFn smallKernelForT(int act) {
   switch(act) {
-    case KB_ACT_IDENTITY: return convSmallKernel<T, KB_ACT_IDENTITY>;
-    case KB_ACT_RELU: return convSmallKernel<T, KB_ACT_RELU>;
-    case KB_ACT_MISH: return convSmallKernel<T, KB_ACT_MISH>;
-    case KB_ACT_SILU: return convSmallKernel<T, KB_ACT_SILU>;
-    case KB_ACT_MISH_SCALE8: return convSmallKernel<T, KB_ACT_MISH_SCALE8>;
+    case KB_ACT_IDENTITY: return convSmallKernel<T, KB_ACT_IDENTITY, BM>;
+    case KB_ACT_RELU: return convSmallKernel<T, KB_ACT_RELU, BM>;
+    case KB_ACT_MISH: return convSmallKernel<T, KB_ACT_MISH, BM>;
+    case KB_ACT_SILU: return convSmallKernel<T, KB_ACT_SILU, BM>;
+    case KB_ACT_MISH_SCALE8: return convSmallKernel<T, KB_ACT_MISH_SCALE8, BM>;
     default: return nullptr;
   }
+}
+template <int BM>
+ConvSmallKernelFn smallKernelFor(int dt, int act) {
+  return dt == DT_F16 ? smallKernelForT<__half, BM>(act) : smallKernelForT<__nv_bfloat16, BM>(act);
 }
 
 }  // namespace
 
 bool convSmallSupports(const Epilogue& ep) {
   if(ep.sumsqOut || ep.rowSumsq || ep.act == KB_ACT_SWIGLU_PAIRS || ep.act == KB_ACT_ROPE_QK) return false;
-  return !ep.outAct || smallKernelForT<__half>(ep.act) != nullptr;
+  // an epilogue thread moves 16 channels of a row in one 32-byte access
+  auto sectors = [](const void* p, int stride) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0 && stride % 16 == 0; };
+  if(ep.outRaw && !sectors(ep.outRaw, ep.rawStride)) return false;
+  if(ep.outAct && !sectors(ep.outAct, ep.actStride)) return false;
+  if(ep.residual && !sectors(ep.residual, ep.resStride)) return false;
+  return !ep.outAct || smallKernelFor<128>(DT_F16, ep.act) != nullptr;
 }
 
-// How wide the tiles of a launch are.  While the tiles are no more than the SMs, each CTA has an SM to itself and the
-// narrowest such tile is the best: its CTAs stream the fewest weights and have the shortest epilogue.  (b18, whole net, 16 /
-// 32 / 64 / 96 wide: one position 714 / 774 / 958 / 1084 us, five 1277 / 836 / 1020 / 1184, eight - / 1426 / 1057 / 1205,
-// twenty - / - / 1954 / 1328; the figures left of the smallest are past one CTA per SM with a full SM's memory each.)
-// Past that, two CTAs share an SM with half of its memory each: with 152 64-wide tiles b28's twelve positions take 2411 us
-// against 2536 in 128-wide tiles with an SM each and 3049 in the wide-tile kernels; with 228 32-wide ones b18's twelve
-// take 1143 us against 1106 in 114 64-wide ones.  Over the whole range of this rule, against the wide-tile kernels: b18 with
-// 24 to 31 boards (225 to 291 64-wide tiles) 1278 to 1299 us against 1426 to 1439, with 96 to 120 boards of 9x9 1290 to 1301
-// against 1437 to 1441, b28 with 12 to 23 boards 2261 to 2359 against 2836 to 2947; one board past it both are the same.
-int convSmallTileWidth(int outC, int rowTiles, int numSMs) {
-  for(int bn : {16, 32, 64, 96})
-    if(outC % bn == 0 && (long long)rowTiles * (outC / bn) <= numSMs) return bn;
-  for(int bn : {32, 64})
-    if(outC % bn == 0 && (long long)rowTiles * (outC / bn) <= 2LL * numSMs) return bn;
-  return 0;
+// Which tile a launch takes.  Device time of the whole net, fp16, 19x19, in us; wide = the kernels of kb_conv_tc.cu / kb_conv_fused.cu.
+//
+// One CTA per SM with all of its shared memory, for layers whose MMAs outweigh the rest (3x3, and 1x1 with a long K loop): the
+// first tile of the list, cheapest MMAs first, of which there are no more than SMs.  Varied for the 3x3 layers of b18: one
+// position 64 x 32 516, 64 x 48 541, 64 x 16 and 128 x 16 553, 128 x 32 577; five 64 x 48 662, 128 x 32 663, 128 x 48 687;
+// eight 128 x 48 774, 128 x 64 811, 64 x 96 838 (its weights do not stay resident); twelve 128 x 64 823, 128 x 96 861, twice as
+// many half tiles on shared SMs 872; twenty 128 x 96 983, 128 x 48 on shared SMs 1034.  b28: twelve 128 x 96 (the last tile of a row 64
+// wide) 1768, 128 x 128 1885, 128 x 64 on shared SMs 2050; twenty 128 x 128 1970, 128 x 64 on shared SMs 2101.
+//
+// Two CTAs per SM, which hide each other's start, loads and epilogue: 1x1 layers with a short K loop (the closing ones, whose
+// epilogue reads a residual and writes two tensors) and whatever does not fit above.  Closing 1x1 of b18: one position 64 x 16
+// 492, 128 x 16 504; five 128 x 32 639, 128 x 64 with an SM each 663; eight 128 x 48 725, 128 x 96 with an SM each 764; b28, twelve
+// 128 x 96 1647, 128 x 192 with an SM each 1659.  3x3 layers past 148 tiles: b18 at 28 positions 128 x 64 1139, wide 1274; at 37
+// 128 x 96 1305, wide 1441; b28 at 30 128 x 96 2728, wide 3283; at 40 128 x 128 3059, wide 3404.  192-wide 3x3 tiles with half an SM
+// have two weight slots and are slower than the wide kernels (b18 at 48: 2353 against 1794).
+//
+// Weight slots of three taps where a wait is a good part of a slot's MMAs (b18, twelve positions, N = 64: 823 against 848 with one
+// tap), of one tap for wide tiles with half an SM (b18, 37 positions, N = 96: 1340 against 1589 with three).
+ConvSmallTile convSmallTile(const ConvSmallShape& s, int rows, int numSMs) {
+  if(const char* e = getenv("KB_SMALL_TILE")) {
+    // "taps:inC:outC=BM:BN:half:group,..."
+    const char* p = e;
+    while(*p) {
+      int tp, ic, oc, bm, bn, hf, gp, used = 0;
+      if(sscanf(p, "%d:%d:%d=%d:%d:%d:%d%n", &tp, &ic, &oc, &bm, &bn, &hf, &gp, &used) == 7) {
+        if(tp == s.taps && ic == s.inC && oc == s.outC) return ConvSmallTile{bm, bn, gp, hf ? CS_SMEM_HALF : CS_SMEM_FULL};
+        p += used;
+      }
+      while(*p && *p != ',') p++;
+      if(*p == ',') p++;
+    }
+  }
+  const int slot = s.taps == 9 ? 3 : 1;
+  auto tiles = [&](int bm, int bn) { return (long long)((rows + bm - 1) / bm) * ((s.outC + bn - 1) / bn); };
+  // one CTA per SM
+  if(s.taps == 9 || s.inC > 256) {
+    const int shapes[][2] = {{64, 32}, {64, 48}, {128, 32}, {128, 48}, {128, 64}, {128, 96}, {128, 128}};
+    for(const auto& t : shapes)
+      if(tiles(t[0], t[1]) <= numSMs) return ConvSmallTile{t[0], t[1], slot, CS_SMEM_FULL};
+  }
+  // two CTAs per SM
+  if(s.taps == 1 && tiles(64, 16) <= 2LL * numSMs) return ConvSmallTile{64, 16, 1, CS_SMEM_HALF};
+  for(int bn : {16, 32, 48, 64, 96, 128, 192})
+    if((s.taps == 1 || bn < 192) && tiles(128, bn) <= 2LL * numSMs) return ConvSmallTile{128, bn, s.taps == 9 && bn < 64 ? 3 : 1, CS_SMEM_HALF};
+  return ConvSmallTile{};
 }
 
-cudaError_t launchConvSmall(cudaStream_t st, const ConvSmallShape& s, int BN, int numSMs, Geom g, const Epilogue& ep, int* statusWord) {
-  if(BN % 16 != 0 || BN > CS_MAX_BN || BN < 16 || s.outC % BN != 0) return cudaErrorInvalidValue;
+cudaError_t launchConvSmall(cudaStream_t st, const ConvSmallShape& s, const ConvSmallTile& tile, Geom g, const Epilogue& ep, int* statusWord) {
+  const int BM = tile.BM, BN = tile.BN, mi = convSmallMapIndex(BN);
+  if((BM != 64 && BM != 128) || mi < 0 || (tile.tapGroup != 1 && (tile.tapGroup != 3 || s.taps != 9))) return cudaErrorInvalidValue;
   ConvSmallArgs a;
   a.g = g; a.ep = ep;
   a.outC = s.outC; a.BN = BN;
-  a.taps = s.taps; a.tapGroup = s.taps == 9 ? 3 : 1;
+  a.taps = s.taps; a.tapGroup = tile.tapGroup;
   a.kChunks = (s.inC + CS_BK - 1) / CS_BK;
   a.haloPad = s.haloPad;
-  a.aSlotBytes = s.aRows * 128;
-  a.bSlotBytes = a.tapGroup * BN * 128;
-  const int totalB = a.kChunks * (a.taps / a.tapGroup);
-  const dim3 grid(s.outC / BN, (g.rows + CS_BM - 1) / CS_BM);
-  const bool roomy = (int)(grid.x * grid.y) <= numSMs;
-  const int budget = (roomy ? CS_SMEM_FULL : CS_SMEM_HALF) - CS_FIXED_SMEM;
-  if(a.taps == 9) {
-    // all weights of the tile if they fit next to at least two activation slots (22.5 KB each on a 19x19 board), which the
-    // MMAs then never wait for; else a ring of them next to two slots (three where there is room)
-    const int allB = totalB * a.bSlotBytes;
-    a.numA = std::min(roomy ? 3 : 2, a.kChunks);
-    a.numB = std::min(std::min(totalB, CS_MAX_SLOTS), (budget - a.numA * a.aSlotBytes) / a.bSlotBytes);
-    if(a.numB < totalB && totalB <= CS_MAX_SLOTS && allB + 2 * a.aSlotBytes <= budget) { a.numA = 2; a.numB = totalB; }
-    while(a.numB == totalB && a.numA < a.kChunks && a.numA < CS_MAX_SLOTS && allB + (a.numA + 1) * a.aSlotBytes <= budget) a.numA++;
+  a.aSlotBytes = (BM == 64 ? s.aRows - 64 : s.aRows) * 128;
+  const dim3 grid((s.outC + BN - 1) / BN, (g.rows + BM - 1) / BM);
+  const int budget = tile.smem - CS_FIXED_SMEM;
+  // all weights of the tile (in slots of three taps) if they fit next to at least two activation slots (three in a full SM); the
+  // MMAs then never wait for them.  Else a ring next to two or three activation slots.
+  const int allB = a.kChunks * s.taps * BN * 128;
+  const int minA = std::min(tile.smem == CS_SMEM_FULL ? 3 : 2, a.kChunks);
+  if(a.kChunks * (s.taps == 9 ? 3 : 1) <= CS_MAX_SLOTS && allB + std::min(2, a.kChunks) * a.aSlotBytes <= budget) {
+    a.tapGroup = s.taps == 9 ? 3 : 1;
+    a.numB = a.kChunks * (s.taps / a.tapGroup);
+    a.bSlotBytes = a.tapGroup * BN * 128;
+    a.numA = std::min(std::min(a.kChunks, CS_MAX_SLOTS), (budget - allB) / a.aSlotBytes);
+  }
+  else if(s.taps == 9) {
+    a.bSlotBytes = a.tapGroup * BN * 128;
+    a.numA = minA;
+    if(budget - a.numA * a.aSlotBytes < 2 * a.bSlotBytes) a.numA = std::min(2, a.kChunks);
+    a.numB = std::min(std::min(a.kChunks * (9 / a.tapGroup), CS_MAX_SLOTS), (budget - a.numA * a.aSlotBytes) / a.bSlotBytes);
   }
   else {
+    a.bSlotBytes = BN * 128;
     a.numA = std::min(std::min(a.kChunks, CS_MAX_SLOTS), budget / (a.aSlotBytes + a.bSlotBytes));
     a.numB = a.numA;
   }
@@ -366,14 +416,15 @@ cudaError_t launchConvSmall(cudaStream_t st, const ConvSmallShape& s, int BN, in
   const size_t smem = (size_t)a.numA * a.aSlotBytes + (size_t)a.numB * a.bSlotBytes + CS_FIXED_SMEM;
   // instruction descriptor: D=f32, A/B format, both K-major, N>>3 at bit 17, M>>4 at bit 24
   const uint32_t fmt = s.dt == DT_F16 ? 0u : 1u;
-  a.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(CS_BM >> 4) << 24);
-  a.tmemCols = BN <= 32 ? 32u : BN <= 64 ? 64u : 128u;
+  a.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+  a.tmemCols = 32;
+  while((int)a.tmemCols < BN) a.tmemCols *= 2;
   a.status = statusWord;
   const int act = ep.outAct ? ep.act : KB_ACT_IDENTITY;
-  ConvSmallKernelFn fn = s.dt == DT_F16 ? smallKernelForT<__half>(act) : smallKernelForT<__nv_bfloat16>(act);
+  ConvSmallKernelFn fn = BM == 64 ? smallKernelFor<64>(s.dt, act) : smallKernelFor<128>(s.dt, act);
   if(!fn) return cudaErrorInvalidValue;
   if(const cudaError_t e = allowSharedMemory((const void*)fn, CS_SMEM_FULL)) return e;
-  return launchDependent(fn, grid, dim3(CS_THREADS), smem, st, *s.tmA, s.tmB[convSmallMapIndex(BN)], a);
+  return launchDependent(fn, grid, dim3(CS_THREADS), smem, st, BM == 64 ? s.tmA64 : *s.tmA, a.tapGroup == 3 ? s.tmB3[mi] : s.tmB[mi], a);
 }
 
 }  // namespace kb

@@ -1440,20 +1440,22 @@ ConvTcPlan* convTcCreate(
   p->numSMs = sms;
   ConvSmallShape& ss = p->smallShape;
   ss.dt = dt; ss.inC = inC; ss.outC = outC; ss.taps = kY * kX; ss.haloPad = p->haloPad; ss.aRows = p->aRows; ss.tmA = &p->tmA;
-  p->smallMaps = 1;
-  for(int bn : CONV_SMALL_WIDTHS)
-    if(!encodeWeights3d(&ss.tmB[convSmallMapIndex(bn)], dt, w, inC, outC, ss.taps, bn, ss.taps == 9 ? 3 : 1)) p->smallMaps = 0;
+  p->smallMaps = encode2d(&ss.tmA64, dt, in, (uint64_t)inC, (uint64_t)rowsPadMax, (uint64_t)inStride * 2, TC_BK, (uint32_t)(p->aRows - 64)) ? 1 : 0;
+  for(int i = 0; i < CONV_SMALL_NUM_WIDTHS; i++) {
+    if(!encodeWeights3d(&ss.tmB[i], dt, w, inC, outC, ss.taps, CONV_SMALL_WIDTHS[i], 1)) p->smallMaps = 0;
+    if(ss.taps == 9 && !encodeWeights3d(&ss.tmB3[i], dt, w, inC, outC, ss.taps, CONV_SMALL_WIDTHS[i], 3)) p->smallMaps = 0;
+  }
   p->small = 0;
   return p;
 }
 
-// Tile width of the small-batch kernel for this convolution and batch, or 0 if the wide-tile kernel runs it.  Decided by
-// the plan and the number of row tiles alone, so that every launch of a batch size takes the same route.
-static int smallWidth(const ConvTcPlan* p, const Geom& g) {
+// Tile of the small-batch kernel for this convolution and batch (BM = 0: the wide-tile kernel runs it).  Decided by the plan
+// and the number of rows alone, so that every launch of a batch size takes the same route.
+static ConvSmallTile smallTile(const ConvTcPlan* p, const Geom& g) {
   static const bool off = getenv("KB_NO_SMALL") != nullptr && atoi(getenv("KB_NO_SMALL")) != 0;
-  return p->small && !off ? convSmallTileWidth(p->outC, (g.rows + TC_BM - 1) / TC_BM, p->numSMs) : 0;
+  return p->small && !off ? convSmallTile(p->smallShape, g.rows, p->numSMs) : ConvSmallTile{};
 }
-bool convTcRunsSmall(const ConvTcPlan* p, const Geom& g) { return p && smallWidth(p, g) > 0; }
+int convTcSmallWidth(const ConvTcPlan* p, const Geom& g) { return p ? smallTile(p, g).BN : 0; }
 
 void convTcDestroy(ConvTcPlan* p) { delete p; }
 
@@ -1546,7 +1548,7 @@ cudaError_t launchConvTc(cudaStream_t st, const ConvTcPlan* p, Geom g, const Epi
   if(ep.outAct && ((ep.actStride % 8) || (ep.actC0 % 16) || (ep.actC1 % 16) || ((ep.actC1 - ep.actC0) > CONV_TC_MAX_ACT && ep.act != KB_ACT_SWIGLU_PAIRS))) return cudaErrorInvalidValue;
   if(ep.residual && (ep.resStride % 8)) return cudaErrorInvalidValue;
   if(!(deps && (deps->done || deps->wait))) {
-    if(const int bn = smallWidth(p, g)) return launchConvSmall(st, p->smallShape, bn, p->numSMs, g, ep, statusWord);
+    if(const ConvSmallTile t = smallTile(p, g); t.BM > 0) return launchConvSmall(st, p->smallShape, t, g, ep, statusWord);
   }
   ConvTcArgs a;
   a.g = g; a.ep = ep;

@@ -36,10 +36,13 @@ struct Op {
   // launches merged into one (multi-layer launches, fused 1x1 pairs): the convolutions themselves, which small batches run
   // one by one (runsSingly)
   std::vector<Op> members;
+  int singlyUpTo = 1 << 30;   // ... while none of their tiles is wider than this
   bool tileCounters = false;  // the merged launch hands tiles over through the tile counters
   bool runsSingly(const Geom& g) const {
-    for(const Op& m : members)
-      if(!convTcRunsSmall(m.tcPlan, g)) return false;
+    for(const Op& m : members) {
+      const int width = convTcSmallWidth(m.tcPlan, g);
+      if(width == 0 || width > singlyUpTo) return false;
+    }
     return !members.empty();
   }
   // tensor-core convolutions only: what the launch reads and writes, and its per-tile dependency record

@@ -233,8 +233,9 @@ struct ConvTcDeps {
 };
 bool convTcDepsCapable(const ConvTcPlan* p);
 int convTcKernelSize(const ConvTcPlan* p);
-// True if a batch of this size runs this convolution in the small-batch kernel: merged launches then make way for single ones.
-bool convTcRunsSmall(const ConvTcPlan* p, const Geom& g);
+// Width of the tiles in which the small-batch kernel runs this convolution for a batch of this size; 0 if it does not.  Merged
+// launches make way for single ones where it runs all of their members.
+int convTcSmallWidth(const ConvTcPlan* p, const Geom& g);
 // True if the tile table marks this shape for multi-layer launches.
 bool convTcChainPreferred(const ConvTcPlan* p);
 int convTcDoneCount(const ConvTcPlan* p);

@@ -87,6 +87,29 @@ __device__ __forceinline__ bool mbarWaitWarp(
   return true;
 }
 
+// The same for a role that runs inside one elected thread, whose loop should hold as little as possible around the first try: a
+// wait that does not succeed at once goes on in a function of its own.  Six steps of a wait on a completed barrier, four MMAs
+// (M=128, N=16: 164 cycles of tensor pipe) and a commit take 223 cycles each in this form, 332 with mbarWaitWarp in the
+// elected thread, 390 with mbarWaitWarp and all lanes.  False: the thread leaves its role.
+static __device__ __noinline__ bool mbarWaitOn(uint32_t bar, uint32_t parity, volatile int* abortFlag, int* status, int code) {
+  const uint64_t t0 = globalTimerNs();
+  for(uint32_t spins = 1;; spins++) {
+    if(mbarTryWait(bar, parity)) return true;
+    if((spins & 63u) == 0u) {
+      if(*abortFlag) return false;
+      if(globalTimerNs() - t0 > 2000000000ull) {
+        *abortFlag = 1;
+        __threadfence_block();
+        atomicCAS(status, 0, code);
+        return false;
+      }
+    }
+  }
+}
+__device__ __forceinline__ bool mbarWaitThread(uint32_t bar, uint32_t parity, volatile int* abortFlag, int* status, int code) {
+  return mbarTryWait(bar, parity) != 0u || mbarWaitOn(bar, parity, abortFlag, status, code);
+}
+
 // Programmatic dependent launch: a kernel launched with the programmatic-stream-serialization attribute may start
 // while the kernel before it in the stream still runs; it must not touch memory that kernel produces (or still
 // reads) before gridDepWait() returns.  gridDepLaunch() lets the next such kernel begin its own preamble.
@@ -174,6 +197,16 @@ __device__ __forceinline__ void bulkWaitPending(int n) {
     case 3: asm volatile("cp.async.bulk.wait_group 3;" ::: "memory"); break;
     default: asm volatile("cp.async.bulk.wait_group 4;" ::: "memory"); break;  // n >= 4: waits for more than asked
   }
+}
+
+// 32 bytes of one thread in one access (a whole sector; the address is a multiple of 32).
+__device__ __forceinline__ void ldGlobal32(const void* p, uint32_t (&r)[8]) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void stGlobal32(void* p, const uint32_t (&r)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
 // shared -> global tile store (asynchronous, tracked by the issuing thread's bulk groups)

@@ -134,6 +134,25 @@ def test_small_batches_give_the_rows_of_a_full_batch(factory, prec, full, edge):
     h.close()
 
 
+@pytest.mark.parametrize("prec,tol", [(capi.PRECISION_FP16, 0.03), (capi.PRECISION_BF16, 0.2)])
+@pytest.mark.parametrize("trunk,mid", [(32, 32), (160, 224), (288, 96)])
+@pytest.mark.parametrize("n", [1, 4, 7, 16, 31])
+def test_tiles_that_end_inside_a_layer(prec, tol, trunk, mid, n, oracle):
+    """Widths that the tiles of the small-batch kernel (32 to 192 channels, 64 or 128 rows) do not divide, at batches from its
+    narrowest tiles to two CTAs per SM: the last tile of a row is short, the last row tile reaches into the padding.  Tolerance as
+    in test_input_widths_between_chunks."""
+    g = mf._Gen(700 + trunk + mid)
+    rng = np.random.default_rng(trunk + mid + n)
+    mask = np.ones((n, 19, 19), np.float32)
+    mask[0, 13:] = 0
+    layer = mf._gen_ordinary(g, trunk, mid, mf.ACT_MISH)
+    x = rng.standard_normal((n, 19, 19, trunk)).astype(np.float32) * mask[..., None]
+    blob = mf.layer_blob(layer)
+    ref = oracle.eval_layer(blob, x, mask, trunk)
+    out = capi.eval_layer(blob, x, mask, trunk, precision=prec)
+    assert np.all(np.abs(out - ref) <= tol * np.maximum(np.maximum(np.abs(out), np.abs(ref)), 3.0))
+
+
 @pytest.mark.parametrize("trunk,mid", [(4, 8), (20, 36), (96, 96), (64, 100), (132, 48)])
 @pytest.mark.parametrize("n,ylen,xlen", [(1, 19, 19), (5, 9, 13), (2, 5, 30)])
 def test_fp32_block_widths(trunk, mid, n, ylen, xlen, oracle):
