@@ -222,9 +222,13 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
     const int bIdx = min(m / a.g.PB, a.g.n - 1);
     const float* biasRow = ep.biasNC ? ep.biasNC + (size_t)bIdx * a.outC + n0 : nullptr;
     const T* resRow = ep.residual ? reinterpret_cast<const T*>(ep.residual) + (size_t)m * ep.resStride + n0 : nullptr;
-    // The residual of the first unit is on its way while the MMAs run, that of the next while a unit is computed.
-    uint32_t res[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    // The residual of the warp's first two units is on its way while the MMAs run (loads behind them wait their turn among the
+    // operand copies of the SM's other CTA: b28 at twelve positions 1622 us with one unit ahead, 1599 with two), that of a third
+    // while the first is computed.  64-row tiles are so narrow that a warp has one unit.
+    constexpr bool AHEAD = BM == 128;
+    uint32_t res[8] = {0, 0, 0, 0, 0, 0, 0, 0}, resNext[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if(resRow && row && part < units) ldGlobal32(resRow + part * 16, res);
+    if(AHEAD && resRow && row && part + CS_PARTS < units) ldGlobal32(resRow + (part + CS_PARTS) * 16, resNext);
     bool ok = mbarWait(accFull, 0u, abortFlag);
     ok = __all_sync(0xffffffffu, ok);
     if(!ok) {
@@ -259,7 +263,12 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
           }
 #pragma unroll
           for(int k = 0; k < 8; k++) v[k] = Pack2<T>::addTo(res[k], v[k]);
-          if(row && u + CS_PARTS < units) ldGlobal32(resRow + (u + CS_PARTS) * 16, res);
+          if(AHEAD) {
+#pragma unroll
+            for(int k = 0; k < 8; k++) res[k] = resNext[k];
+            if(row && u + 2 * CS_PARTS < units) ldGlobal32(resRow + (u + 2 * CS_PARTS) * 16, resNext);
+          }
+          else if(row && u + CS_PARTS < units) ldGlobal32(resRow + (u + CS_PARTS) * 16, res);
         }
         uint32_t o[8];
         if(ep.outRaw && c >= ep.rawC0 && c < ep.rawC1) {

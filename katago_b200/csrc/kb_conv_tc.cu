@@ -28,6 +28,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 #include <algorithm>
 #include <utility>
@@ -106,6 +107,9 @@ constexpr int tcEpiWarps(int cg) { return 4 * cg; }
 constexpr int tcThreads(int cg, bool deps = false) { return 64 + 32 * 4 * cg + (deps ? 32 : 0); }
 
 enum { TC_ERR_PRODUCER_TIMEOUT = 101, TC_ERR_MMA_TIMEOUT = 102, TC_ERR_EPILOGUE_TIMEOUT = 103 };
+
+// forms of the MMA issuing loop
+enum { TC_LOOP_3X3, TC_LOOP_RESIDENT, TC_LOOP_JOINT, TC_LOOP_STREAMED };
 
 constexpr int tcMaxGroups(int cg) { return (16 + cg - 1) / cg; }  // 16-column groups per warp and tile (BN <= 256)
 
@@ -530,7 +534,8 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
       bool live = true;  // this lane's waits have all been met
       // false: this thread leaves its role (single CTAs); in a pair the warp stays together and issues nothing more
       auto wait = [&](uint64_t* bar, uint32_t parity) {
-        const bool met = mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_PRODUCER_TIMEOUT);
+        const bool met = PAIR ? mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_PRODUCER_TIMEOUT)
+                              : mbarWaitThread(smemU32(bar), parity, abortFlag, a.status, TC_ERR_PRODUCER_TIMEOUT);
         if(PAIR && !met) live = false;
         return PAIR || met;
       };
@@ -620,7 +625,8 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
       bool live = true;  // this lane's waits have all been met
       // false: this thread leaves its role (single CTAs); in a pair the warp stays together and issues nothing more
       auto wait = [&](uint64_t* bar, uint32_t parity) {
-        const bool met = mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_MMA_TIMEOUT);
+        const bool met = PAIR ? mbarWaitWarp(smemU32(bar), parity, abortFlag, a.status, TC_ERR_MMA_TIMEOUT)
+                              : mbarWaitThread(smemU32(bar), parity, abortFlag, a.status, TC_ERR_MMA_TIMEOUT);
         if(PAIR && !met) live = false;
         return PAIR || met;
       };
@@ -649,65 +655,72 @@ __global__ void __launch_bounds__(tcThreads(CG, DEPS), 1) convTcKernel(
         tapOff[tap] = (taps == 9) ? (uint32_t)(a.haloPad + dy * a.g.RW + dx) * 8u : 0u;
       }
       uint32_t sa = 0, phA = 0, sb = 0, phB = 0, it = 0;
-      for(int t = tm.first; t < numTiles && !aborted(); t += tm.step, it++) {
-        const uint32_t buf = it & 1u;
-        // wait until the epilogue has drained this accumulator (two tiles ago)
-        if(!wait(&accEmpty[buf], ((it >> 1) & 1u) ^ 1u)) goto issued;
-        tcFenceAfter();
-        TRACE(true, 256 + it * 16);
-        const uint32_t dTmem = tmemBase + buf * (uint32_t)a.BN;
-        for(int kc = 0; kc < a.kChunks; kc++) {
-          if(!wait(&fullA[sa], phA)) goto issued;
-          if(it == 0 && kc == 0) { TLT(2); TL(8, (unsigned long long)clock64()); }
-          TRACE(true, 256 + it * 16 + 1 + kc);
-          const uint32_t aLo = aLoBase + sa * aSlot16, accumulate = kc > 0 ? 1u : 0u;
-          if(taps == 9) {
+      // the form of the loop is chosen once per launch: a choice at every step costs as much as two MMAs
+      auto tiles = [&](auto kind) {
+        constexpr int KIND = decltype(kind)::value;
+        for(int t = tm.first; t < numTiles && !aborted(); t += tm.step, it++) {
+          const uint32_t buf = it & 1u;
+          // wait until the epilogue has drained this accumulator (two tiles ago)
+          if(!wait(&accEmpty[buf], ((it >> 1) & 1u) ^ 1u)) return;
+          tcFenceAfter();
+          TRACE(true, 256 + it * 16);
+          const uint32_t dTmem = tmemBase + buf * (uint32_t)a.BN;
+          for(int kc = 0; kc < a.kChunks; kc++) {
+            if(!wait(&fullA[sa], phA)) return;
+            if(it == 0 && kc == 0) { TLT(2); TL(8, (unsigned long long)clock64()); }
+            TRACE(true, 256 + it * 16 + 1 + kc);
+            const uint32_t aLo = aLoBase + sa * aSlot16, accumulate = kc > 0 ? 1u : 0u;
+            if(KIND == TC_LOOP_3X3) {
 #pragma unroll
-            for(int tap = 0; tap < 9; tap++) {
-              if(!wait(&fullB[sb], phB)) goto issued;
+              for(int tap = 0; tap < 9; tap++) {
+                if(!wait(&fullB[sb], phB)) return;
+                tcFenceAfter();
+                if(one() && live) {
+                  mma4(dTmem, aLo + tapOff[tap], bLoBase + sb * bSlot16, tap == 0 ? accumulate : 1u);
+                  commit(&emptyB[sb]);  // frees the weight slot once these MMAs have read it
+                  if(tap == 8) commit(&emptyA[sa]);
+                }
+                if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
+              }
+            }
+            else if(KIND == TC_LOOP_RESIDENT) {
+              // weights were loaded once; the barrier of chunk kc completed its only phase during the first tile
+              if(it == 0 && !wait(&fullB[kc], 0u)) return;
               tcFenceAfter();
               if(one() && live) {
-                mma4(dTmem, aLo + tapOff[tap], bLoBase + sb * bSlot16, tap == 0 ? accumulate : 1u);
-                commit(&emptyB[sb]);  // frees the weight slot once these MMAs have read it
-                if(tap == 8) commit(&emptyA[sa]);
+                mma4(dTmem, aLo, bLoBase + (uint32_t)kc * bSlot16, accumulate);
+                commit(&emptyA[sa]);
+              }
+            }
+            else if(KIND == TC_LOOP_JOINT) {
+              // the weight chunk arrived on the same barrier as the activation chunk and is released with it
+              tcFenceAfter();
+              if(one() && live) {
+                mma4(dTmem, aLo, bLoBase + sa * bSlot16, accumulate);
+                commit(&emptyA[sa]);
+              }
+            }
+            else {
+              if(!wait(&fullB[sb], phB)) return;
+              tcFenceAfter();
+              if(one() && live) {
+                mma4(dTmem, aLo, bLoBase + sb * bSlot16, accumulate);
+                commit(&emptyB[sb]);
+                commit(&emptyA[sa]);
               }
               if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
             }
+            if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
           }
-          else if(a.residentB) {
-            // weights were loaded once; the barrier of chunk kc completed its only phase during the first tile
-            if(it == 0 && !wait(&fullB[kc], 0u)) goto issued;
-            tcFenceAfter();
-            if(one() && live) {
-              mma4(dTmem, aLo, bLoBase + (uint32_t)kc * bSlot16, accumulate);
-              commit(&emptyA[sa]);
-            }
-          }
-          else if(!PAIR && a.jointAB) {
-            // the weight chunk arrived on the same barrier as the activation chunk and is released with it
-            tcFenceAfter();
-            if(one() && live) {
-              mma4(dTmem, aLo, bLoBase + sa * bSlot16, accumulate);
-              commit(&emptyA[sa]);
-            }
-          }
-          else {
-            if(!wait(&fullB[sb], phB)) goto issued;
-            tcFenceAfter();
-            if(one() && live) {
-              mma4(dTmem, aLo, bLoBase + sb * bSlot16, accumulate);
-              commit(&emptyB[sb]);
-              commit(&emptyA[sa]);
-            }
-            if(++sb == (uint32_t)a.numB) { sb = 0; phB ^= 1u; }
-          }
-          if(++sa == (uint32_t)a.numA) { sa = 0; phA ^= 1u; }
+          if(one() && live) commit(&accFull[buf]);
+          { TLT(3); TL(9, (unsigned long long)clock64()); }
+          TRACE(true, 256 + it * 16 + 15);
         }
-        if(one() && live) commit(&accFull[buf]);
-        { TLT(3); TL(9, (unsigned long long)clock64()); }
-        TRACE(true, 256 + it * 16 + 15);
-      }
-    issued:;
+      };
+      if(taps == 9) tiles(std::integral_constant<int, TC_LOOP_3X3>{});
+      else if(a.residentB) tiles(std::integral_constant<int, TC_LOOP_RESIDENT>{});
+      else if(!PAIR && a.jointAB) tiles(std::integral_constant<int, TC_LOOP_JOINT>{});
+      else tiles(std::integral_constant<int, TC_LOOP_STREAMED>{});
     }
   }
   else if(warp < 2 + TC_EPI_WARPS) {
