@@ -92,7 +92,8 @@ class Engine {
   void profileReset();
   int profileRead(OpClass* out, int cap);
 
-  void sync();
+  void sync();  // waits for the stream; throws if a device-side wait ran out
+  void wait();  // the same where the status word is already on its way to statusHost_
   // Runs the wait self-test on this handle's stream and synchronises: throws CudaError like any timed-out wait.
   void selfTestWaitTimeout(unsigned long long limitNs);
 

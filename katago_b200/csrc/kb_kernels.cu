@@ -146,6 +146,37 @@ __global__ void __launch_bounds__(384) packInputVecKernel(
   }
 }
 
+// A thread moves four 16-byte pieces at a time, so that enough reads are under way to cover the way to the host's memory.
+__global__ void __launch_bounds__(256) transferKernel(const __grid_constant__ TransferList list) {
+  const Transfer& t = list.t[blockIdx.y];
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  size_t done = 0;
+  if(((reinterpret_cast<uintptr_t>(t.src) | reinterpret_cast<uintptr_t>(t.dst)) & 15) == 0) {
+    const uint4* src = reinterpret_cast<const uint4*>(t.src);
+    uint4* dst = reinterpret_cast<uint4*>(t.dst);
+    const size_t n = t.words / 4;
+    for(size_t i = first; i < n; i += 4 * step) {
+      uint4 v[4];
+#pragma unroll
+      for(int k = 0; k < 4; k++)
+        if(i + k * step < n) v[k] = src[i + k * step];
+#pragma unroll
+      for(int k = 0; k < 4; k++)
+        if(i + k * step < n) dst[i + k * step] = v[k];
+    }
+    done = 4 * n;
+  }
+  for(size_t i = done + first; i < t.words; i += step) reinterpret_cast<uint32_t*>(t.dst)[i] = reinterpret_cast<const uint32_t*>(t.src)[i];
+}
+
+cudaError_t launchTransfers(cudaStream_t st, const TransferList& list) {
+  if(list.count == 0) return cudaSuccess;
+  const size_t pieces = (list.mostWords + 3) / 4;
+  const unsigned blocks = (unsigned)std::min<size_t>(std::max<size_t>((pieces + 255) / 256, 1), 148);
+  transferKernel<<<dim3(blocks, (unsigned)list.count), 256, 0, st>>>(list);
+  return cudaGetLastError();
+}
+
 cudaError_t launchPackInput(
   cudaStream_t st, int dt, const float* spatial, const int32_t* symmetry, int inC, void* dst, int dstStride,
   float* mask, float* maskSum, Geom g) {

@@ -88,6 +88,24 @@ struct Epilogue {
   int ropeC1 = 0;
 };
 
+// Copies of 4-byte words between device memory and host memory that the device can reach (page-locked), all in one launch.
+constexpr int MAX_TRANSFERS = 8;
+struct Transfer {
+  const void* src;
+  void* dst;
+  size_t words;
+};
+struct TransferList {
+  Transfer t[MAX_TRANSFERS];
+  int count = 0;
+  size_t mostWords = 0;
+  void add(const void* src, void* dst, size_t words) {
+    t[count++] = Transfer{src, dst, words};
+    if(words > mostWords) mostWords = words;
+  }
+};
+cudaError_t launchTransfers(cudaStream_t st, const TransferList& list);
+
 // --- SIMT kernels (any dtype) ---------------------------------------------------------------------
 
 // Packs NNEvaluator-style inputs into the padded-rows layout, applying the per-row board symmetry

@@ -134,6 +134,37 @@ def test_small_batches_give_the_rows_of_a_full_batch(factory, prec, full, edge):
     h.close()
 
 
+@pytest.mark.parametrize("n", [1, 3, 133])
+def test_host_buffers_of_every_kind(n):
+    """Page-locked buffers (moved by a kernel in small calls, with or without 16-byte alignment), pageable ones and a mixture of
+    the two, and calls that leave outputs out: the same bits.  133 positions are past the kernel's limit."""
+    model = capi.Model(mf.to_blob(mf.make_b6c96()))
+    h = capi.Handle(model, n, precision=capi.PRECISION_FP16)
+    sp, gl = mf.random_positions(n, seed=17)
+    sym = np.arange(n, dtype=np.int32) % 8
+    ref = h.forward(sp, gl, sym)
+    keep = []
+
+    def locked(a, shift):
+        flat = capi.PinnedArray((a.size + shift,), a.dtype)
+        keep.append(flat)
+        view = flat.array[shift:].reshape(a.shape)
+        view[...] = a
+        return view
+
+    for shift in (0, 1):
+        ins = [locked(a, shift) for a in (sp, gl, sym)]
+        outs = {k: locked(np.zeros_like(v), shift) for k, v in ref.items()}
+        for _ in range(2):
+            for v in outs.values():
+                v[...] = -1
+            h.forward(*ins, out=outs)
+            assert all(np.array_equal(outs[k], ref[k]) for k in ref)
+    mixed = h.forward(sp, ins[1], ins[2], out={k: (outs[k] if k == "policy" else np.zeros_like(v)) for k, v in ref.items()})
+    assert all(np.array_equal(mixed[k], ref[k]) for k in ref)
+    h.close()
+
+
 @pytest.mark.parametrize("prec,tol", [(capi.PRECISION_FP16, 0.03), (capi.PRECISION_BF16, 0.2)])
 @pytest.mark.parametrize("trunk,mid", [(32, 32), (160, 224), (288, 96)])
 @pytest.mark.parametrize("n", [1, 4, 7, 16, 31])
