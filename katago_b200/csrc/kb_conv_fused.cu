@@ -3,16 +3,16 @@
 //
 // As two launches the pair is bound by memory: the first writes the activated trunk tensor (the widest tensor of the
 // net) only for the second to read it back once.  Here the activated values never leave the SM: the epilogue of the
-// first GEMM writes them, in the tensor cores' operand layout, into shared memory, from where the second GEMM takes
-// its A operand.  Per 128 rows the kernel reads the block's mid tensor and the residual stream and writes the stream,
-// the next block's mid stream and its activated form: 7/12 of the bytes of the two separate kernels.
+// first GEMM writes them into tensor memory, from where the second GEMM takes its A operand.  Per 128 rows the kernel reads
+// the block's mid tensor and the residual stream and writes the stream, the next block's mid stream and its activated
+// form: 7/12 of the bytes of the two separate kernels.
 //
 // One persistent CTA per SM; warp 0 issues TMA loads, warp 1 issues the MMAs, warps 2..13 are epilogue warps (three per
-// TMEM lane quarter).  GEMM1 (rows x Cm -> Ct) runs in parts of 128 output channels whose accumulators alternate
-// between two TMEM buffers; the epilogue of a part adds the residual, stores the updated stream (TMA), and writes
-// act(norm(.)) * mask into the shared-memory operand buffer; GEMM2 (rows x Ct -> Cn) consumes that buffer part by part
-// (two 64-channel K chunks per part) into a third accumulator, whose epilogue stores the next mid stream and its
-// activated form.  Weights of both GEMMs stream through one ring of slots.  Every wait is bounded.
+// TMEM lane quarter).  GEMM1 (rows x Cm -> Ct) runs in parts of 64 to 192 output channels; the epilogue of a part adds the
+// residual, stores the updated stream (TMA), and writes act(norm(.)) * mask, two 16-bit channels per column, into one of four
+// operand chunks of 64 channels; GEMM2 (rows x Ct -> Cn) multiplies the chunks in turn into an accumulator of its own, whose
+// epilogue stores the next mid stream and its activated form.  Weights of both GEMMs stream through one ring of slots.
+// Every wait is bounded.
 #include "kb_conv_dev.cuh"
 
 #include <cuda.h>
@@ -20,21 +20,23 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 #include <algorithm>
 #include <utility>
 
 namespace kb {
 
-#ifndef KB_PP_CG
-#define KB_PP_CG 3
-#endif
 constexpr int PP_BM = 128;          // rows per tile
-constexpr int PP_CG = KB_PP_CG;            // epilogue warps per TMEM lane quarter
+constexpr int PP_CG = 3;            // epilogue warps per TMEM lane quarter
 constexpr int PP_EPI_WARPS = 4 * PP_CG;
 constexpr int PP_THREADS = 64 + 32 * PP_EPI_WARPS;
 constexpr int PP_UNIT = 32 * 64;    // staging unit: 32 rows x 32 channels of the storage type (64-byte swizzle)
 constexpr int PP_CHUNK = PP_BM * 128;  // one 64-channel K chunk of an A operand: 128 rows x 128 bytes
+constexpr int PP_MAX_SLOTS = 8;     // weight ring
+constexpr int PP_STAGE = 3;         // staging units per epilogue warp: two of the residual / updated stream, one more for GEMM2's outputs
+constexpr int PP_NUM_A2 = 4;        // operand chunks of GEMM2 in tensor memory
+constexpr int PP_A2_COLS = 32;      // 64 channels of 16 bits, two per column
 constexpr int PP_FIXED = 512;       // barriers and the TMEM slot
 
 // Optional timeline (build with -DKB_TC_TRACE): CTA 0 records SM cycle counts of its MMA warp and of its first epilogue
@@ -51,67 +53,69 @@ enum { PP_ERR_PRODUCER = 111, PP_ERR_MMA = 112, PP_ERR_EPILOGUE = 113, PP_ERR_AL
 struct PostPreArgs {
   Geom g;
   int Cm, Ct, Cn;          // GEMM1: Cm -> Ct (+ residual); GEMM2: Ct -> Cn
-  int NP;                  // output channels of GEMM1 per part (a multiple of 96: whole K chunks, units divisible by 3)
-  int parts;               // Ct / NP
+  int NP, parts;           // output channels of GEMM1 per part (64 or 128), Ct / NP
+  int N2, pieces;          // output channels of GEMM2 per weight slot, Cn / N2
   int kc1;                 // Cm / 64
-  int numB1, numB2;        // slots of the two weight rings (GEMM1, GEMM2)
-  int b1Slot, b2Slot;      // bytes per slot
-  uint32_t idesc1, idesc2, tmemCols;
+  int numB, bSlot;         // weight ring: slots and bytes per slot
+  int numD1;               // accumulators of GEMM1 (1 or 2)
+  uint32_t idesc1, idesc2;
   const float* scale1; const float* bias1;   // norm + activation between the two convolutions (Ct channels)
   const float* scale2; const float* bias2;   // norm + activation after the second one (Cn channels)
   const float* mask;
   int* status;
 };
 
-// Schedule of one tile (128 rows), parts p = 0 .. parts-1 of GEMM1, K chunks c of GEMM2 (NP / 64 per part):
-//   MMA warp:  G1(0) | for p: { G2(p, c0) | G1(p+1) | G2(p, c1..) } | G1(0) of the CTA's next tile
-//   epilogue:  for p: e1(p) (residual add, stream store, activation -> operand chunks) | e2 (outputs of GEMM2)
-// GEMM1 has ONE accumulator: its next part is issued as soon as every epilogue warp has loaded its last unit of the
-// current part from TMEM, which is early in that unit, so the MMAs finish long before the epilogue gets to them.  The
-// operand buffer of GEMM2 holds two K chunks that the epilogue fills and the MMA warp drains in turn.
-// The weights of both GEMMs stream through one ring of slots in the order the MMA warp consumes them (a ring per GEMM
-// can be configured for experiments: a slot of GEMM2 is held until the epilogue has produced its operand chunk).
-// shared memory: [A1: kc1 chunks][A2: 2 chunks][weight ring(s)][staging: 3 units per epilogue warp][barriers]
+// What bounds it: shared memory.  A tile of 128 rows (192 -> 384 -> 192) moves 1.3 MB through it (weights written and read 590 KB,
+// operand A1 144 KB, residual and updated stream 390 KB, outputs of GEMM2 196 KB), 10 k cycles at 128 bytes each, next to 9 k
+// cycles of special-function work (two operations per activated value) and 4.7 k of MMAs, in 17 k cycles measured.  With the operand
+// chunks of GEMM2 in shared memory it was 1.5 MB and 18.5 k cycles.  Tried on top of that and slower: parts of 128 channels with two
+// accumulators of GEMM1 (A1 is read three times instead of twice; 97 us a launch at batch 256 against 86), 24 epilogue warps with
+// units of 16 channels (97 us), outputs of GEMM2 from registers in 32-byte pieces (104 us), one reciprocal for two activations
+// (no change).  batch 256: 89.4 -> 85.8 us; 256 -> 512 -> 256 (b28, batch 512, bf16) about 245 us against 265 as two launches.
+//
+// The outputs of GEMM2 are read one tile late, after the warp's first unit of the next tile: nobody waits for GEMM2's last chunk
+// (1.6 k cycles a tile).  Schedule over the CTA's tiles, parts numbered through, with D accumulators for GEMM1:
+//   MMA warp:  G1(0) .. G1(D-1) | for each part P: G2(first chunk of P) | G1(P+D) | G2(other chunks of P)
+//   epilogue:  for each tile: unit cg | outputs of GEMM2 of the tile before | units cg+3, cg+6, ...
+// shared memory: [A1: kc1 chunks][weight ring][staging: 3 units per epilogue warp][barriers]
+// tensor memory: [GEMM1: D x NP columns][GEMM2: Cn][operand chunks: 4 x 32]
 template <typename T, int ACT>
 __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
   const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmW2,
   const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmRaw2, const __grid_constant__ CUtensorMap tmAct2,
-  const PostPreArgs a) {
+  const __grid_constant__ PostPreArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sA1 = smem;
-  uint8_t* sA2 = sA1 + (size_t)a.kc1 * PP_CHUNK;
-  uint8_t* sB1 = sA2 + 2 * PP_CHUNK;
-  uint8_t* sB2 = sB1 + (size_t)a.numB1 * a.b1Slot;
-  uint8_t* sStage = sB2 + (size_t)a.numB2 * a.b2Slot;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStage + (size_t)PP_EPI_WARPS * 3 * PP_UNIT);
-  uint64_t* a1Full = bars;            // 1
-  uint64_t* a1Empty = a1Full + 1;     // 1
-  uint64_t* b1Full = a1Empty + 1;        // [numB1]
-  uint64_t* b1Empty = b1Full + a.numB1;  // [numB1]
-  uint64_t* b2Full = b1Empty + a.numB1;  // [numB2]
-  uint64_t* b2Empty = b2Full + a.numB2;  // [numB2]
-  uint64_t* d1Full = b2Empty + a.numB2;  // 1
-  uint64_t* d1Empty = d1Full + 1;     // 1
-  uint64_t* a2Full = d1Empty + 1;     // [2]
-  uint64_t* a2Empty = a2Full + 2;     // [2]
-  uint64_t* d2Full = a2Empty + 2;     // 1
-  uint64_t* d2Empty = d2Full + 1;     // 1
-  uint64_t* resFull = d2Empty + 1;    // [PP_EPI_WARPS][2]
+  uint8_t* sB = sA1 + (size_t)a.kc1 * PP_CHUNK;
+  uint8_t* sStage = sB + (size_t)a.numB * a.bSlot;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStage + (size_t)PP_EPI_WARPS * PP_STAGE * PP_UNIT);
+  uint64_t* a1Full = bars;
+  uint64_t* a1Empty = a1Full + 1;
+  uint64_t* bFull = a1Empty + 1;             // [PP_MAX_SLOTS]
+  uint64_t* bEmpty = bFull + PP_MAX_SLOTS;   // [PP_MAX_SLOTS]
+  uint64_t* d1Full = bEmpty + PP_MAX_SLOTS;  // [2]
+  uint64_t* d1Empty = d1Full + 2;            // [2]
+  uint64_t* a2Full = d1Empty + 2;            // [PP_NUM_A2]
+  uint64_t* a2Empty = a2Full + PP_NUM_A2;    // [PP_NUM_A2]
+  uint64_t* d2Full = a2Empty + PP_NUM_A2;
+  uint64_t* d2Empty = d2Full + 1;
+  uint64_t* resFull = d2Empty + 1;           // [PP_EPI_WARPS][2]
   uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(resFull + PP_EPI_WARPS * 2);
   volatile int* abortFlag = reinterpret_cast<volatile int*>(tmemSlot + 1);
+  static_assert((2 + 2 * PP_MAX_SLOTS + 4 + 2 * PP_NUM_A2 + 2 + PP_EPI_WARPS * 2) * 8 + 8 <= PP_FIXED, "barriers");
 
   const int warp = warpIndex(), lane = threadIdx.x & 31;
-  const int numTiles = a.g.rowsPad / PP_BM;
   const int grid = (int)gridDim.x;
+  const int allTiles = a.g.rowsPad / PP_BM;
+  const int nTiles = (int)blockIdx.x < allTiles ? (allTiles - 1 - (int)blockIdx.x) / grid + 1 : 0;  // of this CTA
   const int cpp = a.NP / 64;   // K chunks of GEMM2 per part
   const int UP = a.NP / 32;    // 32-channel units per part
 
   if(threadIdx.x == 0) {
     mbarInit(smemU32(a1Full), 1); mbarInit(smemU32(a1Empty), 1);
-    for(int s = 0; s < a.numB1; s++) { mbarInit(smemU32(&b1Full[s]), 1); mbarInit(smemU32(&b1Empty[s]), 1); }
-    for(int s = 0; s < a.numB2; s++) { mbarInit(smemU32(&b2Full[s]), 1); mbarInit(smemU32(&b2Empty[s]), 1); }
-    mbarInit(smemU32(d1Full), 1); mbarInit(smemU32(d1Empty), PP_EPI_WARPS);
-    for(int s = 0; s < 2; s++) { mbarInit(smemU32(&a2Full[s]), 8); mbarInit(smemU32(&a2Empty[s]), 1); }  // a chunk = 2 units x 4 quarters
+    for(int s = 0; s < PP_MAX_SLOTS; s++) { mbarInit(smemU32(&bFull[s]), 1); mbarInit(smemU32(&bEmpty[s]), 1); }
+    for(int s = 0; s < 2; s++) { mbarInit(smemU32(&d1Full[s]), 1); mbarInit(smemU32(&d1Empty[s]), 4 * UP); }  // a part's units x 4 quarters
+    for(int s = 0; s < PP_NUM_A2; s++) { mbarInit(smemU32(&a2Full[s]), 8); mbarInit(smemU32(&a2Empty[s]), 1); }  // a chunk = 2 units x 4 quarters
     mbarInit(smemU32(d2Full), 1); mbarInit(smemU32(d2Empty), PP_EPI_WARPS);
     for(int s = 0; s < PP_EPI_WARPS * 2; s++) mbarInit(smemU32(&resFull[s]), 1);
     // the swizzled operand layouts assume a 1024-byte aligned base
@@ -120,71 +124,60 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if(warp == 1) { tmemAlloc(smemU32(tmemSlot), a.tmemCols); tmemRelinquish(); }
+  if(warp == 1) { tmemAlloc(smemU32(tmemSlot), 512); tmemRelinquish(); }
   tcFenceBefore();
   __syncthreads();
   tcFenceAfter();
   gridDepLaunch();
   const uint32_t tmemBase = *tmemSlot;
-  const uint32_t d1Col = 0u, d2Col = (uint32_t)a.NP;
+  // tensor memory: accumulators of GEMM1, accumulator of GEMM2, operand chunks of GEMM2
+  const uint32_t d2Col = (uint32_t)(a.numD1 * a.NP), a2Col = d2Col + (uint32_t)a.Cn;
   const bool bad = *abortFlag != 0;
 
   if(bad) {
     // misaligned shared memory: nothing runs
   }
   else if(warp == 0) {
-    // ---------------- TMA producer ----------------
+    // ---------------- TMA producer: in the order in which the MMA warp consumes ----------------
     if(electOne()) {
-      uint32_t s1 = 0, ph1 = 0, s2 = 0, ph2 = 0;
+      uint32_t sb = 0, ph = 0;
       bool ok = true;
-      auto loadW1c = [&](int kc, int row, uint32_t bytes) {
+      auto loadW = [&](const CUtensorMap* tm, int kc, int row, uint32_t bytes) {
         if(!ok) return;
-        if(!mbarWait(smemU32(&b1Empty[s1]), ph1 ^ 1u, abortFlag)) { ok = false; return; }
-        const uint32_t bar = smemU32(&b1Full[s1]);
+        if(!mbarWait(smemU32(&bEmpty[sb]), ph ^ 1u, abortFlag)) { ok = false; return; }
+        const uint32_t bar = smemU32(&bFull[sb]);
         mbarExpectTx(bar, bytes);
-        tmaLoad2d(smemU32(sB1 + (size_t)s1 * a.b1Slot), &tmW1, kc * 64, row, bar);
-        if(++s1 == (uint32_t)a.numB1) { s1 = 0; ph1 ^= 1u; }
+        tmaLoad2d(smemU32(sB + (size_t)sb * a.bSlot), tm, kc * 64, row, bar);
+        if(++sb == (uint32_t)a.numB) { sb = 0; ph ^= 1u; }
       };
-      auto loadW2c = [&](int kc, uint32_t bytes) {
-        if(!ok) return;
-        if(a.numB2 == 0) {
-          // one ring for both GEMMs: the slots are taken in the order the MMA warp consumes them
-          if(!mbarWait(smemU32(&b1Empty[s1]), ph1 ^ 1u, abortFlag)) { ok = false; return; }
-          const uint32_t bar = smemU32(&b1Full[s1]);
-          mbarExpectTx(bar, bytes);
-          tmaLoad2d(smemU32(sB1 + (size_t)s1 * a.b1Slot), &tmW2, kc * 64, 0, bar);
-          if(++s1 == (uint32_t)a.numB1) { s1 = 0; ph1 ^= 1u; }
-          return;
+      int gTile = 0, gPart = 0;  // the next part of GEMM1
+      int first = 0;             // its first K chunk whose weights have not been requested
+      auto loadG1 = [&]() {
+        if(gTile >= nTiles) return;
+        if(gPart == 0 && ok) {
+          // the buffer is free once the last part of the tile before has been multiplied
+          if(!mbarWait(smemU32(a1Empty), ((uint32_t)gTile & 1u) ^ 1u, abortFlag)) { ok = false; return; }
+          mbarExpectTx(smemU32(a1Full), (uint32_t)(a.kc1 * PP_CHUNK));
+          const int row = ((int)blockIdx.x + gTile * grid) * PP_BM;
+          for(int kc = 0; kc < a.kc1; kc++) tmaLoad2d(smemU32(sA1 + (size_t)kc * PP_CHUNK), &tmA1, kc * 64, row, smemU32(a1Full));
         }
-        if(!mbarWait(smemU32(&b2Empty[s2]), ph2 ^ 1u, abortFlag)) { ok = false; return; }
-        const uint32_t bar = smemU32(&b2Full[s2]);
-        mbarExpectTx(bar, bytes);
-        tmaLoad2d(smemU32(sB2 + (size_t)s2 * a.b2Slot), &tmW2, kc * 64, 0, bar);
-        if(++s2 == (uint32_t)a.numB2) { s2 = 0; ph2 ^= 1u; }
+        for(int kc = first; kc < a.kc1; kc++) loadW(&tmW1, kc, gPart * a.NP, (uint32_t)a.NP * 128u);
+        first = 0;
+        if(++gPart == a.parts) { gPart = 0; gTile++; }
       };
-      const uint32_t w1Bytes = (uint32_t)a.NP * 128u, w2Bytes = (uint32_t)a.Cn * 128u;
-      uint32_t it = 0;
-      auto loadA1 = [&](int t) {
-        // the buffer is free once the last part of the tile before has been multiplied
-        if(!ok) return;
-        if(!mbarWait(smemU32(a1Empty), (it & 1u) ^ 1u, abortFlag)) { ok = false; return; }
-        mbarExpectTx(smemU32(a1Full), (uint32_t)(a.kc1 * PP_CHUNK));
-        for(int kc = 0; kc < a.kc1; kc++) tmaLoad2d(smemU32(sA1 + (size_t)kc * PP_CHUNK), &tmA1, kc * 64, t * PP_BM, smemU32(a1Full));
-        it++;
+      auto loadG2 = [&](int chunk) {
+        for(int i = 0; i < a.pieces; i++) loadW(&tmW2, chunk, i * a.N2, (uint32_t)a.N2 * 128u);
       };
-      auto loadW1 = [&](int p) { for(int kc = 0; kc < a.kc1; kc++) loadW1c(kc, p * a.NP, w1Bytes); };
+      // the first weights do not wait for the kernels before this one
+      if(nTiles > 0)
+        for(; first < min(a.kc1, a.numB); first++) loadW(&tmW1, first, 0, (uint32_t)a.NP * 128u);
       gridDepWait();
-      int t = (int)blockIdx.x;
-      if(t < numTiles) { loadA1(t); loadW1(0); }
-      for(; t < numTiles && ok; t += grid) {
+      for(int i = 0; i < a.numD1; i++) loadG1();
+      for(int t = 0; t < nTiles && ok; t++) {
         for(int p = 0; p < a.parts && ok; p++) {
-          // the two rings are independent, but one thread issues both: the order follows the MMA warp's
-          loadW2c(p * cpp, w2Bytes);
-          if(p + 1 < a.parts) loadW1(p + 1);
-          for(int c = 1; c < cpp; c++) loadW2c(p * cpp + c, w2Bytes);
-          // the first part of the next tile comes after this tile's last chunk of GEMM2: the second epilogue can then
-          // start as soon as the first one ends, and GEMM1 of the next tile runs underneath it
-          if(p + 1 == a.parts && t + grid < numTiles) { loadA1(t + grid); loadW1(0); }
+          loadG2(p * cpp);
+          loadG1();
+          for(int c = 1; c < cpp; c++) loadG2(p * cpp + c);
         }
       }
       if(!ok && !*abortFlag) { *abortFlag = 1; atomicCAS(a.status, 0, PP_ERR_PRODUCER); }
@@ -195,78 +188,63 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
     if(electOne()) {
       const uint32_t descHi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);
       const uint32_t a1Lo = ((smemU32(sA1) & 0x3FFFFu) >> 4) | (1u << 16);
-      const uint32_t a2Lo = ((smemU32(sA2) & 0x3FFFFu) >> 4) | (1u << 16);
-      const uint32_t b1Lo = ((smemU32(sB1) & 0x3FFFFu) >> 4) | (1u << 16);
-      const uint32_t b2Lo = ((smemU32(sB2) & 0x3FFFFu) >> 4) | (1u << 16);
-      const uint32_t chunk16 = (uint32_t)PP_CHUNK >> 4, b1Slot16 = (uint32_t)a.b1Slot >> 4, b2Slot16 = (uint32_t)a.b2Slot >> 4;
-      uint32_t s1 = 0, ph1 = 0, s2 = 0, ph2 = 0;
+      const uint32_t bLo = ((smemU32(sB) & 0x3FFFFu) >> 4) | (1u << 16);
+      const uint32_t chunk16 = (uint32_t)PP_CHUNK >> 4, bSlot16 = (uint32_t)a.bSlot >> 4;
+      uint32_t sb = 0, ph = 0;
       bool ok = true;
-      uint32_t G1n = 0;   // GEMM1 parts issued so far (over all tiles): phase of the d1 barriers
-      uint32_t GC = 0;    // GEMM2 chunks issued so far: operand buffer GC & 1 and its barrier phases
-      uint32_t tilesA = 0;  // tiles whose A operand has been waited for
-      uint32_t itD2 = 0;    // tiles whose second accumulator has been started
-      auto g1 = [&](bool firstOfTile, bool lastOfTile) {
-        if(!ok) return;
-        if(firstOfTile) {
-          if(!mbarWait(smemU32(a1Full), tilesA & 1u, abortFlag)) { ok = false; return; }
-          tilesA++;
-        }
-        PPT(true, G1n * 4);
-        if(!mbarWait(smemU32(d1Empty), (G1n & 1u) ^ 1u, abortFlag)) { ok = false; return; }
-        PPT(true, G1n * 4 + 1);
+      // the four MMAs of a 64-channel step with the next weight slot
+      // (A from shared memory: descriptor; from tensor memory: column, 8 per 16 channels)
+      auto step = [&](auto fromTmem, uint32_t d, uint32_t aT, uint32_t idesc, uint32_t accumulate) {
+        if(!mbarWait(smemU32(&bFull[sb]), ph, abortFlag)) { ok = false; return; }
         tcFenceAfter();
-        uint32_t acc = 0;
-        for(int kc = 0; kc < a.kc1; kc++) {
-          if(!mbarWait(smemU32(&b1Full[s1]), ph1, abortFlag)) { ok = false; return; }
-          tcFenceAfter();
-          const uint32_t aT = a1Lo + (uint32_t)kc * chunk16, bT = b1Lo + s1 * b1Slot16;
+        const uint32_t bT = bLo + sb * bSlot16;
 #pragma unroll
-          for(int k = 0; k < 4; k++) { ummaLoHi(tmemBase + d1Col, aT + 2 * k, bT + 2 * k, descHi, a.idesc1, acc); acc = 1; }
-          ummaCommit(smemU32(&b1Empty[s1]));
-          if(++s1 == (uint32_t)a.numB1) { s1 = 0; ph1 ^= 1u; }
+        for(int k = 0; k < 4; k++) {
+          if(decltype(fromTmem)::value) ummaTmemA(d, aT + 8 * k, bT + 2 * k, descHi, idesc, k == 0 ? accumulate : 1u);
+          else ummaLoHi(d, aT + 2 * k, bT + 2 * k, descHi, idesc, k == 0 ? accumulate : 1u);
         }
-        ummaCommit(smemU32(d1Full));
-        if(lastOfTile) ummaCommit(smemU32(a1Empty));
+        ummaCommit(smemU32(&bEmpty[sb]));
+        if(++sb == (uint32_t)a.numB) { sb = 0; ph ^= 1u; }
+      };
+      int gTile = 0, gPart = 0;  // the next part of GEMM1
+      uint32_t G1n = 0;          // parts of GEMM1 issued so far: accumulator G1n & 1 and its barrier phases
+      auto g1 = [&]() {
+        if(gTile >= nTiles || !ok) return;
+        if(gPart == 0 && !mbarWait(smemU32(a1Full), (uint32_t)gTile & 1u, abortFlag)) { ok = false; return; }
+        const uint32_t buf = a.numD1 == 2 ? G1n & 1u : 0u, use = a.numD1 == 2 ? G1n >> 1 : G1n;
+        PPT(true, G1n * 4);
+        if(!mbarWait(smemU32(&d1Empty[buf]), (use & 1u) ^ 1u, abortFlag)) { ok = false; return; }
+        PPT(true, G1n * 4 + 1);
+        for(int kc = 0; kc < a.kc1 && ok; kc++) step(std::false_type{}, tmemBase + buf * (uint32_t)a.NP, a1Lo + (uint32_t)kc * chunk16, a.idesc1, kc > 0 ? 1u : 0u);
+        if(!ok) return;
+        ummaCommit(smemU32(&d1Full[buf]));
         PPT(true, G1n * 4 + 2);
         G1n++;
+        if(++gPart == a.parts) { gPart = 0; gTile++; ummaCommit(smemU32(a1Empty)); }
       };
-      auto g2 = [&](bool firstOfTile, bool lastOfTile) {
+      uint32_t A = 0, phA = 0, GC = 0;  // operand chunk to multiply next, its phase, chunks issued so far
+      (void)GC;
+      auto g2 = [&](int tile, bool firstOfTile, bool lastOfTile) {
         if(!ok) return;
-        const uint32_t buf = GC & 1u;
         PPT(true, 256 + GC * 4);
-        if(!mbarWait(smemU32(&a2Full[buf]), (GC >> 1) & 1u, abortFlag)) { ok = false; return; }
+        if(!mbarWait(smemU32(&a2Full[A]), phA, abortFlag)) { ok = false; return; }
         PPT(true, 256 + GC * 4 + 1);
-        if(firstOfTile) {
-          if(!mbarWait(smemU32(d2Empty), (itD2 & 1u) ^ 1u, abortFlag)) { ok = false; return; }
-          itD2++;
-        }
-        const bool shared = a.numB2 == 0;
-        if(!mbarWait(smemU32(shared ? &b1Full[s1] : &b2Full[s2]), shared ? ph1 : ph2, abortFlag)) { ok = false; return; }
-        PPT(true, 256 + GC * 4 + 2);
-        tcFenceAfter();
-        const uint32_t aT = a2Lo + buf * chunk16, bT = shared ? b1Lo + s1 * b1Slot16 : b2Lo + s2 * b2Slot16;
-#pragma unroll
-        for(int k = 0; k < 4; k++) ummaLoHi(tmemBase + d2Col, aT + 2 * k, bT + 2 * k, descHi, a.idesc2, (firstOfTile && k == 0) ? 0u : 1u);
-        if(shared) {
-          ummaCommit(smemU32(&b1Empty[s1]));
-          if(++s1 == (uint32_t)a.numB1) { s1 = 0; ph1 ^= 1u; }
-        }
-        else {
-          ummaCommit(smemU32(&b2Empty[s2]));
-          if(++s2 == (uint32_t)a.numB2) { s2 = 0; ph2 ^= 1u; }
-        }
-        ummaCommit(smemU32(&a2Empty[buf]));
+        if(firstOfTile && !mbarWait(smemU32(d2Empty), ((uint32_t)tile & 1u) ^ 1u, abortFlag)) { ok = false; return; }
+        for(int i = 0; i < a.pieces && ok; i++)
+          step(std::true_type{}, tmemBase + d2Col + (uint32_t)(i * a.N2), tmemBase + a2Col + A * PP_A2_COLS, a.idesc2, firstOfTile ? 0u : 1u);
+        if(!ok) return;
+        ummaCommit(smemU32(&a2Empty[A]));
         if(lastOfTile) ummaCommit(smemU32(d2Full));
+        PPT(true, 256 + GC * 4 + 2);
         GC++;
+        if(++A == (uint32_t)PP_NUM_A2) { A = 0; phA ^= 1u; }
       };
-      int t = (int)blockIdx.x;
-      if(t < numTiles) g1(true, a.parts == 1);
-      for(; t < numTiles && ok; t += grid) {
+      for(int i = 0; i < a.numD1; i++) g1();
+      for(int t = 0; t < nTiles && ok; t++) {
         for(int p = 0; p < a.parts && ok; p++) {
-          g2(p == 0, false);
-          if(p + 1 < a.parts) g1(false, p + 2 == a.parts);
-          for(int c = 1; c < cpp; c++) g2(false, p + 1 == a.parts && c + 1 == cpp);
-          if(p + 1 == a.parts && t + grid < numTiles) g1(true, a.parts == 1);
+          g2(t, p == 0, p + 1 == a.parts && cpp == 1);
+          g1();
+          for(int c = 1; c < cpp; c++) g2(t, false, p + 1 == a.parts && c + 1 == cpp);
         }
       }
       if(!ok && !*abortFlag) { *abortFlag = 1; atomicCAS(a.status, 0, PP_ERR_MMA); }
@@ -277,185 +255,186 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
     const int q = warp & 3;
     const int cg = (warp - 2) >> 2;
     const int ew = warp - 2;
-    uint8_t* sR = sStage + (size_t)ew * 3 * PP_UNIT;  // two residual / raw units, then one unit for the activated output
+    uint8_t* sR = sStage + (size_t)ew * PP_STAGE * PP_UNIT;  // residual units, from which the updated stream leaves again
     uint8_t* sO = sR + 2 * PP_UNIT;
     uint64_t* myRes = resFull + ew * 2;
-    const int U2 = a.Cn / 32;          // units of the second epilogue
+    const int U1 = a.Ct / 32, U2 = a.Cn / 32;  // units of the two epilogues
+    const int mine = (U1 - cg + PP_CG - 1) / PP_CG;  // of the first one, per tile
     const int sw64 = (lane >> 1) & 3;  // 64-byte swizzle of the staging units
-    const int sw128 = lane & 7;        // 128-byte swizzle of the operand buffer (row index modulo 8 = lane modulo 8)
     bool alive = true;
     uint32_t rs = 0;   // residual units consumed so far: ring slot rs % 2, phase (rs / 2) & 1
-    uint32_t P = 0, it = 0;
-    // the sequence of this warp's residual units: (tile, part, unit in part) with unit % PP_CG == cg
-    int nt = (int)blockIdx.x, np = 0, nj = cg - PP_CG;   // the unit before the first one
+    // the sequence of this warp's residual units: (tile, unit)
+    int nt = 0, nu = cg;
     auto fetchNext = [&](uint32_t slotSeq) {
       // an elected thread: request the residual of the next unit of this warp's sequence into ring slot slotSeq % 2
-      nj += PP_CG;
-      if(nj >= UP) { nj = cg; if(++np >= a.parts) { np = 0; nt += grid; } }
-      if(nt >= numTiles) return;
+      if(nt >= nTiles || nu >= U1) return;
       const uint32_t b = slotSeq & 1u;
       mbarExpectTx(smemU32(&myRes[b]), (uint32_t)PP_UNIT);
-      tmaLoad2d(smemU32(sR + (size_t)b * PP_UNIT), &tmS, np * a.NP + nj * 32, nt * PP_BM + q * 32, smemU32(&myRes[b]));
+      tmaLoad2d(smemU32(sR + (size_t)b * PP_UNIT), &tmS, nu * 32, ((int)blockIdx.x + nt * grid) * PP_BM + q * 32, smemU32(&myRes[b]));
+      nu += PP_CG;
+      if(nu >= U1) { nu = cg; nt++; }
     };
+    uint32_t ppUnit = 0;
+    (void)ppUnit;
     gridDepWait();
     if(electOne()) fetchNext(0);
     __syncwarp();
-    for(int t = (int)blockIdx.x; t < numTiles && alive; t += grid, it++) {
-      const int m0 = t * PP_BM;
-      const int m = m0 + q * 32 + lane;
-      const float mk = a.mask[m];
-      const bool on = mk == 1.0f;
-      // ---- first epilogue: parts of GEMM1 ----
-      for(int p = 0; p < a.parts && alive; p++, P++) {
-        PPT(threadIdx.x == 64, 512 + P * 16);
-        bool ok = mbarWait(smemU32(d1Full), P & 1u, abortFlag);
-        ok = __all_sync(0xffffffffu, ok);
-        if(!ok) { alive = false; break; }
-        PPT(threadIdx.x == 64, 512 + P * 16 + 1);
-        tcFenceAfter();
-        for(int j = cg; j < UP && alive; j += PP_CG) {
-          const uint32_t slot = rs & 1u;
-          const int uix = (j - cg) / PP_CG;
-          PPT(threadIdx.x == 64, 512 + P * 16 + 2 + uix * 6);
-          uint32_t r[32];
-          tmemLd32(tmemBase + d1Col + (uint32_t)(j * 32) + ((uint32_t)(q * 32) << 16), r);
-          // the slot of the unit after this one held this warp's store before last: it must have been read; then the
-          // next residual is requested, so that its latency hides behind this unit's arithmetic
-          if(electOne()) { bulkWaitRead0(); fetchNext(rs + 1u); }
-          __syncwarp();
-          bool landed = mbarWait(smemU32(&myRes[slot]), (rs >> 1) & 1u, abortFlag);
-          if(!__all_sync(0xffffffffu, landed)) { alive = false; break; }
-          tmemLdWait();
-          PPT(threadIdx.x == 64, 512 + P * 16 + 2 + uix * 6 + 1);
-          if(j + PP_CG >= UP) {
-            // this warp's last load of the part: the accumulator may be overwritten by the next part
-            tcFenceBefore();
+    bool on = false, onBefore = false;  // this row is a board point: in this tile, in the tile before
+    for(int t = 0; t <= nTiles && alive; t++) {
+      const int m0 = ((int)blockIdx.x + t * grid) * PP_BM;
+      onBefore = on;
+      if(t < nTiles) on = a.mask[m0 + q * 32 + lane] == 1.0f;
+      for(int j = 0; alive && (j < mine || j < 2); j++) {
+        if(j == 1 && t > 0) {
+          // ---- second epilogue, of the tile before: the next block's mid stream and its activated form ----
+          PPT(threadIdx.x == 64, 512 + ppUnit * 6);
+          bool ok = mbarWait(smemU32(d2Full), (uint32_t)(t - 1) & 1u, abortFlag);
+          if(!__all_sync(0xffffffffu, ok)) { alive = false; break; }
+          PPT(threadIdx.x == 64, 512 + ppUnit * 6 + 1);
+          tcFenceAfter();
+          for(int u = cg; u < U2; u += PP_CG) {
+            uint32_t r[32];
+            tmemLd32(tmemBase + d2Col + (uint32_t)(u * 32) + ((uint32_t)(q * 32) << 16), r);
+            tmemLdWait();
+            if(u + PP_CG >= U2) {
+              // this warp's last load: the next tile's GEMM2 may start
+              tcFenceBefore();
+              __syncwarp();
+              if(electOne()) mbarArrive(smemU32(d2Empty));
+            }
+            const int c = u * 32;
+            float2 v[16];
+#pragma unroll
+            for(int k = 0; k < 16; k++) v[k] = make_float2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
+            uint32_t rawP[16], actP[16];
+#pragma unroll
+            for(int k = 0; k < 16; k++) rawP[k] = Pack2<T>::pack(v[k].x, v[k].y);
+            {
+              const float4* sp = reinterpret_cast<const float4*>(a.scale2 + c);
+              const float4* bp = reinterpret_cast<const float4*>(a.bias2 + c);
+#pragma unroll
+              for(int hh = 0; hh < 2; hh++) {
+                float2 x[8];
+#pragma unroll
+                for(int k = 0; k < 4; k++) {
+                  const float4 s4 = __ldg(sp + 4 * hh + k), b4 = __ldg(bp + 4 * hh + k);
+                  x[2 * k] = __ffma2_rn(v[8 * hh + 2 * k], make_float2(s4.x, s4.y), make_float2(b4.x, b4.y));
+                  x[2 * k + 1] = __ffma2_rn(v[8 * hh + 2 * k + 1], make_float2(s4.z, s4.w), make_float2(b4.z, b4.w));
+                }
+                actStaged2<ACT, 8>(x);
+#pragma unroll
+                for(int k = 0; k < 8; k++) actP[8 * hh + k] = onBefore ? Pack2<T>::pack(x[k].x, x[k].y) : 0u;
+              }
+            }
+            // staging: the ring slot that does not hold the residual requested ahead, and the third unit
+            if(electOne()) bulkWaitRead0();
             __syncwarp();
-            if(electOne()) mbarArrive(smemU32(d1Empty));
-          }
-          const int c = p * a.NP + j * 32;  // first output channel of this unit
-          float2 v[16];
+            uint8_t* sRaw = sR + (size_t)((rs + 1u) & 1u) * PP_UNIT;
 #pragma unroll
-          for(int k = 0; k < 16; k++) v[k] = make_float2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
-          uint8_t* rRow = sR + (size_t)slot * PP_UNIT + lane * 64;
-#pragma unroll
-          for(int jj = 0; jj < 4; jj++) {
-            const uint4 x = *reinterpret_cast<const uint4*>(rRow + ((jj ^ sw64) << 4));
-            const uint32_t xu[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-            for(int k = 0; k < 4; k++) v[4 * jj + k] = Pack2<T>::addTo(xu[k], v[4 * jj + k]);
-          }
-          // updated stream: in place of the residual, then out by TMA
-#pragma unroll
-          for(int jj = 0; jj < 4; jj++) {
-            uint4 o;
-            o.x = Pack2<T>::pack(v[4 * jj].x, v[4 * jj].y); o.y = Pack2<T>::pack(v[4 * jj + 1].x, v[4 * jj + 1].y);
-            o.z = Pack2<T>::pack(v[4 * jj + 2].x, v[4 * jj + 2].y); o.w = Pack2<T>::pack(v[4 * jj + 3].x, v[4 * jj + 3].y);
-            *reinterpret_cast<uint4*>(rRow + ((jj ^ sw64) << 4)) = o;
-          }
-          // norm + activation + mask of the layer between the two convolutions
-          uint32_t actP[16];
-          {
-            const float4* sp = reinterpret_cast<const float4*>(a.scale1 + c);
-            const float4* bp = reinterpret_cast<const float4*>(a.bias1 + c);
-#pragma unroll
-            for(int hh = 0; hh < 2; hh++) {
-              float2 x[8];
-#pragma unroll
-              for(int k = 0; k < 4; k++) {
-                const float4 s4 = __ldg(sp + 4 * hh + k), b4 = __ldg(bp + 4 * hh + k);
-                x[2 * k] = __ffma2_rn(v[8 * hh + 2 * k], make_float2(s4.x, s4.y), make_float2(b4.x, b4.y));
-                x[2 * k + 1] = __ffma2_rn(v[8 * hh + 2 * k + 1], make_float2(s4.z, s4.w), make_float2(b4.z, b4.w));
-              }
-              actStaged2<ACT, 8>(x);
-#pragma unroll
-              for(int k = 0; k < 8; k++) actP[8 * hh + k] = on ? Pack2<T>::pack(x[k].x, x[k].y) : 0u;
+            for(int jj = 0; jj < 4; jj++) {
+              *reinterpret_cast<uint4*>(sRaw + lane * 64 + ((jj ^ sw64) << 4)) = make_uint4(rawP[4 * jj], rawP[4 * jj + 1], rawP[4 * jj + 2], rawP[4 * jj + 3]);
+              *reinterpret_cast<uint4*>(sO + lane * 64 + ((jj ^ sw64) << 4)) = make_uint4(actP[4 * jj], actP[4 * jj + 1], actP[4 * jj + 2], actP[4 * jj + 3]);
+            }
+            fenceProxyAsync();
+            __syncwarp();
+            if(electOne()) {
+              const int row = m0 - grid * PP_BM + q * 32;
+              tmaStore2d(&tmRaw2, smemU32(sRaw), c, row);
+              tmaStore2d(&tmAct2, smemU32(sO), c, row);
+              bulkCommit();
             }
           }
-          // K chunk of GEMM2 this unit belongs to: its buffer is free once the chunk two before it has been multiplied
-          const uint32_t gc = P * (uint32_t)cpp + (uint32_t)(j >> 1), abuf = gc & 1u;
-          PPT(threadIdx.x == 64, 512 + P * 16 + 2 + uix * 6 + 2);
-          {
-            bool e = mbarWait(smemU32(&a2Empty[abuf]), ((gc >> 1) & 1u) ^ 1u, abortFlag);
-            if(!__all_sync(0xffffffffu, e)) { alive = false; break; }
+          if(cg >= U2) {
+            __syncwarp();
+            if(electOne()) mbarArrive(smemU32(d2Empty));
           }
-          PPT(threadIdx.x == 64, 512 + P * 16 + 2 + uix * 6 + 3);
-          {
-            uint8_t* aRow = sA2 + (size_t)abuf * PP_CHUNK + (size_t)(q * 32 + lane) * 128;
-            const int col0 = (j & 1) * 4;
-#pragma unroll
-            for(int jj = 0; jj < 4; jj++)
-              *reinterpret_cast<uint4*>(aRow + (((col0 + jj) ^ sw128) << 4)) = make_uint4(actP[4 * jj], actP[4 * jj + 1], actP[4 * jj + 2], actP[4 * jj + 3]);
-          }
-          fenceProxyAsync();
-          __syncwarp();
-          if(electOne()) {
-            mbarArrive(smemU32(&a2Full[abuf]));
-            tmaStore2d(&tmS, smemU32(sR + (size_t)slot * PP_UNIT), c, m0 + q * 32);
-            bulkCommit();
-          }
-          PPT(threadIdx.x == 64, 512 + P * 16 + 2 + uix * 6 + 4);
-          rs++;
+          PPT(threadIdx.x == 64, 512 + ppUnit * 6 + 4);
+          ppUnit++;
         }
-      }
-      if(!alive) break;
-      // ---- second epilogue: the next block's mid stream and its activated form ----
-      {
-        PPT(threadIdx.x == 64, 512 + (P - 1) * 16 + 14);
-        bool ok = mbarWait(smemU32(d2Full), it & 1u, abortFlag);
-        ok = __all_sync(0xffffffffu, ok);
-        if(!ok) { alive = false; break; }
-        PPT(threadIdx.x == 64, 512 + (P - 1) * 16 + 15);
+        if(t == nTiles || j >= mine) continue;
+        // ---- first epilogue: unit u of GEMM1 ----
+        const int u = cg + PP_CG * j;
+        const uint32_t G = (uint32_t)(t * a.parts + u / UP);  // its part, counted over the CTA's tiles
+        const uint32_t buf = a.numD1 == 2 ? G & 1u : 0u, use = a.numD1 == 2 ? G >> 1 : G;
+        PPT(threadIdx.x == 64, 512 + ppUnit * 6);
+        bool ok = mbarWait(smemU32(&d1Full[buf]), use & 1u, abortFlag);
+        if(!__all_sync(0xffffffffu, ok)) { alive = false; break; }
         tcFenceAfter();
-        for(int j = cg; j < U2; j += PP_CG) {
-          uint32_t r[32];
-          tmemLd32(tmemBase + d2Col + (uint32_t)(j * 32) + ((uint32_t)(q * 32) << 16), r);
-          tmemLdWait();
-          const int c = j * 32;
-          float2 v[16];
-#pragma unroll
-          for(int k = 0; k < 16; k++) v[k] = make_float2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
-          uint32_t rawP[16], actP[16];
-#pragma unroll
-          for(int k = 0; k < 16; k++) rawP[k] = Pack2<T>::pack(v[k].x, v[k].y);
-          {
-            const float4* sp = reinterpret_cast<const float4*>(a.scale2 + c);
-            const float4* bp = reinterpret_cast<const float4*>(a.bias2 + c);
-#pragma unroll
-            for(int hh = 0; hh < 2; hh++) {
-              float2 x[8];
-#pragma unroll
-              for(int k = 0; k < 4; k++) {
-                const float4 s4 = __ldg(sp + 4 * hh + k), b4 = __ldg(bp + 4 * hh + k);
-                x[2 * k] = __ffma2_rn(v[8 * hh + 2 * k], make_float2(s4.x, s4.y), make_float2(b4.x, b4.y));
-                x[2 * k + 1] = __ffma2_rn(v[8 * hh + 2 * k + 1], make_float2(s4.z, s4.w), make_float2(b4.z, b4.w));
-              }
-              actStaged2<ACT, 8>(x);
-#pragma unroll
-              for(int k = 0; k < 8; k++) actP[8 * hh + k] = on ? Pack2<T>::pack(x[k].x, x[k].y) : 0u;
-            }
-          }
-          // staging: the ring slot that does not hold the residual requested ahead, and the third unit
-          if(electOne()) bulkWaitRead0();
-          __syncwarp();
-          uint8_t* rawRow = sR + (size_t)((rs + 1u) & 1u) * PP_UNIT + lane * 64;
-          uint8_t* actRow = sO + lane * 64;
-#pragma unroll
-          for(int jj = 0; jj < 4; jj++) {
-            *reinterpret_cast<uint4*>(rawRow + ((jj ^ sw64) << 4)) = make_uint4(rawP[4 * jj], rawP[4 * jj + 1], rawP[4 * jj + 2], rawP[4 * jj + 3]);
-            *reinterpret_cast<uint4*>(actRow + ((jj ^ sw64) << 4)) = make_uint4(actP[4 * jj], actP[4 * jj + 1], actP[4 * jj + 2], actP[4 * jj + 3]);
-          }
-          fenceProxyAsync();
-          __syncwarp();
-          if(electOne()) {
-            tmaStore2d(&tmRaw2, smemU32(sR + (size_t)((rs + 1u) & 1u) * PP_UNIT), c, m0 + q * 32);
-            tmaStore2d(&tmAct2, smemU32(sO), c, m0 + q * 32);
-            bulkCommit();
-          }
-        }
+        const uint32_t slot = rs & 1u;
+        uint32_t r[32];
+        tmemLd32(tmemBase + buf * (uint32_t)a.NP + (uint32_t)((u % UP) * 32) + ((uint32_t)(q * 32) << 16), r);
+        // the slot of the unit after this one held this warp's store before last: it must have been read; then the
+        // next residual is requested, so that its latency hides behind this unit's arithmetic
+        if(electOne()) { bulkWaitRead0(); fetchNext(rs + 1u); }
+        __syncwarp();
+        bool landed = mbarWait(smemU32(&myRes[slot]), (rs >> 1) & 1u, abortFlag);
+        if(!__all_sync(0xffffffffu, landed)) { alive = false; break; }
+        tmemLdWait();
+        PPT(threadIdx.x == 64, 512 + ppUnit * 6 + 1);
         tcFenceBefore();
         __syncwarp();
-        if(electOne()) mbarArrive(smemU32(d2Empty));
+        if(electOne()) mbarArrive(smemU32(&d1Empty[buf]));
+        const int c = u * 32;  // first output channel of this unit
+        float2 v[16];
+#pragma unroll
+        for(int k = 0; k < 16; k++) v[k] = make_float2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
+        uint8_t* rRow = sR + (size_t)slot * PP_UNIT + lane * 64;
+#pragma unroll
+        for(int jj = 0; jj < 4; jj++) {
+          const uint4 x = *reinterpret_cast<const uint4*>(rRow + ((jj ^ sw64) << 4));
+          const uint32_t xu[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for(int k = 0; k < 4; k++) v[4 * jj + k] = Pack2<T>::addTo(xu[k], v[4 * jj + k]);
+        }
+        // updated stream: in place of the residual, then out by TMA
+#pragma unroll
+        for(int jj = 0; jj < 4; jj++) {
+          uint4 o;
+          o.x = Pack2<T>::pack(v[4 * jj].x, v[4 * jj].y); o.y = Pack2<T>::pack(v[4 * jj + 1].x, v[4 * jj + 1].y);
+          o.z = Pack2<T>::pack(v[4 * jj + 2].x, v[4 * jj + 2].y); o.w = Pack2<T>::pack(v[4 * jj + 3].x, v[4 * jj + 3].y);
+          *reinterpret_cast<uint4*>(rRow + ((jj ^ sw64) << 4)) = o;
+        }
+        // norm + activation + mask of the layer between the two convolutions
+        uint32_t actP[16];
+        {
+          const float4* sp = reinterpret_cast<const float4*>(a.scale1 + c);
+          const float4* bp = reinterpret_cast<const float4*>(a.bias1 + c);
+#pragma unroll
+          for(int hh = 0; hh < 2; hh++) {
+            float2 x[8];
+#pragma unroll
+            for(int k = 0; k < 4; k++) {
+              const float4 s4 = __ldg(sp + 4 * hh + k), b4 = __ldg(bp + 4 * hh + k);
+              x[2 * k] = __ffma2_rn(v[8 * hh + 2 * k], make_float2(s4.x, s4.y), make_float2(b4.x, b4.y));
+              x[2 * k + 1] = __ffma2_rn(v[8 * hh + 2 * k + 1], make_float2(s4.z, s4.w), make_float2(b4.z, b4.w));
+            }
+            actStaged2<ACT, 8>(x);
+#pragma unroll
+            for(int k = 0; k < 8; k++) actP[8 * hh + k] = on ? Pack2<T>::pack(x[k].x, x[k].y) : 0u;
+          }
+        }
+        // K chunk of GEMM2 this unit belongs to: its columns are free once the chunk PP_NUM_A2 before it has been multiplied
+        const uint32_t gc = (uint32_t)(t * (U1 / 2) + u / 2), round = gc / (uint32_t)PP_NUM_A2, abuf = gc % (uint32_t)PP_NUM_A2;
+        PPT(threadIdx.x == 64, 512 + ppUnit * 6 + 2);
+        {
+          bool e = mbarWait(smemU32(&a2Empty[abuf]), (round & 1u) ^ 1u, abortFlag);
+          if(!__all_sync(0xffffffffu, e)) { alive = false; break; }
+        }
+        PPT(threadIdx.x == 64, 512 + ppUnit * 6 + 3);
+        tcFenceAfter();
+        tmemSt16(tmemBase + a2Col + abuf * PP_A2_COLS + (uint32_t)((u & 1) * 16) + ((uint32_t)(q * 32) << 16), actP);
+        tmemStWait();
+        tcFenceBefore();
+        fenceProxyAsync();
+        __syncwarp();
+        if(electOne()) {
+          mbarArrive(smemU32(&a2Full[abuf]));
+          tmaStore2d(&tmS, smemU32(sR + (size_t)slot * PP_UNIT), c, m0 + q * 32);
+          bulkCommit();
+        }
+        PPT(threadIdx.x == 64, 512 + ppUnit * 6 + 4);
+        ppUnit++;
+        rs++;
       }
     }
     if(!alive && lane == 0 && !*abortFlag) { *abortFlag = 1; atomicCAS(a.status, 0, PP_ERR_EPILOGUE); }
@@ -472,7 +451,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) convPostPreKernel(
   __syncthreads();
   if(warp == 1) {
     tcFenceAfter();
-    tmemDealloc(tmemBase, a.tmemCols);
+    tmemDealloc(tmemBase, 512);
   }
 }
 
@@ -525,23 +504,28 @@ static PostPreKernelFn postPreKernelForT(int act) {
   }
 }
 
-// Part width of GEMM1: the largest multiple of 96 channels (whole 64-channel K chunks of GEMM2 per pair of 32-channel
-// units, units divisible by the three epilogue warps of a quarter) that divides Ct and fits the tensor memory next to
-// the accumulator of GEMM2.
+// Output channels of GEMM1 per part: whole K chunks of GEMM2, and one accumulator next to GEMM2's and its operand chunks.
 static int postPrePartWidth(int Ct, int Cn) {
-  for(int np = 192; np >= 192; np -= 96)
-    if((Ct % np) == 0 && np + Cn <= 512) return np;
+  for(int np : {192, 128, 64})
+    if(Ct % np == 0 && np + Cn + PP_NUM_A2 * PP_A2_COLS <= 512) return np;
+  return 0;
+}
+// A weight slot holds a 64-channel chunk for one part of GEMM1 or as many output channels of GEMM2.
+static int postPrePieces(int Ct, int Cn) {
+  const int np = postPrePartWidth(Ct, Cn);
+  for(int i = 1; i <= 4; i++)
+    if(Cn % (16 * i) == 0 && Cn / i <= np) return i;
   return 0;
 }
 
 bool convPostPreEligible(int dt, int Cm, int Ct, int Cn) {
   if(dt != DT_F16 && dt != DT_BF16) return false;
-  if((Cm % 64) != 0 || (Cn % 96) != 0 || Cn > 256 || Cn < 96) return false;
+  if((Cm % 64) != 0 || (Ct % 64) != 0 || (Cn % 32) != 0 || Cn > 256 || Cn < 64) return false;
   const int NP = postPrePartWidth(Ct, Cn);
-  if(NP == 0) return false;
-  // shared memory: A1, two chunks of A2, three staging units per epilogue warp, two weight slots of GEMM1, one of GEMM2
-  const long fixed = (long)(Cm / 64) * PP_CHUNK + 2L * PP_CHUNK + (long)PP_EPI_WARPS * 3 * PP_UNIT + PP_FIXED;
-  return 227L * 1024 - fixed >= 3L * std::max(NP, Cn) * 128;
+  if(NP == 0 || postPrePieces(Ct, Cn) == 0) return false;
+  // shared memory: A1, the staging units of the epilogue warps, three weight slots
+  const long fixed = (long)(Cm / 64) * PP_CHUNK + (long)PP_EPI_WARPS * PP_STAGE * PP_UNIT + PP_FIXED;
+  return 227L * 1024 - fixed >= 3L * NP * 128;
 }
 
 // in1: [rows][Cm] activated mid tensor; w1: [Ct][Cm]; stream: [rows][Ct] residual stream, updated in place; w2: [Cn][Ct];
@@ -555,26 +539,22 @@ ConvPostPrePlan* convPostPreCreate(
   std::memset(&p->a, 0, sizeof(p->a));
   p->dt = dt; p->act = act1;
   PostPreArgs& a = p->a;
-  a.NP = postPrePartWidth(Ct, Cn);
-  a.Cm = Cm; a.Ct = Ct; a.Cn = Cn; a.parts = Ct / a.NP; a.kc1 = Cm / 64;
-  a.b1Slot = std::max(a.NP, Cn) * 128; a.b2Slot = a.b1Slot;
-  const long fixed = (long)a.kc1 * PP_CHUNK + 2L * PP_CHUNK + (long)PP_EPI_WARPS * 3 * PP_UNIT + PP_FIXED;
-  // what shared memory is left goes to the rings: GEMM1 first (its parts are short bursts of kc1 slots), then GEMM2
-  long left = 227L * 1024 - fixed;
-  // One ring shared by both GEMMs (numB2 = 0) keeps the most loads in flight: measured on B200 for 192 -> 384 -> 192 with
-  // three slots, shared 94 us per launch, split 2 + 1 105 us, 1 + 2 110 us.  KB_PP_RINGS="n1:n2" splits for experiments.
-  a.numB1 = (int)std::min<long>(left / a.b1Slot, 8); a.numB2 = 0;
-  if(const char* e = getenv("KB_PP_RINGS")) { int n1 = 0, n2 = 0; if(sscanf(e, "%d:%d", &n1, &n2) == 2 && n1 >= 1 && n2 >= 0 && (long)n1 * a.b1Slot + (long)n2 * a.b2Slot <= left) { a.numB1 = n1; a.numB2 = n2; } }
-  p->smemBytes = (size_t)fixed + (size_t)a.numB1 * a.b1Slot + (size_t)a.numB2 * a.b2Slot;
+  a.Cm = Cm; a.Ct = Ct; a.Cn = Cn; a.kc1 = Cm / 64;
+  a.NP = postPrePartWidth(Ct, Cn); a.parts = Ct / a.NP;
+  a.pieces = postPrePieces(Ct, Cn); a.N2 = Cn / a.pieces;
+  a.numD1 = 2 * a.NP + Cn + PP_NUM_A2 * PP_A2_COLS <= 512 ? 2 : 1;
+  a.bSlot = a.NP * 128;
+  const long fixed = (long)a.kc1 * PP_CHUNK + (long)PP_EPI_WARPS * PP_STAGE * PP_UNIT + PP_FIXED;
+  a.numB = (int)std::min<long>((227L * 1024 - fixed) / a.bSlot, PP_MAX_SLOTS);
+  p->smemBytes = (size_t)fixed + (size_t)a.numB * a.bSlot;
   const uint32_t fmt = dt == DT_F16 ? 0u : 1u;
   a.idesc1 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a.NP >> 3) << 17) | ((uint32_t)(PP_BM >> 4) << 24);
-  a.idesc2 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(Cn >> 3) << 17) | ((uint32_t)(PP_BM >> 4) << 24);
-  a.tmemCols = 512;
+  a.idesc2 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(a.N2 >> 3) << 17) | ((uint32_t)(PP_BM >> 4) << 24);
   a.scale1 = scale1; a.bias1 = bias1; a.scale2 = scale2; a.bias2 = bias2; a.mask = mask;
   const uint64_t rows = (uint64_t)rowsPadMax;
   bool ok = enc2d(&p->tmA1, dt, in1, (uint64_t)Cm, rows, (uint64_t)Cm * 2, 64, PP_BM, CU_TENSOR_MAP_SWIZZLE_128B) &&
             enc2d(&p->tmW1, dt, w1, (uint64_t)Cm, (uint64_t)Ct, (uint64_t)Cm * 2, 64, (uint32_t)a.NP, CU_TENSOR_MAP_SWIZZLE_128B) &&
-            enc2d(&p->tmW2, dt, w2, (uint64_t)Ct, (uint64_t)Cn, (uint64_t)Ct * 2, 64, (uint32_t)Cn, CU_TENSOR_MAP_SWIZZLE_128B) &&
+            enc2d(&p->tmW2, dt, w2, (uint64_t)Ct, (uint64_t)Cn, (uint64_t)Ct * 2, 64, (uint32_t)a.N2, CU_TENSOR_MAP_SWIZZLE_128B) &&
             enc2d(&p->tmS, dt, stream, (uint64_t)Ct, rows, (uint64_t)Ct * 2, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B) &&
             enc2d(&p->tmRaw2, dt, raw2, (uint64_t)Cn, rows, (uint64_t)Cn * 2, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B) &&
             enc2d(&p->tmAct2, dt, act2, (uint64_t)Cn, rows, (uint64_t)Cn * 2, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);

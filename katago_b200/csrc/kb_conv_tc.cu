@@ -958,10 +958,11 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
     // (the loops of this kernel run inside the elected threads: with all lanes in them, as in convTcKernel, chains of four
     // 192-wide layers took 1.5 to 2 % longer)
     if(electOne()) {
+      // Weights depend on nothing in the stream.  While a tile's inputs are not ready yet (the kernel before this launch, then
+      // the tile's gate) its first weight slots are requested as the ring frees them; `ahead` counts them.
       uint32_t sa = 0, phA = 0, sb = 0, phB = 0;
-      bool ok = true;
+      bool ok = true, started = false;
       int item = 0, base = 0;
-      gridDepWait();  // the chain's inputs belong to the kernels before this launch
       for(int L = 0; L < c.numLayers && ok; L++) {
         const ConvTcArgs& la = sArgs[L];
         const CUtensorMap* tmA = &layers[L].tmA;
@@ -970,9 +971,23 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
         const uint32_t aBytes = (uint32_t)la.aSlotBytes, bBytes = (uint32_t)la.bSlotBytes;
         for(int t = firstOf(base); t < numTiles && ok; t += grid, item++) {
           const int m0 = (t / numNTiles) * TC_BM, n0 = (t % numNTiles) * la.BN;
+          auto requestB = [&](int kc, int tap) {
+            const uint32_t bar = smemU32(&fullB[sb]);
+            mbarExpectTx(bar, bBytes);
+            tmaLoad2d(smemU32(smemB + (size_t)sb * c.bSlotStride), tmB, kc * TC_BK, tap * la.outC + n0, bar);
+            if(++sb == (uint32_t)c.numB) { sb = 0; phB ^= 1u; }
+          };
+          int ahead = 0;
           {
+            const int most = min(c.numB, taps);
             uint32_t spins = 0;
+            if(!started) {
+              for(; ahead < most; ahead++) requestB(0, ahead);
+              gridDepWait();  // the chain's inputs belong to the kernels before this launch
+              started = true;
+            }
             while(*gateItems <= item) {
+              if(ahead < most && mbarTestWait(smemU32(&emptyB[sb]), phB ^ 1u)) { requestB(0, ahead); ahead++; }
               if((++spins & 63u) == 0u && *abortFlag) { ok = false; break; }
             }
             if(!ok) break;
@@ -988,12 +1003,9 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
               tmaLoad2d(smemU32(smemA + (size_t)sa * c.aSlotStride), tmA, kc * TC_BK, m0 - la.haloPad, bar);
             }
             if(++sa == (uint32_t)c.numA) { sa = 0; phA ^= 1u; }
-            for(int tap = 0; tap < taps; tap++) {
+            for(int tap = kc == 0 ? ahead : 0; tap < taps; tap++) {
               if(!mbarWait(smemU32(&emptyB[sb]), phB ^ 1u, abortFlag)) { ok = false; break; }
-              const uint32_t bar = smemU32(&fullB[sb]);
-              mbarExpectTx(bar, bBytes);
-              tmaLoad2d(smemU32(smemB + (size_t)sb * c.bSlotStride), tmB, kc * TC_BK, tap * la.outC + n0, bar);
-              if(++sb == (uint32_t)c.numB) { sb = 0; phB ^= 1u; }
+              requestB(kc, tap);
             }
           }
         }

@@ -33,6 +33,18 @@ __device__ __forceinline__ uint32_t mbarTryWait(uint32_t bar, uint32_t parity) {
     : "memory");
   return ok;
 }
+// The same without waiting.
+__device__ __forceinline__ uint32_t mbarTestWait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+    "{\n\t.reg .pred p;\n\t"
+    "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+    "selp.u32 %0, 1, 0, p;\n\t}"
+    : "=r"(ok)
+    : "r"(bar), "r"(parity)
+    : "memory");
+  return ok;
+}
 __device__ __forceinline__ uint64_t globalTimerNs() {
   uint64_t t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -209,6 +221,11 @@ __device__ __forceinline__ void stGlobal32(void* p, const uint32_t (&r)[8]) {
                ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
+// Asks for a run of global memory to be brought into L2 (address and size: multiples of 16 bytes).  A hint: it orders nothing.
+__device__ __forceinline__ void l2Prefetch(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // shared -> global tile store (asynchronous, tracked by the issuing thread's bulk groups)
 __device__ __forceinline__ void tmaStore2d(const CUtensorMap* tmap, uint32_t src, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(tmap), "r"(src), "r"(c0), "r"(c1) : "memory");
@@ -252,6 +269,16 @@ __device__ __forceinline__ void ummaLoHi(uint32_t dTmem, uint32_t aLo, uint32_t 
     "setp.ne.b32 p, %5, 0;\n\t"
     "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
     ::"r"(dTmem), "r"(aLo), "r"(bLo), "r"(descHi), "r"(idesc), "r"(accumulate)
+    : "memory");
+}
+// The same with A in tensor memory: 128 lanes (rows), two 16-bit elements of K per column, aTmem = first of its 8 columns.
+__device__ __forceinline__ void ummaTmemA(uint32_t dTmem, uint32_t aTmem, uint32_t bLo, uint32_t descHi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+    "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+    "mov.b64 db, {%2, %3};\n\t"
+    "setp.ne.b32 p, %5, 0;\n\t"
+    "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+    ::"r"(dTmem), "r"(aTmem), "r"(bLo), "r"(descHi), "r"(idesc), "r"(accumulate)
     : "memory");
 }
 // mbarrier arrives once all MMAs issued so far by this thread have completed.
@@ -365,7 +392,15 @@ __device__ __forceinline__ void tmemSt32(uint32_t taddr, const uint32_t (&r)[32]
       "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
     : "memory");
 }
-// All earlier tmemSt32 of this thread have been written (needed before the thread reads those columns back).
+// 16 registers per thread -> 32 lanes x 16 consecutive columns.
+__device__ __forceinline__ void tmemSt16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+    "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+    ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+    : "memory");
+}
+// All earlier tmemSt16 / tmemSt32 of this thread have been written (needed before the thread reads those columns back).
 __device__ __forceinline__ void tmemStWait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows 128 B apart, 8-row groups

@@ -134,6 +134,35 @@ def test_small_batches_give_the_rows_of_a_full_batch(factory, prec, full, edge):
     h.close()
 
 
+@pytest.mark.parametrize("trunk,mid", [(512, 256), (256, 128), (128, 64), (320, 192), (384, 128), (192, 64)])
+@pytest.mark.parametrize("prec", [capi.PRECISION_FP16, capi.PRECISION_BF16])
+def test_fused_closing_and_opening_convolutions(trunk, mid, prec):
+    """The fused 1x1 pair at every part width (64, 128, 192 channels), with one and two accumulators of its first GEMM and weights of
+    the second in one or several pieces, at more tiles than SMs: the bits of separate launches."""
+    blob = mf.to_blob(mf.make_nbt("pair", 3, 4, trunk, mid, 32, (32, 32, 64, 96)))
+    n = 70
+    sp, gl = mf.random_positions(n, seed=5, board_sizes=([19, 13, 9, 19] * n)[:n])
+    outs = {}
+    old = os.environ.get("KB_FUSE_1X1")
+    try:
+        for mode in ("0", "1"):
+            os.environ["KB_FUSE_1X1"] = mode
+            h = capi.Handle(capi.Model(blob), n, precision=prec)
+            outs[mode] = [h.forward(sp, gl) for _ in range(3)]
+            h.profile_enable(True)
+            h.forward_resident(n)
+            assert any("fused" in e["name"] and e["launches"] for e in h.profile_read()) == (mode == "1")
+            h.close()
+    finally:
+        if old is None:
+            os.environ.pop("KB_FUSE_1X1", None)
+        else:
+            os.environ["KB_FUSE_1X1"] = old
+    for run in outs["0"] + outs["1"]:
+        for k in run:
+            assert np.array_equal(run[k], outs["0"][0][k]), k
+
+
 @pytest.mark.parametrize("n", [1, 3, 133])
 def test_host_buffers_of_every_kind(n):
     """Page-locked buffers (moved by a kernel in small calls, with or without 16-byte alignment), pageable ones and a mixture of
