@@ -71,7 +71,7 @@ struct PostPreArgs {
 // chunks of GEMM2 in shared memory it was 1.5 MB and 18.5 k cycles.  Tried on top of that and slower: parts of 128 channels with two
 // accumulators of GEMM1 (A1 is read three times instead of twice; 97 us a launch at batch 256 against 86), 24 epilogue warps with
 // units of 16 channels (97 us), outputs of GEMM2 from registers in 32-byte pieces (104 us), one reciprocal for two activations
-// (no change).  batch 256: 89.4 -> 85.8 us; 256 -> 512 -> 256 (b28, batch 512, bf16) about 245 us against 265 as two launches.
+// (no change).  batch 256: 89.4 -> 85.8 us; 256 -> 512 -> 256 (b28, batch 512, bf16) 254 us against 265 as two launches.
 //
 // The outputs of GEMM2 are read one tile late, after the warp's first unit of the next tile: nobody waits for GEMM2's last chunk
 // (1.6 k cycles a tile).  Schedule over the CTA's tiles, parts numbered through, with D accumulators for GEMM1:

@@ -1063,8 +1063,9 @@ void Engine::planPostPre() {
       op.run = [plan, status](cudaStream_t st, const Geom& g) { return launchConvPostPre(st, plan, g, status); };
       op.members.assign(ops_.begin() + (long)i, ops_.begin() + (long)i + 2);
       // Past 96-wide tiles the pair is the better choice: b18 at 28 boards 1139 us with fused pairs, 1155 with 128-wide members;
-      // at 37 boards 1340 against 1502 with 192-wide ones
-      op.singlyUpTo = 96;
+      // at 37 boards 1340 against 1502 with 192-wide ones.  A 512-channel pair takes longer for its one tile: b28 at 20 boards 2009
+      // fused, 1905 with 128-wide members; at 32 2858 fused, 2948 with 192-wide ones.
+      op.singlyUpTo = ops_[i].convOutC >= 512 ? 128 : 96;
       out.push_back(std::move(op));
       i += 2;
     }
