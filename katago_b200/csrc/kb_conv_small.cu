@@ -27,8 +27,6 @@
 #include "kb_conv_small.cuh"
 
 #include <algorithm>
-#include <cstdio>
-#include <cstdlib>
 #include <type_traits>
 
 namespace kb {
@@ -40,14 +38,45 @@ constexpr int CS_EPI_WARPS = 12;                    // three per TMEM lane quart
 constexpr int CS_PARTS = CS_EPI_WARPS / 4;
 constexpr int CS_THREADS = 64 + 32 * CS_EPI_WARPS;  // producer warp, MMA warp, epilogue warps
 constexpr int CS_MAX_SLOTS = 32;
-constexpr int CS_MAX_BN = 192;
+constexpr int CS_MAX_BN = 256;
 // barriers (full and empty of both rings, accumulator), the TMEM slot and flags, the norm parameters of the tile, and the
 // slack of the 1024-byte alignment
 constexpr int CS_FIXED_SMEM = (4 * CS_MAX_SLOTS + 1) * 8 + 64 + 2 * CS_MAX_BN * 4 + 1024;
 // Shared memory of a CTA: half of an SM's (228 KB, 1 KB reserved per CTA) or all of it
 constexpr int CS_SMEM_HALF = 113 * 1024, CS_SMEM_FULL = 226 * 1024;
 
+// Kernel variant that records the sums of squares of its raw output (Epilogue::sumsqOut) and has no activated one.
+constexpr int CS_ACT_ROW_SUMS = 102;
+
 enum { CS_ERR_PRODUCER_TIMEOUT = 121, CS_ERR_MMA_TIMEOUT = 122, CS_ERR_EPILOGUE_TIMEOUT = 123 };
+
+// Sum of the partials that the small-batch kernel wrote for row m, twelve loads at a time (a 384-channel row).
+__device__ __forceinline__ float rowSumOfUnits(const float* sums, int stride, int slots, uint32_t ends, int m) {
+  float ss = 0.0f, part = 0.0f;
+  for(int k0 = 0; k0 < slots; k0 += 12) {
+    float t[12];
+#pragma unroll
+    for(int k = 0; k < 12; k++) t[k] = sums[(size_t)min(k0 + k, slots - 1) * stride + m];
+#pragma unroll
+    for(int k = 0; k < 12; k++) {
+      // past the last slot no group ends
+      part += t[k];
+      const bool end = k0 + k < 32 && ((ends >> ((k0 + k) & 31)) & 1u);
+      ss += end ? part : 0.0f;
+      part = end ? 0.0f : part;
+    }
+  }
+  return ss;
+}
+// The factor of a row-normalised convolution (Epilogue::rowSumsq) for row m, whose mask is mk; 1 without one.
+__device__ __forceinline__ float rowNormScale(const Epilogue& ep, int m, float mk) {
+  if(!ep.rowSumsq) return 1.0f;
+  float ss = 0.0f;
+  if(ep.rowSumsqEnds != 0u) ss = rowSumOfUnits(ep.rowSumsq, ep.sumsqRowStride, ep.rowSumsqSlots, ep.rowSumsqEnds, m);
+  else
+    for(int k = 0; k < ep.rowSumsqSlots; k++) ss += ep.rowSumsq[(size_t)k * ep.sumsqRowStride + m];
+  return mk == 1.0f ? rsqrtf(fmaf(ss, ep.rowInvC, ep.rowEps)) : 0.0f;
+}
 
 struct ConvSmallArgs {
   Geom g;
@@ -61,6 +90,7 @@ struct ConvSmallArgs {
   int numA, numB;  // ring depths
   uint32_t idesc, tmemCols;
   int* status;
+  uint8_t sumRank[32];  // row sums: slot of each 32-channel unit (rowSumRank; a table, as its divisions took 0.5 us)
 };
 
 template <typename T, int ACT, int BM>
@@ -110,6 +140,10 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
       sScale[i] = in ? ep.scale[ca] : 0.0f;
       sBias[i] = in ? ep.bias[ca] : 0.0f;
     }
+  }
+  if(ACT == KB_ACT_ROPE_QK && warp >= 2) {
+    // rotary frequencies of this tile's query and key channels
+    for(int i = (int)threadIdx.x - 64; i < a.BN; i += CS_THREADS - 64) sScale[i] = n0 + i < ep.ropeC1 ? ep.ropeFreq[n0 + i] : 0.0f;
   }
   tcFenceBefore();
   __syncthreads();
@@ -211,24 +245,39 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
     // ---------------- Epilogue: TMEM lane quarter = warp % 4; three warps per quarter take the 16-channel units in turn ----------------
     // A thread owns 16 channels of a row: 32 bytes, a whole sector, in one access per tensor.  A 64-row accumulator lies in
     // the first 16 lanes of each quarter.
-    constexpr int QROWS = BM / 4;
+    // Row sums and SwiGLU go by 32 channels: a warp then takes both 16-channel halves in turn.
+    constexpr int QROWS = BM / 4, HALVES = (ACT == CS_ACT_ROW_SUMS || ACT == KB_ACT_SWIGLU_PAIRS) ? 2 : 1;
     const int q = warp & 3, part = (warp - 2) >> 2;
     const bool row = lane < QROWS;
     const int m = m0 + q * QROWS + (lane & (QROWS - 1));
-    const int units = min(a.BN, a.outC - n0) / 16;
+    const int units = min(a.BN, a.outC - n0) / (16 * HALVES);
     gridDepWait();
     const float mk = ep.mask ? ep.mask[m] : 1.0f;
     const bool on = mk == 1.0f;
     const int bIdx = min(m / a.g.PB, a.g.n - 1);
     const float* biasRow = ep.biasNC ? ep.biasNC + (size_t)bIdx * a.outC + n0 : nullptr;
     const T* resRow = ep.residual ? reinterpret_cast<const T*>(ep.residual) + (size_t)m * ep.resStride + n0 : nullptr;
-    // The residual of the warp's first two units is on its way while the MMAs run (loads behind them wait their turn among the
-    // operand copies of the SM's other CTA: b28 at twelve positions 1622 us with one unit ahead, 1599 with two), that of a third
-    // while the first is computed.  64-row tiles are so narrow that a warp has one unit.
-    constexpr bool AHEAD = BM == 128;
+    // This warp's 16-channel pieces in order: piece i is number (part + CS_PARTS * (i / HALVES)) * HALVES + i % HALVES of the tile.
+    const int pieces = part < units ? ((units - 1 - part) / CS_PARTS + 1) * HALVES : 0;
+    auto pieceAt = [&](int i) { return (part + CS_PARTS * (i / HALVES)) * HALVES + i % HALVES; };
+    const float rowScale = rowNormScale(ep, m, mk);
+    // rotary embedding: this thread's board point; rows that are not board points turn by the angle of (0,0), which is 0
+    float ropePx = 0.0f, ropePy = 0.0f;
+    if(ACT == KB_ACT_ROPE_QK) {
+      const int br = m % a.g.PB, y = br / a.g.RW, x = br - y * a.g.RW;
+      if(y < a.g.Y && x < a.g.X) { ropePx = (float)x; ropePy = (float)y; }
+    }
+    // slots of the row sums of this warp's first two units, read while the MMAs run
+    const int slot0 = ACT == CS_ACT_ROW_SUMS ? a.sumRank[(n0 / 32 + part) & 31] : 0;
+    const int slot1 = ACT == CS_ACT_ROW_SUMS ? a.sumRank[(n0 / 32 + part + CS_PARTS) & 31] : 0;
+    float2 held[ACT == KB_ACT_SWIGLU_PAIRS ? 8 : 2];  // SwiGLU: silu of the unit's first half; row sums: the two running sums
+    // The residual of the warp's first two pieces is on its way while the MMAs run (loads behind them wait their turn among the
+    // operand copies of the SM's other CTA: b28 at twelve positions 1622 us with one piece ahead, 1599 with two), that of a third
+    // while the first is computed.  64-row tiles are so narrow that a warp has one piece (two with row sums).
+    constexpr bool AHEAD = BM == 128 || HALVES == 2;
     uint32_t res[8] = {0, 0, 0, 0, 0, 0, 0, 0}, resNext[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if(resRow && row && part < units) ldGlobal32(resRow + part * 16, res);
-    if(AHEAD && resRow && row && part + CS_PARTS < units) ldGlobal32(resRow + (part + CS_PARTS) * 16, resNext);
+    if(resRow && row && pieces > 0) ldGlobal32(resRow + pieceAt(0) * 16, res);
+    if(AHEAD && resRow && row && pieces > 1) ldGlobal32(resRow + pieceAt(1) * 16, resNext);
     bool ok = mbarWait(accFull, 0u, abortFlag);
     ok = __all_sync(0xffffffffu, ok);
     if(!ok) {
@@ -237,8 +286,8 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
     else {
       tcFenceAfter();
 #pragma unroll 1
-      for(int u = part; u < units; u += CS_PARTS) {
-        const int c = n0 + u * 16;
+      for(int i = 0; i < pieces; i++) {
+        const int u = pieceAt(i), c = n0 + u * 16;
         uint32_t r[16];
         tmemLd16(tmemBase + ((uint32_t)(q * 32) << 16) + (uint32_t)(u * 16), r);
         tmemLdWait();
@@ -246,6 +295,11 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
         float2 v[8];
 #pragma unroll
         for(int k = 0; k < 8; k++) v[k] = make_float2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
+        if(ep.rowSumsq) {
+          const float2 rs = make_float2(rowScale, rowScale);
+#pragma unroll
+          for(int k = 0; k < 8; k++) v[k] = __fmul2_rn(v[k], rs);
+        }
         if(biasRow) {
           const float4* bp = reinterpret_cast<const float4*>(biasRow + u * 16);
 #pragma unroll
@@ -266,17 +320,55 @@ __global__ void __launch_bounds__(CS_THREADS, 2) convSmallKernel(
           if(AHEAD) {
 #pragma unroll
             for(int k = 0; k < 8; k++) res[k] = resNext[k];
-            if(row && u + 2 * CS_PARTS < units) ldGlobal32(resRow + (u + 2 * CS_PARTS) * 16, resNext);
+            if(row && i + 2 < pieces) ldGlobal32(resRow + pieceAt(i + 2) * 16, resNext);
           }
-          else if(row && u + CS_PARTS < units) ldGlobal32(resRow + (u + CS_PARTS) * 16, res);
+          else if(row && i + 1 < pieces) ldGlobal32(resRow + pieceAt(i + 1) * 16, res);
+        }
+        if(ACT == KB_ACT_ROPE_QK && c < ep.ropeC1) {
+          const float4* fq = reinterpret_cast<const float4*>(sScale + u * 16);
+#pragma unroll
+          for(int k = 0; k < 4; k++) {
+            const float4 f = fq[k];
+            float sn0, cs0, sn1, cs1;
+            __sincosf(fmaf(ropePy, f.y, ropePx * f.x), &sn0, &cs0);
+            __sincosf(fmaf(ropePy, f.w, ropePx * f.z), &sn1, &cs1);
+            const float2 t0 = v[2 * k], t1 = v[2 * k + 1];
+            v[2 * k] = make_float2(t0.x * cs0 - t0.y * sn0, t0.x * sn0 + t0.y * cs0);
+            v[2 * k + 1] = make_float2(t1.x * cs1 - t1.y * sn1, t1.x * sn1 + t1.y * cs1);
+          }
         }
         uint32_t o[8];
+        if(ACT == CS_ACT_ROW_SUMS && c >= ep.rawC0 && c < ep.rawC1) {
+          if((i & 1) == 0) { held[0] = make_float2(0.0f, 0.0f); held[1] = make_float2(0.0f, 0.0f); }
+#pragma unroll
+          for(int k = 0; k < 8; k++) held[k & 1] = __ffma2_rn(v[k], v[k], held[k & 1]);
+          if((i & 1) == 1 && row) ep.sumsqOut[(size_t)(i < 2 ? slot0 : i < 4 ? slot1 : a.sumRank[c / 32]) * ep.sumsqRowStride + m] = (held[0].x + held[0].y) + (held[1].x + held[1].y);
+        }
         if(ep.outRaw && c >= ep.rawC0 && c < ep.rawC1) {
 #pragma unroll
           for(int k = 0; k < 8; k++) o[k] = Pack2<T>::pack(v[k].x, v[k].y);
           if(row) stGlobal32(reinterpret_cast<T*>(ep.outRaw) + (size_t)m * ep.rawStride + (c - ep.rawC0), o);
         }
-        if(ep.outAct && c >= ep.actC0 && c < ep.actC1) {
+        if(ACT == KB_ACT_SWIGLU_PAIRS) {
+          // pieces alternate between 16 "up" channels and their 16 "gate" channels: h = silu(up) * gate
+          if(ep.outAct && c >= ep.actC0 && c < ep.actC1) {
+            if((i & 1) == 0) {
+              const float2 kk2 = make_float2(-1.4426950408889634f, -1.4426950408889634f), one2 = make_float2(1.0f, 1.0f);
+#pragma unroll
+              for(int k = 0; k < 8; k++) {
+                float2 n = __fmul2_rn(v[k], kk2);
+                n = __fadd2_rn(one2, make_float2(ex2Approx(n.x), ex2Approx(n.y)));
+                held[k % (sizeof(held) / sizeof(float2))] = __fmul2_rn(v[k], make_float2(rcpApprox(n.x), rcpApprox(n.y)));
+              }
+            }
+            else {
+#pragma unroll
+              for(int k = 0; k < 8; k++) { const float2 h = __fmul2_rn(held[k % (sizeof(held) / sizeof(float2))], v[k]); o[k] = Pack2<T>::pack(h.x, h.y); }
+              if(row) stGlobal32(reinterpret_cast<T*>(ep.outAct) + (size_t)m * ep.actStride + (c - 16 - ep.actC0) / 2, o);
+            }
+          }
+        }
+        else if(ep.outAct && c >= ep.actC0 && c < ep.actC1) {
           const float4* sp = reinterpret_cast<const float4*>(sScale + u * 16);
           const float4* bp = reinterpret_cast<const float4*>(sBias + u * 16);
 #pragma unroll
@@ -321,6 +413,9 @@ ConvSmallKernelFn smallKernelForT(int act) {
     case KB_ACT_MISH: return convSmallKernel<T, KB_ACT_MISH, BM>;
     case KB_ACT_SILU: return convSmallKernel<T, KB_ACT_SILU, BM>;
     case KB_ACT_MISH_SCALE8: return convSmallKernel<T, KB_ACT_MISH_SCALE8, BM>;
+    case KB_ACT_SWIGLU_PAIRS: return convSmallKernel<T, KB_ACT_SWIGLU_PAIRS, BM>;
+    case KB_ACT_ROPE_QK: return convSmallKernel<T, KB_ACT_ROPE_QK, BM>;
+    case CS_ACT_ROW_SUMS: return convSmallKernel<T, CS_ACT_ROW_SUMS, BM>;
     default: return nullptr;
   }
 }
@@ -329,16 +424,24 @@ ConvSmallKernelFn smallKernelFor(int dt, int act) {
   return dt == DT_F16 ? smallKernelForT<__half, BM>(act) : smallKernelForT<__nv_bfloat16, BM>(act);
 }
 
+// The kernel's variant for an epilogue, or -1.
+int smallVariant(const Epilogue& ep) {
+  if(ep.sumsqOut) return !ep.outAct && ep.act != KB_ACT_ROPE_QK ? CS_ACT_ROW_SUMS : -1;
+  if(ep.act == KB_ACT_ROPE_QK) return !ep.outAct ? KB_ACT_ROPE_QK : -1;
+  if(ep.act == KB_ACT_SWIGLU_PAIRS) return ep.outAct && !ep.outRaw ? KB_ACT_SWIGLU_PAIRS : -1;
+  return ep.outAct ? ep.act : KB_ACT_IDENTITY;
+}
+
 }  // namespace
 
 bool convSmallSupports(const Epilogue& ep) {
-  if(ep.sumsqOut || ep.rowSumsq || ep.act == KB_ACT_SWIGLU_PAIRS || ep.act == KB_ACT_ROPE_QK) return false;
   // an epilogue thread moves 16 channels of a row in one 32-byte access
   auto sectors = [](const void* p, int stride) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0 && stride % 16 == 0; };
   if(ep.outRaw && !sectors(ep.outRaw, ep.rawStride)) return false;
   if(ep.outAct && !sectors(ep.outAct, ep.actStride)) return false;
   if(ep.residual && !sectors(ep.residual, ep.resStride)) return false;
-  return !ep.outAct || smallKernelFor<128>(DT_F16, ep.act) != nullptr;
+  const int variant = smallVariant(ep);
+  return variant >= 0 && smallKernelFor<128>(DT_F16, variant) != nullptr;
 }
 
 // Which tile a launch takes.  Device time of the whole net, fp16, 19x19, in us; wide = the kernels of kb_conv_tc.cu / kb_conv_fused.cu.
@@ -357,24 +460,19 @@ bool convSmallSupports(const Epilogue& ep) {
 // 128 x 96 1305, wide 1441; b28 at 30 128 x 96 2728, wide 3283; at 40 128 x 128 3059, wide 3404.  192-wide 3x3 tiles with half an SM
 // have two weight slots and are slower than the wide kernels (b18 at 48: 2353 against 1794).
 //
+// The projections of a transformer follow the same rules, with tiles of whole 32-channel units where row sums or SwiGLU pairs
+// need them.  Producers of row sums keep to one CTA per SM (12-layer transformer, 32 boards: 1252 us with wide tiles, 1345 with
+// 192-wide ones on shared SMs); the up|gate projection takes 256-wide tiles on shared SMs (11 boards, relative-position bias: 695
+// us against 753 with 192-wide ones, wide 783) and, past those, up to one and a half rounds of 192-wide ones (12 boards 704, wide
+// 768).  Plain transformer at 1 / 4 / 8 / 16 boards: 570 -> 367, 586 -> 417, 665 -> 519, 808 (wide).
+//
 // Weight slots of three taps where a wait is a good part of a slot's MMAs (b18, twelve positions, N = 64: 823 against 848 with one
 // tap), of one tap for wide tiles with half an SM (b18, 37 positions, N = 96: 1340 against 1589 with three).
-ConvSmallTile convSmallTile(const ConvSmallShape& s, int rows, int numSMs) {
-  if(const char* e = getenv("KB_SMALL_TILE")) {
-    // "taps:inC:outC=BM:BN:half:group,..."
-    const char* p = e;
-    while(*p) {
-      int tp, ic, oc, bm, bn, hf, gp, used = 0;
-      if(sscanf(p, "%d:%d:%d=%d:%d:%d:%d%n", &tp, &ic, &oc, &bm, &bn, &hf, &gp, &used) == 7) {
-        if(tp == s.taps && ic == s.inC && oc == s.outC) return ConvSmallTile{bm, bn, gp, hf ? CS_SMEM_HALF : CS_SMEM_FULL};
-        p += used;
-      }
-      while(*p && *p != ',') p++;
-      if(*p == ',') p++;
-    }
-  }
+ConvSmallTile convSmallTile(const ConvSmallShape& s, const Epilogue& ep, int rows, int numSMs) {
   const int slot = s.taps == 9 ? 3 : 1;
-  auto tiles = [&](int bm, int bn) { return (long long)((rows + bm - 1) / bm) * ((s.outC + bn - 1) / bn); };
+  // row sums and SwiGLU go by 32 channels
+  const int unit = ep.sumsqOut || ep.act == KB_ACT_SWIGLU_PAIRS ? 32 : 16;
+  auto tiles = [&](int bm, int bn) { return bn % unit != 0 ? 1LL << 40 : (long long)((rows + bm - 1) / bm) * ((s.outC + bn - 1) / bn); };
   // one CTA per SM
   if(s.taps == 9 || s.inC > 256) {
     const int shapes[][2] = {{64, 32}, {64, 48}, {128, 32}, {128, 48}, {128, 64}, {128, 96}, {128, 128}};
@@ -382,9 +480,12 @@ ConvSmallTile convSmallTile(const ConvSmallShape& s, int rows, int numSMs) {
       if(tiles(t[0], t[1]) <= numSMs) return ConvSmallTile{t[0], t[1], slot, CS_SMEM_FULL};
   }
   // two CTAs per SM
+  if(ep.sumsqOut) return ConvSmallTile{};  // see above
   if(s.taps == 1 && tiles(64, 16) <= 2LL * numSMs) return ConvSmallTile{64, 16, 1, CS_SMEM_HALF};
   for(int bn : {16, 32, 48, 64, 96, 128, 192})
     if((s.taps == 1 || bn < 192) && tiles(128, bn) <= 2LL * numSMs) return ConvSmallTile{128, bn, s.taps == 9 && bn < 64 ? 3 : 1, CS_SMEM_HALF};
+  if(ep.act == KB_ACT_SWIGLU_PAIRS && tiles(128, 256) <= 2LL * numSMs) return ConvSmallTile{128, 256, 1, CS_SMEM_HALF};
+  if(ep.act == KB_ACT_SWIGLU_PAIRS && tiles(128, 192) <= 3LL * numSMs) return ConvSmallTile{128, 192, 1, CS_SMEM_HALF};
   return ConvSmallTile{};
 }
 
@@ -429,7 +530,8 @@ cudaError_t launchConvSmall(cudaStream_t st, const ConvSmallShape& s, const Conv
   a.tmemCols = 32;
   while((int)a.tmemCols < BN) a.tmemCols *= 2;
   a.status = statusWord;
-  const int act = ep.outAct ? ep.act : KB_ACT_IDENTITY;
+  for(int u = 0; u < 32; u++) a.sumRank[u] = ep.sumsqOut ? (uint8_t)rowSumRank(u, ep.sumsqTile, ep.sumsqWarps) : 0;
+  const int act = smallVariant(ep);
   ConvSmallKernelFn fn = BM == 64 ? smallKernelFor<64>(s.dt, act) : smallKernelFor<128>(s.dt, act);
   if(!fn) return cudaErrorInvalidValue;
   if(const cudaError_t e = allowSharedMemory((const void*)fn, CS_SMEM_FULL)) return e;

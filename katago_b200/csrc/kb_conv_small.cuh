@@ -7,7 +7,7 @@
 namespace kb {
 
 // Tile widths the kernel is launched with.
-constexpr int CONV_SMALL_WIDTHS[] = {16, 32, 48, 64, 96, 128, 192};
+constexpr int CONV_SMALL_WIDTHS[] = {16, 32, 48, 64, 96, 128, 192, 256};
 constexpr int CONV_SMALL_NUM_WIDTHS = sizeof(CONV_SMALL_WIDTHS) / sizeof(int);
 inline int convSmallMapIndex(int BN) {
   for(int i = 0; i < CONV_SMALL_NUM_WIDTHS; i++)
@@ -30,9 +30,9 @@ struct ConvSmallTile {
   int BM = 0, BN = 0, tapGroup = 1, smem = 0;
 };
 
-// True if the kernel has a variant for this epilogue (staged-epilogue convolutions without row sums).
+// True if the kernel has a variant for this epilogue (of a convolution whose wide-tile form has the staged epilogue).
 bool convSmallSupports(const Epilogue& ep);
-ConvSmallTile convSmallTile(const ConvSmallShape& s, int rows, int numSMs);
+ConvSmallTile convSmallTile(const ConvSmallShape& s, const Epilogue& ep, int rows, int numSMs);
 cudaError_t launchConvSmall(cudaStream_t st, const ConvSmallShape& s, const ConvSmallTile& tile, Geom g, const Epilogue& ep, int* statusWord);
 
 }  // namespace kb

@@ -1296,6 +1296,8 @@ struct ConvTcPlan {
   CUtensorMap tmRes, tmRaw, tmAct;
   int smallMaps;  // the weight maps of the small-batch kernel exist
   int small;  // the small-batch kernel (kb_conv_small.cu) can run this convolution
+  Epilogue ep;  // as given to convTcSetEpilogue
+  std::vector<const ConvTcPlan*> rowSumsTo;  // the convolutions that read its row sums
   ConvSmallShape smallShape;
 };
 
@@ -1478,8 +1480,13 @@ ConvTcPlan* convTcCreate(
 // and the number of rows alone, so that every launch of a batch size takes the same route.
 static ConvSmallTile smallTile(const ConvTcPlan* p, const Geom& g) {
   static const bool off = getenv("KB_NO_SMALL") != nullptr && atoi(getenv("KB_NO_SMALL")) != 0;
-  return p->small && !off ? convSmallTile(p->smallShape, g.rows, p->numSMs) : ConvSmallTile{};
+  if(!p->small || off) return ConvSmallTile{};
+  // the wide-tile kernels read row sums in their own form only
+  for(const ConvTcPlan* c : p->rowSumsTo)
+    if(smallTile(c, g).BM == 0) return ConvSmallTile{};
+  return convSmallTile(p->smallShape, p->ep, g.rows, p->numSMs);
 }
+void convTcLinkRowSums(ConvTcPlan* producer, const ConvTcPlan* consumer) { producer->rowSumsTo.push_back(consumer); }
 int convTcSmallWidth(const ConvTcPlan* p, const Geom& g) { return p ? smallTile(p, g).BN : 0; }
 
 void convTcDestroy(ConvTcPlan* p) { delete p; }
@@ -1488,7 +1495,7 @@ void convTcDestroy(ConvTcPlan* p) { delete p; }
 // multiple of 32 channels the residual is fetched and the outputs are written by TMA through swizzled
 // shared-memory units; otherwise the epilogue threads access global memory directly.
 bool convTcSetEpilogue(ConvTcPlan* p, const Epilogue& ep) {
-  p->tmaEpi = 0; p->cg = TC_EPI_CG; p->small = 0;
+  p->tmaEpi = 0; p->cg = TC_EPI_CG; p->small = 0; p->ep = ep;
   const bool force = getenv("KB_TC_NO_TMA_EPI") != nullptr && atoi(getenv("KB_TC_NO_TMA_EPI")) != 0;
   auto aligned32 = [](int c0, int c1) { return (c0 % 32) == 0 && (c1 % 32) == 0 && c1 > c0; };
   bool ok = !force && (p->BN % 32) == 0 && p->BN <= 256;
@@ -1546,7 +1553,7 @@ bool convTcSetEpilogue(ConvTcPlan* p, const Epilogue& ep) {
   if(!enc) { p->cg = TC_EPI_CG; return needsStaged ? false : sizeRings(p, 0); }
   p->tmaEpi = 1;
   // the small-batch kernel repeats the arithmetic of the staged epilogue
-  p->small = p->smallMaps && convSmallSupports(ep) ? 1 : 0;
+  p->small = p->smallMaps && convSmallSupports(ep) && !(ep.sumsqOut && p->outC > 32 * 32) ? 1 : 0;
   return true;
 }
 
@@ -1567,7 +1574,23 @@ int convTcGridSize(const ConvTcPlan* p, const Geom& g) {
   return p->pair ? 2 * units : units;
 }
 
-cudaError_t launchConvTc(cudaStream_t st, const ConvTcPlan* p, Geom g, const Epilogue& ep, int* statusWord, const ConvTcDeps* deps) {
+// The slots (rowSumRank) at which a consumer of the small-batch kernel's partials has a whole slot of the wide-tile kernels'.
+static uint32_t rowSumEnds(const ConvTcPlan* p) {
+  const int tile = p->BN / 32;
+  uint32_t ends = 0;
+  for(int unit = 0; unit < p->outC / 32; unit++)
+    if(unit % tile + p->cg >= tile) ends |= 1u << rowSumRank(unit, tile, p->cg);
+  return ends;
+}
+
+cudaError_t launchConvTc(cudaStream_t st, const ConvTcPlan* p, Geom g, const Epilogue& epGiven, int* statusWord, const ConvTcDeps* deps) {
+  Epilogue ep = epGiven;
+  if(ep.rowSumsq && ep.rowSumsqFrom && convTcSmallWidth(ep.rowSumsqFrom, g) > 0) {
+    ep.rowSumsqSlots = ep.rowSumsqFrom->outC / 32;
+    ep.rowSumsqEnds = rowSumEnds(ep.rowSumsqFrom);
+  }
+  ep.sumsqTile = (uint8_t)(p->BN / 32);
+  ep.sumsqWarps = (uint8_t)p->cg;
   // vector accesses in the epilogue need 16-byte aligned rows and 16-channel aligned ranges
   if(ep.outRaw && ((ep.rawStride % 8) || (ep.rawC0 % 16) || (ep.rawC1 % 16))) return cudaErrorInvalidValue;
   if(ep.outAct && ((ep.actStride % 8) || (ep.actC0 % 16) || (ep.actC1 % 16) || ((ep.actC1 - ep.actC0) > CONV_TC_MAX_ACT && ep.act != KB_ACT_SWIGLU_PAIRS))) return cudaErrorInvalidValue;

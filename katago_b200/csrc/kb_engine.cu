@@ -252,7 +252,9 @@ void Engine::addConvOp(const ConvDev& c, Epilogue ep, const std::string& tag) {
       const int slots = convTcPlanRowSumSlots(c.plan);
       if(slots < 1 || slots > rowSumsSlotsMax_) throw std::runtime_error("internal: row-sum slots of a convolution exceed the buffer");
       rowSumsCur_ = slots;
+      rowSumsFrom_ = c.plan;
     }
+    if(ep.rowSumsq && ep.rowSumsqFrom) convTcLinkRowSums(ep.rowSumsqFrom, c.plan);
     const ConvTcPlan* plan = c.plan;
     std::shared_ptr<ConvTcDeps> deps = std::make_shared<ConvTcDeps>();
     addOp(name, flops, bytes, [plan, ep, status, deps](cudaStream_t st, const Geom& g) { return launchConvTc(st, plan, g, ep, status, deps.get()); });
@@ -576,7 +578,7 @@ void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* 
       // the norm is folded into the projection: it reads the stream itself and scales its rows
       foldGain(qkvW, b.preLN.weight);
       ConvDev cq = makeConv({&qkvW}, raw, C, C);
-      eq.rowSumsq = rowSums_; eq.rowSumsqSlots = rowSumsCur_; eq.sumsqRowStride = rowsPadMax_; eq.rowInvC = 1.0f / (float)C; eq.rowEps = eps;
+      eq.rowSumsq = rowSums_; eq.rowSumsqSlots = rowSumsCur_; eq.rowSumsqFrom = rowSumsFrom_; eq.sumsqRowStride = rowsPadMax_; eq.rowInvC = 1.0f / (float)C; eq.rowEps = eps;
       ropeEpilogue(cq);
       addConvOp(cq, eq, ropeInProjection ? "norm+qkv+rope" : "norm+qkv");
     }
@@ -661,7 +663,7 @@ void Engine::emitBlock(const BlockW& b, int C, void* raw, void* act, const BNW* 
     if(foldNorm) foldGain(upW, b.preLN.weight);
     ConvDev cu = makeConv({&upW}, ffnIn, C, C);
     Epilogue eu;
-    if(foldNorm) { eu.rowSumsq = rowSums_; eu.rowSumsqSlots = rowSumsCur_; eu.sumsqRowStride = rowsPadMax_; eu.rowInvC = 1.0f / (float)C; eu.rowEps = eps; }
+    if(foldNorm) { eu.rowSumsq = rowSums_; eu.rowSumsqSlots = rowSumsCur_; eu.rowSumsqFrom = rowSumsFrom_; eu.sumsqRowStride = rowsPadMax_; eu.rowInvC = 1.0f / (float)C; eu.rowEps = eps; }
     if(fuseSwiglu) {
       // one kernel: the projection's epilogue writes silu(up) * gate; the 2F-wide intermediate never reaches memory
       if(!cu.tc) throw std::runtime_error("internal: fused SwiGLU projection is not on the tensor-core path");

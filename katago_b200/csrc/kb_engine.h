@@ -122,6 +122,7 @@ class Engine {
   // stream leaves per-row partial sums of squares, the consuming projection turns them into its row scale.
   float* rowSums_ = nullptr;   // [slot][rowsPadMax] partial sums of squares of the current stream's rows
   int rowSumsSlotsMax_ = 0;
+  ConvTcPlan* rowSumsFrom_ = nullptr;  // the convolution that writes the row sums at this point of the launch list
   int rowSumsCur_ = -1;        // number of slots the current stream's producer filled, or -1: no sums available
   bool rowNormFold_ = false;
   void produceRowSums(Epilogue& ep, int k, int inC, int outC);

@@ -74,9 +74,16 @@ struct Epilogue {
   // on any ordering.  A consumer adds rowSumsqSlots partials in slot order and multiplies each accumulator row by
   // rsqrt(sum/C + eps) (0 where the mask is 0) before anything else; with the norm's gain folded into its weights that
   // equals conv(rmsnorm(x)).  convTcRowSumSlots gives the producer's slot count.
+  // The small-batch kernel writes one partial per unit of 32 channels, in an order (rowSumRank, from the wide tile's units
+  // sumsqTile and its warps sumsqWarps) in which those of one slot of the wide-tile kernels follow each other; rowSumsqEnds marks
+  // where they end.  A consumer adds them slot by slot first, so the sums are the same bits.  launchConvTc fills these in, by
+  // what rowSumsqFrom, the producer, runs as in the batch at hand; it runs in small tiles only where all its consumers do.
   float* sumsqOut = nullptr;
   const float* rowSumsq = nullptr;
   int rowSumsqSlots = 0;
+  struct ConvTcPlan* rowSumsqFrom = nullptr;
+  uint32_t rowSumsqEnds = 0;
+  uint8_t sumsqTile = 0, sumsqWarps = 0;
   int sumsqRowStride = 0;
   float rowInvC = 0.0f, rowEps = 0.0f;
   // act == KB_ACT_ROPE_QK: output channels [0, ropeC1) are the query and key heads (ropeC1 <= 1024, a multiple of 32).
@@ -105,6 +112,15 @@ struct TransferList {
   }
 };
 cudaError_t launchTransfers(cudaStream_t st, const TransferList& list);
+
+// Place of a 32-channel unit among the row-sum partials of the small-batch kernel: tile by tile of `tile` units, warp by warp
+// (a wide tile's units go to its `warps` warps in turn).
+inline int rowSumRank(int unit, int tile, int warps) {
+  const int r = unit % tile;
+  int rank = unit - r + r / warps;
+  for(int w = 0; w < r % warps; w++) rank += (tile - w + warps - 1) / warps;
+  return rank;
+}
 
 // --- SIMT kernels (any dtype) ---------------------------------------------------------------------
 
@@ -254,6 +270,8 @@ int convTcKernelSize(const ConvTcPlan* p);
 // Width of the tiles in which the small-batch kernel runs this convolution for a batch of this size; 0 if it does not.  Merged
 // launches make way for single ones where it runs all of their members.
 int convTcSmallWidth(const ConvTcPlan* p, const Geom& g);
+// Tells the producer of row sums (Epilogue::sumsqOut) who reads them.
+void convTcLinkRowSums(ConvTcPlan* producer, const ConvTcPlan* consumer);
 // True if the tile table marks this shape for multi-layer launches.
 bool convTcChainPreferred(const ConvTcPlan* p);
 int convTcDoneCount(const ConvTcPlan* p);
