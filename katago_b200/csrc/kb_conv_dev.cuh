@@ -12,43 +12,9 @@ namespace kb {
 // ---------------------------------------------------------------------------------------------
 // Fast activations for the reduced-precision epilogue
 
-// G values at once, stage by stage, so that G independent dependency chains are in flight per thread: the special
-// function unit has a long latency and an epilogue warp has only one other warp to share its scheduler with.
-template <int ACT, int G>
-__device__ __forceinline__ void actStaged(float (&x)[G]) {
-  if(ACT == KB_ACT_RELU) {
-#pragma unroll
-    for(int i = 0; i < G; i++) x[i] = fmaxf(x[i], 0.0f);
-  }
-  else if(ACT == KB_ACT_MISH || ACT == KB_ACT_MISH_SCALE8) {
-    const float kk = (ACT == KB_ACT_MISH ? 1.0f : 8.0f) * 1.4426950408889634f;
-    float n[G];
-#pragma unroll
-    for(int i = 0; i < G; i++) n[i] = x[i] * kk;
-#pragma unroll
-    for(int i = 0; i < G; i++) n[i] = ex2Approx(n[i]);
-#pragma unroll
-    for(int i = 0; i < G; i++) n[i] = fmaf(n[i], n[i] + 2.0f, 2.0f);
-#pragma unroll
-    for(int i = 0; i < G; i++) n[i] = rcpApprox(n[i]);
-#pragma unroll
-    for(int i = 0; i < G; i++) x[i] = fmaf(-2.0f, x[i] * n[i], x[i]);
-  }
-  else if(ACT == KB_ACT_SILU) {
-    float n[G];
-#pragma unroll
-    for(int i = 0; i < G; i++) n[i] = x[i] * -1.4426950408889634f;
-#pragma unroll
-    for(int i = 0; i < G; i++) n[i] = ex2Approx(n[i]);
-#pragma unroll
-    for(int i = 0; i < G; i++) n[i] = rcpApprox(1.0f + n[i]);
-#pragma unroll
-    for(int i = 0; i < G; i++) x[i] *= n[i];
-  }
-}
-
-// The same on pairs of values with the packed fp32 instructions of sm_100 (two IEEE operations per instruction, half
-// the issue slots; results are bit-identical to the scalar form).  The special-function calls stay scalar.
+// G2 pairs of values at once, stage by stage, so that many independent dependency chains are in flight per thread: the special
+// function unit has a long latency and an epilogue warp has only one or two other warps to share its scheduler with.  The packed
+// fp32 instructions of sm_100 do two IEEE operations each; the special-function calls stay scalar.
 template <int ACT, int G2>
 __device__ __forceinline__ void actStaged2(float2 (&x)[G2]) {
   if(ACT == KB_ACT_RELU) {

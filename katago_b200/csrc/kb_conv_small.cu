@@ -1,4 +1,4 @@
-// Tensor-core convolution for small batches: one CTA per tile of 64 or 128 rows x 16 to 192 output channels.
+// Tensor-core convolution for small batches: one CTA per tile of 64 or 128 rows x 16 to 256 output channels.
 //
 // convTcKernel (kb_conv_tc.cu) gives every CTA a wide tile and a deep pipeline, which is right when there are more tiles
 // than SMs.  A batch of a few positions has 4 to 40 row tiles: with 192- or 256-wide tiles most SMs idle, and a layer
@@ -15,11 +15,11 @@
 //   (programmatic dependent launch); what is left after it is the activations, the MMAs and the epilogue;
 // * the MMAs come from one elected thread whose loops are chosen once per launch and whose waits cost a single try: with a run-time
 //   choice of the loop's form and a bounded wait spelled out inside it, every step cost 470 cycles beyond its MMAs
-//   (3x3 192->192 of one position: 6.2 k cycles from the first MMA to the last, 1x1 384->192 3.7 k; now 3.1 k and 1.1 k);
+//   (3x3 192->192 of one position: 6.2 k cycles from the first MMA to the last, 1x1 384->192 3.7 k; now 3.5 k and 1.6 k);
 // * the epilogue goes straight from registers to global memory, 32 bytes (a sector) per thread and access: with 16-byte accesses
 //   the closing 1x1 of five positions took 1.5 to 4.5 us for its epilogue alone, every sector being written twice.
 //
-// What is left of a launch (5 us for a 3x3 layer of one position before these changes, 3.7 us now) is the launch boundary (about 1 us),
+// What is left of a launch (5.6 us for a 3x3 layer of one position before these changes, 4.5 us now) is the launch boundary (about 1 us),
 // the first activations (0.6 us), the MMAs and the epilogue (0.5 us).
 //
 // Each CTA computes one tile and leaves.  Every wait is bounded; see kb_conv_tc.cu.

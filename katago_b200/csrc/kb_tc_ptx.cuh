@@ -221,11 +221,6 @@ __device__ __forceinline__ void stGlobal32(void* p, const uint32_t (&r)[8]) {
                ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
-// Asks for a run of global memory to be brought into L2 (address and size: multiples of 16 bytes).  A hint: it orders nothing.
-__device__ __forceinline__ void l2Prefetch(const void* p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
 // shared -> global tile store (asynchronous, tracked by the issuing thread's bulk groups)
 __device__ __forceinline__ void tmaStore2d(const CUtensorMap* tmap, uint32_t src, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(tmap), "r"(src), "r"(c0), "r"(c1) : "memory");
