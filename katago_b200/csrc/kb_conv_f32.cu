@@ -9,7 +9,10 @@
 // channels of every slice, up to 5 x 8 outputs per thread, and the eight sums are added in warp order at the end.  Measured
 // per 96->96 layer of eight boards (event overhead of 4.5 us included): 72 us before; 37 us with 4 x 4 outputs per thread, whose
 // shared-memory loads took twice the time of the FMAs; 35 us with 8 x 8 from eight warps (two per scheduler, 41 % FMA
-// utilisation, and 156 tiles of 64 rows on 148 SMs); 27 us as it is.  The order of the additions is the same in every batch size.
+// utilisation, and 156 tiles of 64 rows on 148 SMs); 27 us with up to 5 x 8 from sixteen.  The issue slots (62 % taken) were then
+nearer their limit than the FMA units (43 %): packed FMAs on pairs of channels take half of them, same bits.  Device time of the
+net before and after: b6c96 at 1 / 8 / 33 / 64 boards 232 / 342 / 1011 / 1796 -> 229 / 311 / 954 / 1691 us, b18 at 1 / 4 / 8
+3439 / 3891 / 6887 -> 3351 / 3512 / 6450.  The order of the additions is the same in every batch size.
 #include "kb_kernels.cuh"
 #include "kb_act.cuh"
 #include "kb_tc_ptx.cuh"
@@ -73,11 +76,12 @@ __global__ void __launch_bounds__(CF_THREADS) convF32Kernel(
   loadA(0);
   asm volatile("cp.async.commit_group;" ::: "memory");
 
-  float acc[NR][8];
+  // pairs of neighbouring channels: the packed fp32 instructions do two IEEE operations in one issue slot
+  float2 acc[NR][4];
 #pragma unroll
   for(int i = 0; i < NR; i++)
 #pragma unroll
-    for(int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+    for(int j = 0; j < 4; j++) acc[i][j] = make_float2(0.0f, 0.0f);
 
   for(int s = 0; s < slices; s++) {
     if(s + 1 < slices) { loadB(s + 1); loadA(s + 1); }
@@ -99,11 +103,10 @@ __global__ void __launch_bounds__(CF_THREADS) convF32Kernel(
         const float4 b0 = *reinterpret_cast<const float4*>(b + k * CF_BN), b1 = *reinterpret_cast<const float4*>(b + k * CF_BN + 16);
 #pragma unroll
         for(int i = 0; i < NR; i++) {
-          const float x = k == 0 ? av[i].x : av[i].y;
-          acc[i][0] = fmaf(x, b0.x, acc[i][0]); acc[i][1] = fmaf(x, b0.y, acc[i][1]);
-          acc[i][2] = fmaf(x, b0.z, acc[i][2]); acc[i][3] = fmaf(x, b0.w, acc[i][3]);
-          acc[i][4] = fmaf(x, b1.x, acc[i][4]); acc[i][5] = fmaf(x, b1.y, acc[i][5]);
-          acc[i][6] = fmaf(x, b1.z, acc[i][6]); acc[i][7] = fmaf(x, b1.w, acc[i][7]);
+          const float x1 = k == 0 ? av[i].x : av[i].y;
+          const float2 x = make_float2(x1, x1);
+          acc[i][0] = __ffma2_rn(x, make_float2(b0.x, b0.y), acc[i][0]); acc[i][1] = __ffma2_rn(x, make_float2(b0.z, b0.w), acc[i][1]);
+          acc[i][2] = __ffma2_rn(x, make_float2(b1.x, b1.y), acc[i][2]); acc[i][3] = __ffma2_rn(x, make_float2(b1.z, b1.w), acc[i][3]);
         }
       }
     }
@@ -114,8 +117,8 @@ __global__ void __launch_bounds__(CF_THREADS) convF32Kernel(
 #pragma unroll
   for(int i = 0; i < NR; i++) {
     float4* o = reinterpret_cast<float4*>(sm + (kg * BM + r0 + ty + 8 * i) * CF_BN);
-    o[tx] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    o[4 + tx] = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+    o[tx] = make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
+    o[4 + tx] = make_float4(acc[i][2].x, acc[i][2].y, acc[i][3].x, acc[i][3].y);
   }
   __syncthreads();
   for(int i = tid; i < BM * (CF_BN / 4); i += CF_THREADS) {
