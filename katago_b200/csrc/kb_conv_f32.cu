@@ -10,9 +10,9 @@
 // per 96->96 layer of eight boards (event overhead of 4.5 us included): 72 us before; 37 us with 4 x 4 outputs per thread, whose
 // shared-memory loads took twice the time of the FMAs; 35 us with 8 x 8 from eight warps (two per scheduler, 41 % FMA
 // utilisation, and 156 tiles of 64 rows on 148 SMs); 27 us with up to 5 x 8 from sixteen.  The issue slots (62 % taken) were then
-nearer their limit than the FMA units (43 %): packed FMAs on pairs of channels take half of them, same bits.  Device time of the
-net before and after: b6c96 at 1 / 8 / 33 / 64 boards 232 / 342 / 1011 / 1796 -> 229 / 311 / 954 / 1691 us, b18 at 1 / 4 / 8
-3439 / 3891 / 6887 -> 3351 / 3512 / 6450.  The order of the additions is the same in every batch size.
+// nearer their limit than the FMA units (43 %): packed FMAs on pairs of channels take half of them, same bits.  Device time of the
+// net before and after: b6c96 at 1 / 8 / 33 / 64 boards 232 / 342 / 1011 / 1796 -> 229 / 311 / 954 / 1691 us, b18 at 1 / 4 / 8
+// 3439 / 3891 / 6887 -> 3351 / 3512 / 6450.  The order of the additions is the same in every batch size.
 #include "kb_kernels.cuh"
 #include "kb_act.cuh"
 #include "kb_tc_ptx.cuh"
