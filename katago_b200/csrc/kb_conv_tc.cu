@@ -1296,6 +1296,7 @@ struct ConvTcPlan {
   CUtensorMap tmRes, tmRaw, tmAct;
   int smallMaps;  // the weight maps of the small-batch kernel exist
   int small;  // the small-batch kernel (kb_conv_small.cu) can run this convolution
+  int tileDeps;  // its launches report or wait per tile, which the small-batch kernel does not
   Epilogue ep;  // as given to convTcSetEpilogue
   std::vector<const ConvTcPlan*> rowSumsTo;  // the convolutions that read its row sums
   ConvSmallShape smallShape;
@@ -1472,20 +1473,22 @@ ConvTcPlan* convTcCreate(
     if(!encodeWeights3d(&ss.tmB[i], dt, w, inC, outC, ss.taps, CONV_SMALL_WIDTHS[i], 1)) p->smallMaps = 0;
     if(ss.taps == 9 && !encodeWeights3d(&ss.tmB3[i], dt, w, inC, outC, ss.taps, CONV_SMALL_WIDTHS[i], 3)) p->smallMaps = 0;
   }
-  p->small = 0;
+  p->small = 0; p->tileDeps = 0;
   return p;
 }
 
 // Tile of the small-batch kernel for this convolution and batch (BM = 0: the wide-tile kernel runs it).  Decided by the plan
-// and the number of rows alone, so that every launch of a batch size takes the same route.
+// and the number of rows alone, so that every launch of a batch size takes the same route; a producer and the consumers of its
+// row sums rely on that.
 static ConvSmallTile smallTile(const ConvTcPlan* p, const Geom& g) {
   static const bool off = getenv("KB_NO_SMALL") != nullptr && atoi(getenv("KB_NO_SMALL")) != 0;
-  if(!p->small || off) return ConvSmallTile{};
+  if(!p->small || p->tileDeps || off) return ConvSmallTile{};
   // the wide-tile kernels read row sums in their own form only
   for(const ConvTcPlan* c : p->rowSumsTo)
     if(smallTile(c, g).BM == 0) return ConvSmallTile{};
   return convSmallTile(p->smallShape, p->ep, g.rows, p->numSMs);
 }
+void convTcUseTileDeps(ConvTcPlan* p) { p->tileDeps = 1; }
 void convTcLinkRowSums(ConvTcPlan* producer, const ConvTcPlan* consumer) { producer->rowSumsTo.push_back(consumer); }
 int convTcSmallWidth(const ConvTcPlan* p, const Geom& g) { return p ? smallTile(p, g).BN : 0; }
 
@@ -1595,9 +1598,8 @@ cudaError_t launchConvTc(cudaStream_t st, const ConvTcPlan* p, Geom g, const Epi
   if(ep.outRaw && ((ep.rawStride % 8) || (ep.rawC0 % 16) || (ep.rawC1 % 16))) return cudaErrorInvalidValue;
   if(ep.outAct && ((ep.actStride % 8) || (ep.actC0 % 16) || (ep.actC1 % 16) || ((ep.actC1 - ep.actC0) > CONV_TC_MAX_ACT && ep.act != KB_ACT_SWIGLU_PAIRS))) return cudaErrorInvalidValue;
   if(ep.residual && (ep.resStride % 8)) return cudaErrorInvalidValue;
-  if(!(deps && (deps->done || deps->wait))) {
-    if(const ConvSmallTile t = smallTile(p, g); t.BM > 0) return launchConvSmall(st, p->smallShape, t, g, ep, statusWord);
-  }
+  if(deps && (deps->done || deps->wait) && !p->tileDeps) return cudaErrorInvalidValue;
+  if(const ConvSmallTile t = smallTile(p, g); t.BM > 0) return launchConvSmall(st, p->smallShape, t, g, ep, statusWord);
   ConvTcArgs a;
   a.g = g; a.ep = ep;
   a.inC = p->inC; a.outC = p->outC; a.kY = p->kY; a.kX = p->kX;

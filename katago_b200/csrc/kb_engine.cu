@@ -255,7 +255,7 @@ void Engine::addConvOp(const ConvDev& c, Epilogue ep, const std::string& tag) {
       rowSumsFrom_ = c.plan;
     }
     if(ep.rowSumsq && ep.rowSumsqFrom) convTcLinkRowSums(ep.rowSumsqFrom, c.plan);
-    const ConvTcPlan* plan = c.plan;
+    ConvTcPlan* plan = c.plan;
     std::shared_ptr<ConvTcDeps> deps = std::make_shared<ConvTcDeps>();
     addOp(name, flops, bytes, [plan, ep, status, deps](cudaStream_t st, const Geom& g) { return launchConvTc(st, plan, g, ep, status, deps.get()); });
     ops_.back().tcPlan = plan;
@@ -1171,6 +1171,8 @@ void Engine::planTileDeps() {
     cur.deps->wait = prev.deps->done;
     cur.deps->waitPlan = prev.tcPlan;
   }
+  for(Op& op : ops_)
+    if(op.deps && (op.deps->done || op.deps->wait)) convTcUseTileDeps(op.tcPlan);
 }
 
 void Engine::selfTestWaitTimeout(unsigned long long limitNs) {

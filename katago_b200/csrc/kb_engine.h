@@ -46,7 +46,7 @@ struct Op {
     return !members.empty();
   }
   // tensor-core convolutions only: what the launch reads and writes, and its per-tile dependency record
-  const ConvTcPlan* tcPlan = nullptr;
+  ConvTcPlan* tcPlan = nullptr;
   Epilogue ep;
   const void* convIn = nullptr;   // input tensor, its row stride, weights and shape of the convolution
   const void* convW = nullptr;

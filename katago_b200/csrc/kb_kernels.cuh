@@ -266,6 +266,8 @@ struct ConvTcDeps {
   const ConvTcPlan* waitPlan = nullptr;
 };
 bool convTcDepsCapable(const ConvTcPlan* p);
+// Says that this convolution will be launched with a dependency record: it then runs in wide tiles in every batch.
+void convTcUseTileDeps(ConvTcPlan* p);
 int convTcKernelSize(const ConvTcPlan* p);
 // Width of the tiles in which the small-batch kernel runs this convolution for a batch of this size; 0 if it does not.  Merged
 // launches make way for single ones where it runs all of their members.

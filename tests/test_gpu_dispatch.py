@@ -134,6 +134,25 @@ def test_small_batches_give_the_rows_of_a_full_batch(factory, prec, full, edge):
     h.close()
 
 
+@pytest.mark.parametrize("make", [mf.make_transformer, mf.make_transformer_relbias])
+@pytest.mark.parametrize("n", [1, 3])
+def test_tile_dependencies_leave_row_sums_in_the_form_they_are_read(make, n, monkeypatch):
+    """With KB_TILE_DEPS a convolution that reports its tiles runs in wide tiles in every batch: the row sums of its output then have to
+    be read in the form of the wide tiles.  The same bits as without the switch."""
+    model = capi.Model(mf.to_blob(make(layers=2)))
+    sp, gl = mf.random_positions(n, seed=18, board_sizes=[19, 13, 9][:n])
+    outs = {}
+    for mode in ("0", "1", "2"):
+        monkeypatch.setenv("KB_TILE_DEPS", mode)  # read when a handle is created
+        h = capi.Handle(model, n, precision=capi.PRECISION_FP16)
+        outs[mode] = [h.forward(sp, gl) for _ in range(3)]
+        h.close()
+    for mode in outs:
+        for run in outs[mode]:
+            for k in run:
+                assert np.array_equal(run[k], outs["0"][0][k]), (mode, k)
+
+
 @pytest.mark.parametrize("trunk,mid", [(512, 256), (256, 128), (128, 64), (320, 192), (384, 128), (192, 64)])
 @pytest.mark.parametrize("prec", [capi.PRECISION_FP16, capi.PRECISION_BF16])
 def test_fused_closing_and_opening_convolutions(trunk, mid, prec):
