@@ -14,6 +14,7 @@
 // epilogue stores the next mid stream and its activated form.  Weights of both GEMMs stream through one ring of slots.
 // Every wait is bounded.
 #include "kb_conv_dev.cuh"
+#include "kb_fused_shape.h"
 
 #include <cuda.h>
 #include <cstdio>
@@ -28,15 +29,12 @@
 namespace kb {
 
 constexpr int PP_BM = 128;          // rows per tile
-constexpr int PP_CG = 3;            // epilogue warps per TMEM lane quarter
 constexpr int PP_EPI_WARPS = 4 * PP_CG;
 constexpr int PP_THREADS = 64 + 32 * PP_EPI_WARPS;
 constexpr int PP_UNIT = 32 * 64;    // staging unit: 32 rows x 32 channels of the storage type (64-byte swizzle)
 constexpr int PP_CHUNK = PP_BM * 128;  // one 64-channel K chunk of an A operand: 128 rows x 128 bytes
 constexpr int PP_MAX_SLOTS = 8;     // weight ring
 constexpr int PP_STAGE = 3;         // staging units per epilogue warp: two of the residual / updated stream, one more for GEMM2's outputs
-constexpr int PP_NUM_A2 = 4;        // operand chunks of GEMM2 in tensor memory
-constexpr int PP_A2_COLS = 32;      // 64 channels of 16 bits, two per column
 constexpr int PP_FIXED = 512;       // barriers and the TMEM slot
 
 // Optional timeline (build with -DKB_TC_TRACE): CTA 0 records SM cycle counts of its MMA warp and of its first epilogue
@@ -53,7 +51,7 @@ enum { PP_ERR_PRODUCER = 111, PP_ERR_MMA = 112, PP_ERR_EPILOGUE = 113, PP_ERR_AL
 struct PostPreArgs {
   Geom g;
   int Cm, Ct, Cn;          // GEMM1: Cm -> Ct (+ residual); GEMM2: Ct -> Cn
-  int NP, parts;           // output channels of GEMM1 per part (64 or 128), Ct / NP
+  int NP, parts;           // output channels of GEMM1 per part (64, 128 or 192), Ct / NP
   int N2, pieces;          // output channels of GEMM2 per weight slot, Cn / N2
   int kc1;                 // Cm / 64
   int numB, bSlot;         // weight ring: slots and bytes per slot
@@ -504,20 +502,6 @@ static PostPreKernelFn postPreKernelForT(int act) {
   }
 }
 
-// Output channels of GEMM1 per part: whole K chunks of GEMM2, and one accumulator next to GEMM2's and its operand chunks.
-static int postPrePartWidth(int Ct, int Cn) {
-  for(int np : {192, 128, 64})
-    if(Ct % np == 0 && np + Cn + PP_NUM_A2 * PP_A2_COLS <= 512) return np;
-  return 0;
-}
-// A weight slot holds a 64-channel chunk for one part of GEMM1 or as many output channels of GEMM2.
-static int postPrePieces(int Ct, int Cn) {
-  const int np = postPrePartWidth(Ct, Cn);
-  for(int i = 1; i <= 4; i++)
-    if(Cn % (16 * i) == 0 && Cn / i <= np) return i;
-  return 0;
-}
-
 bool convPostPreEligible(int dt, int Cm, int Ct, int Cn) {
   if(dt != DT_F16 && dt != DT_BF16) return false;
   if((Cm % 64) != 0 || (Ct % 64) != 0 || (Cn % 32) != 0 || Cn > 256 || Cn < 64) return false;
@@ -542,7 +526,7 @@ ConvPostPrePlan* convPostPreCreate(
   a.Cm = Cm; a.Ct = Ct; a.Cn = Cn; a.kc1 = Cm / 64;
   a.NP = postPrePartWidth(Ct, Cn); a.parts = Ct / a.NP;
   a.pieces = postPrePieces(Ct, Cn); a.N2 = Cn / a.pieces;
-  a.numD1 = 2 * a.NP + Cn + PP_NUM_A2 * PP_A2_COLS <= 512 ? 2 : 1;
+  a.numD1 = postPreAccumulators(a.NP, Cn);
   a.bSlot = a.NP * 128;
   const long fixed = (long)a.kc1 * PP_CHUNK + (long)PP_EPI_WARPS * PP_STAGE * PP_UNIT + PP_FIXED;
   a.numB = (int)std::min<long>((227L * 1024 - fixed) / a.bSlot, PP_MAX_SLOTS);
