@@ -1291,12 +1291,23 @@ static bool reachableHostMemory(const void* p, size_t bytes) {
   return type == CU_MEMORYTYPE_HOST && dev == at && (at & 3) == 0 && start != 0 && start <= at && at + bytes <= start + size;
 }
 
-// Up to this many bytes of positions, a call whose buffers are all page-locked moves them with one kernel each way: a copy
-// engine takes several microseconds for every buffer and for the change between it and the kernels.  Wall time of a whole call, copy
-// engine / kernel, in us: b6c96 fp16 at 1 position 134 / 105, 16 167 / 142, 100 320 / 296, 200 496 / 486, 400 904 / 902; b18 fp16 at 1
-// 550 / 522, 37 1391 / 1373, 128 3150 / 3165.  Past about 130 positions both wait for the bus, and the copy engine leaves the
-// multiprocessors to other streams.
-constexpr size_t TRANSFER_KERNEL_MAX_BYTES = 4u << 20;
+// Up to these many bytes of positions, and of policy and ownership, a call whose buffers of that direction are all page-locked moves
+// them with one kernel.  A copy engine takes several microseconds for every buffer and for the change between it and the
+// kernels, but it works beside the kernels of other streams; a transfer kernel waits for the bus on SMs that another handle's
+// persistent launches wait for in turn.  Wall time of a call of b6c96 fp16 in us, copy engine both ways / kernel out only / kernel both
+// ways, with one, two and three handles called from as many threads:
+//   1 position     129 / 104 / 104   139 / 116 / 117   145 / 125 / 125
+//   32             197 / 177 / 173   207 / 206 / 195   246 / 241 / 245
+//   48             238 / 221 / 216   255 / 247 / 251   291 / 291 / 305
+//   64             253 / 235 / 234   281 / 279 / 285   339 / 340 / 354
+//   100            309 / 293 / 292   357 / 362 / 486   509 / 524 / 651
+//   128            353 / 332 / 333   413 / 423 / 565   600 / 616 / 774
+//   256            597 / 579 / 589   744 / 754 / 1027  1125 / 1183 / 1458
+// (b18 at 1 to 37 positions gains 10 to 20 us with one handle and is within 1 % with more.)  The lines: 33 positions of 19x19 in, 121 out.
+constexpr size_t TRANSFER_IN_MAX_BYTES = 1u << 20, TRANSFER_OUT_MAX_BYTES = 512u << 10;
+// Blocks per buffer.  Eight keep the bus busy and hold few SMs: with two handles of 64 positions 287 us a call, 299 with 16, 319 with 148;
+// four are enough for writes, which wait for nothing (reads: 243 us with four, 236 with eight).
+constexpr int TRANSFER_IN_BLOCKS = 8, TRANSFER_OUT_BLOCKS = 4;
 
 void Engine::uploadInputs(int n, const float* spatial, const float* global, const int32_t* symmetry, const float* meta) {
   if(n < 1 || n > maxBatch_) throw std::runtime_error("batch size out of range for this handle");
@@ -1316,7 +1327,7 @@ void Engine::uploadInputs(int n, const float* spatial, const float* global, cons
                          {dMeta_, meta, (size_t)n * inMetaC_, "H2D metadata"},
                          {dSym_, symmetry, (size_t)n, "H2D symmetry"}};
   TransferList list;
-  bool direct = copies[0].words * 4 <= TRANSFER_KERNEL_MAX_BYTES;
+  bool direct = copies[0].words * 4 <= TRANSFER_IN_MAX_BYTES;
   for(const Copy& c : copies) {
     if(!direct) break;
     if(!c.src) continue;
@@ -1324,7 +1335,7 @@ void Engine::uploadInputs(int n, const float* spatial, const float* global, cons
     list.add(c.src, c.dst, c.words);
   }
   if(direct) {
-    cudaCheck(launchTransfers(stream_, list), "input transfer");
+    cudaCheck(launchTransfers(stream_, list, TRANSFER_IN_BLOCKS), "input transfer");
     return;
   }
   for(const Copy& c : copies)
@@ -1347,7 +1358,7 @@ void Engine::downloadOutputs(int n, float* policy, float* policyPass, float* val
                          {scoreValue, dScore_, (size_t)n * scoreValueC_, "D2H score"},
                          {ownership, dOwnership_, (size_t)n * S, "D2H ownership"}};
   TransferList list;
-  bool direct = (copies[0].words + copies[4].words) * 4 <= TRANSFER_KERNEL_MAX_BYTES;
+  bool direct = (copies[0].words + copies[4].words) * 4 <= TRANSFER_OUT_MAX_BYTES;
   for(const Copy& c : copies) {
     if(!direct) break;
     if(!c.dst) continue;
@@ -1356,7 +1367,7 @@ void Engine::downloadOutputs(int n, float* policy, float* policyPass, float* val
   }
   if(direct) {
     list.add(statusWord_, statusHost_, 1);
-    cudaCheck(launchTransfers(stream_, list), "output transfer");
+    cudaCheck(launchTransfers(stream_, list, TRANSFER_OUT_BLOCKS), "output transfer");
     wait();
     return;
   }

@@ -169,10 +169,10 @@ __global__ void __launch_bounds__(256) transferKernel(const __grid_constant__ Tr
   for(size_t i = done + first; i < t.words; i += step) reinterpret_cast<uint32_t*>(t.dst)[i] = reinterpret_cast<const uint32_t*>(t.src)[i];
 }
 
-cudaError_t launchTransfers(cudaStream_t st, const TransferList& list) {
+cudaError_t launchTransfers(cudaStream_t st, const TransferList& list, int maxBlocks) {
   if(list.count == 0) return cudaSuccess;
   const size_t pieces = (list.mostWords + 3) / 4;
-  const unsigned blocks = (unsigned)std::min<size_t>(std::max<size_t>((pieces + 255) / 256, 1), 148);
+  const unsigned blocks = (unsigned)std::min<size_t>(std::max<size_t>((pieces + 255) / 256, 1), (size_t)maxBlocks);
   transferKernel<<<dim3(blocks, (unsigned)list.count), 256, 0, st>>>(list);
   return cudaGetLastError();
 }

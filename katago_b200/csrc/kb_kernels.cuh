@@ -111,7 +111,7 @@ struct TransferList {
     if(words > mostWords) mostWords = words;
   }
 };
-cudaError_t launchTransfers(cudaStream_t st, const TransferList& list);
+cudaError_t launchTransfers(cudaStream_t st, const TransferList& list, int maxBlocks);  // maxBlocks: per buffer
 
 // Place of a 32-channel unit among the row-sum partials of the small-batch kernel: tile by tile of `tile` units, warp by warp
 // (a wide tile's units go to its `warps` warps in turn).

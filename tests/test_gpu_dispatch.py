@@ -182,35 +182,69 @@ def test_fused_closing_and_opening_convolutions(trunk, mid, prec):
             assert np.array_equal(run[k], outs["0"][0][k]), k
 
 
-@pytest.mark.parametrize("n", [1, 3, 133])
+def _locked(a, keep, shift=0):
+    """A copy of `a` in page-locked memory, `shift` elements behind an aligned address."""
+    flat = capi.PinnedArray((a.size + shift,), a.dtype)
+    keep.append(flat)
+    view = flat.array[shift:].reshape(a.shape)
+    view[...] = a
+    return view
+
+
+@pytest.mark.parametrize("n", [1, 3, 60, 133])
 def test_host_buffers_of_every_kind(n):
     """Page-locked buffers (moved by a kernel in small calls, with or without 16-byte alignment), pageable ones and a mixture of
-    the two, and calls that leave outputs out: the same bits.  133 positions are past the kernel's limit."""
+    the two, and calls that leave outputs out: the same bits.  60 positions are past the limit of the kernel that reads, 133 past
+    that of the one that writes too."""
     model = capi.Model(mf.to_blob(mf.make_b6c96()))
     h = capi.Handle(model, n, precision=capi.PRECISION_FP16)
     sp, gl = mf.random_positions(n, seed=17)
     sym = np.arange(n, dtype=np.int32) % 8
     ref = h.forward(sp, gl, sym)
     keep = []
-
-    def locked(a, shift):
-        flat = capi.PinnedArray((a.size + shift,), a.dtype)
-        keep.append(flat)
-        view = flat.array[shift:].reshape(a.shape)
-        view[...] = a
-        return view
-
     for shift in (0, 1):
-        ins = [locked(a, shift) for a in (sp, gl, sym)]
-        outs = {k: locked(np.zeros_like(v), shift) for k, v in ref.items()}
-        for _ in range(2):
+        ins = [_locked(a, keep, shift) for a in (sp, gl, sym)]
+        outs = {k: _locked(np.zeros_like(v), keep, shift) for k, v in ref.items()}
+        for left_out in ((), ("policy", "value"), ("ownership",), tuple(ref)):
             for v in outs.values():
                 v[...] = -1
-            h.forward(*ins, out=outs)
-            assert all(np.array_equal(outs[k], ref[k]) for k in ref)
+            h.forward(*ins, out={k: None if k in left_out else v for k, v in outs.items()})
+            assert all(np.all(outs[k] == -1) if k in left_out else np.array_equal(outs[k], ref[k]) for k in ref), left_out
     mixed = h.forward(sp, ins[1], ins[2], out={k: (outs[k] if k == "policy" else np.zeros_like(v)) for k, v in ref.items()})
     assert all(np.array_equal(mixed[k], ref[k]) for k in ref)
     h.close()
+
+
+@pytest.mark.parametrize("n", [2, 60])
+def test_page_locked_metadata_and_two_handles_at_once(n):
+    """Metadata rows in page-locked memory, and two handles whose calls share the GPU from two threads: every call's own outputs."""
+    model = capi.Model(mf.to_blob(mf.add_meta_encoder(mf.make_b6c96())))
+    keep, states, errors = [], [], []
+    for seed in (18, 19):
+        h = capi.Handle(model, n, precision=capi.PRECISION_FP16)
+        ins = mf.random_positions(n, seed=seed) + (np.arange(n, dtype=np.int32) % 8,)
+        meta = mf.random_meta_rows(n, seed=seed, channels=model.meta_c)
+        ref = h.forward(*ins, meta=meta)
+        states.append((h, [_locked(a, keep) for a in ins], _locked(meta, keep), {k: _locked(np.zeros_like(v), keep) for k, v in ref.items()}, ref))
+
+    def work(h, ins, meta, outs, ref):
+        try:
+            for _ in range(200):
+                for v in outs.values():
+                    v[...] = -1
+                h.forward(*ins, out=outs, meta=meta)
+                assert all(np.array_equal(outs[k], ref[k]) for k in ref)
+        except Exception as e:  # handed to the test's own thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=s) for s in states]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for s in states:
+        s[0].close()
 
 
 @pytest.mark.parametrize("prec,tol", [(capi.PRECISION_FP16, 0.03), (capi.PRECISION_BF16, 0.2)])
