@@ -1839,27 +1839,35 @@ cudaError_t launchConvChain(cudaStream_t st, const ConvChainPlan* c, Geom g, int
 }
 
 // ---------------------------------------------------------------------------------------------
-// Self-test of the bounded waits: one warp waits, half of the given limit in each of the two forms, on a barrier that nothing
+// Self-test of the bounded waits: one warp waits, a third of the given limit in each of the three forms, on a barrier that nothing
 // ever arrives at.  The waits give up, the kernel records its code in the status word exactly as the convolution kernels do
-// on a time-out, and returns; the context stays usable.  The second form is used as a feeding warp uses it, on a slot that
-// is never given back: a slot armed again behind the failed wait, or a wait that reports success, is recorded as 198.
+// on a time-out, and returns; the context stays usable.  mbarWaitThread has to record its code and raise the flag, and to leave at
+// once where the flag is raised already.  mbarWaitWarp is used as a feeding warp uses it, on a slot that is never given back: a
+// slot armed again behind the failed wait, or a wait that reports success, is recorded as 198.
 
 enum { TC_ERR_SELFTEST_FAILED = 198, TC_ERR_SELFTEST_TIMEOUT = 199 };
 
 __global__ void waitTimeoutSelfTestKernel(int* status, unsigned long long limitNs) {
   __shared__ uint64_t empty, full;
-  __shared__ int abortFlag;
+  __shared__ int abortFlag, ownStatus;
+  const uint64_t limit = (uint64_t)limitNs / 3;
   bool ok = true;
   if(threadIdx.x == 0) {
-    abortFlag = 0;
+    volatile int* raised = &abortFlag;
+    *raised = 0;
+    ownStatus = 0;
     mbarInit(smemU32(&empty), 1); mbarInit(smemU32(&full), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    ok = !mbarWait(smemU32(&empty), 0u, &abortFlag, (uint64_t)limitNs / 2);
+    ok = !mbarWait(smemU32(&empty), 0u, raised, limit) && *raised == 0;
+    ok = ok && !mbarWaitThread(smemU32(&empty), 0u, raised, &ownStatus, TC_ERR_SELFTEST_TIMEOUT, limit) && *raised == 1;
+    ok = ok && atomicExch(&ownStatus, 0) == TC_ERR_SELFTEST_TIMEOUT;
+    ok = ok && !mbarWaitThread(smemU32(&empty), 0u, raised, &ownStatus, TC_ERR_SELFTEST_TIMEOUT, limit) && atomicAdd(&ownStatus, 0) == 0;
+    *raised = 0;
   }
   __syncwarp();
   bool live = true;
   for(int use = 0; use < 2; use++) {
-    if(use > 0) live = mbarWaitWarp(smemU32(&empty), 0u, &abortFlag, status, TC_ERR_SELFTEST_TIMEOUT, (uint64_t)limitNs / 2);
+    if(use > 0) live = mbarWaitWarp(smemU32(&empty), 0u, &abortFlag, status, TC_ERR_SELFTEST_TIMEOUT, limit);
     if(electOne() && live) mbarArrive(smemU32(&full));
   }
   __syncwarp();

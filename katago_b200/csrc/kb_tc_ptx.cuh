@@ -103,13 +103,13 @@ __device__ __forceinline__ bool mbarWaitWarp(
 // wait that does not succeed at once goes on in a function of its own.  Six steps of a wait on a completed barrier, four MMAs
 // (M=128, N=16: 164 cycles of tensor pipe) and a commit take 223 cycles each in this form, 332 with mbarWaitWarp in the
 // elected thread, 390 with mbarWaitWarp and all lanes.  False: the thread leaves its role.
-static __device__ __noinline__ bool mbarWaitOn(uint32_t bar, uint32_t parity, volatile int* abortFlag, int* status, int code) {
+static __device__ __noinline__ bool mbarWaitOn(uint32_t bar, uint32_t parity, volatile int* abortFlag, int* status, int code, uint64_t limitNs) {
   const uint64_t t0 = globalTimerNs();
   for(uint32_t spins = 1;; spins++) {
     if(mbarTryWait(bar, parity)) return true;
     if((spins & 63u) == 0u) {
       if(*abortFlag) return false;
-      if(globalTimerNs() - t0 > 2000000000ull) {
+      if(globalTimerNs() - t0 > limitNs) {
         *abortFlag = 1;
         __threadfence_block();
         atomicCAS(status, 0, code);
@@ -118,8 +118,9 @@ static __device__ __noinline__ bool mbarWaitOn(uint32_t bar, uint32_t parity, vo
     }
   }
 }
-__device__ __forceinline__ bool mbarWaitThread(uint32_t bar, uint32_t parity, volatile int* abortFlag, int* status, int code) {
-  return mbarTryWait(bar, parity) != 0u || mbarWaitOn(bar, parity, abortFlag, status, code);
+__device__ __forceinline__ bool mbarWaitThread(
+  uint32_t bar, uint32_t parity, volatile int* abortFlag, int* status, int code, uint64_t limitNs = 2000000000ull) {
+  return mbarTryWait(bar, parity) != 0u || mbarWaitOn(bar, parity, abortFlag, status, code, limitNs);
 }
 
 // Programmatic dependent launch: a kernel launched with the programmatic-stream-serialization attribute may start

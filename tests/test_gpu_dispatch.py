@@ -382,7 +382,8 @@ def test_profile_counts_what_a_small_batch_launches():
 
 
 def test_both_forms_of_the_bounded_wait_give_up():
-    """199 is the time-out itself; 198 would be a wait that reported success, or a slot armed again behind a failed one."""
+    """Those of feeding and issuing warps, and the plain one.  199 is the time-out itself; 198 would be a wait that reported success or
+    recorded nothing, or a slot armed again behind a failed one."""
     h = capi.Handle(capi.Model(mf.to_blob(mf.make_b18c384nbt(num_blocks=1))), 1, precision=capi.PRECISION_FP16)
     with pytest.raises(capi.KBError, match="status 199:"):
         h.selftest_wait_timeout(1_000_000)

@@ -66,3 +66,35 @@ def test_nothing_is_issued_behind_a_wait_that_ran_out(name):
     for w in re.finditer(r"\bwait\(&|mbarWaitWarp\(smemU32\(&", body):
         behind = next((i for i in issues if i.start() > w.start()), None)
         assert behind is not None and re.match(r" && (?:go\(\)|live|!\*abortFlag)\)", behind.group(1)), body[w.start():w.start() + 200]
+
+
+LEAVING = [n for n, _, b in KERNELS if "mbarWaitThread" in b and n != "waitTimeoutSelfTestKernel"]
+
+
+def test_the_kernels_whose_roles_run_in_one_thread_are_found():
+    assert set(LEAVING) == {"convTcKernel", "convSmallKernel"}
+
+
+@pytest.mark.parametrize("name", LEAVING)
+def test_a_thread_leaves_its_role_behind_a_wait_that_ran_out(name):
+    """The same for a role inside one thread (mbarWaitThread): whatever follows a wait that failed is left, out of its loops."""
+    body = next(b for n, _, b in KERNELS if n == name)
+    waits = [m.start() for m in re.finditer(r"(?<!auto )\bwait\((?!\[)", body)]
+    assert len(waits) >= 5
+    for w in waits:
+        line = body[body.rindex("\n", 0, w) + 1:body.index("\n", w)]
+        before, behind = body[:w].splitlines()[-1], body[w:].split("\n", 1)[0]
+        assert re.search(r"if\((?:[^;{}]* (?:&&|\|\|) )?!$", before), line
+        assert re.search(r"\)\) (?:goto \w+;|return;|return false;|\{ ok = false; break; \})$", behind.rstrip()), line
+    # a `break` ends one loop; its header, and those around it, ask for `ok`
+    for m in re.finditer(r"\{ ok = false; break; \}", body):
+        depth, loops = 0, []
+        for i in range(m.start() - 1, -1, -1):
+            depth += {"}": 1, "{": -1}.get(body[i], 0)
+            if depth < 0:
+                depth = 0
+                header = body[body.rindex("\n", 0, i) + 1:i]
+                if "for(" not in header:
+                    break
+                loops.append(header)
+        assert loops and all(re.search(r"&& ok;", h) for h in loops), loops
