@@ -117,6 +117,19 @@ def test_more_activated_channels_than_the_tensor_core_kernel_holds(trunk, mid, o
     (lambda: mf.make_b6c96(), capi.PRECISION_FP16, 256, 19),
     (lambda: mf.make_transformer(layers=2), capi.PRECISION_FP16, 64, 19),
     (lambda: mf.make_transformer_relbias(layers=2), capi.PRECISION_FP16, 64, 19),
+    # widths that the small tiles do not divide, and a layer (96->288) that keeps to the wide ones among layers that do not
+    (lambda: mf.make_convnet("tiles", 81, 15, 160, ["plain", "plain"], (32, 32, 32, 64), mf.ACT_MISH, mid_c=224, regular_c=64, gpool_c=32),
+     capi.PRECISION_FP16, 128, 19),
+    (lambda: mf.make_convnet("tiles", 82, 15, 320, ["plain", "gpool", "plain"], (32, 32, 32, 64), mf.ACT_MISH, mid_c=96, regular_c=64, gpool_c=32),
+     capi.PRECISION_BF16, 128, 19),
+    (lambda: mf.make_convnet("tiles", 83, 15, 288, ["plain", "plain"], (32, 32, 32, 64), mf.ACT_MISH, mid_c=96, regular_c=64, gpool_c=32),
+     capi.PRECISION_FP16, 128, 19),
+    # transformers of other widths: other wide tiles and warps behind the order of the row sums, and consumers of row sums without small
+    # tiles (832 = 4 x 208 channels), whose producers then have none either
+    (lambda: mf.make_transformer(layers=2, d=96, heads=3, head_dim=32, ffn=160), capi.PRECISION_FP16, 128, 19),
+    (lambda: mf.make_transformer(layers=2, d=160, heads=5, head_dim=64, ffn=416), capi.PRECISION_FP16, 64, 19),
+    (lambda: mf.make_transformer(layers=2, d=224, heads=4, head_dim=64, ffn=320, rope="none", rel_bias=True), capi.PRECISION_BF16, 64, 19),
+    (lambda: mf.make_transformer(layers=2, d=512, heads=8, head_dim=64, ffn=1024, rope="fixed"), capi.PRECISION_FP16, 64, 13),
 ])
 def test_small_batches_give_the_rows_of_a_full_batch(factory, prec, full, edge):
     """Small batches run in narrow tiles (kb_conv_small.cu), full ones in wide tiles and merged launches.  The order of an
@@ -248,12 +261,15 @@ def test_page_locked_metadata_and_two_handles_at_once(n):
 
 
 @pytest.mark.parametrize("prec,tol", [(capi.PRECISION_FP16, 0.03), (capi.PRECISION_BF16, 0.2)])
-@pytest.mark.parametrize("trunk,mid", [(32, 32), (160, 224), (288, 96)])
+@pytest.mark.parametrize("trunk,mid", [(32, 32), (160, 224), (288, 96), (320, 96), (448, 160)])
 @pytest.mark.parametrize("n", [1, 4, 7, 16, 31])
 def test_tiles_that_end_inside_a_layer(prec, tol, trunk, mid, n, oracle):
     """Widths that the tiles of the small-batch kernel (32 to 192 channels, 64 or 128 rows) do not divide, at batches from its
-    narrowest tiles to two CTAs per SM: the last tile of a row is short, the last row tile reaches into the padding.  Tolerance as
+    narrowest tiles to two CTAs per SM: the last tile of a row is short, the last row tile reaches into the padding.  (Of 288 and 96
+    the layer to 288 keeps to the wide kernels, whose tile of 144 channels is no multiple of 32; its neighbour does not.)  Tolerance as
     in test_input_widths_between_chunks."""
+    small = [capi.tile_plan(3, i, o)["bn"] % 32 == 0 for i, o in ((trunk, mid), (mid, trunk))]
+    assert small == [True, trunk != 288]
     g = mf._Gen(700 + trunk + mid)
     rng = np.random.default_rng(trunk + mid + n)
     mask = np.ones((n, 19, 19), np.float32)
