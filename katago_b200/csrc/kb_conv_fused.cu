@@ -63,13 +63,15 @@ struct PostPreArgs {
   int* status;
 };
 
-// What bounds it: shared memory.  A tile of 128 rows (192 -> 384 -> 192) moves 1.3 MB through it (weights written and read 590 KB,
-// operand A1 144 KB, residual and updated stream 390 KB, outputs of GEMM2 196 KB), 10 k cycles at 128 bytes each, next to 9 k
-// cycles of special-function work (two operations per activated value) and 4.7 k of MMAs, in 17 k cycles measured.  With the operand
-// chunks of GEMM2 in shared memory it was 1.5 MB and 18.5 k cycles.  Tried on top of that and slower: parts of 128 channels with two
-// accumulators of GEMM1 (A1 is read three times instead of twice; 97 us a launch at batch 256 against 86), 24 epilogue warps with
-// units of 16 channels (97 us), outputs of GEMM2 from registers in 32-byte pieces (104 us), one reciprocal for two activations
-// (no change).  batch 256: 89.4 -> 85.8 us; 256 -> 512 -> 256 (b28, batch 512, bf16) 254 us against 265 as two launches.
+// What bounds it: no unit alone.  b18 at batch 256 (profiles/conv_kernels_by_shape_ncu.md): special-function pipe busy for 50 % of
+// the cycles (two operations per activated value), issue slots 40 %, L1 and shared memory 43 %, DRAM 37 %, tensor pipe 23 %; the 3.5 warps of
+// a scheduler mostly wait for results of fixed latency and for tensor memory.  256 -> 512 -> 256 (bf16) stays lower: 39, 32, 35, 32 and
+// 25 %, with twice the waits for tensor memory per instruction and one accumulator for GEMM1.
+// With the operand chunks of GEMM2 in shared memory a tile of 128 rows moved 1.5 MB through it and took 18.5 k cycles, now 1.3 MB and 17 k.
+// Tried on top of that and slower: parts of 128 channels with two accumulators of GEMM1 (A1 is read three times instead of
+// twice; 97 us a launch at batch 256 against 86), 24 epilogue warps with units of 16 channels (97 us), outputs of GEMM2 from registers in
+// 32-byte pieces (104 us), one reciprocal for two activations (no change).  batch 256: 89.4 -> 85.8 us; 256 -> 512 -> 256 (b28, batch
+// 512, bf16) 254 us against 265 as two launches.
 //
 // The outputs of GEMM2 are read one tile late, after the warp's first unit of the next tile: nobody waits for GEMM2's last chunk
 // (1.6 k cycles a tile).  Schedule over the CTA's tiles, parts numbered through, with D accumulators for GEMM1:
@@ -502,6 +504,13 @@ static PostPreKernelFn postPreKernelForT(int act) {
   }
 }
 
+// Which widths: all that fit.  Whole nets of 18 blocks, fp16, in seconds of steady load (power-limited), two launches / fused in us, at 128
+// and at 256 boards: 384 channels with 192 inside 3311 / 3114, 6608 / 6243; 320 with 192 3228 / 3096, 6473 / 6284; 256 with 192 3112 / 2982,
+// 6244 / 6043; 384 with 256 5128 / 5003, 9783 / 9599; 256 with 256 4878 / 4746, 9340 / 9101; 512 with 192 3620 / 3425, 7204 / 6908; 192 with
+// 256 4725 / 4621, 9053 / 8915; b28 (512 with 256) 8236 / 7986, 15706 / 15402, at 24 and 48 boards 2451 / 2457, 4521 / 4574.  Single calls behind
+// idle gaps gain 1 to 6 % at 100 to 256 boards.  Narrow pairs gain more (six blocks at 256 boards: 256 with 128 1166 / 1100, 128 with 64
+// 697 / 642, 64 with 64 624 / 578).  The exception found: bursts of some tens of milliseconds of six-block nets with unscaled random weights,
+// in which pairs with 192 and more channels inside were up to 8 % slower fused at 256 boards.
 bool convPostPreEligible(int dt, int Cm, int Ct, int Cn) {
   if(dt != DT_F16 && dt != DT_BF16) return false;
   if((Cm % 64) != 0 || (Ct % 64) != 0 || (Cn % 32) != 0 || Cn > 256 || Cn < 64) return false;

@@ -463,8 +463,10 @@ bool convSmallSupports(const Epilogue& ep) {
 // The projections of a transformer follow the same rules, with tiles of whole 32-channel units where row sums or SwiGLU pairs
 // need them.  Producers of row sums keep to one CTA per SM (12-layer transformer, 32 boards: 1252 us with wide tiles, 1345 with
 // 192-wide ones on shared SMs); the up|gate projection takes 256-wide tiles on shared SMs (11 boards, relative-position bias: 695
-// us against 753 with 192-wide ones, wide 783) and, past those, up to one and a half rounds of 192-wide ones (12 boards 704, wide
-// 768).  Plain transformer at 1 / 4 / 8 / 16 boards: 570 -> 367, 586 -> 417, 665 -> 519, 808 (wide).
+// us against 753 with 192-wide ones, wide 783) and, past those, up to one and a half rounds of 192-wide ones.  Of those batches, four
+// layers, these / wide tiles: 384 channels with an FFN of 1024 at 12 boards 260 / 265, of 768 at 16 290 / 299 and 17 320 / 328, of 1536 at 8
+// 233 / 253; 256 channels 219 / 229; 512 channels 340 / 341; 13x13 boards 25 281 / 286, 26 284 / 288; 9x9 49 262 / 265, 51 283 / 287.
+// Plain transformer at 1 / 4 / 8 / 16 boards: 570 -> 367, 586 -> 417, 665 -> 519, 808 (wide).
 //
 // Weight slots of three taps where a wait is a good part of a slot's MMAs (b18, twelve positions, N = 64: 823 against 848 with one
 // tap), of one tap for wide tiles with half an SM (b18, 37 positions, N = 96: 1340 against 1589 with three).

@@ -955,7 +955,7 @@ __global__ void __launch_bounds__(tcThreads(TC_EPI_CG, true), 1) convChainKernel
 
   if(warp == 0) {
     // ---------------- TMA producer ----------------
-    // (the loops of this kernel run inside the elected threads: with all lanes in them, as in convTcKernel, chains of four
+    // (the loops of this kernel run inside the elected threads: with all lanes in them, as in CTA pairs, chains of four
     // 192-wide layers took 1.5 to 2 % longer)
     if(electOne()) {
       // Weights depend on nothing in the stream.  While a tile's inputs are not ready yet (the kernel before this launch, then

@@ -129,7 +129,7 @@ __device__ __forceinline__ bool mbarWaitThread(
 //
 // A kernel that allocates tensor memory calls gridDepLaunch() only after the block barrier behind its allocation.  An
 // allocation blocks without a limit, and two kernels fit one SM where registers and shared memory allow it: 96 registers x
-// 320 threads of a convTcKernel with the direct epilogue and 56 x 576 of convSmallKernel are 62 976 of 65 536.  If the later
+// 320 threads of a convTcKernel with the direct epilogue and 72 x 448 of convSmallKernel are 62 976 of 65 536.  If the later
 // of the two could start before the earlier one's CTA holds its columns, it could take the ones that are left (a 192-wide
 // tile's accumulators are all 512), and then wait for a kernel that waits for it.
 __device__ __forceinline__ void gridDepWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -341,14 +341,6 @@ __device__ __forceinline__ void ummaCommitPair(uint32_t clusterBar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(clusterBar) : "memory");
 }
 
-// 32 lanes x 8 consecutive 32-bit columns -> 8 registers per thread (thread t reads lane base+t).
-__device__ __forceinline__ void tmemLd8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile(
-    "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-    : "r"(taddr)
-    : "memory");
-}
 // 32 lanes x 32 consecutive 32-bit columns -> 32 registers per thread (thread t reads lane base+t).
 __device__ __forceinline__ void tmemLd32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
